@@ -1,0 +1,369 @@
+// Expert products for batches of more than a few rows per expert: the TOKENS are the M side of the MMA (one token row
+// per TMEM lane), the weights the N side.
+//
+// With the weights on the M side (expert_tc.cu, right for a few token columns) a lane of the accumulator holds one
+// weight row, so the 16-element blocks of the re-quantisation run ACROSS lanes: a warp reduction, a select tree, a
+// shuffle per column and a nibble transposition - about 65 instructions per SwiGLU value, which is what bounded the
+// kernel at 4,096 tokens (201 µs).  With the tokens on the M side a lane holds one token's 32 neighbouring values:
+// maximum, scale, packing and store need no other lane.  And one MMA covers 128 tokens x 256 weight rows (gate box and
+// up box of a chunk are one 256-row operand), so an operand byte in shared memory is read half as often as with
+// N = 64.
+#include "expert_common.cuh"
+
+#include <cstdlib>
+
+namespace p92b {
+
+using namespace ptx;
+using namespace expert;
+
+namespace {
+
+constexpr int kTok = 128;                                   // token rows of a tile (M)
+constexpr int kWRows = 256;                                 // weight rows of a tile (N)
+constexpr int kEpiWarps = 16;                               // four per TMEM quarter
+constexpr int kThreads = 64 + 32 * kEpiWarps;
+
+constexpr int kTmemAll = 512;
+
+// Eight sums of one row scaled and rounded to BF16: 16 bytes.
+__device__ __forceinline__ uint4 scale_to_bf16x8(const std::uint32_t* v, float alpha) {
+    std::uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = bf16x2_bits(__uint_as_float(v[2 * k]) * alpha, __uint_as_float(v[2 * k + 1]) * alpha);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Stores 32 rows x 64 BF16 values; lane l holds row l's eight 16-byte pieces.  Stored as they are, one instruction
+// would touch 32 lines and write 16 bytes of each (a down product over 147,456 rows took 506 µs that way against 326).
+// An 8 x 8 transposition of the pieces inside every group of eight lanes - three exchange rounds - makes lane j of a
+// group hold piece j of the group's eight rows: one instruction then stores four whole 128-byte lines.  `row` = this lane's row number in the output, `valid` = rows that exist (warp uniform).
+__device__ __forceinline__ void store_rows64(std::uint16_t* out, int pitch, long row, int valid, uint4 (&w)[8]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 4; d >= 1; d >>= 1) {
+        const bool upper = (lane & d) != 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if ((q & d) != 0) continue;
+            // the lane with bit d set keeps piece q + d and gives piece q away; the other one the reverse
+            const uint4 give = upper ? w[q] : w[q + d];
+            uint4 got;
+            got.x = __shfl_xor_sync(0xffffffffU, give.x, d);
+            got.y = __shfl_xor_sync(0xffffffffU, give.y, d);
+            got.z = __shfl_xor_sync(0xffffffffU, give.z, d);
+            got.w = __shfl_xor_sync(0xffffffffU, give.w, d);
+            if (upper) w[q] = got; else w[q + d] = got;
+        }
+    }
+    // now w[r] is piece (lane & 7) of row (lane & ~7) + r
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int from = (lane & ~7) + r;
+        const long to = __shfl_sync(0xffffffffU, row, from);
+        if (from < valid) *reinterpret_cast<uint4*>(out + to * pitch + (lane & 7) * 8) = w[r];
+    }
+}
+
+// 32 consecutive columns of this warp's 32 TMEM lanes.
+__device__ __forceinline__ void tmem_load32(std::uint32_t addr, std::uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(addr)
+        : "memory");
+}
+
+// 64 columns of this warp's 32 rows, scaled and rounded, half of them at a time to stay within the registers.
+__device__ __forceinline__ void load_scale_rows64(std::uint32_t tmem, float alpha, uint4 (&w)[8]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        std::uint32_t v[32];
+        tmem_load32(tmem + h * 32, v);
+        tmem_load_wait();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[h * 4 + q] = scale_to_bf16x8(v + q * 8, alpha);
+    }
+}
+
+// One 16-element block of a token's intermediate row from its gate and up sums: bf16(alpha * sum) for both, SwiGLU
+// rounded to BF16 (cuda/nvfp4_ops.cu:97-105), block maximum, E4M3 scale, E2M1 values (cuda/nvfp4_ops.cu:818-841) -
+// the arithmetic of the other gate/up epilogues value for value, all of it in one lane.
+__device__ __forceinline__ uint2 swiglu_block16(const std::uint32_t* g, const std::uint32_t* u, float alpha_g, float alpha_u,
+                                                float quant_scale, std::uint32_t* scale_bits) {
+    std::uint32_t hh[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        float h[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int j = 2 * k + i;
+            const std::uint32_t gu = bf16x2_bits(__uint_as_float(g[j]) * alpha_g, __uint_as_float(u[j]) * alpha_u);
+            const float gv = __uint_as_float(gu << 16);
+            const float uv = __uint_as_float(gu & 0xffff0000U);
+            h[i] = (gv / (1.0F + expf(-gv))) * uv;
+        }
+        hh[k] = bf16x2_bits(h[0], h[1]);
+    }
+    // |BF16| bit patterns order like unsigned integers: the maximum of 16 as packed 16-bit maxima
+    std::uint32_t m = hh[0] & 0x7fff7fffU;
+#pragma unroll
+    for (int k = 1; k < 8; ++k) m = __vmaxu2(m, hh[k] & 0x7fff7fffU);
+    const float amax = __uint_as_float(max(m << 16, m & 0xffff0000U));
+    const __nv_fp8_e4m3 scale(amax * (quant_scale / 6.0F));
+    *scale_bits = scale.__x;
+    const float decoded = static_cast<float>(scale);
+    const float multiplier = decoded == 0.0F ? 0.0F : quant_scale / decoded;
+    std::uint32_t words[2] = {0U, 0U};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float2 pair = make_float2(__uint_as_float(hh[k] << 16) * multiplier, __uint_as_float(hh[k] & 0xffff0000U) * multiplier);
+        const std::uint32_t byte = __nv_fp4x2_e2m1(pair).__x;
+        words[k >> 2] |= byte << ((k & 3) * 8);
+    }
+    return make_uint2(words[0], words[1]);
+}
+
+// A ring stage: one K block (256 values) of the weight tile and of the token tile.  The weight part of a gate/up
+// stage is exactly one chunk of the bank's stream: gate box, up box, their two scale slabs.
+struct Stage {
+    static constexpr int kOffW = 0;
+    static constexpr int kOffSfW = kWRows * kBlockKBytes;                   // 32,768
+    static constexpr int kOffT = kChunkBytes;                               // 36,864
+    static constexpr int kOffSfT = kOffT + kTok * kBlockKBytes;
+    static constexpr int kBytes = kOffSfT + kSfSlab;                        // 55,296
+    static constexpr int kCount = 4;
+    static constexpr int kBarriers = 3 * kCount + 2;
+    static constexpr int kSmem = kCount * kBytes + kBarriers * 8 + 16 + 1024;
+    // TMEM: the accumulator (256 columns), then two buffers of scale factors: 16 columns for the tokens, 32 for the weights
+    static constexpr int kSfBase = 256, kSfBufferCols = 64, kSfWeights = 16;
+};
+
+// MODE 0: gate/up + SwiGLU + re-quantisation; p.m_tiles row tiles of 128 intermediate rows (gate and up rows of each).
+// MODE 1: one matrix, BF16 rows out; p.m_tiles pairs of the bank's 128-row tiles.
+// Roles as in expert_tc.cu: producer warp, MMA warp, sixteen epilogue warps; items (128-row token tile, weight tile).
+// One accumulator only - two of 256 columns and the scale factors do not fit TMEM - so the epilogue warps take their
+// 64 columns into registers at once and the next item's products start after that read, not after the arithmetic.
+// What bounds it with full tiles: the shared-memory port.  A K block costs 48 KB of operand reads, 54 KB of arriving
+// copies and 6 KB of scale copies, 844 cycles at 128 bytes against 512 of tensor work; it runs at 907 (16,384 tokens:
+// 556 -> 393 us; 4,096 tokens: 202 -> 168 us, HBM floor 116).  A pair of blocks sharing the weight rows (cta_group::2,
+// 256-row token tiles) needs 594 cycles but pads every expert to 256 rows: 376 us and 200 us, not kept.  Token rows
+// gathered from token order (TMA tile::gather4, four rows per operation) take 46 ns per operation: 1,023 us.
+template <int MODE>
+__global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_constant__ CUtensorMap map_t32,
+                                                                  const __grid_constant__ CUtensorMap map_t128, const TcParams p) {
+    extern __shared__ std::uint8_t smem_raw[];
+    __shared__ RouteTable route_table;
+    const std::uint32_t base = (smem_u32(smem_raw) + 1023U) & ~1023U;
+    const std::uint32_t bars = base + Stage::kCount * Stage::kBytes;
+    auto weight_bar = [&](int s) { return bars + 8U * s; };
+    auto token_bar = [&](int s) { return bars + 8U * (Stage::kCount + s); };
+    auto empty_bar = [&](int s) { return bars + 8U * (2 * Stage::kCount + s); };
+    const std::uint32_t accum_full = bars + 8U * (3 * Stage::kCount);
+    const std::uint32_t accum_empty = accum_full + 8U;
+    const std::uint32_t tmem_slot = bars + 8U * Stage::kBarriers;
+    volatile std::uint32_t* tmem_slot_ptr =
+        reinterpret_cast<volatile std::uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+    volatile std::uint32_t* abort_ptr = tmem_slot_ptr + 1;
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int k_blocks = p.k_bytes / kBlockKBytes;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < Stage::kCount; ++s) {
+            mbar_init(weight_bar(s), 1);
+            mbar_init(token_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        mbar_init(accum_full, 1);
+        mbar_init(accum_empty, kEpiWarps);
+        *abort_ptr = 0;
+        fence_mbar_init();
+        prefetch_tensormap(&map_t32);
+        prefetch_tensormap(&map_t128);
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, kTmemAll);
+        tmem_relinquish();
+    }
+    pdl_wait();                       // routing lists and token rows come from the kernels upstream
+    load_route_table(p, &route_table);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_launch_dependents();
+    const std::uint32_t tmem_base = *tmem_slot_ptr;
+    const int total_items = route_table.prefix[route_table.active_count] * p.m_tiles;       // the prefix counts 128-row slabs here
+    auto give_up = [&]() {
+        *abort_ptr = 1;
+        atomicCAS(p.status, kStatusOk, kStatusWaitExpired);
+    };
+
+    if (warp == 0) {
+        if (elect_one()) {
+            int stage = 0;
+            std::uint32_t phase = 0;
+            for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
+                Item it;
+                if (!decode_item<kTok>(p, route_table, item, &it)) continue;
+                // token rows beyond the tile's last one are not loaded: their lanes compute on what the stage held
+                // before, and nothing reads them
+                const int boxes = (it.valid + 31) >> 5;
+                const std::uint8_t* t_sf = p.b_sf + static_cast<std::size_t>(it.pp0 >> 7) * (p.k_bytes / 32) * 512;
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!mbar_wait(empty_bar(stage), phase ^ 1U)) { give_up(); break; }
+                    const std::uint32_t st = base + stage * Stage::kBytes;
+                    mbar_arrive_expect_tx(weight_bar(stage), kChunkBytes);
+                    if constexpr (MODE == 0) {
+                        bulk_load(st + Stage::kOffW,
+                                  p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes,
+                                  kChunkBytes, weight_bar(stage));
+                    } else {
+                        // K block kb of two neighbouring row tiles: a box and a scale slab from either tile's chunk
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const std::uint8_t* chunk = p.bank.g2 +
+                                ((static_cast<std::size_t>(it.entry) * p.m_tiles * 2 + it.m_tile * 2 + h) * (k_blocks / 2) + (kb >> 1)) * kChunkBytes;
+                            bulk_load(st + Stage::kOffW + h * kChunkBox, chunk + (kb & 1) * kChunkBox, kChunkBox, weight_bar(stage));
+                            bulk_load(st + Stage::kOffSfW + h * kSfSlab, chunk + kChunkScaleOffset + (kb & 1) * kChunkScaleBytes, kSfSlab,
+                                      weight_bar(stage));
+                        }
+                    }
+                    mbar_arrive_expect_tx(token_bar(stage), boxes * (32 * kBlockKBytes) + kSfSlab);
+                    if (boxes == 4) {
+                        tma_load_2d(st + Stage::kOffT, &map_t128, token_bar(stage), kb * kBlockKBytes, it.pp0);
+                    } else {
+                        for (int b = 0; b < boxes; ++b) {
+                            tma_load_2d(st + Stage::kOffT + b * 32 * kBlockKBytes, &map_t32, token_bar(stage), kb * kBlockKBytes, it.pp0 + b * 32);
+                        }
+                    }
+                    bulk_load(st + Stage::kOffSfT, t_sf + static_cast<std::size_t>(kb) * 4 * 512, kSfSlab, token_bar(stage));
+                    if (++stage == Stage::kCount) { stage = 0; phase ^= 1U; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
+            int stage = 0;
+            std::uint32_t phase = 0;
+            std::uint32_t accum_phase = 0;
+            constexpr std::uint32_t idesc = idesc_nvf4(kTok, kWRows);
+            int sf_buffer = 0;
+            for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
+                Item it;
+                if (!decode_item<kTok>(p, route_table, item, &it)) continue;
+                bool ok = true;
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!mbar_wait(weight_bar(stage), phase) || !mbar_wait(token_bar(stage), phase)) {
+                        give_up();
+                        ok = false;
+                        break;
+                    }
+                    if (kb == 0 && !mbar_wait(accum_empty, accum_phase ^ 1U)) { give_up(); ok = false; break; }
+                    tc_fence_after();
+                    const std::uint32_t st = base + stage * Stage::kBytes;
+                    const std::uint32_t sf_t = tmem_base + Stage::kSfBase + sf_buffer * Stage::kSfBufferCols;
+                    const std::uint32_t sf_w = sf_t + Stage::kSfWeights;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        tc_copy_sf(sf_t + k * 4, desc_scale_atom(st + Stage::kOffSfT + k * 512));
+                        // a 256-row operand takes eight columns per K step: its rows 0..127, then 128..255
+                        tc_copy_sf(sf_w + k * 8, desc_scale_atom(st + Stage::kOffSfW + k * 512));
+                        tc_copy_sf(sf_w + k * 8 + 4, desc_scale_atom(st + Stage::kOffSfW + kSfSlab + k * 512));
+                    }
+                    const std::uint64_t a_desc = desc_k_major_sw128(st + Stage::kOffT);
+                    const std::uint64_t b_desc = desc_k_major_sw128(st + Stage::kOffW);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        mma_nvf4(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, sf_t + k * 4, sf_w + k * 8, kb > 0 || k > 0);
+                    }
+                    tc_commit(empty_bar(stage));
+                    sf_buffer ^= 1;
+                    if (++stage == Stage::kCount) { stage = 0; phase ^= 1U; }
+                }
+                if (!ok) break;
+                tc_commit(accum_full);
+                accum_phase ^= 1U;
+            }
+        }
+    } else {
+        const int quarter = warp & 3;
+        const int group = (warp - 2) >> 2;                  // which 32 intermediate rows (MODE 0) or 64 output columns (MODE 1)
+        const std::uint32_t lane_base = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16);
+        const int row = quarter * 32 + lane;                // token row of the tile
+        std::uint32_t accum_phase = 0;
+        for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
+            Item it;
+            if (!decode_item<kTok>(p, route_table, item, &it)) continue;
+            if (!mbar_wait(accum_full, accum_phase)) { give_up(); break; }
+            accum_phase ^= 1U;
+            tc_fence_after();
+            const bool mine = quarter * 32 < it.valid;      // warp uniform
+            const int pp = it.pp0 + row;
+            if constexpr (MODE == 0) {
+                std::uint32_t first[32], second[32];
+                if (mine) {
+                    tmem_load32(lane_base + group * 32, first);
+                    tmem_load32(lane_base + 128 + group * 32, second);
+                    tmem_load_wait();
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accum_empty);
+                if (row < it.valid) {
+                    const float alpha_g = p.bank.alpha[it.entry * 3 + 0];
+                    const float alpha_u = p.bank.alpha[it.entry * 3 + 1];
+                    const int inter = p.m_total;
+                    std::uint32_t scale0, scale1;
+                    const uint2 q0 = swiglu_block16(first, second, alpha_g, alpha_u, p.quant_scale, &scale0);
+                    const uint2 q1 = swiglu_block16(first + 16, second + 16, alpha_g, alpha_u, p.quant_scale, &scale1);
+                    const int column = it.m_tile * kTileM + group * 32;
+                    *reinterpret_cast<uint4*>(p.hq + static_cast<std::size_t>(pp) * (inter / 2) + (column >> 1)) = make_uint4(q0.x, q0.y, q1.x, q1.y);
+                    const int sf_col = column >> 4;         // even: the two bytes are neighbours in the tiled layout
+                    std::uint8_t* sf = p.hs + (static_cast<std::size_t>(pp >> 7) * (inter / 64) + (sf_col >> 2)) * 512 + (pp & 31) * 16 +
+                                       ((pp >> 5) & 3) * 4 + (sf_col & 3);
+                    *reinterpret_cast<std::uint16_t*>(sf) = static_cast<std::uint16_t>(scale0 | (scale1 << 8));
+                }
+                __syncwarp();                               // the next accumulator read is warp wide
+            } else {
+                const float alpha = p.bank.alpha[it.entry * 3 + 2];
+                uint4 w[8];
+                if (mine) load_scale_rows64(lane_base + group * 64, alpha, w);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accum_empty);
+                if (!mine) continue;
+                const long my_row = p.out_row != nullptr ? (row < it.valid ? p.out_row[it.dense0 + row] : 0) : pp;
+                store_rows64(p.out + static_cast<std::size_t>(it.m_tile) * kWRows + group * 64, p.m_total, my_row, it.valid - quarter * 32, w);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, kTmemAll);
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_expert_rows_gate_up(const p92b_plan* plan, const TcParams& p, cudaStream_t stream, bool pdl) {
+    if (cudaError_t st = ensure_dynamic_smem<expert_rows_kernel<0>>(Stage::kSmem); st != cudaSuccess) return st;
+    return launch_kernel(expert_rows_kernel<0>, dim3(plan->sm_count), dim3(kThreads), Stage::kSmem, stream, pdl, plan->map_x[1],
+                         plan->map_x[3], p);
+}
+
+cudaError_t launch_expert_rows_matrix(const p92b_plan* plan, TcParams p, cudaStream_t stream, bool pdl) {
+    p.m_tiles = p.m_total / kWRows;
+    if (cudaError_t st = ensure_dynamic_smem<expert_rows_kernel<1>>(Stage::kSmem); st != cudaSuccess) return st;
+    return launch_kernel(expert_rows_kernel<1>, dim3(plan->sm_count), dim3(kThreads), Stage::kSmem, stream, pdl, plan->map_h[1],
+                         plan->map_h[3], p);
+}
+
+}  // namespace p92b

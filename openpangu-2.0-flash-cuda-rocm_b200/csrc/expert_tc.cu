@@ -24,15 +24,14 @@
 //           up rows un-fused (MODE 2, the reference's project_expert_gate_up result).
 // Every role turns an item number into work from a copy of the routing lists in shared memory (RouteTable), and an
 // epilogue warp hands its accumulator buffer back as soon as it has read its columns into registers.
-// Two more kernels in this file serve large batches with the same three roles: expert_gu_pair_kernel (one weight stage
-// against two 64-row token tiles) and expert_down_slab_kernel (a 128-token slab resident, weights streaming past).
+// expert_down_slab_kernel serves the down product of large batches with the same three roles (a 128-token slab resident,
+// weights streaming past); their gate/up product, with the tokens on the M side, is in expert_rows.cu.
 // Scale factors stay in the 128x4-tiled layout the reference keeps them in
 // (cuda/nvfp4_ops.cu:869-890): one 512-byte tile is exactly one tcgen05.cp atom.
 //
 // Every mbarrier wait is bounded; on expiry the block records kStatusWaitExpired,
 // stops issuing work, frees its TMEM and returns.
-#include "p92b_common.cuh"
-#include "tc_ptx.cuh"
+#include "expert_common.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -40,12 +39,10 @@
 namespace p92b {
 
 using namespace ptx;
+using namespace expert;
 
 namespace {
 
-constexpr int kTileM = 128;
-constexpr int kBlockKBytes = 128;                 // one swizzle row: 256 E2M1 values
-constexpr int kSfSlab = 2048;                     // 128 rows x 16 scales of one K block
 constexpr int kEpilogueWarps = 16;                // four per TMEM quarter: they split the 16-column chunks
 constexpr int kThreadsTc = 64 + 32 * kEpilogueWarps;
 
@@ -77,107 +74,12 @@ struct Tc {
     static_assert(kNeedCols <= 512, "accumulators and scale factors must fit TMEM");
 };
 
-struct TcParams {
-    BankView bank;
-    RouteView route;
-    const std::int32_t* pp_off;        // [258]
-    const std::int32_t* tile_prefix;   // [active_count + 1]
-    const std::uint8_t* b_sf;          // token-side scales, 128x4 tiled over padded positions
-    std::uint8_t* hq;                  // MODE 0 out: packed SwiGLU rows [PP][I/2]
-    std::uint8_t* hs;                  // MODE 0 out: their scales, 128x4 tiled over padded positions
-    std::uint16_t* out;                // MODE 1 out: BF16 down rows [PP][H]
-    std::int32_t* status;
-    float quant_scale;                 // 1.0, passed at run time so the quantiser's divisions stay run-time operations
-    int k_bytes;                       // K/2: bytes per operand row
-    int m_total;                       // output rows per expert matrix
-    int m_tiles;
-    int routing_is_upstream;           // 1: the routing lists are written by the kernel just before this one in the stream
-    // optional redirections (stage entry points, p92b_nvfp4_grouped_rows)
-    const std::int32_t* out_row;       // null: output rows sit at their padded position; else [dense position] -> output row
-    std::uint16_t* gate_out;           // MODE 2: BF16 [output row][m_total]
-    std::uint16_t* up_out;
-    const p92b_expert_projection* table;   // SRC 1: device table of reference-format matrices, entry expert * 3 + kind
-    int table_kind;                    // SRC 1, MODE 1: which of an expert's three matrices
-    int skip_shared;                   // 1: the shared expert's items are not computed (the caller has none)
-    std::uint16_t* const* row_dest;    // slab kernel of the down product: null, or [padded position] -> destination row
-};
-
-struct Item {
-    int expert;
-    int entry;
-    int count;
-    int m_tile;
-    int pp0;
-    int valid;     // tokens of this tile that exist
-    int dense0;    // dense (unpadded) position of the tile's first row
-};
-
-// The routing lists a block needs to turn an item number into work, copied to shared memory once per block:
-// every role decodes every item, and from global memory that is a dozen dependent loads (a binary search over
-// the tile prefix, then the expert's entries) - about 1.4 µs per item, which in the MMA lane is time the tensor
-// pipe runs dry.  Indexed by active slot.
-struct RouteTable {
-    std::int32_t prefix[kExperts + 2];      // exclusive prefix of token tiles over the active list, total at [active_count]
-    std::int32_t expert[kExperts + 1];
-    std::int32_t count[kExperts + 1];
-    std::int32_t pp_off[kExperts + 1];
-    std::int32_t offset[kExperts + 1];
-    std::int32_t active_count;
-};
-
-// All threads of the block, after the lists are known to be written; the caller synchronises the block afterwards.
-__device__ __forceinline__ void load_route_table(const TcParams& p, RouteTable* t) {
-    const int n = min(*p.route.active_count, kExperts + 1);
-    for (int a = threadIdx.x; a <= n; a += blockDim.x) {
-        t->prefix[a] = p.tile_prefix[a];
-        if (a < n) {
-            const int e = p.route.active[a];
-            t->expert[a] = e;
-            t->count[a] = p.route.counts[e];
-            t->pp_off[a] = p.pp_off[e];
-            t->offset[a] = p.route.offsets[e];
-        }
-    }
-    if (threadIdx.x == 0) t->active_count = n;
-}
-
-template <int N>
-__device__ __forceinline__ bool decode_item(const TcParams& p, const RouteTable& t, int item, Item* it) {
-    const int tt = item / p.m_tiles;
-    it->m_tile = item - tt * p.m_tiles;
-    int lo = 0, hi = t.active_count;         // find a: prefix[a] <= tt < prefix[a+1]
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (t.prefix[mid] <= tt) lo = mid; else hi = mid;
-    }
-    const int n_tile = tt - t.prefix[lo];
-    it->expert = t.expert[lo];
-    it->entry = it->expert == kExperts ? p.bank.local_experts : it->expert - p.bank.first_expert;
-    it->count = t.count[lo];
-    it->pp0 = t.pp_off[lo] + n_tile * N;
-    it->valid = min(N, it->count - n_tile * N);
-    it->dense0 = t.offset[lo] + n_tile * N;
-    if (p.skip_shared && it->expert == kExperts) return false;
-    if (p.table != nullptr) {          // weights in place: the table is indexed by the global expert id
-        it->entry = it->expert;
-        return it->expert >= 0 && it->expert < kExperts;
-    }
-    return it->entry >= 0 && it->entry <= p.bank.local_experts;
-}
-
 // 16-byte asynchronous copy global -> shared (through the load/store unit, not the bulk-copy engine).
 __device__ __forceinline__ void async_copy16_tc(std::uint32_t dst_smem, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
 
-// Two floats rounded to BF16 (nearest even) in one conversion: the first in the low half.
-__device__ __forceinline__ std::uint32_t bf16x2_bits(float low, float high) {
-    const __nv_bfloat162 pair = __floats2bfloat162_rn(low, high);
-    return *reinterpret_cast<const std::uint32_t*>(&pair);
-}
-
-// The gate/up epilogue for one chunk of 16 token columns (shared by expert_tc_kernel<0, N> and
-// expert_gu_pair_kernel).  A lane holds one weight row (row0 + lane of the intermediate dimension): gate g[j] and
+// The gate/up epilogue for one chunk of 16 token columns (of expert_tc_kernel<0, N>).  A lane holds one weight row (row0 + lane of the intermediate dimension): gate g[j] and
 // up u[j] for token column c0 + j.  bf16(alpha * product) for both, SwiGLU rounded to BF16
 // (cuda/nvfp4_ops.cu:97-105), then the activation quantiser (cuda/nvfp4_ops.cu:818-841) along the intermediate
 // dimension, whose 16-element blocks are the two 16-lane halves of the warp:
@@ -594,230 +496,6 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
             __syncwarp();
             if (lane == 0) mbar_arrive(accum_empty(buffer));
             if (C::kAccumBuffers == 2) buffer ^= 1;
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc(tmem_base, C::kTmemCols);
-    }
-}
-
-// ---- gate/up for large batches: two 64-row token tiles per weight stage ---------------------------
-// At thousands of tokens the gate/up product is bound by L2-to-SM traffic: every 64-row token tile of an
-// expert pulls the expert's 128-row weight tile (36 KB per K block) across again.  Here an item is a PAIR
-// of neighbouring token tiles (one 128-row slab of the padded position space): a weight stage is loaded
-// once and multiplied with both, which halves the weight traffic of experts with more than 64 rows.
-// Each half keeps its own accumulator pair (gate | up, 64 columns each); three such buffers rotate, so
-// the epilogue of one item still overlaps the loads and MMAs of the next.
-struct GuPair {
-    static constexpr int kN = 64;
-    static constexpr int kChunk = 2 * (kTileM * kBlockKBytes + kSfSlab);            // 36,864: one chunk of the bank's stream
-    static constexpr int kOffSfA = 2 * kTileM * kBlockKBytes;
-    static constexpr int kOffB0 = kChunk;
-    static constexpr int kOffB1 = kOffB0 + kN * kBlockKBytes;
-    static constexpr int kOffSfB = kOffB1 + kN * kBlockKBytes;
-    static constexpr int kStageBytes = kOffSfB + kSfSlab;                           // 55,296
-    static constexpr int kStages = 4;
-    static constexpr int kAccumCols = 2 * kN;                                       // gate at +0, up at +64
-    static constexpr int kAccumBuffers = 3;
-    static constexpr int kSfCols = 3 * 16;                                          // SFA gate, SFA up, SFB
-    static constexpr int kTmemCols = 512;                                           // 3 * 128 + 2 * 48 = 480
-    static constexpr int kBarriers = 3 * kStages + 2 * kAccumBuffers;
-    static constexpr int kSmemBytes = kStages * kStageBytes + kBarriers * 8 + 16 + 1024;
-    // the epilogue (SwiGLU + re-quantisation, about 40 instructions per element) is what the issue slots are spent
-    // on: four warps per TMEM quarter, each taking one 16-column chunk of a half
-    static constexpr int kEpilogueWarps = 16;
-    static constexpr int kThreads = 64 + 32 * kEpilogueWarps;
-};
-
-__global__ void __launch_bounds__(GuPair::kThreads, 1) expert_gu_pair_kernel(const __grid_constant__ CUtensorMap map_b,
-                                                                        const TcParams p) {
-    using C = GuPair;
-    extern __shared__ std::uint8_t smem_raw[];
-    __shared__ RouteTable route_table;
-    const std::uint32_t base = (smem_u32(smem_raw) + 1023U) & ~1023U;
-    const std::uint32_t bars = base + C::kStages * C::kStageBytes;
-    auto weight_bar = [&](int s) { return bars + 8U * s; };
-    auto token_bar = [&](int s) { return bars + 8U * (C::kStages + s); };
-    auto empty_bar = [&](int s) { return bars + 8U * (2 * C::kStages + s); };
-    auto accum_full = [&](int b) { return bars + 8U * (3 * C::kStages + b); };
-    auto accum_empty = [&](int b) { return bars + 8U * (3 * C::kStages + C::kAccumBuffers + b); };
-    const std::uint32_t tmem_slot = bars + 8U * C::kBarriers;
-    volatile std::uint32_t* tmem_slot_ptr =
-        reinterpret_cast<volatile std::uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
-    volatile std::uint32_t* abort_ptr = tmem_slot_ptr + 1;
-
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int k_blocks = p.k_bytes / kBlockKBytes;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < C::kStages; ++s) {
-            mbar_init(weight_bar(s), 1);
-            mbar_init(token_bar(s), 1);
-            mbar_init(empty_bar(s), 1);
-        }
-        for (int b = 0; b < C::kAccumBuffers; ++b) {
-            mbar_init(accum_full(b), 1);
-            mbar_init(accum_empty(b), C::kEpilogueWarps);
-        }
-        *abort_ptr = 0;
-        fence_mbar_init();
-        prefetch_tensormap(&map_b);
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, C::kTmemCols);
-        tmem_relinquish();
-    }
-    pdl_wait();                       // routing lists and token rows come from the kernels upstream
-    load_route_table(p, &route_table);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    pdl_launch_dependents();
-    const std::uint32_t tmem_base = *tmem_slot_ptr;
-    const int total_items = route_table.prefix[route_table.active_count] * p.m_tiles;       // the prefix counts 128-row slabs here
-    auto give_up = [&]() {
-        *abort_ptr = 1;
-        atomicCAS(p.status, kStatusOk, kStatusWaitExpired);
-    };
-
-    if (warp == 0) {
-        if (elect_one()) {
-            int stage = 0;
-            std::uint32_t phase = 0;
-            for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
-                Item it;
-                if (!decode_item<2 * C::kN>(p, route_table, item, &it)) continue;
-                const bool two = it.valid > C::kN;
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(empty_bar(stage), phase ^ 1U)) { give_up(); break; }
-                    const std::uint32_t st = base + stage * C::kStageBytes;
-                    mbar_arrive_expect_tx(weight_bar(stage), C::kChunk);
-                    bulk_load(st, p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) *
-                                                   kChunkBytes,
-                              kChunkBytes, weight_bar(stage));
-                    mbar_arrive_expect_tx(token_bar(stage), (two ? 2 : 1) * C::kN * kBlockKBytes + kSfSlab);
-                    tma_load_2d(st + C::kOffB0, &map_b, token_bar(stage), kb * kBlockKBytes, it.pp0);
-                    if (two) tma_load_2d(st + C::kOffB1, &map_b, token_bar(stage), kb * kBlockKBytes, it.pp0 + C::kN);
-                    bulk_load(st + C::kOffSfB,
-                              p.b_sf + (static_cast<std::size_t>(it.pp0 >> 7) * (p.k_bytes / 32) + kb * 4) * 512, kSfSlab,
-                              token_bar(stage));
-                    if (++stage == C::kStages) { stage = 0; phase ^= 1U; }
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (elect_one()) {
-            int stage = 0;
-            std::uint32_t phase = 0;
-            int next_buffer = 0;
-            std::uint32_t accum_phase = 0;                      // bit b = phase of buffer b
-            constexpr std::uint32_t idesc = idesc_nvf4(kTileM, C::kN);
-            const std::uint32_t sf_tmem = tmem_base + C::kAccumBuffers * C::kAccumCols;
-            int sf_buffer = 0;
-            for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
-                Item it;
-                if (!decode_item<2 * C::kN>(p, route_table, item, &it)) continue;
-                const int halves = it.valid > C::kN ? 2 : 1;
-                int buffer[2];
-                bool ok = true;
-                for (int h = 0; h < halves && ok; ++h) {
-                    buffer[h] = next_buffer;
-                    next_buffer = (next_buffer + 1) % C::kAccumBuffers;
-                    if (!mbar_wait(accum_empty(buffer[h]), ((accum_phase >> buffer[h]) & 1U) ^ 1U)) { give_up(); ok = false; }
-                }
-                if (!ok) break;
-                tc_fence_after();
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(weight_bar(stage), phase) || !mbar_wait(token_bar(stage), phase)) {
-                        give_up();
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const std::uint32_t st = base + stage * C::kStageBytes;
-                    const std::uint32_t sfc = sf_tmem + sf_buffer * C::kSfCols;
-#pragma unroll
-                    for (int o = 0; o < 3; ++o) {
-                        const std::uint32_t slab = o < 2 ? st + C::kOffSfA + o * kSfSlab : st + C::kOffSfB;
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) tc_copy_sf(sfc + o * 16 + k * 4, desc_scale_atom(slab + k * 512));
-                    }
-                    for (int h = 0; h < halves; ++h) {
-                        const std::uint32_t accum = tmem_base + buffer[h] * C::kAccumCols;
-                        const std::uint64_t b_desc = desc_k_major_sw128(st + (h == 0 ? C::kOffB0 : C::kOffB1));
-                        // rows 64..127 of the slab are quarters 2 and 3 of its 128-row scale tile: two TMEM columns further
-                        const std::uint32_t b_quarter = h == 0 ? 0U : 2U;
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-#pragma unroll
-                            for (int a = 0; a < 2; ++a) {
-                                const std::uint64_t a_desc = desc_k_major_sw128(st + a * kTileM * kBlockKBytes);
-                                mma_nvf4(accum + a * C::kN, a_desc + 2 * k, b_desc + 2 * k, idesc, sfc + a * 16 + k * 4,
-                                         sfc + 32 + k * 4 + b_quarter, kb > 0 || k > 0);
-                            }
-                        }
-                    }
-                    tc_commit(empty_bar(stage));
-                    sf_buffer ^= 1;
-                    if (++stage == C::kStages) { stage = 0; phase ^= 1U; }
-                }
-                if (!ok) break;
-                for (int h = 0; h < halves; ++h) {
-                    tc_commit(accum_full(buffer[h]));
-                    accum_phase ^= 1U << buffer[h];
-                }
-            }
-        }
-    } else {
-        // epilogue: the code of expert_tc_kernel<0, 64>, once per half of the item
-        const int quarter = warp & 3;
-        const int sub = (warp - 2) >> 2;                  // 0..3: which 16-column chunk of every 64
-        int next_buffer = 0;
-        std::uint32_t accum_phase = 0;
-        for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
-            Item it;
-            if (!decode_item<2 * C::kN>(p, route_table, item, &it)) continue;
-            const int halves = it.valid > C::kN ? 2 : 1;
-            const float alpha_g = p.bank.alpha[it.entry * 3 + 0];
-            const float alpha_u = p.bank.alpha[it.entry * 3 + 1];
-            const int inter = p.m_total;
-            const int row0 = it.m_tile * kTileM + quarter * 32;
-            bool ok = true;
-            for (int hh = 0; hh < halves; ++hh) {
-                const int buffer = next_buffer;
-                next_buffer = (next_buffer + 1) % C::kAccumBuffers;
-                if (!mbar_wait(accum_full(buffer), (accum_phase >> buffer) & 1U)) { give_up(); ok = false; break; }
-                accum_phase ^= 1U << buffer;
-                tc_fence_after();
-                const int pp0 = it.pp0 + hh * C::kN;
-                const int valid = hh == 0 ? min(C::kN, it.valid) : it.valid - C::kN;
-                const std::uint32_t lane_base =
-                    tmem_base + buffer * C::kAccumCols + (static_cast<std::uint32_t>(quarter * 32) << 16);
-                std::uint8_t* hs_tile = p.hs + static_cast<std::size_t>(pp0 >> 7) * (inter / 64) * 512;
-                std::uint8_t* hq_rows = p.hq + static_cast<std::size_t>(pp0) * (inter / 2);
-                const int n_base = pp0 & 127;
-                // Sixteen warps, sixteen (quarter, 16-column chunk) pieces per half: a warp has exactly one.  It takes its
-                // piece into registers and gives the buffer back at once - the arithmetic that follows is several times
-                // longer than the read, and the MMA lane needs two free buffers to start the next item.
-                static_assert(C::kN == 16 * (C::kEpilogueWarps / 4), "one chunk per warp and half");
-                const int c0 = sub * 16;
-                const bool mine = c0 < valid;                                        // warp uniform
-                std::uint32_t g[16], u[16];
-                if (mine) {
-                    tmem_load16(lane_base + c0, g);
-                    tmem_load16(lane_base + C::kN + c0, u);
-                    tmem_load_wait();
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(accum_empty(buffer));
-                if (mine) swiglu_requant_chunk(g, u, alpha_g, alpha_u, p.quant_scale, lane, c0, valid, n_base, inter, row0, hq_rows, hs_tile);
-            }
-            if (!ok) break;
         }
     }
     tc_fence_before();
@@ -1329,13 +1007,13 @@ cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int 
             case 0: return launch_tc<0, 16>(plan, plan->map_x[0], p, stream, pdl);
             case 1: return launch_tc<0, 32>(plan, plan->map_x[1], p, stream, pdl);
             default:
-                if (plan->wide_rows == 128 && std::getenv("P92B_NO_GU_PAIR") == nullptr) {
-                    // large batches: pairs of 64-row token tiles share one weight stage (one 128-column tile was
-                    // tried too: a single accumulator buffer and three stages then, 377 µs against 283 µs at T=4096)
+                // Lists with 128-row tiles (every call of more than 32 rows except the expert-parallel ones that build
+                // their lists themselves): tokens on the M side.  It is the quicker form over the whole range: 107 against
+                // 109 us at 64 rows, 123 against 129 at 512 (both near the HBM time of the weights), 168 against 201 at
+                // 4,096, 389 against 563 at 16,384.
+                if (plan->wide_rows == 128) {
                     p.tile_prefix = plan->tile_prefix_wide;
-                    if (cudaError_t st = ensure_dynamic_smem<expert_gu_pair_kernel>(GuPair::kSmemBytes); st != cudaSuccess) return st;
-                    return launch_kernel(expert_gu_pair_kernel, dim3(plan->sm_count), dim3(GuPair::kThreads), GuPair::kSmemBytes,
-                                         stream, pdl, plan->map_x[2], p);
+                    return launch_expert_rows_gate_up(plan, p, stream, pdl);
                 }
                 return launch_tc<0, 64>(plan, plan->map_x[2], p, stream, pdl);
         }
@@ -1368,6 +1046,11 @@ cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int 
                                          stream, pdl, plan->map_h[3], p);
                 }
                 if (p.row_dest != nullptr) return cudaErrorNotSupported;
+                // any K: 128 x 256 tiles with the tokens on the M side (dense MLP, 3,807 rows: both products together 196 ->
+                // 141 us per layer); it stores 16 bytes at a time and computes whole token tiles of every entry
+                if (!(io != nullptr && io->skip_shared) && (reinterpret_cast<std::uintptr_t>(p.out) & 15U) == 0U) {
+                    return launch_expert_rows_matrix(plan, p, stream, pdl);
+                }
                 return launch_tc<1, 128>(plan, plan->map_h[3], p, stream, pdl);
             }
             if (p.row_dest != nullptr) return cudaErrorNotSupported;
