@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(kEpThreads, 1) moe_decode_ep_kernel(const __gr
             const std::uint32_t mask = rt.slot_mask[slot];
             const int pp0 = slab_of_slot(slot, rt.n_active);
             const std::uint32_t lane_base = tmem_base + buffer * kAccumCols + (static_cast<std::uint32_t>(quarter * 32) << 16);
-            const int row = m_tile * kTile + quarter * 32 + lane;
+            const int row = m_tile * kTile + (kind == 0 ? gu_tile_row(quarter, lane) : quarter * 32 + lane);
             if (kind == 0) {
                 const float alpha_g = p.bank.alpha[entry * 3 + 0];
                 const float alpha_u = p.bank.alpha[entry * 3 + 1];
@@ -643,6 +643,7 @@ __global__ void __launch_bounds__(kEpThreads, 1) moe_decode_ep_kernel(const __gr
                         const int token = 16 * c + n;
                         if (!(mask >> token & 1U)) continue;                          // warp uniform
                         const std::size_t pp = static_cast<std::size_t>(pp0 + __popc(mask & ((1U << token) - 1U)));
+                        gu_exchange(g[n], u[n], lane, &g[n], &u[n]);
                         const float gv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(g[n]) * alpha_g));
                         const float uv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(u[n]) * alpha_u));
                         const float h = bf16_bits_to_float(float_to_bf16_bits((gv / (1.0F + expf(-gv))) * uv));

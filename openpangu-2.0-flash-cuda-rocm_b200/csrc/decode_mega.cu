@@ -14,15 +14,16 @@
 //       every token (cuda/nvfp4_ops.cu:357-433), histogram, stable permutation
 //       (cuda/nvfp4_grouped.cu:117-132), active-expert list; block 0 also writes the
 //       routing products to global memory;
-//   P2  gate/up tiles and P3 down tiles through ONE TMA ring and one tcgen05 pipeline
-//       (same operand formats as expert_tc.cu).  The token side of gate/up is simply all
+//   P2  gate/up tiles (64 intermediate rows: one box of mixed gate and up rows) and P3 down tiles (128 output
+//       rows) through ONE TMA ring and one tcgen05 pipeline (same operand formats as expert_tc.cu).  The token side of gate/up is simply all
 //       tokens in token order (N=16 columns cost nothing at M=128), so it does not depend
 //       on routing; the epilogue keeps the columns routed to the tile's expert.  A down
-//       tile needs the eight gate/up tiles of its expert: per-expert counters, no barrier,
+//       tile needs the sixteen gate/up tiles of its expert: per-expert counters, no barrier,
 //       and its weights are already in flight while the producer waits.  Tiles are handed
 //       out dynamically from one device-wide counter, gate/up tiles first, both in expert
-//       order: a block that falls behind simply takes fewer (a gate/up tile is 10 ring
-//       stages, a down tile 2, so the tail is fine-grained);
+//       order: a block that falls behind simply takes fewer (a gate/up tile is 5 ring
+//       stages, a down tile 2, so the tail is fine-grained).  With one token the 144 gate/up tiles are
+//       one round of the 148 blocks (72 tiles of 128 rows left half the chip idle: 22.0 -> 18.8 us);
 //   P4  weighted combine in slot order + shared expert (cuda/nvfp4_ops.cu:124-142,92-95):
 //       the down epilogue publishes its rows as {two BF16, launch number} words and the
 //       combining threads poll the words they need, so the combine of a token starts when
@@ -41,7 +42,19 @@ using namespace decode;
 
 namespace {
 
-constexpr int kMegaThreads = 192;
+// Warps 0 and 1 are the producer and the MMA lane, 2..5 the epilogue; the others only work before the first tile and
+// after the last one: staging, norms, logits, quantisation and top-8 are a handful of short dependent chains per token,
+// and with 13 tokens six warps went round three times for each of them
+// (T=13: 81 instead of 100 us per layer with both norms; T=1: 18.8 against 19.2 with eight warps, T=4: the same).
+constexpr int kMegaThreads = 512;
+constexpr int kMegaWarps = kMegaThreads / 32;
+// Every logit is published in eight places and a block polls one of them: all blocks need all words at the same moment,
+// and 148 readers of the same few lines queue up at the L2 slices that hold them.  For the same reason a block starts to
+// poll only when its own logits are out, asks again only for what is missing, and nobody polls the arrival counter
+// while it is being counted up: at four tokens the last reader had the logits 2.2 us after the average block was done
+// with its own, now 1.0 us.
+constexpr int kReplicas = 8;
+constexpr int kEpilogueEnd = 6;                    // first warp behind the epilogue warps
 constexpr int kMegaMaxRows = 16;                   // = kN: the token side of every MMA holds them all; the kernel is built
                                                    // for 8 (the decode sizes, leaner loops) and for 16 rows
 constexpr int kN = 16;                             // token columns of every MMA
@@ -69,7 +82,7 @@ struct MegaParams {
     std::uint8_t* hq;              // [PP][I/2]
     std::uint8_t* hs;              // tiled scales of hq
     std::uint16_t* mixed;          // [PP][H]
-    unsigned long long* logits_tagged;   // [8][256] {value, launch number}
+    unsigned long long* logits_tagged;   // [kReplicas][R][256] {value, launch number}
     unsigned long long* ret;             // [8][9][1280] {two BF16, launch number}
     unsigned* sync;                // [0]: blocks that have finished P0 (monotonic across launches)
     std::int32_t* gu_done;         // [2][264] by launch parity: gate/up tiles finished per active slot, [257] tile counter
@@ -78,6 +91,7 @@ struct MegaParams {
     const std::uint16_t* post_norm_w;    // optional: RMSNorm weight applied to the block's output rows
     unsigned long long* hidden_tagged;   // [8][H/2] {two BF16 of the un-normalised output, launch number} (post-norm only)
     float norm_eps;
+    int norm_w_aligned;                  // both norm weights (where given) start on a 16-byte boundary
     unsigned long long* trace;     // optional [grid][64] %globaltimer stamps per block (null: off)
     unsigned epoch;                // launches of this kernel on the plan before this one
     float routed_scale;
@@ -102,19 +116,32 @@ struct Routing {                   // shared-memory copy, identical in every blo
     std::uint32_t expert_mask[kExperts];             // tokens routed to each expert
     std::int32_t before[kExperts];                   // assignments with a smaller expert id
     std::int32_t slot_of[kExperts];                  // active slot an expert has (if any token picked it)
-    float logits[R * kExperts];
-    float bias[kExperts];
+    __align__(16) float logits[R * kExperts];
+    __align__(16) float bias[kExperts];
 };
 
-// One arrival per block on a device-wide counter; whoever needs all blocks to have arrived waits for
-// the count itself (wait_counter).
-__device__ __forceinline__ void grid_arrive(unsigned* counter) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        fence_proxy_async_all();          // what the block wrote is later read by TMA in other blocks
-        atomicAdd(counter, 1U);
+// Eight norm weights, one 16-byte load where the pointer allows it.
+__device__ __forceinline__ uint4 load_norm_weight(const std::uint16_t* w, bool aligned, int vec) {
+    if (aligned) return __ldg(reinterpret_cast<const uint4*>(w) + vec);
+    std::uint32_t words[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        words[i] = static_cast<std::uint32_t>(__ldg(w + vec * 8 + 2 * i)) | (static_cast<std::uint32_t>(__ldg(w + vec * 8 + 2 * i + 1)) << 16);
     }
+    return make_uint4(words[0], words[1], words[2], words[3]);
+}
+
+// bf16(x * inverse * w) of eight columns.
+__device__ __forceinline__ uint4 normalise8(uint4 x, float inverse, uint4 w) {
+    const std::uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ws[4] = {w.x, w.y, w.z, w.w};
+    std::uint32_t out[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const std::uint16_t lo = float_to_bf16_bits(__uint_as_float(xs[i] << 16) * inverse * __uint_as_float(ws[i] << 16));
+        const std::uint16_t hi = float_to_bf16_bits(__uint_as_float(xs[i] & 0xffff0000U) * inverse * __uint_as_float(ws[i] & 0xffff0000U));
+        out[i] = static_cast<std::uint32_t>(lo) | (static_cast<std::uint32_t>(hi) << 16);
+    }
+    return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
 template <int R>
@@ -129,7 +156,6 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     __shared__ volatile std::uint32_t abort_word;
     __shared__ volatile int tile_queue[kTileQueue];
     __shared__ volatile int first_tile_word;
-    __shared__ volatile int rows_ready_word;
     __shared__ float norm_partial[R][8];
     __shared__ float norm_inverse[R];
 
@@ -177,23 +203,30 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     // the router rows and the bias do not depend on the kernel upstream: fetch them before waiting for it
     const int my_experts = block + grid < kExperts ? 2 : (block < kExperts ? 1 : 0);
     std::uint16_t* w_rows = reinterpret_cast<std::uint16_t*>(smem_raw + (base - smem_u32(smem_raw)));
-    std::uint16_t* x_rows = w_rows + 2 * hidden;
+    // rows 64 bytes further apart than they are long: two neighbouring rows, read side by side by the halves of a warp,
+    // then lie in different banks
+    const int row_pitch = hidden + 32;
+    std::uint16_t* x_rows = w_rows + 2 * row_pitch;
     const int vec_per_row = hidden / 8;
     // (asynchronous 16-byte copies: the token rows below are requested behind them without waiting for these, so the
     // block pays one round trip to the L2 for both, not two)
     for (int i = threadIdx.x; i < my_experts * vec_per_row; i += kMegaThreads) {
         const int r = i / vec_per_row;
         const int c = i - r * vec_per_row;
-        async_copy16(reinterpret_cast<uint4*>(w_rows + r * hidden) + c,
+        async_copy16(reinterpret_cast<uint4*>(w_rows + r * row_pitch) + c,
                      reinterpret_cast<const uint4*>(p.router_w + static_cast<std::size_t>(block + r * grid) * hidden) + c);
     }
     for (int e = threadIdx.x; e < kExperts; e += kMegaThreads) async_copy4(&rt.bias[e], p.bias + e);
+    // a thread below hidden / 8 owns eight columns of every row in the pre-norm: their weights, too, do not depend on upstream
+    const bool norm_thread = static_cast<int>(threadIdx.x) < vec_per_row;
+    uint4 pre_w = make_uint4(0U, 0U, 0U, 0U);
+    if (p.pre_norm_w != nullptr && norm_thread) pre_w = load_norm_weight(p.pre_norm_w, p.norm_w_aligned, threadIdx.x);
     pdl_wait();                       // the token rows come from the kernel before this one
     pdl_launch_dependents();
     for (int i = threadIdx.x; i < rows * vec_per_row; i += kMegaThreads) {
         const int r = i / vec_per_row;
         const int c = i - r * vec_per_row;
-        async_copy16(reinterpret_cast<uint4*>(x_rows + r * hidden) + c,
+        async_copy16(reinterpret_cast<uint4*>(x_rows + r * row_pitch) + c,
                      reinterpret_cast<const uint4*>(p.x + static_cast<std::size_t>(r) * hidden) + c);
     }
     // the first tile number is asked for now and used after the routing, the atomic's latency in between; behind the
@@ -205,22 +238,30 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     tc_fence_after();
     // RMSNorm, the reference operator's arithmetic (cuda/nvfp4_ops.cu:67-90): 256 chains per row (chain t: elements
     // t, t+256, ... with fmaf), a shuffle-down tree per 32 chains, a second tree over the eight results, then
-    // rsqrtf(sum / H + eps).  Eight "virtual warps" of 32 chains per row are dealt to the block's six warps.
+    // rsqrtf(sum / H + eps).  A lane runs two neighbouring chains (one 4-byte read per step), so a warp does two groups of
+    // 32 chains of a row at once, and a tree step over `off` chains is a shuffle over off / 2 lanes; the last step adds the
+    // lane's own two.
     auto row_sum_of_squares = [&](const std::uint16_t* rows_bf16, int n_rows) {
-        for (int vw = warp; vw < n_rows * 8; vw += kMegaThreads / 32) {
-            const int r = vw >> 3, w8 = vw & 7;
-            const std::uint16_t* xr = rows_bf16 + r * hidden;
-            float square_sum = 0.0F;
-            for (int i = w8 * 32 + lane; i < hidden; i += 256) {
-                const float value = bf16_bits_to_float(xr[i]);
-                square_sum = fmaf(value, value, square_sum);
+        for (int job = warp; job < n_rows * 4; job += kMegaWarps) {
+            const int r = job >> 2, w4 = job & 3;
+            const std::uint32_t* xr = reinterpret_cast<const std::uint32_t*>(rows_bf16 + r * row_pitch) + w4 * 32 + lane;
+            float even = 0.0F, odd = 0.0F;
+#pragma unroll 5
+            for (int i = 0; i < hidden / 256; ++i) {
+                const std::uint32_t pair = xr[i * 128];
+                const float lo = __uint_as_float(pair << 16), hi = __uint_as_float(pair & 0xffff0000U);
+                even = fmaf(lo, lo, even);
+                odd = fmaf(hi, hi, odd);
             }
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) square_sum += __shfl_down_sync(0xffffffffU, square_sum, off);
-            if (lane == 0) norm_partial[r][w8] = square_sum;
+            for (int off = 8; off > 0; off >>= 1) {
+                even += __shfl_down_sync(0xffffffffU, even, off);
+                odd += __shfl_down_sync(0xffffffffU, odd, off);
+            }
+            if ((lane & 15) == 0) norm_partial[r][w4 * 2 + (lane >> 4)] = even + odd;
         }
         __syncthreads();
-        for (int r = warp; r < n_rows; r += kMegaThreads / 32) {
+        for (int r = warp; r < n_rows; r += kMegaWarps) {
             float total = lane < 8 ? norm_partial[r][lane] : 0.0F;
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) total += __shfl_down_sync(0xffffffffU, total, off);
@@ -232,11 +273,11 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
         // every block normalises all token rows for itself, in place in shared memory: from here on the kernel sees
         // the rows the reference's rmsnorm(pre_mlp_norm) would have written (src/model.cpp:211-212,1210-1211)
         row_sum_of_squares(x_rows, rows);
-        for (int i = threadIdx.x; i < rows * hidden; i += kMegaThreads) {
-            const int r = i / hidden;
-            const int c = i - r * hidden;
-            x_rows[i] = float_to_bf16_bits(bf16_bits_to_float(x_rows[i]) * norm_inverse[r] *
-                                           bf16_bits_to_float(__ldg(p.pre_norm_w + c)));
+        if (norm_thread) {
+            for (int r = 0; r < rows; ++r) {
+                uint4* at = reinterpret_cast<uint4*>(x_rows + r * row_pitch) + threadIdx.x;
+                *at = normalise8(*at, norm_inverse[r], pre_w);
+            }
         }
         __syncthreads();
     }
@@ -255,11 +296,11 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
         if (rows == 1) {
             // T = 1 order: 256 partial chains (thread t: columns t, t+256, ...), a shuffle-down tree
             // per 32 of them, then a tree over the eight results (cuda/nvfp4_ops.cu:38-51,161-176)
-            // The block's (router row, group of 32 chains) pairs are dealt to its six warps - one warp per row would walk
-            // eight dependent rounds while four warps idle - and a warp per row then adds the eight group sums.
-            for (int job = warp; job < my_experts * 8; job += kMegaThreads / 32) {
+            // The block's (router row, group of 32 chains) pairs are dealt to its warps, one each, and a warp per row then
+            // adds the eight group sums.
+            for (int job = warp; job < my_experts * 8; job += kMegaWarps) {
                 const int q = job >> 3, v = job & 7;
-                const std::uint16_t* wr = w_rows + q * hidden;
+                const std::uint16_t* wr = w_rows + q * row_pitch;
                 float partial = 0.0F;
                 for (int c = lane + 32 * v; c < hidden; c += 256) {
                     partial = fmaf(bf16_bits_to_float(x_rows[c]), bf16_bits_to_float(wr[c]), partial);
@@ -269,48 +310,45 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 if (lane == 0) norm_partial[q][v] = partial;
             }
             __syncthreads();
-            for (int q = warp; q < my_experts; q += kMegaThreads / 32) {
+            for (int q = warp; q < my_experts; q += kMegaWarps) {
                 float value = lane < 8 ? norm_partial[q][lane] : 0.0F;
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) value += __shfl_down_sync(0xffffffffU, value, off);
-                if (lane == 0) {
-                    const int e = block + q * grid;
-                    p.logits[e] = value;
-                    st_tagged(p.logits_tagged + e, __float_as_uint(value), tag);
-                }
+                value = __shfl_sync(0xffffffffU, value, 0);
+                const int e = block + q * grid;
+                if (lane == 0) p.logits[e] = value;
+                if (lane < kReplicas) st_tagged(p.logits_tagged + lane * R * kExperts + e, __float_as_uint(value), tag);
             }
         } else {
             // T > 1 order: lane l sums columns l, l+32, ...; shuffle-down tree (cuda/nvfp4_ops.cu:178-207).
-            // A warp runs the chains of two tokens against one router row side by side (same order within
-            // each chain), so four tokens x two rows are one round of the six warps.
-            const int token_pairs = (rows + 1) / 2;
-            for (int q = warp; q < my_experts * token_pairs; q += kMegaThreads / 32) {
-                const int r = q / token_pairs;
-                const int t0 = 2 * (q - r * token_pairs);
-                const bool second = t0 + 1 < rows;
-                const std::uint16_t* wr = w_rows + r * hidden;
-                const std::uint16_t* xa = x_rows + t0 * hidden;
-                const std::uint16_t* xb = x_rows + (second ? t0 + 1 : t0) * hidden;
-                float va = 0.0F, vb = 0.0F;
+            // Half a warp per chain set: lane l of a half runs columns 2l and 2l + 1 (mod 32) of one (token, router row)
+            // pair with one 4-byte read per operand and step - 2-byte reads, a lane per column, keep the shared-memory
+            // pipe busy for twice as long, which is what this phase is bound by.  The halves take the block's two router
+            // rows with the same token, or two tokens where the block has one router row.
+            const int half = lane >> 4, l16 = lane & 15;
+            for (int q = warp; my_experts == 2 ? q < rows : 2 * q < rows; q += kMegaWarps) {
+                const int t = my_experts == 2 ? q : min(2 * q + half, rows - 1);
+                const int r = my_experts == 2 ? half : 0;
+                const std::uint32_t* wr = reinterpret_cast<const std::uint32_t*>(w_rows + r * row_pitch) + l16;
+                const std::uint32_t* xr = reinterpret_cast<const std::uint32_t*>(x_rows + t * row_pitch) + l16;
+                float even = 0.0F, odd = 0.0F;
 #pragma unroll 8
-                for (int c = lane; c < hidden; c += 32) {
-                    const float wv = bf16_bits_to_float(wr[c]);
-                    va = fmaf(bf16_bits_to_float(xa[c]), wv, va);
-                    vb = fmaf(bf16_bits_to_float(xb[c]), wv, vb);
+                for (int j = 0; j < hidden / 32; ++j) {
+                    const std::uint32_t wv = wr[16 * j], xv = xr[16 * j];
+                    even = fmaf(__uint_as_float(xv << 16), __uint_as_float(wv << 16), even);
+                    odd = fmaf(__uint_as_float(xv & 0xffff0000U), __uint_as_float(wv & 0xffff0000U), odd);
                 }
+                // the tree over the 32 chains: steps of 16, 8, 4, 2 chains are 8, 4, 2, 1 lanes, the last one is this lane's own
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    va += __shfl_down_sync(0xffffffffU, va, off);
-                    vb += __shfl_down_sync(0xffffffffU, vb, off);
+                for (int off = 8; off > 0; off >>= 1) {
+                    even += __shfl_down_sync(0xffffffffU, even, off);
+                    odd += __shfl_down_sync(0xffffffffU, odd, off);
                 }
-                if (lane == 0) {
+                const float value = __shfl_sync(0xffffffffU, even + odd, lane & 16);
+                if (my_experts == 2 || 2 * q + half < rows) {
                     const int e = block + r * grid;
-                    p.logits[static_cast<std::size_t>(t0) * kExperts + e] = va;
-                    st_tagged(p.logits_tagged + t0 * kExperts + e, __float_as_uint(va), tag);
-                    if (second) {
-                        p.logits[static_cast<std::size_t>(t0 + 1) * kExperts + e] = vb;
-                        st_tagged(p.logits_tagged + (t0 + 1) * kExperts + e, __float_as_uint(vb), tag);
-                    }
+                    if (l16 == 0) p.logits[static_cast<std::size_t>(t) * kExperts + e] = value;
+                    if (l16 < kReplicas) st_tagged(p.logits_tagged + (l16 * R + t) * kExperts + e, __float_as_uint(value), tag);
                 }
             }
         }
@@ -321,7 +359,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
         if (g < rows * blocks16) {
             const int t = g / blocks16;
             const int b = g - t * blocks16;
-            const uint4* src = reinterpret_cast<const uint4*>(x_rows + t * hidden + b * 16);
+            const uint4* src = reinterpret_cast<const uint4*>(x_rows + t * row_pitch + b * 16);
             const uint4 lo = src[0];
             const uint4 hi = src[1];
             const std::uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
@@ -341,58 +379,59 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
         }
     }
     if (threadIdx.x == 0) stamp(1);
-    grid_arrive(p.sync + 0);          // quantised rows and zeroed counters of this block are out
+    // One arrival per block on a device-wide counter when all its warps are past P0 (quantised rows and zeroed counters
+    // are out); the producer lane waits for the count of all blocks before it asks the TMA for the token rows.
+    __syncthreads();
+    if (threadIdx.x == kMegaThreads - 32) {
+        __threadfence();
+        fence_proxy_async_all();              // what the block wrote is later read by TMA in other blocks
+        atomicAdd(p.sync + 0, 1U);
+    }
 
     // ------------------------------------------------------------------ P1
-    {
-        // logits come from all blocks of this launch: each word is polled until it carries this launch's
-        // number.  All of a thread's words are requested before the first is looked at.
-        constexpr int kPerThread = (R * kExperts + kMegaThreads - 1) / kMegaThreads;
-        uint2 word[kPerThread];
+    // (the last warp is left out: it is the one that waits for the fence above)
+    constexpr int kPollers = kMegaThreads - 32;
+    if (warp < kMegaWarps - 1) {
+        for (int i = threadIdx.x; i < kMaxActive * R; i += kPollers) (&rt.pp_tok[0][0])[i] = -1;
+        for (int i = threadIdx.x; i < kExperts; i += kPollers) rt.expert_mask[i] = 0U;
+        // logits come from all blocks of this launch: each word is polled until it carries this launch's number.  All of a
+        // thread's words are requested before the first is looked at, and only the missing ones again.
+        constexpr int kPerThread = (R * kExperts / 2 + kPollers - 1) / kPollers;        // pairs of words
+        const unsigned long long* const mine = p.logits_tagged + (block % kReplicas) * R * kExperts;
+        uint4 pair[kPerThread];
+        unsigned missing = 0U;
+#pragma unroll
+        for (int j = 0; j < kPerThread; ++j) {
+            if (2 * (static_cast<int>(threadIdx.x) + j * kPollers) < rows * kExperts) missing |= 1U << j;
+        }
         const std::uint64_t poll_start = global_timer_ns();
-        while (true) {
-            // every word still missing is requested again in one batch: one round trip per round, not per word
-            bool missing = false;
+        while (missing != 0U) {
 #pragma unroll
             for (int j = 0; j < kPerThread; ++j) {
-                const int i = threadIdx.x + j * kMegaThreads;
-                if (i < rows * kExperts) word[j] = ld_tagged(p.logits_tagged + i);
+                if (missing >> j & 1U) pair[j] = ld_tagged_pair(mine + 2 * (threadIdx.x + j * kPollers));
             }
 #pragma unroll
             for (int j = 0; j < kPerThread; ++j) {
-                const int i = threadIdx.x + j * kMegaThreads;
-                if (i < rows * kExperts) {
-                    if (word[j].y == tag) {
-                        rt.logits[i] = __uint_as_float(word[j].x);
-                    } else {
-                        missing = true;
-                    }
+                if ((missing >> j & 1U) && pair[j].y == tag && pair[j].w == tag) {
+                    reinterpret_cast<float2*>(rt.logits)[threadIdx.x + j * kPollers] = make_float2(__uint_as_float(pair[j].x), __uint_as_float(pair[j].z));
+                    missing &= ~(1U << j);
                 }
             }
-            if (!missing) break;
-            if (global_timer_ns() - poll_start > 1000000000ULL) {
+            if (missing != 0U && global_timer_ns() - poll_start > 1000000000ULL) {
                 give_up(kStatusWaitExpired);
                 break;
             }
         }
-        // a thread of the last warp (free unless there are six or more tokens) makes sure every block's share of
-        // the quantised rows is written before the producer lane asks the TMA for them
-        if (threadIdx.x == kMegaThreads - 32) {
-            const bool arrived = wait_counter(p.sync + 0, (p.epoch + 1U) * static_cast<unsigned>(grid));
-            fence_proxy_async_all();      // ordinary stores of other blocks -> this block's TMA loads
-            rows_ready_word = arrived ? 1 : 0;
-        }
-        for (int i = threadIdx.x; i < kMaxActive * R; i += kMegaThreads) (&rt.pp_tok[0][0])[i] = -1;
-        for (int i = threadIdx.x; i < kExperts; i += kMegaThreads) rt.expert_mask[i] = 0U;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) stamp(2);
-    if (!abort_word) {
-        for (int t = warp; t < rows; t += kMegaThreads / 32) {
+        __syncwarp();
+        asm volatile("bar.sync 3, %0;" ::"n"(kPollers) : "memory");
+        if (threadIdx.x == 0) stamp(2);
+        for (int t = warp; t < rows && !abort_word; t += kMegaWarps - 1) {
             warp_top8(rt.logits + t * kExperts, rt.bias, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
         }
         if (threadIdx.x == 0) stamp(13);
-        __syncthreads();
+    }
+    __syncthreads();
+    if (!abort_word) {
         if (threadIdx.x == 0) stamp(14);
         // The ranking law of cuda/nvfp4_grouped.cu:117-132, position = #(smaller expert id) + #(same id,
         // smaller flat index), through one bit mask of tokens per expert (a token picks an expert at most
@@ -457,10 +496,10 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     }
     if (threadIdx.x == 0) stamp(3);
     // ------------------------------------------------------------ P2 + P3
-    const int gu_tiles = inter / kTile;          // 8
+    const int gu_tiles = inter / (kTile / 2);    // 16: one box of a chunk, 64 intermediate rows
     const int dn_tiles = hidden / kTile;         // 20
-    const int gu_kblocks = (hidden / 2) / kKB;   // 10 stages per gate/up tile
-    const int dn_stages = (inter / 2) / kKB / 2; // 2 stages per down tile (two K blocks each)
+    const int gu_stages = (hidden / 2) / kKB / 2; // 5 stages per gate/up tile, two K blocks each
+    const int dn_stages = (inter / 2) / kKB / 2; // 2 stages per down tile, two K blocks each
     const int gu_items = abort_word ? 0 : rt.n_active * gu_tiles;
     const int total_items = abort_word ? 0 : rt.n_active * (gu_tiles + dn_tiles);
 
@@ -469,7 +508,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
             int stage = 0;
             std::uint32_t phase = 0;
             int sequence = 0;
-            if (rows_ready_word == 0) give_up(kStatusWaitExpired);
+            bool rows_ready = false;
             const std::uint64_t stream_policy = l2_policy_evict_first();     // weights are read once per launch
             int current = first_tile_word;
             while (!abort_word) {
@@ -481,7 +520,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                     mbar_arrive(token_bar(stage));
                     break;
                 }
-                const int following = static_cast<int>(atomicAdd(tile_counter, 1U));
+                int following = 0;
                 int kind, slot, m_tile;
                 if (current < gu_items) {
                     kind = 0; slot = current / gu_tiles; m_tile = current - slot * gu_tiles;
@@ -491,7 +530,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 }
                 const int expert = rt.active[slot];
                 const int entry = expert == kExperts ? p.bank.local_experts : expert - p.bank.first_expert;
-                const int n_stages = kind == 0 ? gu_kblocks : dn_stages;
+                const int n_stages = kind == 0 ? gu_stages : dn_stages;
                 bool tokens_ready = kind == 0;
                 bool ok = true;
                 for (int s = 0; s < n_stages; ++s) {
@@ -501,18 +540,32 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                     if (sequence == 0 && s < 10) stamp(16 + s);
                     mbar_arrive_expect_tx(weight_bar(stage), kWeightTx);
                     if (kind == 0) {
-                        bulk_load_hint(st, p.bank.g13 + ((static_cast<std::size_t>(entry) * gu_tiles + m_tile) * gu_kblocks + s) *
-                                                            kChunkBytes,
-                                       kChunkBytes, weight_bar(stage), stream_policy);
-                        mbar_arrive_expect_tx(token_bar(stage), 2 * kSlab);
-                        tma_load_2d(st + kOffB0, &map_x, token_bar(stage), s * kKB, 0);
-                        bulk_load(st + kOffSfB0, p.xs_tok + static_cast<std::size_t>(s * 4) * 512, kSlab, token_bar(stage));
+                        // K blocks 2s and 2s + 1 of one box: the same half of two neighbouring chunks
+                        const std::uint8_t* chunk = p.bank.g13 +
+                            ((static_cast<std::size_t>(entry) * (gu_tiles / 2) + (m_tile >> 1)) * (2 * gu_stages) + 2 * s) * kChunkBytes;
+                        const int half = m_tile & 1;
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            bulk_load_hint(st + k * kChunkBox, chunk + k * kChunkBytes + half * kChunkBox, kChunkBox, weight_bar(stage), stream_policy);
+                            bulk_load_hint(st + kChunkScaleOffset + k * kChunkScaleBytes,
+                                           chunk + k * kChunkBytes + kChunkScaleOffset + half * kChunkScaleBytes, kChunkScaleBytes, weight_bar(stage),
+                                           stream_policy);
+                        }
+                        if (!rows_ready) {
+                            if (!wait_counter(p.sync + 0, (p.epoch + 1U) * static_cast<unsigned>(grid))) { give_up(kStatusWaitExpired); ok = false; break; }
+                            fence_proxy_async_all();      // ordinary stores of other blocks -> this block's TMA loads
+                            rows_ready = true;
+                        }
+                        mbar_arrive_expect_tx(token_bar(stage), 4 * kSlab);
+                        tma_load_2d(st + kOffB0, &map_x, token_bar(stage), (2 * s) * kKB, 0);
+                        tma_load_2d(st + kOffB1, &map_x, token_bar(stage), (2 * s + 1) * kKB, 0);
+                        bulk_load(st + kOffSfB0, p.xs_tok + static_cast<std::size_t>(s * 8) * 512, 2 * kSlab, token_bar(stage));
                     } else {
                         bulk_load_hint(st, p.bank.g2 + ((static_cast<std::size_t>(entry) * dn_tiles + m_tile) * dn_stages + s) *
                                                            kChunkBytes,
                                        kChunkBytes, weight_bar(stage), stream_policy);
                         if (!tokens_ready) {
-                            // the SwiGLU rows of this expert exist once its eight gate/up tiles are done
+                            // the SwiGLU rows of this expert exist once all its gate/up tiles are done
                             if (!wait_counter(reinterpret_cast<const unsigned*>(done + slot),
                                               static_cast<unsigned>(gu_tiles))) {
                                 give_up(kStatusWaitExpired);
@@ -530,6 +583,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                         bulk_load(st + kOffSfB0, bsf, kSlab, token_bar(stage));
                         bulk_load(st + kOffSfB1, bsf + 4 * 512, kSlab, token_bar(stage));
                     }
+                    // the next tile's number is asked for behind the first loads of this one: its answer is a round trip away
+                    if (s == 0) following = static_cast<int>(atomicAdd(tile_counter, 1U));
                     if (++stage == kStages) { stage = 0; phase ^= 1U; }
                 }
                 if (!ok) break;
@@ -561,7 +616,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 decode_tile(code, &kind, &slot, &m_tile);
                 tc_fence_after();
                 const std::uint32_t accum = tmem_base + buffer * kAccumCols;
-                const int n_stages = kind == 0 ? gu_kblocks : dn_stages;
+                const int n_stages = kind == 0 ? gu_stages : dn_stages;
                 bool ok = true;
                 for (int s = 0; s < n_stages; ++s) {
                     if (s > 0 && (!mbar_wait(weight_bar(stage), phase) || !mbar_wait(token_bar(stage), phase))) {
@@ -571,7 +626,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                     }
                     tc_fence_after();
                     if (sequence == 0 && s < 10) stamp(26 + s);
-                    issue_stage(kind, base + stage * kStage, kOffB1, kOffSfB0, sf_tmem + sf_buffer * kSfColsPerBuffer, accum,
+                    issue_stage(1, base + stage * kStage, kOffB1, kOffSfB0, sf_tmem + sf_buffer * kSfColsPerBuffer, accum,
                                 idesc, s == 0);
                     tc_commit(empty_bar(stage));
                     if (sequence == 0 && s < 10) stamp(36 + s);
@@ -586,12 +641,11 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
             }
             stamp(8);
         }
-    } else if (!abort_word) {
-        if (block == 0) {
-            // The routing products go to global memory for the caller (ids, weights, permutation,
-            // histogram); these four warps would otherwise idle until the first accumulator is ready.
-            const int t = threadIdx.x - 64;
-            if (t < assignments) {
+    } else if (warp >= kEpilogueEnd) {
+        // the routing products go to global memory for the caller (ids, weights, permutation, histogram)
+        constexpr int kHelpers = kMegaThreads - 32 * kEpilogueEnd;
+        if (block == 0 && !abort_word) {
+            for (int t = threadIdx.x - 32 * kEpilogueEnd; t < assignments; t += kHelpers) {
                 const int pos = rt.less[t] + rt.rank[t];
                 p.ids[t] = rt.ids[t];
                 p.route_weights[t] = rt.weights[t];
@@ -599,8 +653,9 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 p.position[t] = pos;
                 p.pp_of_flat[t] = rt.pp_tok[rt.slot_a[t]][t / kTop];
             }
-            if (t < rows) p.pp_of_flat[assignments + t] = rt.pp_tok[0][t];
-            for (int e = t; e <= kExperts; e += 128) {
+            const int h = threadIdx.x - 32 * kEpilogueEnd;
+            if (h < rows) p.pp_of_flat[assignments + h] = rt.pp_tok[0][h];
+            for (int e = h; e <= kExperts; e += kHelpers) {
                 if (e < kExperts) {
                     p.counts[e] = __popc(rt.expert_mask[e]);
                     p.offsets[e] = rt.before[e];
@@ -609,6 +664,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 }
             }
         }
+    } else if (!abort_word) {
         const int quarter = warp & 3;
         int buffer = 0;
         std::uint32_t accum_phase = 0;
@@ -623,21 +679,28 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
             const int expert = rt.active[slot];
             const int entry = expert == kExperts ? p.bank.local_experts : expert - p.bank.first_expert;
             const std::uint32_t lane_base = tmem_base + buffer * kAccumCols + (static_cast<std::uint32_t>(quarter * 32) << 16);
-            const int row = m_tile * kTile + quarter * 32 + lane;
             if (kind == 0) {
+                // lanes 0..15 of the quarter hold the gate sums of 16 intermediate rows, lanes 16..31 their up sums.  Of a
+                // pair of token columns the lower half finishes the even one and the upper half the odd one: one exchange
+                // per pair and every lane has a gate and an up value.
                 const float alpha_g = p.bank.alpha[entry * 3 + 0];
                 const float alpha_u = p.bank.alpha[entry * 3 + 1];
+                const int row = m_tile * (kTile / 2) + quarter * 16 + (lane & 15);
                 const int sf_col = row >> 4;
-                std::uint32_t g[16], u[16];
-                tmem_load16(lane_base, g);
-                tmem_load16(lane_base + kAccumStride, u);
+                const bool upper = (lane & 16) != 0;
+                std::uint32_t d[16];
+                tmem_load16(lane_base, d);
                 tmem_load_wait();
 #pragma unroll
-                for (int n = 0; n < R; ++n) {
-                    const int pp_signed = n < rows ? rt.pp_tok[slot][n] : -1;        // warp uniform
-                    if (pp_signed < 0) continue;
-                    const float gv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(g[n]) * alpha_g));
-                    const float uv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(u[n]) * alpha_u));
+                for (int n = 0; n < R; n += 2) {
+                    const int pp_even = n < rows ? rt.pp_tok[slot][n] : -1;
+                    const int pp_odd = n + 1 < rows ? rt.pp_tok[slot][n + 1] : -1;
+                    if (pp_even < 0 && pp_odd < 0) continue;                         // warp uniform
+                    const std::uint32_t got = __shfl_xor_sync(0xffffffffU, upper ? d[n] : d[n + 1], 16);
+                    const std::uint32_t g = upper ? got : d[n];
+                    const std::uint32_t u = upper ? d[n + 1] : got;
+                    const float gv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(g) * alpha_g));
+                    const float uv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(u) * alpha_u));
                     const float h = bf16_bits_to_float(float_to_bf16_bits((gv / (1.0F + expf(-gv))) * uv));
                     float amax = fabsf(h);
 #pragma unroll
@@ -647,6 +710,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                     const float multiplier = decoded == 0.0F ? 0.0F : p.quant_scale / decoded;
                     const float q = h * multiplier;
                     const float q_next = __shfl_xor_sync(0xffffffffU, q, 1);
+                    const int pp_signed = upper ? pp_odd : pp_even;
+                    if (pp_signed < 0) continue;                                     // no shuffle left in this round
                     const std::size_t pp = static_cast<std::size_t>(pp_signed);
                     if ((lane & 1) == 0) {
                         p.hq[pp * (inter / 2) + (row >> 1)] =
@@ -657,6 +722,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                              (sf_col & 3)] = scale.__x;
                     }
                 }
+                __syncwarp();
                 tc_fence_before();
                 __threadfence();
                 fence_proxy_async_all();
@@ -670,6 +736,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 }
             } else {
                 const float alpha = p.bank.alpha[entry * 3 + 2];
+                const int row = m_tile * kTile + quarter * 32 + lane;
                 const int pp0 = slab_of_slot(slot, rt.n_active);
                 std::uint32_t d[16];
                 tmem_load16(lane_base, d);
@@ -716,7 +783,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     // One thread per four output features: eight routed slots in slot order, then the shared expert;
     // each operand is polled until its words carry this launch's number.
     const int quads = hidden / 4;
-    for (int v = block * kMegaThreads + threadIdx.x; v < rows * quads; v += grid * kMegaThreads) {
+    // 32 quads to a warp, neighbouring groups to neighbouring blocks: at four tokens 80 blocks have one group each
+    for (int v = (warp * grid + block) * 32 + lane; v < rows * quads; v += grid * kMegaThreads) {
         const int row = v / quads;
         const int q = v - row * quads;
         float acc[4] = {0.0F, 0.0F, 0.0F, 0.0F};
@@ -764,24 +832,41 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
         // over the grid; this block collects the row, sums the squares in the operator's order and writes the row out
         std::uint16_t* h_row = reinterpret_cast<std::uint16_t*>(smem_raw + (base - smem_u32(smem_raw)));
         bool ok = true;
-        for (int i = threadIdx.x; i < hidden / 2; i += kMegaThreads) {
-            std::uint32_t pair = 0;
-            ok = poll_tagged(p.hidden_tagged + static_cast<std::size_t>(block) * (hidden / 2) + i, tag, &pair) && ok;
-            reinterpret_cast<std::uint32_t*>(h_row)[i] = pair;
+        const unsigned long long* words = p.hidden_tagged + static_cast<std::size_t>(block) * (hidden / 2);
+        constexpr int kPerThread = (640 + kMegaThreads - 1) / kMegaThreads;       // 640 pairs of words (hidden is 2560 here)
+        uint4 got[kPerThread];
+#pragma unroll
+        for (int j = 0; j < kPerThread; ++j) {
+            const int i = threadIdx.x + j * kMegaThreads;
+            if (i < hidden / 4) got[j] = ld_tagged_pair(words + 2 * i);             // all requested before the first is looked at
+        }
+#pragma unroll
+        for (int j = 0; j < kPerThread; ++j) {
+            const int i = threadIdx.x + j * kMegaThreads;
+            if (i >= hidden / 4) continue;
+            if (got[j].y != tag || got[j].w != tag) ok = poll_tagged_pair(words + 2 * i, tag, &got[j].x, &got[j].z) && ok;
+            reinterpret_cast<uint2*>(h_row)[i] = make_uint2(got[j].x, got[j].z);
         }
         if (!ok) give_up(kStatusWaitExpired);
         __syncthreads();
         row_sum_of_squares(h_row, 1);
-        const float inverse = norm_inverse[0];
-        for (int i = threadIdx.x; i < hidden; i += kMegaThreads) {
-            p.out[static_cast<std::size_t>(block) * hidden + i] =
-                float_to_bf16_bits(bf16_bits_to_float(h_row[i]) * inverse * bf16_bits_to_float(__ldg(p.post_norm_w + i)));
+        if (norm_thread) {
+            const uint4 w = load_norm_weight(p.post_norm_w, p.norm_w_aligned, threadIdx.x);
+            const uint4 out = normalise8(reinterpret_cast<const uint4*>(h_row)[threadIdx.x], norm_inverse[0], w);
+            std::uint16_t* to = p.out + static_cast<std::size_t>(block) * hidden + threadIdx.x * 8;
+            if ((reinterpret_cast<std::uintptr_t>(to) & 15U) == 0U) {
+                *reinterpret_cast<uint4*>(to) = out;
+            } else {
+                const std::uint32_t words4[4] = {out.x, out.y, out.z, out.w};
+                for (int i = 0; i < 8; ++i) to[i] = static_cast<std::uint16_t>(words4[i >> 1] >> (16 * (i & 1)));
+            }
         }
     }
     if (threadIdx.x == 0) stamp(12);
 }
 
 constexpr int kMegaSmem = kStages * kStage + 1024;
+static_assert(kReplicas == kLogitReplicas, "size of the plan's words");
 
 }  // namespace
 
@@ -828,6 +913,7 @@ cudaError_t launch_decode_mega(p92b_plan* plan, const p92b_bank* bank, const std
     p.post_norm_w = post_norm_w;
     p.hidden_tagged = plan->mega_hidden;
     p.norm_eps = norm_eps;
+    p.norm_w_aligned = ((reinterpret_cast<std::uintptr_t>(pre_norm_w) | reinterpret_cast<std::uintptr_t>(post_norm_w)) & 15U) == 0U;
     p.trace = plan->trace_on ? plan->mega_trace : nullptr;
     p.epoch = plan->mega_epoch++;
     p.routed_scale = routed_scale;

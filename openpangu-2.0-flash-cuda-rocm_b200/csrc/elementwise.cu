@@ -333,10 +333,12 @@ __device__ __forceinline__ void retile_piece(const std::uint8_t* __restrict__ we
         const int piece = static_cast<int>(index - static_cast<long>(row) * pieces_per_row);
         const int tile = row >> 7, r = row & 127;
         const int kb = piece >> 3, j = piece & 7;
-        const int which = blocks_per_chunk == 1 ? slot : (kb & 1);
+        // gate (slot 0) and up (slot 1) rows are mixed in both boxes of a chunk; a down tile's boxes are two K blocks
+        const int which = blocks_per_chunk == 1 ? r >> 6 : (kb & 1);
+        const int to = blocks_per_chunk == 1 ? gu_box_row(r & 63) + 16 * slot : r;
         const std::size_t chunk = static_cast<std::size_t>(tile) * chunks_per_tile + kb / blocks_per_chunk;
         const uint4 v = *reinterpret_cast<const uint4*>(weight + static_cast<std::size_t>(row) * k_bytes + piece * 16);
-        *reinterpret_cast<uint4*>(chunks + chunk * kChunkBytes + which * kChunkBox + r * 128 + ((j ^ (r & 7)) * 16)) = v;
+        *reinterpret_cast<uint4*>(chunks + chunk * kChunkBytes + which * kChunkBox + to * 128 + ((j ^ (to & 7)) * 16)) = v;
         return;
     }
     const long scale_piece = index - weight_pieces;                     // 16 scale bytes each
@@ -347,12 +349,24 @@ __device__ __forceinline__ void retile_piece(const std::uint8_t* __restrict__ we
     const int within = static_cast<int>(scale_piece - block_index * per_block);
     const int tile = static_cast<int>(block_index / k_blocks);
     const int kb = static_cast<int>(block_index - static_cast<long>(tile) * k_blocks);
-    const int which = blocks_per_chunk == 1 ? slot : (kb & 1);
     const std::size_t chunk = static_cast<std::size_t>(tile) * chunks_per_tile + kb / blocks_per_chunk;
     // source: tile row-block `tile`, scale column blocks 4*kb .. 4*kb+3, 512 bytes each, contiguous
     const uint4 v = *reinterpret_cast<const uint4*>(
         scales + (static_cast<std::size_t>(tile) * (k_blocks * 4) + kb * 4) * 512 + within * 16);
-    *reinterpret_cast<uint4*>(chunks + chunk * kChunkBytes + kChunkScaleOffset + which * kChunkScaleBytes + within * 16) = v;
+    std::uint8_t* slabs = chunks + chunk * kChunkBytes + kChunkScaleOffset;
+    if (blocks_per_chunk != 1) {
+        *reinterpret_cast<uint4*>(slabs + (kb & 1) * kChunkScaleBytes + within * 16) = v;
+        return;
+    }
+    // the piece holds four scale columns of rows r, r + 32, r + 64, r + 96: each row's word goes where its values went
+    const std::uint32_t words[4] = {v.x, v.y, v.z, v.w};
+    const int column_block = within >> 5;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = q * 32 + (within & 31);
+        const int to = gu_box_row(r & 63) + 16 * slot;
+        *reinterpret_cast<std::uint32_t*>(slabs + (r >> 6) * kChunkScaleBytes + column_block * 512 + (to & 31) * 16 + (to >> 5) * 4) = words[q];
+    }
 }
 
 // All entries of one kind in one launch: blockIdx.y = entry, the matrix pointers come from the

@@ -5,8 +5,8 @@
 // weight row, so the 16-element blocks of the re-quantisation run ACROSS lanes: a warp reduction, a select tree, a
 // shuffle per column and a nibble transposition - about 65 instructions per SwiGLU value, which is what bounded the
 // kernel at 4,096 tokens (201 µs).  With the tokens on the M side a lane holds one token's 32 neighbouring values:
-// maximum, scale, packing and store need no other lane.  And one MMA covers 128 tokens x 256 weight rows (gate box and
-// up box of a chunk are one 256-row operand), so an operand byte in shared memory is read half as often as with
+// maximum, scale, packing and store need no other lane.  And one MMA covers 128 tokens x 256 weight rows (the two boxes
+// of a chunk are one 256-row operand), so an operand byte in shared memory is read half as often as with
 // N = 64.
 #include "expert_common.cuh"
 
@@ -129,7 +129,7 @@ __device__ __forceinline__ uint2 swiglu_block16(const std::uint32_t* g, const st
 }
 
 // A ring stage: one K block (256 values) of the weight tile and of the token tile.  The weight part of a gate/up
-// stage is exactly one chunk of the bank's stream: gate box, up box, their two scale slabs.
+// stage is exactly one chunk of the bank's stream: two boxes of mixed gate and up rows, their two scale slabs.
 struct Stage {
     static constexpr int kOffW = 0;
     static constexpr int kOffSfW = kWRows * kBlockKBytes;                   // 32,768
@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
             if constexpr (MODE == 0) {
                 std::uint32_t first[32], second[32];
                 if (mine) {
-                    tmem_load32(lane_base + group * 32, first);
-                    tmem_load32(lane_base + 128 + group * 32, second);
+                    tmem_load32(lane_base + group * 64, first);            // gate and up sums of 16 intermediate rows
+                    tmem_load32(lane_base + group * 64 + 32, second);       // ... and of the next 16
                     tmem_load_wait();
                 }
                 tc_fence_before();
@@ -320,8 +320,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                     const float alpha_u = p.bank.alpha[it.entry * 3 + 1];
                     const int inter = p.m_total;
                     std::uint32_t scale0, scale1;
-                    const uint2 q0 = swiglu_block16(first, second, alpha_g, alpha_u, p.quant_scale, &scale0);
-                    const uint2 q1 = swiglu_block16(first + 16, second + 16, alpha_g, alpha_u, p.quant_scale, &scale1);
+                    const uint2 q0 = swiglu_block16(first, first + 16, alpha_g, alpha_u, p.quant_scale, &scale0);
+                    const uint2 q1 = swiglu_block16(second, second + 16, alpha_g, alpha_u, p.quant_scale, &scale1);
                     const int column = it.m_tile * kTileM + group * 32;
                     *reinterpret_cast<uint4*>(p.hq + static_cast<std::size_t>(pp) * (inter / 2) + (column >> 1)) = make_uint4(q0.x, q0.y, q1.x, q1.y);
                     const int sf_col = column >> 4;         // even: the two bytes are neighbours in the tiled layout

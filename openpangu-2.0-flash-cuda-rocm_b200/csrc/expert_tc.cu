@@ -134,7 +134,7 @@ __device__ __forceinline__ void swiglu_requant_chunk(const std::uint32_t (&g)[16
     const float my_multiplier = decoded == 0.0F ? 0.0F : quant_scale / decoded;
     const int n_mine = c0 + c;
     if (n_mine < valid) {
-        const int sf_col = (row0 >> 4) + half;
+        const int sf_col = row0 >> 4;
         const int tn = n_base + n_mine;
         hs_tile[static_cast<std::size_t>(sf_col >> 2) * 512 + (sf_col & 3) + (tn & 31) * 16 + (tn >> 5) * 4] = scale.__x;
     }
@@ -166,7 +166,7 @@ __device__ __forceinline__ void swiglu_requant_chunk(const std::uint32_t (&g)[16
         w1 = (upper ? w1 & ~low : w1 & low) | r1;
     }
     if (n_mine < valid) {
-        *reinterpret_cast<uint2*>(hq_rows + static_cast<std::size_t>(n_mine) * (inter / 2) + ((row0 + 16 * half) >> 1)) =
+        *reinterpret_cast<uint2*>(hq_rows + static_cast<std::size_t>(n_mine) * (inter / 2) + (row0 >> 1)) =
             make_uint2(w0, w1);
     }
 }
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
                     // weights never depend on the upstream kernel: they start streaming at once
                     mbar_arrive_expect_tx(weight_bar(stage), C::kWeightBytes);
                     if constexpr (MODE != 1) {
-                        // one chunk = gate box, up box and both scale slabs of this (row tile, K block)
+                        // one chunk = both boxes and both scale slabs of this (row tile, K block)
                         const std::uint8_t* chunk = p.bank.g13 +
                             ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes;
                         bulk_load(st, chunk, kChunkBytes, weight_bar(stage));
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
                 std::uint8_t* hs_tile = p.hs + static_cast<std::size_t>(it.pp0 >> 7) * (inter / 64) * 512;
                 std::uint8_t* hq_rows = p.hq + static_cast<std::size_t>(it.pp0) * (inter / 2);
                 const int n_base = it.pp0 & 127;
-                const int row0 = it.m_tile * kTileM + quarter * 32;
+                const int row0 = it.m_tile * kTileM + gu_tile_row(quarter, lane & 16);      // of this half warp's 16 rows
 #pragma unroll 1
                 for (int c0 = half * 16; c0 < N; c0 += 16 * (kEpilogueWarps / 4)) {
                     if (c0 >= it.valid) break;                                    // warp uniform
@@ -448,6 +448,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
                     tmem_load16(lane_base + c0, g);
                     tmem_load16(lane_base + C::kAccumStride + c0, u);
                     tmem_load_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) gu_exchange(g[j], u[j], lane, &g[j], &u[j]);
                     swiglu_requant_chunk(g, u, alpha_g, alpha_u, p.quant_scale, lane, c0, it.valid, n_base, inter, row0, hq_rows, hs_tile);
                 }
             } else if constexpr (MODE == 2) {
@@ -456,6 +458,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
                 const float alpha_g = SRC == 1 ? *p.table[it.entry * 3 + 0].alpha : p.bank.alpha[it.entry * 3 + 0];
                 const float alpha_u = SRC == 1 ? *p.table[it.entry * 3 + 1].alpha : p.bank.alpha[it.entry * 3 + 1];
                 const int inter = p.m_total;
+                // a caller's table is read in place, gate rows and up rows apart; the bank's boxes mix them
+                const int my_row = SRC == 1 ? row : it.m_tile * kTileM + gu_tile_row(quarter, lane);
 #pragma unroll 1
                 for (int c0 = half * 16; c0 < N; c0 += 16 * (kEpilogueWarps / 4)) {
                     if (c0 >= it.valid) break;
@@ -463,13 +467,17 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
                     tmem_load16(lane_base + c0, g);
                     tmem_load16(lane_base + C::kAccumStride + c0, u);
                     tmem_load_wait();
+                    if constexpr (SRC == 0) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) gu_exchange(g[j], u[j], lane, &g[j], &u[j]);
+                    }
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const int n = c0 + j;
                         if (n < it.valid) {
                             const std::size_t r = static_cast<std::size_t>(p.out_row != nullptr ? p.out_row[it.dense0 + n] : it.pp0 + n);
-                            p.gate_out[r * inter + row] = float_to_bf16_bits(__uint_as_float(g[j]) * alpha_g);
-                            p.up_out[r * inter + row] = float_to_bf16_bits(__uint_as_float(u[j]) * alpha_u);
+                            p.gate_out[r * inter + my_row] = float_to_bf16_bits(__uint_as_float(g[j]) * alpha_g);
+                            p.up_out[r * inter + my_row] = float_to_bf16_bits(__uint_as_float(u[j]) * alpha_u);
                         }
                     }
                 }

@@ -75,14 +75,15 @@ __device__ __forceinline__ uint2 quantize_block16(const float (&v)[16], float gl
     return make_uint2(words[0], words[1]);
 }
 
-// Top-8 of one token by one warp: lane l holds experts l, l+32, ..., l+224 in registers.
+// Top-8 of one token by one warp for any scores, equal ones included (warp_top8 below calls it when it meets scores too
+// close for its 24-bit keys): lane l holds experts l, l+32, ..., l+224 in registers.
 // Eight rounds of (local best, warp butterfly arg-max) with the reference's total order: higher
 // corrected score first, equal scores -> lower id (cuda/nvfp4_ops.cu:391-392,411-412).  Weights
 // are the uncorrected sigmoid of the winners, summed in slot order and scaled by
 // routed_scale/total (:420,425-432).  The score is written exactly as the reference writes it and
 // every file using this is compiled with --use_fast_math like the reference, so expf and the
 // divisions lower to the same hardware approximations.  lg/ids/weights point at this token's row.
-__device__ __forceinline__ void warp_top8(const float* __restrict__ lg, const float* __restrict__ bias,
+static __device__ __noinline__ void warp_top8_by_id(const float* __restrict__ lg, const float* __restrict__ bias,
                                           std::int32_t* __restrict__ ids, float* __restrict__ weights,
                                           float routed_scale) {
     const int lane = threadIdx.x & 31;
@@ -147,6 +148,67 @@ __device__ __forceinline__ void warp_top8(const float* __restrict__ lg, const fl
     }
 }
 
+// The same for scores whose nine highest differ in the upper 24 bits of their order-preserving image - all but about one
+// token in a thousand: the low byte of a 32-bit word then carries the expert id, so that one warp reduction per
+// round gives winner and id together, and a comparator of the lane-local ordering is one minimum and one maximum.  The
+// ninth round is there to see that the eighth and ninth differ; any two neighbours that agree in 24 bits send the whole
+// token through warp_top8_by_id, so ids, order and weights are the same bits in every case.
+__device__ __forceinline__ void warp_top8(const float* __restrict__ lg, const float* __restrict__ bias,
+                                          std::int32_t* __restrict__ ids, float* __restrict__ weights,
+                                          float routed_scale) {
+    const int lane = threadIdx.x & 31;
+    std::uint32_t cand[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = lane + 32 * i;
+        const float raw = 1.0F / (1.0F + expf(-lg[e]));
+        const float corrected = raw + bias[e];
+        const std::uint32_t bits = __float_as_uint(corrected);
+        const std::uint32_t key = corrected != corrected ? 0U : (bits & 0x80000000U ? ~bits : bits | 0x80000000U);
+        cand[i] = (key & 0xffffff00U) | static_cast<std::uint32_t>(kExperts - 1 - e);
+    }
+#define P92B_ORDER(a, b)                                       \
+    {                                                          \
+        const std::uint32_t hi = max(cand[a], cand[b]);        \
+        cand[b] = min(cand[a], cand[b]);                       \
+        cand[a] = hi;                                          \
+    }
+    P92B_ORDER(0, 1) P92B_ORDER(2, 3) P92B_ORDER(4, 5) P92B_ORDER(6, 7)
+    P92B_ORDER(0, 2) P92B_ORDER(1, 3) P92B_ORDER(4, 6) P92B_ORDER(5, 7)
+    P92B_ORDER(1, 2) P92B_ORDER(5, 6)
+    P92B_ORDER(0, 4) P92B_ORDER(1, 5) P92B_ORDER(2, 6) P92B_ORDER(3, 7)
+    P92B_ORDER(2, 4) P92B_ORDER(3, 5)
+    P92B_ORDER(1, 2) P92B_ORDER(3, 4) P92B_ORDER(5, 6)
+#undef P92B_ORDER
+    std::uint32_t mine = 0U;      // lane k keeps the word of slot k, lane 8 the ninth
+#pragma unroll 3
+    for (int slot = 0; slot <= kTop; ++slot) {
+        const std::uint32_t top = __reduce_max_sync(0xffffffffU, cand[0]);
+        if (cand[0] == top) {
+#pragma unroll
+            for (int i = 0; i < 7; ++i) cand[i] = cand[i + 1];
+            cand[7] = 0U;
+        }
+        if (lane == slot) mine = top;
+    }
+    const std::uint32_t above = __shfl_up_sync(0xffffffffU, mine, 1);
+    if (__any_sync(0xffffffffU, lane >= 1 && lane <= kTop && (above >> 8) == (mine >> 8))) {
+        warp_top8_by_id(lg, bias, ids, weights, routed_scale);
+        return;
+    }
+    const int chosen_id = kExperts - 1 - static_cast<int>(mine & 0xffU);
+    // weights: the uncorrected sigmoid of the winners, summed in slot order and scaled by routed_scale / total (:420,425-432)
+    const float chosen_weight = lane < 8 ? 1.0F / (1.0F + expf(-lg[chosen_id])) : 0.0F;
+    float total = 0.0F;
+#pragma unroll
+    for (int slot = 0; slot < 8; ++slot) total += __shfl_sync(0xffffffffU, chosen_weight, slot);
+    const float multiplier = routed_scale / total;
+    if (lane < 8) {
+        ids[lane] = chosen_id;
+        weights[lane] = chosen_weight * multiplier;
+    }
+}
+
 // Layout of one layer's expert weights inside the library (device memory).
 // Entry e = local expert index, entry local_experts = the shared expert.
 //
@@ -157,12 +219,17 @@ __device__ __forceinline__ void warp_top8(const float* __restrict__ lg, const fl
 //   box    = 128 rows x 128 bytes (256 E2M1 values of one K block), 16-byte pieces XOR-swizzled by
 //            (row & 7): the 128-byte swizzle a TMA tile load would have produced
 //   scales = the matching four 512-byte tiles of the 128x4-tiled E4M3 layout
-//   g13: [entry][row tile of I][K block of H]    box0/1 = gate/up rows of the same K block
+//   g13: [entry][row tile of I][K block of H]    both boxes the same K block; box b holds the 64 gate rows and the 64 up
+//        rows of intermediate rows 64 b .. 64 b + 63 of the tile, interleaved by 16 (gu_box_row), so that half a tile is
+//        a unit of work of its own and a gate row meets its up row in the same 32 TMEM lanes
 //   g2:  [entry][row tile of H][pair of K blocks] box0/1 = K blocks 2s, 2s+1 of the down matrix
 constexpr int kChunkBytes = 36864;
 constexpr int kChunkBox = 16384;
 constexpr int kChunkScaleOffset = 32768;
 constexpr int kChunkScaleBytes = 2048;
+
+// Row of a g13 box that holds gate row `i` of its 64 intermediate rows (its up row: 16 further).
+__host__ __device__ __forceinline__ constexpr int gu_box_row(int i) { return (i >> 4) * 32 + (i & 15); }
 
 struct BankView {
     const std::uint8_t* g13;
@@ -255,7 +322,7 @@ struct p92b_plan {
     std::int32_t* gu_done = nullptr;      // [2][264] per launch parity: gate/up tiles finished per active slot, [257] the tile counter
     std::int32_t* ep_gu_done = nullptr;   // [2][264] the same for the fused expert-parallel kernel
     unsigned long long* ep_logits = nullptr;    // [8][256] its router logits as tagged words
-    unsigned long long* mega_logits = nullptr;  // [8][256] router logits as {value, launch number} words
+    unsigned long long* mega_logits = nullptr;  // [8][16][256] router logits as {value, launch number} words, in eight copies
     unsigned long long* mega_ret = nullptr;     // [8][9][1280] down rows as {two BF16, launch number} words
     float* w_norms = nullptr;                   // [2][256] norms of the router rows (tensor-core router), alternating by call
     int norms_parity = 0;
@@ -420,6 +487,7 @@ cudaError_t host_pipeline_begin(p92b_plan* plan, const std::uint16_t* pinned_inp
                                 std::uint16_t** rows_in, std::uint16_t** rows_out, int* set);
 cudaError_t host_pipeline_end(p92b_plan* plan, std::uint16_t* pinned_output, int rows, cudaStream_t stream, int set);
 // fused decode kernel (decode_mega.cu)
+constexpr int kLogitReplicas = 8;
 int decode_mega_max_rows();
 cudaError_t launch_decode_mega(p92b_plan* plan, const p92b_bank* bank, const std::uint16_t* x,
                                const std::uint16_t* router_w, const float* bias, std::uint16_t* out, int rows,

@@ -223,6 +223,18 @@ __device__ __forceinline__ void tmem_load16(std::uint32_t addr, std::uint32_t (&
 
 __device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Gate and up sums of a 128-row tile of intermediate rows whose two boxes (gu_box_row) were multiplied into two
+// accumulators: a lane reads `first` (box 0) and `second` (box 1) at its own TMEM lane, where lanes 0..15 of a quarter are
+// gate rows and lanes 16..31 the up rows of the same 16 intermediate rows.  One exchange between the two halves of
+// the warp leaves a lane with gate and up of ONE intermediate row of the tile: row gu_tile_row().
+__device__ __forceinline__ int gu_tile_row(int quarter, int lane) { return (lane >> 4) * 64 + quarter * 16 + (lane & 15); }
+__device__ __forceinline__ void gu_exchange(std::uint32_t first, std::uint32_t second, int lane, std::uint32_t* gate, std::uint32_t* up) {
+    const bool upper = (lane & 16) != 0;
+    const std::uint32_t got = __shfl_xor_sync(0xffffffffU, upper ? first : second, 16);
+    *gate = upper ? got : first;
+    *up = upper ? second : got;
+}
+
 // ---- descriptors -------------------------------------------------------------------
 // Shared-memory matrix descriptor (64 bit): start address >> 4 in bits [0,14),
 // leading byte offset >> 4 in [16,30), stride byte offset >> 4 in [32,46),
