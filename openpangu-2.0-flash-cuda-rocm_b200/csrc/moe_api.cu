@@ -203,6 +203,7 @@ int p92b_plan_create(p92b_plan** out, int max_rows, int hidden, int intermediate
         plan->ep_zero_counts = c.take<std::int32_t>(kExperts + 1);
         plan->epg_counts = c.take<std::int32_t>(kExperts + 1);
         plan->epg_offsets = c.take<std::int32_t>(kExperts + 2);
+        plan->dense_parts_done = c.take<unsigned>(static_cast<std::size_t>(hidden / 128));
         plan->stage_in = c.take<std::uint16_t>(rows * hidden);
         plan->stage_out = c.take<std::uint16_t>(rows * hidden);
         plan->stage_in_b = c.take<std::uint16_t>(rows * hidden);
@@ -487,6 +488,7 @@ int p92b_dense_forward(p92b_plan* plan, const p92b_bank* bank, const uint16_t* i
     static const bool pdl = std::getenv("P92B_NO_PDL") == nullptr;
     plan->last_launches = 0;
     plan->last_path = 2;
+    if (dense_few_rows_applies(plan, rows)) return launch_dense_few_rows(plan, bank, input, output, rows, stream, pdl);
     // the MLP is the bank's last entry; every row is "routed" to it and to nothing else, so its rows sit at padded
     // positions 0 .. rows-1 in token order and the down product can write the caller's rows directly
     cudaError_t st = launch_dense_lists(plan, rows, tc_tile_rows(rows), stream, pdl);

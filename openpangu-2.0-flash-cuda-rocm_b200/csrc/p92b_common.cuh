@@ -342,6 +342,7 @@ struct p92b_plan {
     std::int32_t* epg_counts = nullptr;   // [257] histogram and [258] offsets of the whole gathered batch
     std::int32_t* epg_offsets = nullptr;
     int ep_words = 0;
+    unsigned* dense_parts_done = nullptr; // [H/128] K parts of a down tile that have finished (dense MLP of a few rows; zero between calls)
     // optional stage timing (host side)
     bool timing = false;
     cudaEvent_t stage_events[P92B_STAGES + 1] = {};
@@ -476,6 +477,10 @@ cudaError_t launch_gather_quantized_rows(const std::uint8_t* packed, const std::
                                          int k_bytes, bool distinct_rows, cudaStream_t stream, bool pdl = false);
 cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int rows, bool down,
                               cudaStream_t stream, bool pdl = false, const TcIo* io = nullptr);
+// The dense MLP of up to 32 rows (dense_rows.cu).
+bool dense_few_rows_applies(const p92b_plan* plan, int rows);
+cudaError_t launch_dense_few_rows(p92b_plan* plan, const p92b_bank* bank, const std::uint16_t* x, std::uint16_t* out, int rows,
+                                  cudaStream_t stream, bool pdl);
 // Routing lists of a call in which every row goes to the bank's last entry only (the dense MLP).
 cudaError_t launch_dense_lists(p92b_plan* plan, int rows, int tile_rows, cudaStream_t stream, bool pdl = false);
 // Pipelined host-buffer calls (moe_api.cu).  Three streams: the caller's (the block), one for rows coming in, one

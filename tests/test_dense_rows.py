@@ -1,0 +1,59 @@
+"""The dense MLP of a few rows (its own pair of kernels up to 32 rows) against the CPU oracle.
+
+Row counts sit on both sides of the column counts of the MMA (16, 32) and of the hand-over to the large-batch kernels;
+shapes cover a K extent of the down product that its parts do not divide, fewer K blocks than parts, one part per tile
+(hidden 4096 has 32 tiles for 148 SMs: 4 parts) and the model's own MLP.  Both products accumulate in FP32 over FP4
+operands, so a result differs from the oracle's only where another order of the sums moves a SwiGLU value to the
+neighbouring FP4 value: the 1e-2 of the block's parity bound."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(256, 512), (512, 1536), (2560, 1024), (4096, 512), (2560, 9216)]
+
+
+def _u16(t):
+    import torch
+
+    return t.view(torch.int16).cpu().numpy().view(np.uint16)
+
+
+@pytest.mark.parametrize("hidden,inter", SHAPES)
+def test_dense_few_rows_against_the_oracle(cuda, pkg, orc, hidden, inter):
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(hidden + inter)
+    entries, packed_np, scales_np, alphas = [], [], [], []
+    for rows, cols in ((inter, hidden), (inter, hidden), (hidden, inter)):
+        w = torch.empty((rows, cols), dtype=torch.float32, device="cuda").normal_(0, 0.02, generator=g).to(torch.bfloat16)
+        packed = torch.empty((rows, cols // 2), dtype=torch.uint8, device="cuda")
+        linear = torch.empty((rows, cols // 16), dtype=torch.uint8, device="cuda")
+        alpha = torch.empty(1, dtype=torch.float32, device="cuda")
+        pkg.nvfp4_pack_weight(w, packed, linear, alpha)
+        swizzled = torch.empty(pkg.nvfp4_swizzled_scale_bytes(rows, cols // 16), dtype=torch.uint8, device="cuda")
+        pkg.nvfp4_swizzle_scales(linear, swizzled, rows, cols // 16)
+        entries.append((packed, swizzled, alpha))
+        packed_np.append(packed.cpu().numpy().reshape(-1))
+        scales_np.append(linear.cpu().numpy().reshape(-1))
+        alphas.append(float(alpha))
+    bank = pkg.ExpertBank(entries, first_expert=0, local_experts=0, hidden=hidden, intermediate=inter)
+    # the oracle is row by row, so one call at the largest size has every row's result
+    most = 33 if inter < 9216 else 17
+    x = torch.empty((most, hidden), dtype=torch.float32, device="cuda").normal_(0, 1, generator=g).to(torch.bfloat16)
+    want = orc.bf16_to_f32(orc.dense_forward(_u16(x), np.stack(packed_np), np.stack(scales_np), np.array(alphas, np.float32),
+                                             hidden, inter))
+    plan = pkg.MoePlan(max_rows=most, hidden=hidden, intermediate=inter)
+    for rows in (1, 2, 15, 16, 17, 31, 32, 33):
+        if rows > most:
+            continue
+        out = torch.full((rows, hidden), float("nan"), dtype=torch.bfloat16, device="cuda")
+        pkg.run_dense_rows(plan, bank, x[:rows].contiguous(), out, rows)
+        first = out.clone()
+        pkg.run_dense_rows(plan, bank, x[:rows].contiguous(), out, rows)
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        assert torch.equal(first.view(torch.int16), out.view(torch.int16))      # the parts are added in a fixed order
+        got = orc.bf16_to_f32(_u16(out))
+        assert np.linalg.norm(got - want[:rows]) <= 1e-2 * np.linalg.norm(want[:rows]), rows
+    plan.close()
+    bank.close()
