@@ -18,6 +18,8 @@ __global__ void __launch_bounds__(256) quantize_kernel(const std::uint16_t* __re
                                                        std::uint8_t* __restrict__ scales, long groups,
                                                        float global_scale,
                                                        const float* __restrict__ weight_scale_2) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const long group = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (group >= groups) return;
     if (weight_scale_2 != nullptr) global_scale = __fdiv_rn(1.0F, *weight_scale_2);   // host IEEE division in the reference (cuda/nvfp4_pack.cu:256)
@@ -110,20 +112,35 @@ __global__ void __launch_bounds__(256) quantize_batch_kernel(const std::uint16_t
     scales[group] = scale_bits;
 }
 
-// cuda/nvfp4_ops.cu:869-890: linear [row][K/16] -> 128-row x 4-column tiles.
+// cuda/nvfp4_ops.cu:869-890: linear [row][K/16] -> 128-row x 4-column tiles, rows and columns beyond the last one zero.
+// A thread writes one row's four columns of a tile, in the order of the destination, so the padding needs no pass
+// (and no launch) of its own.
 __global__ void __launch_bounds__(256) swizzle_kernel(const std::uint8_t* __restrict__ linear,
                                                       std::uint8_t* __restrict__ swizzled, int rows,
                                                       int scale_columns, int column_blocks) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const long index = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (index >= static_cast<long>(rows) * scale_columns) return;
-    const int row = static_cast<int>(index / scale_columns);
-    const int column = static_cast<int>(index - static_cast<long>(row) * scale_columns);
-    const int row_block = row >> 7;
-    const int row_in_block = row & 127;
-    const std::size_t destination =
-        (static_cast<std::size_t>(row_block) * column_blocks + (column >> 2)) * 512 + (row_in_block & 31) * 16 +
-        (row_in_block >> 5) * 4 + (column & 3);
-    swizzled[destination] = linear[index];
+    const long tile = index >> 7;
+    const int row_block = static_cast<int>(tile / column_blocks);
+    const int column = static_cast<int>(tile - static_cast<long>(row_block) * column_blocks) * 4;
+    const int row = row_block * 128 + (static_cast<int>(index) & 3) * 32 + ((static_cast<int>(index) & 127) >> 2);
+    if (row_block * 128L >= rows) return;
+    std::uint8_t scale[4] = {0, 0, 0, 0};
+    if (row < rows) {
+        const std::uint8_t* from = linear + static_cast<std::size_t>(row) * scale_columns + column;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (column + i < scale_columns) scale[i] = from[i];
+        }
+    }
+    std::uint8_t* to = swizzled + index * 4;
+    if ((reinterpret_cast<std::uintptr_t>(swizzled) & 3U) == 0U) {
+        *reinterpret_cast<uchar4*>(to) = make_uchar4(scale[0], scale[1], scale[2], scale[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) to[i] = scale[i];
+    }
 }
 
 // The three element-wise operators of the block's stage interface.  Each thread takes eight BF16 values through one
@@ -158,6 +175,8 @@ __device__ __forceinline__ float silu_times(float g, float u) { return (g / (1.0
 __global__ void __launch_bounds__(256) swiglu_kernel(const std::uint16_t* __restrict__ gate,
                                                      const std::uint16_t* __restrict__ up,
                                                      std::uint16_t* __restrict__ output, long elements, long vectors) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const long t = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < vectors) {
         const Bf16x8 g(__ldg(reinterpret_cast<const uint4*>(gate) + t));
@@ -178,6 +197,8 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(const std::uint16_t* 
                                                            const float* __restrict__ route_weights,
                                                            std::uint16_t* __restrict__ output, int experts,
                                                            int elements, int vectors) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const std::size_t route_base = static_cast<std::size_t>(blockIdx.y) * experts;
     std::uint16_t* out_row = output + static_cast<std::size_t>(blockIdx.y) * elements;
@@ -205,6 +226,8 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(const std::uint16_t* 
 // destination = bf16(destination + source), the residual add of cuda/nvfp4_ops.cu:92-95.
 __global__ void __launch_bounds__(256) add_kernel(std::uint16_t* __restrict__ destination,
                                                   const std::uint16_t* __restrict__ source, long elements, long vectors) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
     const long t = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < vectors) {
         const Bf16x8 d(reinterpret_cast<const uint4*>(destination)[t]);
@@ -388,10 +411,10 @@ inline unsigned blocks_for(long n, int per_block) { return static_cast<unsigned>
 }  // namespace
 
 cudaError_t launch_quantize(const std::uint16_t* input, std::uint8_t* output, std::uint8_t* scales,
-                            long groups, float global_scale, cudaStream_t stream) {
+                            long groups, float global_scale, cudaStream_t stream, bool pdl) {
     if (input == nullptr || output == nullptr || scales == nullptr || groups <= 0) return cudaErrorInvalidValue;
-    quantize_kernel<<<blocks_for(groups, 256), 256, 0, stream>>>(input, output, scales, groups, global_scale, nullptr);
-    return cudaGetLastError();
+    return launch_kernel(quantize_kernel, dim3(blocks_for(groups, 256)), dim3(256), 0, stream, pdl, input, output, scales, groups,
+                         global_scale, static_cast<const float*>(nullptr));
 }
 
 cudaError_t launch_combine_shared(const std::uint16_t* mixed, const std::int32_t* mixed_index,
@@ -432,7 +455,7 @@ extern "C" {
 int p92b_nvfp4_quantize(const uint16_t* input, uint8_t* output, uint8_t* scales, int elements,
                         float global_scale, void* stream) {
     if (elements <= 0 || elements % 16 != 0) return cudaErrorInvalidValue;
-    return launch_quantize(input, output, scales, elements / 16, global_scale, static_cast<cudaStream_t>(stream));
+    return launch_quantize(input, output, scales, elements / 16, global_scale, static_cast<cudaStream_t>(stream), pdl_enabled());
 }
 
 size_t p92b_nvfp4_swizzled_scale_bytes(int rows, int scale_columns) {
@@ -445,12 +468,9 @@ size_t p92b_nvfp4_swizzled_scale_bytes(int rows, int scale_columns) {
 int p92b_nvfp4_swizzle_scales(const uint8_t* linear, uint8_t* swizzled, int rows, int scale_columns,
                               void* stream) {
     if (linear == nullptr || swizzled == nullptr || rows <= 0 || scale_columns <= 0) return cudaErrorInvalidValue;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaError_t st = cudaMemsetAsync(swizzled, 0, p92b_nvfp4_swizzled_scale_bytes(rows, scale_columns), s);
-    if (st != cudaSuccess) return st;
-    const long n = static_cast<long>(rows) * scale_columns;
-    swizzle_kernel<<<blocks_for(n, 256), 256, 0, s>>>(linear, swizzled, rows, scale_columns, (scale_columns + 3) / 4);
-    return cudaGetLastError();
+    const long words = static_cast<long>(p92b_nvfp4_swizzled_scale_bytes(rows, scale_columns) / 4);
+    return launch_kernel(swizzle_kernel, dim3(blocks_for(words, 256)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                         pdl_enabled(), linear, swizzled, rows, scale_columns, (scale_columns + 3) / 4);
 }
 
 int p92b_nvfp4_pack_weight(const uint16_t* input, uint8_t* packed, uint8_t* scales, size_t elements,
@@ -494,9 +514,8 @@ int p92b_nvfp4_pack_weight_batch(const uint16_t* input, uint8_t* packed, uint8_t
 int p92b_swiglu(const uint16_t* gate, const uint16_t* up, uint16_t* output, int elements, void* stream) {
     if (gate == nullptr || up == nullptr || output == nullptr || elements <= 0) return cudaErrorInvalidValue;
     const long vectors = aligned16(gate, up, output) ? elements / 8 : 0;
-    swiglu_kernel<<<blocks_for(vectors + (elements - vectors * 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        gate, up, output, elements, vectors);
-    return cudaGetLastError();
+    return launch_kernel(swiglu_kernel, dim3(blocks_for(vectors + (elements - vectors * 8), 256)), dim3(256), 0,
+                         static_cast<cudaStream_t>(stream), pdl_enabled(), gate, up, output, elements, vectors);
 }
 
 int p92b_expert_combine_rows(const uint16_t* expert_rows, const float* route_weights, uint16_t* output,
@@ -507,9 +526,8 @@ int p92b_expert_combine_rows(const uint16_t* expert_rows, const float* route_wei
     }
     const int vectors = aligned16(expert_rows, output) && elements % 8 == 0 ? elements / 8 : 0;
     dim3 grid(blocks_for(vectors + (elements - vectors * 8), 256), batch_rows);
-    combine_rows_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(expert_rows, route_weights, output,
-                                                                            experts, elements, vectors);
-    return cudaGetLastError();
+    return launch_kernel(combine_rows_kernel, grid, dim3(256), 0, static_cast<cudaStream_t>(stream), pdl_enabled(), expert_rows,
+                         route_weights, output, experts, elements, vectors);
 }
 
 int p92b_expert_combine(const uint16_t* expert_rows, const float* route_weights, uint16_t* output,
@@ -532,9 +550,8 @@ int p92b_rmsnorm_strided(const uint16_t* input, int input_stride, const uint16_t
 int p92b_add_inplace(uint16_t* destination, const uint16_t* source, int elements, void* stream) {
     if (destination == nullptr || source == nullptr || elements <= 0) return cudaErrorInvalidValue;
     const long vectors = aligned16(destination, source) ? elements / 8 : 0;
-    add_kernel<<<blocks_for(vectors + (elements - vectors * 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        destination, source, elements, vectors);
-    return cudaGetLastError();
+    return launch_kernel(add_kernel, dim3(blocks_for(vectors + (elements - vectors * 8), 256)), dim3(256), 0,
+                         static_cast<cudaStream_t>(stream), pdl_enabled(), destination, source, elements, vectors);
 }
 
 }  // extern "C"

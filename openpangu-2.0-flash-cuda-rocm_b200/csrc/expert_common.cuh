@@ -35,6 +35,7 @@ struct TcParams {
     std::uint16_t* gate_out;           // MODE 2: BF16 [output row][m_total]
     std::uint16_t* up_out;
     const p92b_expert_projection* table;   // SRC 1: device table of reference-format matrices, entry expert * 3 + kind
+    const CUtensorMap* table_maps;     // SRC 1: maps of the matrices of the active experts, expert * 3 + kind
     int table_kind;                    // SRC 1, MODE 1: which of an expert's three matrices
     int skip_shared;                   // 1: the shared expert's items are not computed (the caller has none)
     std::uint16_t* const* row_dest;    // slab kernel of the down product: null, or [padded position] -> destination row

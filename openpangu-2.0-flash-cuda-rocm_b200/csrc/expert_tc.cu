@@ -13,8 +13,7 @@
 //           weight side is one untiled bulk copy of a contiguous chunk of the bank's tile stream (boxes already in
 //           the swizzled shared-memory image, scale slabs behind them), the token side a tiled box load plus its
 //           2 KB scale slab; weights and tokens complete on separate mbarriers.  When the weights are read in place
-//           from a caller's table of reference-format matrices (SRC 1) the whole warp gathers the box with 16-byte
-//           asynchronous copies, writing the same swizzled image;
+//           from a caller's table of reference-format matrices (SRC 1) the box is a tiled load as well;
 //   warp 1  MMA issuer: owns TMEM; per K block copies the scale slabs SMEM->TMEM (tcgen05.cp) and issues 4 MMAs of
 //           K=64 per weight operand; commits the stage back to the producer and, after the last K block, the
 //           accumulator to the epilogue;
@@ -73,11 +72,6 @@ struct Tc {
     static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 1024;   // + alignment slack
     static_assert(kNeedCols <= 512, "accumulators and scale factors must fit TMEM");
 };
-
-// 16-byte asynchronous copy global -> shared (through the load/store unit, not the bulk-copy engine).
-__device__ __forceinline__ void async_copy16_tc(std::uint32_t dst_smem, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
-}
 
 // The gate/up epilogue for one chunk of 16 token columns (of expert_tc_kernel<0, N>).  A lane holds one weight row (row0 + lane of the intermediate dimension): gate g[j] and
 // up u[j] for token column c0 + j.  bf16(alpha * product) for both, SwiGLU rounded to BF16
@@ -196,9 +190,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::kStages; ++s) {
-            // in-place weights: the scale slabs arrive by bulk copy (one arrival with the byte count), the boxes by
-            // the 32 producer lanes' own copies (one arrival each, after their copies have landed)
-            mbar_init(weight_bar(s), SRC == 1 ? 33 : 1);
+            mbar_init(weight_bar(s), 1);
             mbar_init(token_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
@@ -231,72 +223,49 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
 
     if (warp == 0 && SRC == 1) {
         // ------------------------------------------------ producer, weights read in place
-        // The matrices are row-major [rows][K/2] wherever the caller keeps them, so a stage's box is gathered: 128
-        // rows x eight 16-byte pieces per box, piece j of row r to r * 128 + ((j ^ (r & 7)) * 16) - the image a
-        // 128-byte-swizzle tile load would have written.  A lane's copies of a stage form one group; a stage is
-        // handed to the MMA lane (fence to the asynchronous proxy, arrival) when its group has landed, kLag stages
-        // behind the one being issued, so kLag stages of copies are always in flight.
-        constexpr int kLag = C::kStages - 1;
-        int stage = 0, oldest = 0, in_flight = 0;
-        std::uint32_t phase = 0;
-        bool ok = true;
-        for (int item = blockIdx.x; item < total_items && !*abort_ptr && ok; item += gridDim.x) {
-            Item it;
-            if (!decode_item<N>(p, route_table, item, &it)) continue;
-            const p92b_expert_projection first = p.table[it.entry * 3 + (MODE == 1 ? p.table_kind : 0)];
-            const p92b_expert_projection second = MODE == 1 ? first : p.table[it.entry * 3 + 1];
-            if (((reinterpret_cast<std::uintptr_t>(first.weight) | reinterpret_cast<std::uintptr_t>(second.weight) |
-                  reinterpret_cast<std::uintptr_t>(first.scales_swizzled) | reinterpret_cast<std::uintptr_t>(second.scales_swizzled)) & 15U) != 0U) {
-                *abort_ptr = 1;                                       // the copies need 16-byte aligned matrices
-                atomicCAS(p.status, kStatusOk, kStatusBadPointer);
-                break;
-            }
-            for (int kb = 0; kb < k_blocks; ++kb) {
-                if (!mbar_wait(empty_bar(stage), phase ^ 1U)) { give_up(); ok = false; break; }
-                const std::uint32_t st = base + stage * C::kStageBytes;
+        // The matrices are row-major [rows][K/2] wherever the caller keeps them; the kernel upstream has built a tensor
+        // map of each (gather_quantized_rows_kernel), so a box of 128 rows is one tiled load.  (Gathered in 16-byte
+        // pieces by this warp, 31 experts at 4 tokens took 35 us for gate and up against 20 from the bank's stream.)
+        if (elect_one()) {
+            int stage = 0;
+            std::uint32_t phase = 0;
+            for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
+                Item it;
+                if (!decode_item<N>(p, route_table, item, &it)) continue;
+                const int which = it.entry * 3 + (MODE == 1 ? p.table_kind : 0);
+                bool aligned = true;
+                const std::uint8_t* scales[C::kA];
 #pragma unroll
                 for (int a = 0; a < C::kA; ++a) {
-                    const std::uint8_t* src = (a == 0 ? first.weight : second.weight) +
-                                              static_cast<std::size_t>(it.m_tile) * kTileM * p.k_bytes + kb * kBlockKBytes;
-#pragma unroll 8
-                    for (int q = 0; q < kTileM * 8 / 32; ++q) {
-                        const int piece = lane + 32 * q;
-                        const int r = piece >> 3, j = piece & 7;
-                        async_copy16_tc(st + a * C::kABytes + r * 128 + ((j ^ (r & 7)) * 16),
-                                        src + static_cast<std::size_t>(r) * p.k_bytes + j * 16);
-                    }
+                    scales[a] = p.table[which + a].scales_swizzled;
+                    aligned = aligned && ((reinterpret_cast<std::uintptr_t>(p.table[which + a].weight) |
+                                           reinterpret_cast<std::uintptr_t>(scales[a])) & 15U) == 0U;
                 }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                if (lane == 0) {
-                    // scale slabs: row block m_tile, scale column blocks 4 kb .. 4 kb + 3 of the 128x4 tiling: 2 KB contiguous
-                    mbar_arrive_expect_tx(weight_bar(stage), C::kA * kSfSlab);
+                if (!aligned) {
+                    *abort_ptr = 1;                                   // the copies need 16-byte aligned matrices
+                    atomicCAS(p.status, kStatusOk, kStatusBadPointer);
+                    break;
+                }
+#pragma unroll
+                for (int a = 0; a < C::kA; ++a) tensormap_acquire(p.table_maps + which + a);
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!mbar_wait(empty_bar(stage), phase ^ 1U)) { give_up(); break; }
+                    const std::uint32_t st = base + stage * C::kStageBytes;
+                    mbar_arrive_expect_tx(weight_bar(stage), C::kWeightBytes);
 #pragma unroll
                     for (int a = 0; a < C::kA; ++a) {
-                        const std::uint8_t* sf = (a == 0 ? first.scales_swizzled : second.scales_swizzled) +
-                                                 (static_cast<std::size_t>(it.m_tile) * (k_blocks * 4) + kb * 4) * 512;
-                        bulk_load(st + C::kOffSfA + a * kSfSlab, sf, kSfSlab, weight_bar(stage));
+                        tma_load_2d(st + a * C::kABytes, p.table_maps + which + a, weight_bar(stage), kb * kBlockKBytes, it.m_tile * kTileM);
+                        // scale slabs: row block m_tile, scale column blocks 4 kb .. 4 kb + 3 of the 128x4 tiling: 2 KB contiguous
+                        bulk_load(st + C::kOffSfA + a * kSfSlab, scales[a] + (static_cast<std::size_t>(it.m_tile) * (k_blocks * 4) + kb * 4) * 512,
+                                  kSfSlab, weight_bar(stage));
                     }
                     mbar_arrive_expect_tx(token_bar(stage), C::kTokenBytes);
                     tma_load_2d(st + C::kOffB, &map_b, token_bar(stage), kb * kBlockKBytes, it.pp0);
                     const std::uint8_t* bsf = p.b_sf + (static_cast<std::size_t>(it.pp0 >> 7) * (p.k_bytes / 32) + kb * 4) * 512;
                     bulk_load(st + C::kOffSfB, bsf, kSfSlab, token_bar(stage));
+                    if (++stage == C::kStages) { stage = 0; phase ^= 1U; }
                 }
-                if (++in_flight > kLag) {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(kLag) : "memory");
-                    fence_proxy_async();
-                    mbar_arrive(weight_bar(oldest));
-                    if (++oldest == C::kStages) oldest = 0;
-                    --in_flight;
-                }
-                if (++stage == C::kStages) { stage = 0; phase ^= 1U; }
             }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        fence_proxy_async();
-        while (in_flight > 0) {
-            mbar_arrive(weight_bar(oldest));
-            if (++oldest == C::kStages) oldest = 0;
-            --in_flight;
         }
     } else if (warp == 0) {
         // ------------------------------------------------------------ producer
@@ -975,6 +944,7 @@ cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int 
         p.up_out = io->up_out;
         p.table = io->table;
         p.table_kind = io->table_kind;
+        p.table_maps = plan->table_maps;
         p.skip_shared = io->skip_shared ? 1 : 0;
         p.row_dest = io->row_dest;
     }
@@ -1074,11 +1044,31 @@ __global__ void __launch_bounds__(256) gather_quantized_rows_kernel(const std::u
                                                                     const std::uint8_t* __restrict__ scales_swizzled,
                                                                     const std::int32_t* __restrict__ pp_of_flat,
                                                                     std::uint8_t* __restrict__ xq, std::uint8_t* __restrict__ xs,
-                                                                    int assignments, int k_bytes, int distinct_rows) {
+                                                                    int assignments, int k_bytes, int distinct_rows,
+                                                                    const __grid_constant__ TableMaps maps) {
+    __shared__ __align__(128) std::uint32_t map_image[8][32];
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int warp = threadIdx.x >> 5;
+    const int gather_blocks = (assignments + 7) / 8;
+    const int i = blockIdx.x * 8 + warp;
+    if (static_cast<int>(blockIdx.x) >= gather_blocks) {
+        // a warp per matrix: the host's map of a matrix of this shape with the matrix's own address, so that the product
+        // kernel loads whole boxes by TMA; maps of matrices off a 16-byte boundary are not built (it rejects them)
+        const int m = i - gather_blocks * 8;
+        const int slot = 1 + m / maps.kinds;                          // slot 0 is the shared expert, which has no rows here
+        if (slot >= *maps.active_count) return;
+        const int which = maps.active[slot] * 3 + maps.first_kind + m % maps.kinds;
+        const std::uint8_t* matrix = maps.table[which].weight;
+        if ((reinterpret_cast<std::uintptr_t>(matrix) & 15U) != 0U) return;
+        map_image[warp][lane] = reinterpret_cast<const std::uint32_t*>(&maps.box)[lane];
+        __syncwarp();
+        if (lane == 0) tensormap_set_address(map_image[warp], matrix);
+        __syncwarp();
+        tensormap_publish(maps.maps + which, map_image[warp]);
+        return;
+    }
     if (i >= assignments) return;
     const std::size_t src = static_cast<std::size_t>(distinct_rows ? i : i / kTop);
     const std::size_t pp = static_cast<std::size_t>(pp_of_flat[i]);
@@ -1095,13 +1085,14 @@ __global__ void __launch_bounds__(256) gather_quantized_rows_kernel(const std::u
 
 cudaError_t launch_gather_quantized_rows(const std::uint8_t* packed, const std::uint8_t* scales_swizzled,
                                          const std::int32_t* pp_of_flat, std::uint8_t* xq, std::uint8_t* xs, int assignments,
-                                         int k_bytes, bool distinct_rows, cudaStream_t stream, bool pdl) {
+                                         int k_bytes, bool distinct_rows, const TableMaps& maps, cudaStream_t stream, bool pdl) {
     if (packed == nullptr || scales_swizzled == nullptr || assignments <= 0 || k_bytes % 16 != 0 ||
         (reinterpret_cast<std::uintptr_t>(packed) & 15U) != 0U) {
         return cudaErrorInvalidValue;
     }
-    return launch_kernel(gather_quantized_rows_kernel, dim3((assignments + 7) / 8), dim3(256), 0, stream, pdl, packed,
-                         scales_swizzled, pp_of_flat, xq, xs, assignments, k_bytes, distinct_rows ? 1 : 0);
+    const int map_warps = std::min(assignments, kExperts) * maps.kinds;
+    return launch_kernel(gather_quantized_rows_kernel, dim3((assignments + 7) / 8 + (map_warps + 7) / 8), dim3(256), 0, stream, pdl,
+                         packed, scales_swizzled, pp_of_flat, xq, xs, assignments, k_bytes, distinct_rows ? 1 : 0, maps);
 }
 
 }  // namespace p92b

@@ -208,6 +208,7 @@ int p92b_plan_create(p92b_plan** out, int max_rows, int hidden, int intermediate
         plan->stage_out = c.take<std::uint16_t>(rows * hidden);
         plan->stage_in_b = c.take<std::uint16_t>(rows * hidden);
         plan->stage_out_b = c.take<std::uint16_t>(rows * hidden);
+        plan->table_maps = c.take<CUtensorMap>(static_cast<std::size_t>(kExperts) * 3);
         plan->status = c.take<std::int32_t>(1);
         if (pass == 0) {
             plan->bytes = c.used;
@@ -233,6 +234,8 @@ int p92b_plan_create(p92b_plan** out, int max_rows, int hidden, int intermediate
                            cudaSuccess;
         }
         ok = ok && make_operand_map(&plan->map_x_tok, plan->xq_tok, 16, hidden / 2, 16) == cudaSuccess;
+        ok = ok && make_operand_map(&plan->map_table[0], plan->xq_pp, intermediate, hidden / 2, 128) == cudaSuccess;
+        ok = ok && make_operand_map(&plan->map_table[1], plan->xq_pp, hidden, intermediate / 2, 128) == cudaSuccess;
         plan->tc_ready = ok;
     }
     *out = plan;
@@ -309,19 +312,19 @@ int p92b_plan_get_views(const p92b_plan* plan, p92b_plan_views* v) {
 
 int p92b_bf16_gemv_f32(const uint16_t* input, const uint16_t* weight, float* output, int rows, int columns,
                        void* stream) {
-    return launch_router_logits(input, weight, output, 1, rows, columns, true, static_cast<cudaStream_t>(stream));
+    return launch_router_logits(input, weight, output, 1, rows, columns, true, static_cast<cudaStream_t>(stream), pdl_enabled());
 }
 
 int p92b_bf16_gemm_f32(const uint16_t* input, const uint16_t* weight, float* output, int batch_rows, int rows,
                        int columns, void* stream) {
     return launch_router_logits(input, weight, output, batch_rows, rows, columns, false,
-                                static_cast<cudaStream_t>(stream));
+                                static_cast<cudaStream_t>(stream), pdl_enabled());
 }
 
 int p92b_router_top8_rows(const float* logits, const float* correction_bias, int32_t* expert_ids,
                           float* expert_weights, int rows, float routed_scale, void* stream) {
     return launch_router_top8(logits, correction_bias, expert_ids, expert_weights, rows, routed_scale,
-                              static_cast<cudaStream_t>(stream));
+                              static_cast<cudaStream_t>(stream), pdl_enabled());
 }
 
 int p92b_router_top8(const float* logits, const float* correction_bias, int32_t* expert_ids,
@@ -618,7 +621,7 @@ int p92b_project_expert_gate_up(p92b_plan* plan, const p92b_bank* bank, const in
     // permutation of the caller's ids -> token rows quantised into the padded position space -> the grouped
     // tcgen05 product with the epilogue that stores gate and up un-fused at their (row, slot) rows
     cudaError_t st = launch_permute(plan, expert_ids, rows * kTop, plan->order, plan->position, plan->counts,
-                                    plan->offsets, true, tc_pad_align(rows), tc_tile_rows(rows), stream);
+                                    plan->offsets, true, tc_pad_align(rows), tc_tile_rows(rows), stream, pdl);
     if (st != cudaSuccess) return st;
     st = launch_quantize_padded(plan, input, rows, stream, pdl);
     if (st != cudaSuccess) return st;
@@ -644,7 +647,7 @@ int p92b_project_expert_down(p92b_plan* plan, const p92b_bank* bank, const int32
     plan->last_launches = 0;
     plan->last_path = 2;
     cudaError_t st = launch_permute(plan, expert_ids, rows * kTop, plan->order, plan->position, plan->counts,
-                                    plan->offsets, true, tc_pad_align(rows), tc_tile_rows(rows), stream);
+                                    plan->offsets, true, tc_pad_align(rows), tc_tile_rows(rows), stream, pdl);
     if (st != cudaSuccess) return st;
     // every (row, slot) intermediate row is quantised on its own (src/executor.cpp:85-91), to its padded position
     st = launch_quantize_rows_to_pp(input_rows, plan->pp_of_flat, plan->hq_pp, plan->hs_sw, rows * kTop, plan->intermediate,
@@ -727,11 +730,19 @@ int p92b_nvfp4_grouped_rows(p92b_grouped_plan* plan, const uint8_t* packed_input
     // the reference orders its problems by (kind, expert) with ties in the original order
     // (cuda/nvfp4_grouped.cu:117-132); the same stable order groups the rows per expert here
     cudaError_t st = launch_permute(p, expert_ids, assignments, p->order, p->position, p->counts, p->offsets, true,
-                                    tc_pad_align(batch_rows), tc_tile_rows(batch_rows), stream);
+                                    tc_pad_align(batch_rows), tc_tile_rows(batch_rows), stream, pdl);
     if (st != cudaSuccess) return st;
+    TableMaps maps {};
+    maps.table = expert_bank;
+    maps.active = p->active;
+    maps.active_count = p->active_count;
+    maps.maps = p->table_maps;
+    maps.box = p->map_table[down ? 1 : 0];
+    maps.first_kind = projection_kind;
+    maps.kinds = second_output != nullptr ? 2 : 1;
     st = launch_gather_quantized_rows(packed_input, input_scales_swizzled, p->pp_of_flat, down ? p->hq_pp : p->xq_pp,
                                       down ? p->hs_sw : p->xs_sw, assignments, plan->columns / 2,
-                                      expert_distinct_input_rows != 0, stream, pdl);
+                                      expert_distinct_input_rows != 0, maps, stream, pdl);
     if (st != cudaSuccess) return st;
     TcIo io {};
     io.table = expert_bank;

@@ -11,6 +11,7 @@
 #include <cfloat>
 #include <cstddef>
 #include <cstdint>
+#include <cstdlib>
 
 #include "p92b_moe.h"
 
@@ -342,6 +343,8 @@ struct p92b_plan {
     std::int32_t* epg_counts = nullptr;   // [257] histogram and [258] offsets of the whole gathered batch
     std::int32_t* epg_offsets = nullptr;
     int ep_words = 0;
+    CUtensorMap map_table[2] = {};        // weights read in place: box of a gate/up matrix, of a down matrix; the address is filled in on the device
+    CUtensorMap* table_maps = nullptr;    // [256 * 3] maps of the active experts' matrices, built by each in-place call
     unsigned* dense_parts_done = nullptr; // [H/128] K parts of a down tile that have finished (dense MLP of a few rows; zero between calls)
     // optional stage timing (host side)
     bool timing = false;
@@ -388,6 +391,12 @@ cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, std::
     return cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
 }
 
+// Programmatic dependent launch is on unless P92B_NO_PDL is set (A/B timing).
+inline bool pdl_enabled() {
+    static const bool on = std::getenv("P92B_NO_PDL") == nullptr;
+    return on;
+}
+
 // Opt-in to more than 48 KB of dynamic shared memory.  The attribute belongs to the (kernel, device)
 // pair, not to the process: a host that drives several GPUs from one process has to set it once on
 // each of them, so the "already done" flag is kept per device (one table per kernel through the
@@ -425,7 +434,7 @@ int route_fused_max_rows();
 cudaError_t launch_route_fused(p92b_plan* plan, const float* bias, float routed_scale, const std::uint16_t* x,
                                int rows, int pad_align, int tile_rows, cudaStream_t stream, bool pdl);
 cudaError_t launch_quantize(const std::uint16_t* input, std::uint8_t* output, std::uint8_t* scales,
-                            long groups, float global_scale, cudaStream_t stream);
+                            long groups, float global_scale, cudaStream_t stream, bool pdl = false);
 // Writes the matrices of one kind (0/1/2 = gate/up/down) of all `entries` of a table of reference-format
 // projections (device copy, entry * 3 + kind) into the chunk stream, and their alpha values.
 // blocks_per_chunk 1: gate (slot 0) or up (slot 1) of a K block; 2: K blocks 2s, 2s+1 of a down matrix.
@@ -472,9 +481,20 @@ struct TcIo {
 // True when launch_experts_tc(..., down = true) with the lists last built for `rows` runs the slab kernel, the one
 // that honours TcIo::row_dest.
 bool down_slab_applies(const p92b_plan* plan, int rows);
+// Tensor maps of the matrices that an in-place call will read: kinds first_kind .. first_kind + kinds - 1 of every active expert.
+struct TableMaps {
+    const p92b_expert_projection* table;
+    const std::int32_t* active;             // the routing lists' active entries, the shared expert first
+    const std::int32_t* active_count;
+    CUtensorMap* maps;                      // out, expert * 3 + kind
+    CUtensorMap box;                        // the map with any address
+    int first_kind;
+    int kinds;
+};
 cudaError_t launch_gather_quantized_rows(const std::uint8_t* packed, const std::uint8_t* scales_swizzled,
                                          const std::int32_t* pp_of_flat, std::uint8_t* xq, std::uint8_t* xs, int assignments,
-                                         int k_bytes, bool distinct_rows, cudaStream_t stream, bool pdl = false);
+                                         int k_bytes, bool distinct_rows, const TableMaps& maps, cudaStream_t stream,
+                                         bool pdl = false);
 cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int rows, bool down,
                               cudaStream_t stream, bool pdl = false, const TcIo* io = nullptr);
 // The dense MLP of up to 32 rows (dense_rows.cu).

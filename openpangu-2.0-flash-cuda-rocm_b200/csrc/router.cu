@@ -87,10 +87,10 @@ __global__ void __launch_bounds__(WE* WT * 32) logits_rows_kernel(
         for (int j = 0; j < TT; ++j) acc[i][j] = 0.0F;
 
     pdl_launch_dependents();
+    pdl_wait();
     for (int k0 = 0; k0 < columns; k0 += kc) {
         if (k0 != 0) __syncthreads();
-        // 16-byte coalesced staging; rows beyond the edge are zero filled.  The router weight does
-        // not depend on the upstream kernel, the token rows do.
+        // 16-byte coalesced staging; rows beyond the edge are zero filled
         for (int idx = threadIdx.x; idx < BE * kc8; idx += THREADS) {
             const int r = idx / kc8;
             const int c8 = idx - r * kc8;
@@ -100,7 +100,6 @@ __global__ void __launch_bounds__(WE* WT * 32) logits_rows_kernel(
             }
             *reinterpret_cast<uint4*>(ws + static_cast<std::size_t>(r) * kc + c8 * 8) = v;
         }
-        if (k0 == 0) pdl_wait();
         for (int idx = threadIdx.x; idx < BT * kc8; idx += THREADS) {
             const int r = idx / kc8;
             const int c8 = idx - r * kc8;
@@ -136,6 +135,58 @@ __global__ void __launch_bounds__(WE* WT * 32) logits_rows_kernel(
             const int tok = t0 + wt * TT + t;
             if (lane == 0 && e < rows && tok < batch_rows) out[static_cast<std::size_t>(tok) * rows + e] = value;
         }
+    }
+}
+
+// ---- T > 1 order, up to eight tokens ----------------------------------------
+// A block takes two experts and all tokens, four warps: (expert, half of the tokens).  Both expert rows and the token rows
+// arrive by asynchronous 16-byte copies that are all in flight at once; with loads into registers on the way to shared
+// memory, 64 blocks took 15.4 us for four tokens.  The chains are the ones above.
+template <int TT>
+__global__ void __launch_bounds__(128) logits_few_rows_kernel(const std::uint16_t* __restrict__ x, const std::uint16_t* __restrict__ w,
+                                                              float* __restrict__ out, int batch_rows, int rows, int columns) {
+    extern __shared__ __align__(16) std::uint16_t staged[];            // [2 experts + 2 TT tokens][columns]
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int pieces = columns / 8;
+    const int e0 = blockIdx.x * 2;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int staged_rows = 2 + min(batch_rows, 2 * TT);
+    for (int r = warp; r < staged_rows; r += 4) {
+        const std::uint16_t* src = r < 2 ? w + static_cast<std::size_t>(min(e0 + r, rows - 1)) * columns
+                                         : x + static_cast<std::size_t>(r - 2) * columns;
+        for (int piece = lane; piece < pieces; piece += 32) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                         ::"r"(static_cast<std::uint32_t>(__cvta_generic_to_shared(staged + static_cast<std::size_t>(r) * columns + piece * 8))),
+                         "l"(src + piece * 8) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int e = e0 + (warp & 1);
+    const int t0 = (warp >> 1) * TT;
+    if (e >= rows || t0 >= batch_rows) return;
+    const std::uint16_t* wr = staged + static_cast<std::size_t>(warp & 1) * columns + lane;
+    const std::uint16_t* xr = staged + static_cast<std::size_t>(2 + t0) * columns + lane;
+    float acc[TT];
+#pragma unroll
+    for (int t = 0; t < TT; ++t) acc[t] = 0.0F;
+#pragma unroll 8
+    for (int c = 0; c < columns; c += 32) {
+        const float wv = bf16_bits_to_float(wr[c]);
+#pragma unroll
+        for (int t = 0; t < TT; ++t) {
+            // rows beyond the batch were not staged: what lies there goes into sums that nobody reads
+            acc[t] = fmaf(bf16_bits_to_float(xr[static_cast<std::size_t>(t) * columns + c]), wv, acc[t]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < TT; ++t) {
+        float value = acc[t];
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) value += __shfl_down_sync(0xffffffffU, value, offset);
+        if (lane == 0 && t0 + t < batch_rows) out[static_cast<std::size_t>(t0 + t) * rows + e] = value;
     }
 }
 
@@ -308,17 +359,17 @@ cudaError_t launch_router_logits(const std::uint16_t* x, const std::uint16_t* w,
         if (batch_rows != 1) return cudaErrorInvalidValue;
         return launch_kernel(logits_gemv_kernel, dim3(rows), dim3(256), 0, stream, pdl, x, w, out, rows, columns);
     } else if (batch_rows <= 8) {
-        // decode: the whole K extent of 2 expert rows and of every token sits in
-        // shared memory, so all global loads of a block are in flight at once
-        constexpr int TE = 1, TT = 8, WE = 4, WT = 1;
-        const std::size_t smem = static_cast<std::size_t>(TE * WE + TT * WT) * columns * 2;
-        if (smem > 200 * 1024) return cudaErrorInvalidValue;
-        auto kernel = logits_rows_kernel<TE, TT, WE, WT>;
-        if (cudaError_t st = ensure_dynamic_smem<logits_rows_kernel<TE, TT, WE, WT>>(200 * 1024); st != cudaSuccess) return st;
-        dim3 grid((rows + TE * WE - 1) / (TE * WE), 1);
-        return launch_kernel(kernel, grid, dim3(WE * WT * 32), smem, stream, pdl, x, w, out, batch_rows, rows, columns,
-                             columns);
-    } else if (batch_rows >= 256 && columns % 256 == 0) {
+        // decode: the whole K extent of two expert rows and of every token in shared memory
+        if (static_cast<std::size_t>(12) * columns * 2 > 200 * 1024) return cudaErrorInvalidValue;
+        const dim3 grid((rows + 1) / 2);
+        const std::size_t row_bytes = static_cast<std::size_t>(columns) * 2;
+        if (batch_rows <= 4) {
+            if (cudaError_t st = ensure_dynamic_smem<logits_few_rows_kernel<2>>(200 * 1024); st != cudaSuccess) return st;
+            return launch_kernel(logits_few_rows_kernel<2>, grid, dim3(128), 6 * row_bytes, stream, pdl, x, w, out, batch_rows, rows, columns);
+        }
+        if (cudaError_t st = ensure_dynamic_smem<logits_few_rows_kernel<4>>(200 * 1024); st != cudaSuccess) return st;
+        return launch_kernel(logits_few_rows_kernel<4>, grid, dim3(128), 10 * row_bytes, stream, pdl, x, w, out, batch_rows, rows, columns);
+    } else if (columns % 256 == 0) {
         // 16 experts x 16 tokens per block of four warps.  (Measured at T=4096 with the chunk copied asynchronously
         // into shared memory and transposed there: 230 µs with this block shape, 237 - 296 µs with three others.)
         dim3 grid((rows + 15) / 16, (batch_rows + 15) / 16);

@@ -170,6 +170,19 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 
+// A tensor map in shared memory (128-byte aligned) gets another base address; the whole warp then copies it to global
+// memory for a later kernel, whose loading thread acquires it before its first use.
+__device__ __forceinline__ void tensormap_set_address(const void* smem_map, const void* address) {
+    asm volatile("tensormap.replace.tile.global_address.shared::cta.b1024.b64 [%0], %1;" ::"r"(smem_u32(smem_map)), "l"(address) : "memory");
+}
+__device__ __forceinline__ void tensormap_publish(CUtensorMap* global_map, const void* smem_map) {
+    asm volatile("tensormap.cp_fenceproxy.global.shared::cta.tensormap::generic.release.gpu.sync.aligned [%0], [%1], 128;"
+                 ::"l"(global_map), "r"(smem_u32(smem_map)) : "memory");
+}
+__device__ __forceinline__ void tensormap_acquire(const CUtensorMap* global_map) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(global_map) : "memory");
+}
+
 // ---- tcgen05 --------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(std::uint32_t smem_slot, std::uint32_t columns) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_slot), "r"(columns)
