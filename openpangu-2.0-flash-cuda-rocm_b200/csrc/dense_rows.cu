@@ -22,6 +22,7 @@ using namespace ptx;
 namespace {
 
 constexpr int kRowsMax = 32;
+constexpr int kPartsMax = 8;                                 // of K, down product
 constexpr int kTile = 128;
 constexpr int kKB = 128;                                     // bytes of a K block per row: 256 values
 constexpr int kSlab = kChunkScaleBytes;
@@ -162,13 +163,16 @@ __global__ void __launch_bounds__(kGuThreads, 1) dense_gate_up_kernel(const Dens
     } else {
         // token rows -> NVFP4 in the operand's shared-memory image (cuda/nvfp4_ops.cu:818-841; 16-byte pieces XOR-swizzled by
         // the row, scales 128x4 tiled); columns beyond the last row hold whatever was there and nothing reads them
+        const float alpha_g = __ldg(p.bank.alpha + p.entry * 3 + 0);
+        const float alpha_u = __ldg(p.bank.alpha + p.entry * 3 + 1);
         pdl_wait();
         const int blocks = p.hidden / 16;
+#pragma unroll 2
         for (int i = threadIdx.x - 64; i < p.rows * blocks; i += 32 * kQuantWarps) {
             const int row = i / blocks;
             const int b = i - row * blocks;
             const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<std::size_t>(row) * p.hidden + b * 16);
-            const uint4 lo = src[0], hi = src[1];
+            const uint4 lo = __ldg(src), hi = __ldg(src + 1);
             const std::uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
             float v[16];
 #pragma unroll
@@ -193,8 +197,6 @@ __global__ void __launch_bounds__(kGuThreads, 1) dense_gate_up_kernel(const Dens
                 // lanes 0..15 of a quarter hold the gate sums of 16 intermediate rows, lanes 16..31 their up sums: of a
                 // pair of tokens the lower half finishes the even one, the upper half the odd one
                 const int quarter = warp & 3;
-                const float alpha_g = p.bank.alpha[p.entry * 3 + 0];
-                const float alpha_u = p.bank.alpha[p.entry * 3 + 1];
                 const int row = blockIdx.x * (kTile / 2) + quarter * 16 + (lane & 15);
                 const int sf_col = row >> 4;
                 const bool upper = (lane & 16) != 0;
@@ -337,12 +339,12 @@ __global__ void __launch_bounds__(kDownThreads, 1) dense_down_kernel(const __gri
             if (ok) tc_commit(accum_full); else give_up();
         }
     } else {
+        const float alpha = __ldg(p.bank.alpha + p.entry * 3 + 2);
         const bool done = mbar_wait(accum_full, 0);
         if (!done) give_up();
         tc_fence_after();
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;                     // of the tile
-        const float alpha = p.bank.alpha[p.entry * 3 + 2];
         std::uint16_t* out = p.out + static_cast<std::size_t>(tile) * kTile + row;
         float* mine = p.partial + (static_cast<std::size_t>(tile) * p.parts + part) * p.rows * kTile + row;
         if (__all_sync(0xffffffffU, done)) {
@@ -368,11 +370,17 @@ __global__ void __launch_bounds__(kDownThreads, 1) dense_down_kernel(const __gri
             if (arrived == static_cast<unsigned>(p.parts - 1)) {
                 __threadfence();
                 const float* all = p.partial + static_cast<std::size_t>(tile) * p.parts * p.rows * kTile + row;
-#pragma unroll 2
+#pragma unroll 4
                 for (int n = 0; n < p.rows; ++n) {
-                    float sum = 0.0F;
-#pragma unroll 8
-                    for (int q = 0; q < p.parts; ++q) sum += __ldcg(all + (static_cast<std::size_t>(q) * p.rows + n) * kTile);
+                    // all requests before the first sum: a loop over the parts pays a round trip to the L2 for each
+                    float part_sum[kPartsMax];
+#pragma unroll
+                    for (int q = 0; q < kPartsMax; ++q) {
+                        part_sum[q] = q < p.parts ? __ldcg(all + (static_cast<std::size_t>(q) * p.rows + n) * kTile) : 0.0F;
+                    }
+                    float sum = part_sum[0];
+#pragma unroll
+                    for (int q = 1; q < kPartsMax; ++q) sum = q < p.parts ? sum + part_sum[q] : sum;
                     out[static_cast<std::size_t>(n) * p.hidden] = float_to_bf16_bits(sum * alpha);
                 }
             }
@@ -422,7 +430,7 @@ cudaError_t launch_dense_few_rows(p92b_plan* plan, const p92b_bank* bank, const 
     // parts of K: as many blocks as there are SMs (20 tiles: 7 parts), at least one K block each.  The sums lie in the
     // grouped kernels' output rows, which this call does not use: (257 * 127 or fewer, at least 1,152) rows x hidden
     // BF16 values hold 8 parts x 32 rows x hidden FP32 values.
-    p.parts = std::max(1, std::min({8, plan->sm_count / (plan->hidden / kTile), plan->intermediate / 256}));
+    p.parts = std::max(1, std::min({kPartsMax, plan->sm_count / (plan->hidden / kTile), plan->intermediate / 256}));
     p.partial = reinterpret_cast<float*>(plan->mixed_pp);
     if (static_cast<std::size_t>(p.parts) * rows * 4 > plan->pp_rows * 2) return cudaErrorInvalidValue;
     plan->last_launches += 2;
