@@ -192,9 +192,9 @@ int p92b_plan_create(p92b_plan** out, int max_rows, int hidden, int intermediate
         plan->mega_logits = c.take<unsigned long long>(static_cast<std::size_t>(kLogitReplicas) * 16 * kExperts);
         plan->mega_ret = c.take<unsigned long long>(static_cast<std::size_t>(16) * (kTop + 1) * 1280);
         plan->mega_trace = c.take<unsigned long long>(static_cast<std::size_t>(plan->sm_count) * 64);
-        plan->w_norms = c.take<float>(2 * kExperts);
+        plan->w_norms = c.take<float>(kExperts);
         plan->router_stats = c.take<int>(2);
-        plan->logit_partials = c.take<float>(static_cast<std::size_t>(kRouterSplits) * std::min(max_rows, kRouterSplitRows) * kExperts);
+        plan->logit_partials = c.take<float>(std::min<std::size_t>(kRouterSplits * rows, kRouterPartialRows) * kExperts);
         plan->mega_hidden = c.take<unsigned long long>(static_cast<std::size_t>(16) * (hidden / 2));
         plan->normed = c.take<std::uint16_t>(rows * hidden);
         plan->ep_words = 16 * (kExperts + 1);
@@ -414,7 +414,7 @@ int p92b_moe_forward_normed(p92b_plan* plan, const p92b_bank* bank, const uint16
     }
     if ((st = mark()) != cudaSuccess) return st;
     // large batches: tensor-core logits with exact repair of the candidates (ids and weights still the reference's bit
-    // for bit); in the stage table its three kernels are the "router logits" stage and the top-8 stage is empty
+    // for bit); in the stage table its two kernels are the "router logits" stage and the top-8 stage is empty
     bool routed = false;
     if (rows >= router_fast_min_rows()) {
         st = launch_router_fast(plan, input, router_weight, correction_bias, rows, routed_scale, stream, pdl);

@@ -3,13 +3,13 @@
 // The reference's logits are FP32 fmaf chains in a fixed order (cuda/nvfp4_ops.cu:178-207): lane l of a warp sums
 // columns l, l+32, ... and a shuffle-down tree adds the 32 partial sums.  Expert ids must equal the reference's, so
 // every logit that can influence the top-8 has to be THAT number - but almost none can: of 256 logits per token only
-// those near the top-8 boundary matter.  Three kernels:
+// those near the top-8 boundary matter.  Two kernels:
 //
-//   1. expert_norms_kernel   ||w_e||_2 of the 256 router rows (the error bound below needs them);
-//   2. logits_tc_kernel      approximate logits of every (token, expert) as one BF16 x BF16 -> FP32 product on the
+//   1. logits_tc_kernel      approximate logits of every (token, expert) as one BF16 x BF16 -> FP32 product on the
 //                            5th-generation tensor cores (tcgen05.mma kind::f16, M = 128 tokens, N = 64 experts per
-//                            block, operands by TMA, accumulator in TMEM);
-//   3. route_repair_kernel   one warp per token: corrected scores from the approximate logits, the approximate 8th
+//                            block, operands by TMA, accumulator in TMEM), and beside it ||w_e||_2 of the 256 router
+//                            rows (the error bound below needs them);
+//   2. route_repair_kernel   one warp per token: corrected scores from the approximate logits, the approximate 8th
 //                            best, the candidate set = every expert whose approximate score is within 2 delta of it,
 //                            the candidates' logits recomputed in the reference's exact order, and the reference's
 //                            top-8 (cuda/nvfp4_ops.cu:357-433: higher corrected score first, ties to the lower id,
@@ -30,6 +30,7 @@
 #include "p92b_common.cuh"
 #include "tc_ptx.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 
 namespace p92b {
@@ -68,22 +69,12 @@ __host__ __device__ constexpr std::uint32_t idesc_bf16(int m, int n) {
            (static_cast<std::uint32_t>(m >> 4) << 24);
 }
 
-__global__ void __launch_bounds__(256) expert_norms_kernel(const std::uint16_t* __restrict__ w, float* __restrict__ norms,
-                                                           int experts, int hidden) {
-    // Nothing here reads the upstream kernel's output, so the work comes first and overlaps that kernel's tail; the wait
-    // comes last (the kernels behind this one rely on the chain: a kernel that finished without waiting would let them
-    // start before the token rows are written).  `norms` alternates between two buffers from call to call, so a repair
-    // kernel of the call before cannot still be reading what this one writes.
-    pdl_launch_dependents();
-    const int e = blockIdx.x * 8 + (threadIdx.x >> 5);
+// ||w_e|| of one router row, by a warp.
+__device__ __forceinline__ void row_norm(const std::uint16_t* __restrict__ w, float* __restrict__ norms, int e, int hidden) {
     const int lane = threadIdx.x & 31;
-    if (e >= experts) {
-        pdl_wait();
-        return;
-    }
     float s = 0.0F;
     const uint4* row = reinterpret_cast<const uint4*>(w + static_cast<std::size_t>(e) * hidden);
-#pragma unroll 4
+#pragma unroll 10
     for (int v = lane; v < hidden / 8; v += 32) {
         const uint4 q = __ldg(row + v);
         const std::uint32_t words[4] = {q.x, q.y, q.z, q.w};
@@ -97,13 +88,13 @@ __global__ void __launch_bounds__(256) expert_norms_kernel(const std::uint16_t* 
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffU, s, off);
     if (lane == 0) norms[e] = sqrtf(s) * 1.0001F;             // rounded up a little: it feeds a bound
-    pdl_wait();
 }
 
 __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                      const __grid_constant__ CUtensorMap map_w,
                                                                      float* __restrict__ logits, int rows, int hidden,
-                                                                     std::int32_t* status) {
+                                                                     std::int32_t* status, const std::uint16_t* __restrict__ w,
+                                                                     float* __restrict__ norms) {
     // gridDim.z > 1: block z takes a slice of the K blocks and writes its partial sums to slice z of `logits`
     // ([gridDim.z][rows][256]); the repair kernel adds the slices (small batches: 4 blocks would otherwise walk all of
     // K one after the other while 144 SMs idle)
@@ -184,9 +175,17 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
             }
             if (ok && k_blocks > 0) tc_commit(accum_bar);
         }
-    } else if (k_blocks > 0) {
+    } else {
+        // while the products run, the epilogue warps take the norms of the 64 router rows, shared out over the blocks of
+        // this expert tile (a kernel of its own in front of this one cost the chain 2 us)
+        const int sharers = static_cast<int>(gridDim.x * gridDim.z) * 4;
+        for (int i = static_cast<int>(blockIdx.x * gridDim.z + blockIdx.z) * 4 + (warp - 2); i < kExpTile; i += sharers) {
+            row_norm(w, norms, e0 + i, hidden);
+        }
         const int quarter = warp & 3;                       // TMEM lanes 32 * quarter ..: the token rows of this warp
-        if (mbar_wait(accum_bar, 0)) {
+        if (k_blocks == 0) {
+            // an empty slice: nothing was issued
+        } else if (mbar_wait(accum_bar, 0)) {
             tc_fence_after();
             const int token = t0 + quarter * 32 + lane;
             const std::uint32_t lane_base = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16);
@@ -514,10 +513,14 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     if ((st = ensure_dynamic_smem<logits_tc_kernel>(kLogitSmem)) != cudaSuccess) return st;
     const bool in_registers = hidden == 2560;
     // small batches: K split over blocks of the logits kernel, and a block of eight warps per token in the repair
-    const bool small = rows <= kRouterSplitRows && plan->logit_partials != nullptr && plan->max_rows >= rows &&
-                       std::getenv("P92B_ROUTER_NO_SPLIT") == nullptr;
+    const bool may_split = plan->logit_partials != nullptr && plan->max_rows >= rows && std::getenv("P92B_ROUTER_NO_SPLIT") == nullptr;
+    const bool small = rows <= kRouterWideRows && may_split;
     const int k_blocks = hidden * 2 / kKBytes;
-    const int per_split = small ? (k_blocks + kRouterSplits - 1) / kRouterSplits : k_blocks;
+    // as many slices as fill the chip: 8 up to 512 rows, 4 up to 1,024, 2 up to 2,304 (512 rows, 16 blocks: 12 us)
+    const int tiles = (rows + kTokTile - 1) / kTokTile * (kExperts / kExpTile);
+    const int wanted = may_split && rows <= kRouterSplitRows
+                           ? std::max(1, std::min({kRouterSplits, plan->sm_count / tiles, kRouterPartialRows / rows})) : 1;
+    const int per_split = (k_blocks + wanted - 1) / wanted;
     const int splits = (k_blocks + per_split - 1) / per_split;                    // no empty slice
     constexpr int kWide = 8;
     const int repair_warps = small ? kWide : kRepairWarps;
@@ -531,12 +534,10 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
                           : ensure_dynamic_smem<route_repair_kernel<0, 1>>(static_cast<int>(repair_smem));
     }
     if (st != cudaSuccess) return st;
-    float* norms = plan->w_norms + (plan->norms_parity ^= 1) * kExperts;
-    st = launch_kernel(expert_norms_kernel, dim3(kExperts / 8), dim3(256), 0, stream, pdl, router_w, norms, kExperts, hidden);
-    if (st != cudaSuccess) return st;
+    float* norms = plan->w_norms;
     float* approx_out = splits > 1 ? plan->logit_partials : plan->logits;
     st = launch_kernel(logits_tc_kernel, dim3((rows + kTokTile - 1) / kTokTile, kExperts / kExpTile, splits), dim3(kLogitThreads),
-                       kLogitSmem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status);
+                       kLogitSmem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status, router_w, norms);
     if (st != cudaSuccess) return st;
     const float* partials = splits > 1 ? plan->logit_partials : nullptr;
     if (small) {
@@ -550,7 +551,7 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
                            router_w, bias, static_cast<const float*>(norms), plan->logits, plan->ids,
                            plan->route_weights, rows, hidden, routed_scale, plan->router_stats, partials, splits);
     }
-    plan->last_launches += 3;
+    plan->last_launches += 2;
     return st;
 }
 
