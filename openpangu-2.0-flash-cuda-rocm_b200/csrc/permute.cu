@@ -8,7 +8,7 @@
 // (cuda/nvfp4_grouped.cu:117-132) and the order its host-scheduled path walks
 // rows in (src/model.cpp:1528-1540).  No atomics touch the ordering, so the
 // result is deterministic: each warp owns a contiguous chunk of flat indices,
-// ranks inside a 32-wide step come from __match_any_sync + popcount of the
+// ranks inside a 32-wide step come from a vote per id bit + popcount of the
 // lower lanes, and chunk bases come from an exclusive scan over (expert, chunk).
 #include "p92b_common.cuh"
 #include "tc_ptx.cuh"
@@ -24,6 +24,9 @@ namespace {
 
 constexpr int kChunk = 256;          // flat indices per warp in the multi-block path
 constexpr int kWarps = 8;
+constexpr int kSmallWarps = 32;      // of the one-block path
+constexpr int kSmallChunk = 128;     // ids per warp there, at most
+constexpr int kSmallMax = kSmallWarps * kSmallChunk;      // 4,096: from there on the three-kernel form is quicker
 
 // Which expert ids take part.  The whole range by default; an expert-parallel GPU that holds the ids of the whole
 // batch restricts the permutation to its own experts [first, first + count) - ids outside (other GPUs' experts, and
@@ -34,10 +37,24 @@ struct IdRange {
     int restricted = 0;
 };
 
+// The lanes of the warp that are valid and hold the same id (0..255) as this one, from a vote per bit: 8 votes where
+// __match_any_sync goes through the distinct values (4,096 assignments: 14.3 us with it).
+__device__ __forceinline__ unsigned same_id_lanes(int e, bool valid) {
+    unsigned peers = __ballot_sync(0xffffffffU, valid);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool set = (e >> b) & 1;
+        const unsigned with = __ballot_sync(0xffffffffU, set);
+        peers &= set ? with : ~with;
+    }
+    return peers;
+}
+
 // Counts the experts of one chunk into hist[256] (owned by the calling warp).
 // `cached` (optional): the chunk's ids already in shared memory, cached[i - begin].
+template <class T>
 __device__ __forceinline__ void warp_histogram(const std::int32_t* __restrict__ ids, int begin, int end,
-                                               std::int32_t* hist, std::int32_t* status,
+                                               T* hist, std::int32_t* status,
                                                const std::int16_t* cached = nullptr, IdRange range = IdRange()) {
     const int lane = threadIdx.x & 31;
     for (int e = lane; e < kExperts; e += 32) hist[e] = 0;
@@ -54,8 +71,8 @@ __device__ __forceinline__ void warp_histogram(const std::int32_t* __restrict__ 
             atomicCAS(status, kStatusOk, kStatusBadExpertId);
             e = e < 0 ? 0 : kExperts - 1;
         }
-        const unsigned peers = __match_any_sync(0xffffffffU, e);
-        if (valid && (peers & ((1U << lane) - 1U)) == 0U) hist[e] += __popc(peers);
+        const unsigned peers = same_id_lanes(e, valid);
+        if (valid && (peers & ((1U << lane) - 1U)) == 0U) hist[e] += static_cast<T>(__popc(peers));
         __syncwarp();
     }
 }
@@ -71,20 +88,20 @@ __device__ __forceinline__ void load_chunk_ids(const std::int32_t* __restrict__ 
     __syncwarp();
 }
 
-// Scatters one chunk.  base[e] = first position of this chunk's rows of expert e; running[256] is warp-private
-// scratch; pp_delta[e] (shared memory, read only with pp_of_flat) = padded offset - offset of expert e.  The steps
+// Scatters one chunk.  running[e] (warp private) = first position of this chunk's rows of expert e, counted from
+// expert_base[e] (null: from 0); pp_delta[e] (shared memory, read only with pp_of_flat) = padded offset - offset of expert e.  The steps
 // of a chunk depend on one another through running[], so whatever a step reads has to be in shared memory or in
 // registers already: a global load per step is a round trip to the L2 per step.
+template <class T, class Order>
 __device__ __forceinline__ void warp_scatter(const std::int32_t* __restrict__ ids, int begin, int end,
-                                             const std::int32_t* base, std::int32_t* running,
-                                             std::int32_t* __restrict__ order,
+                                             T* running, const std::int32_t* expert_base,
+                                             Order* __restrict__ order,
                                              std::int32_t* __restrict__ position,
                                              std::int32_t* __restrict__ row_token,
                                              const std::int32_t* pp_delta,
                                              std::int32_t* __restrict__ pp_of_flat,
                                              const std::int16_t* cached = nullptr, IdRange range = IdRange()) {
     const int lane = threadIdx.x & 31;
-    for (int e = lane; e < kExperts; e += 32) running[e] = base[e];
     __syncwarp();
     for (int step = begin; step < end; step += 32) {
         const int i = step + lane;
@@ -99,23 +116,29 @@ __device__ __forceinline__ void warp_scatter(const std::int32_t* __restrict__ id
             e = -1;
         }
         if (valid) e = e < 0 ? 0 : (e >= kExperts ? kExperts - 1 : e);
-        const unsigned peers = __match_any_sync(0xffffffffU, e);
+        const unsigned peers = same_id_lanes(e, valid);
         const int rank = __popc(peers & ((1U << lane) - 1U));
         int pos = 0;
         if (valid) {
-            pos = running[e] + rank;
-            if (order != nullptr) order[pos] = i;
+            pos = running[e] + rank + (expert_base != nullptr ? expert_base[e] : 0);
+            if (order != nullptr) order[pos] = static_cast<Order>(i);
             if (position != nullptr) position[i] = pos;
             if (row_token != nullptr) row_token[pos] = i / kTop;
             if (pp_of_flat != nullptr) pp_of_flat[i] = pp_delta[e] + pos;
         }
         __syncwarp();
-        if (valid && rank == 0) running[e] += __popc(peers);
+        if (valid && rank == 0) running[e] += static_cast<T>(__popc(peers));
         __syncwarp();
     }
 }
 
-// Exclusive scan of 256 per-expert totals by one 256-thread block.
+// Exclusive scan of 256 per-expert totals by the first 256 threads of a block: all threads that the block (still) has,
+// or, with PART, the first 256 of more (named barrier 1).
+template <bool PART>
+__device__ __forceinline__ void scan_sync() {
+    if constexpr (PART) asm volatile("bar.sync 1, 256;" ::: "memory"); else __syncthreads();
+}
+template <bool PART = false>
 __device__ __forceinline__ int block_exclusive_scan_256(int value, std::int32_t* warp_totals) {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -126,10 +149,10 @@ __device__ __forceinline__ int block_exclusive_scan_256(int value, std::int32_t*
         if (lane >= offset) inclusive += other;
     }
     if (lane == 31) warp_totals[warp] = inclusive;
-    __syncthreads();
+    scan_sync<PART>();
     int before = 0;
     for (int wi = 0; wi < warp; ++wi) before += warp_totals[wi];
-    __syncthreads();
+    scan_sync<PART>();
     return before + inclusive - value;
 }
 
@@ -153,13 +176,14 @@ struct RouteLists {
     bool enabled;
 };
 
+template <bool PART = false>
 __device__ __forceinline__ void write_route_lists(int e, int count, int offset, int assignments, int rows,
                                                   const RouteLists& lists, std::int32_t* scan_scratch) {
     lists.counts[e] = count;
     lists.offsets[e] = offset;
     if (e == kExperts - 1) lists.offsets[kExperts] = assignments;
     if (!lists.enabled) return;
-    const int slot = block_exclusive_scan_256(count > 0 ? 1 : 0, scan_scratch);
+    const int slot = block_exclusive_scan_256<PART>(count > 0 ? 1 : 0, scan_scratch);
     if (count > 0) lists.active[1 + slot] = e;
     if (e == kExperts - 1) {
         lists.counts[kExperts] = rows;
@@ -170,11 +194,11 @@ __device__ __forceinline__ void write_route_lists(int e, int count, int offset, 
     if (lists.pp_off == nullptr) return;
     const int align = lists.pad_align;
     const int padded = (count + align - 1) / align * align;
-    const int pp = block_exclusive_scan_256(padded, scan_scratch);
+    const int pp = block_exclusive_scan_256<PART>(padded, scan_scratch);
     lists.pp_off[e] = pp;
     const int tiles = (count + lists.tile_rows - 1) / lists.tile_rows;
     const int shared_tiles = (rows + lists.tile_rows - 1) / lists.tile_rows;
-    const int before = block_exclusive_scan_256(tiles, scan_scratch);
+    const int before = block_exclusive_scan_256<PART>(tiles, scan_scratch);
     if (count > 0) lists.tile_prefix[1 + slot] = shared_tiles + before;
     if (e == kExperts - 1) {
         lists.pp_off[kExperts] = pp + padded;
@@ -186,7 +210,7 @@ __device__ __forceinline__ void write_route_lists(int e, int count, int offset, 
     const int wide = lists.tile_rows_wide;
     const int tiles_w = (count + wide - 1) / wide;
     const int shared_w = (rows + wide - 1) / wide;
-    const int before_w = block_exclusive_scan_256(tiles_w, scan_scratch);
+    const int before_w = block_exclusive_scan_256<PART>(tiles_w, scan_scratch);
     if (count > 0) lists.tile_prefix_wide[1 + slot] = shared_w + before_w;
     if (e == kExperts - 1) {
         lists.tile_prefix_wide[0] = 0;
@@ -194,44 +218,76 @@ __device__ __forceinline__ void write_route_lists(int e, int count, int offset, 
     }
 }
 
-// ---- single-block path (assignments <= 8 * 1024) ---------------------------
-__global__ void __launch_bounds__(256) permute_small_kernel(
+// ---- single-block path (assignments <= kSmallMax) ---------------------------
+// Both passes of a warp are chains of dependent 32-wide steps, so the ids are spread over 32 warps (4,096 assignments: four
+// steps).  What lies in position order is put together in shared memory and leaves as whole lines: scattered 4-byte
+// stores of one SM and the matching of ids bound the kernel before (15.5 us at 4,096 assignments, now 11.4).
+constexpr int kSmallThreads = 32 * kSmallWarps;
+__global__ void __launch_bounds__(kSmallThreads) permute_small_kernel(
     const std::int32_t* __restrict__ ids, int assignments, std::int32_t* order,
     std::int32_t* position, RouteLists lists, std::int32_t* row_token, std::int32_t* pp_of_flat,
     std::int32_t* status, IdRange range, int shared_rows) {
-    __shared__ std::int32_t hist[kWarps][kExperts];
-    __shared__ std::int32_t running[kWarps][kExperts];
+    __shared__ std::uint16_t hist[kSmallWarps][kExperts];            // counts, then positions within the expert
+    __shared__ std::int16_t cached_ids[kSmallWarps][kSmallChunk];
+    __shared__ std::uint16_t order_image[kSmallMax];
+    __shared__ std::int32_t segment_total[kSmallThreads];
+    __shared__ std::int32_t positions;
+    __shared__ std::int32_t expert_base[kExperts];
     __shared__ std::int32_t scan_scratch[kWarps];
     __shared__ std::int32_t pp_delta[kExperts];
     pdl_launch_dependents();
     pdl_wait();
     const int warp = threadIdx.x >> 5;
-    const int per_warp = ((assignments + kWarps - 1) / kWarps + 31) / 32 * 32;
+    const int per_warp = ((assignments + kSmallWarps - 1) / kSmallWarps + 31) / 32 * 32;
     const int begin = min(assignments, warp * per_warp);
     const int end = min(assignments, begin + per_warp);
-    // the warp's ids once into shared memory, all loads in flight together: the two passes below are chains of
-    // dependent 32-wide steps and would otherwise pay a global-memory round trip per step
-    __shared__ std::int16_t cached_ids[kWarps][1024];
+    // the warp's ids once into shared memory, all loads in flight together: the two passes below would otherwise pay a
+    // global-memory round trip per step
     load_chunk_ids(ids, begin, end, cached_ids[warp]);
     warp_histogram(ids, begin, end, hist[warp], status, cached_ids[warp], range);
     __syncthreads();
-    const int e = threadIdx.x;
-    int total = 0;
+    // exclusive prefix over the warps, per expert: four threads of eight warps' counts each
+    const int e = threadIdx.x % kExperts;
+    constexpr int kPerSegment = kSmallWarps * kExperts / kSmallThreads;
+    const int first_warp = threadIdx.x / kExperts * kPerSegment;
+    int count[kPerSegment];
+    int sum = 0;
 #pragma unroll
-    for (int wi = 0; wi < kWarps; ++wi) {
-        const int c = hist[wi][e];
-        hist[wi][e] = total;      // exclusive prefix over chunks
-        total += c;
+    for (int wi = 0; wi < kPerSegment; ++wi) {
+        count[wi] = hist[first_warp + wi][e];
+        sum += count[wi];
     }
-    const int offset = block_exclusive_scan_256(total, scan_scratch);
-#pragma unroll
-    for (int wi = 0; wi < kWarps; ++wi) hist[wi][e] += offset;
-    const int rows = shared_rows >= 0 ? shared_rows : assignments / kTop;
-    write_route_lists(e, total, offset, assignments, rows, lists, scan_scratch);
-    pp_delta[e] = (pp_of_flat != nullptr && lists.pp_off != nullptr) ? lists.pp_off[e] - offset : 0;       // write_route_lists stored both just above
+    segment_total[threadIdx.x] = sum;
     __syncthreads();
-    warp_scatter(ids, begin, end, hist[warp], running[warp], order, position, row_token, pp_delta, pp_of_flat,
-                 cached_ids[warp], range);
+    int before = 0, total = 0;
+#pragma unroll
+    for (int s = 0; s < kSmallThreads / kExperts; ++s) {
+        const int v = segment_total[s * kExperts + e];
+        if (s * kPerSegment < first_warp) before += v;
+        total += v;
+    }
+#pragma unroll
+    for (int wi = 0; wi < kPerSegment; ++wi) {
+        hist[first_warp + wi][e] = static_cast<std::uint16_t>(before);
+        before += count[wi];
+    }
+    const int rows = shared_rows >= 0 ? shared_rows : assignments / kTop;
+    if (threadIdx.x < kExperts) {
+        const int offset = block_exclusive_scan_256<true>(total, scan_scratch);
+        write_route_lists<true>(e, total, offset, assignments, rows, lists, scan_scratch);
+        expert_base[e] = offset;
+        if (e == kExperts - 1) positions = offset + total;
+        pp_delta[e] = (pp_of_flat != nullptr && lists.pp_off != nullptr) ? lists.pp_off[e] - offset : 0;       // write_route_lists stored both just above
+    }
+    __syncthreads();
+    warp_scatter(ids, begin, end, hist[warp], expert_base, order_image, position, static_cast<std::int32_t*>(nullptr), pp_delta,
+                 pp_of_flat, cached_ids[warp], range);
+    __syncthreads();
+    for (int at = threadIdx.x; at < positions; at += kSmallThreads) {
+        const int i = order_image[at];
+        if (order != nullptr) order[at] = i;
+        if (row_token != nullptr) row_token[at] = i / kTop;
+    }
     if (row_token != nullptr) {
         for (int t = threadIdx.x; t < rows; t += blockDim.x) {
             row_token[assignments + t] = t;
@@ -326,7 +382,6 @@ __global__ void __launch_bounds__(256) permute_scatter_kernel(
     const std::int32_t* __restrict__ offsets, std::int32_t* order, std::int32_t* position,
     std::int32_t* row_token, const std::int32_t* __restrict__ pp_off, std::int32_t* pp_of_flat, IdRange range,
     int shared_rows) {
-    __shared__ std::int32_t base[kWarps][kExperts];
     __shared__ std::int32_t running[kWarps][kExperts];
     __shared__ std::int32_t pp_delta[kExperts];
     __shared__ std::int16_t cached_ids[kWarps][kChunk];
@@ -341,11 +396,11 @@ __global__ void __launch_bounds__(256) permute_scatter_kernel(
     pp_delta[threadIdx.x] = pp_of_flat != nullptr ? pp_off[threadIdx.x] - offsets[threadIdx.x] : 0;
     if (begin < assignments) {
         for (int e = lane; e < kExperts; e += 32) {
-            base[warp][e] = offsets[e] + chunk_hist[static_cast<std::size_t>(chunk) * kExperts + e];
+            running[warp][e] = offsets[e] + chunk_hist[static_cast<std::size_t>(chunk) * kExperts + e];
         }
     }
     __syncthreads();
-    warp_scatter(ids, begin, end, base[warp], running[warp], order, position, row_token, pp_delta, pp_of_flat,
+    warp_scatter(ids, begin, end, running[warp], nullptr, order, position, row_token, pp_delta, pp_of_flat,
                  cached_ids[warp], range);
     if (row_token != nullptr) {
         const int rows = shared_rows >= 0 ? shared_rows : assignments / kTop;
@@ -542,10 +597,10 @@ cudaError_t launch_permute(p92b_plan* plan, const std::int32_t* ids, int assignm
     plan->wide_rows = wide ? 128 : 0;
     std::int32_t* row_token = route_lists ? plan->row_token : nullptr;
     std::int32_t* pp_of_flat = padded ? plan->pp_of_flat : nullptr;
-    // one block takes up to 8,192 assignments, but from 4,097 on the three-kernel form is quicker (33 against 22 µs at 8,192)
-    if (assignments <= 4096) {
+    // one block up to 4,096 assignments; at 8,192 the three-kernel form was quicker (22 against 33 µs)
+    if (assignments <= kSmallMax) {
         plan->last_launches += 1;
-        return launch_kernel(permute_small_kernel, dim3(1), dim3(256), 0, stream, pdl, ids, assignments, order, position,
+        return launch_kernel(permute_small_kernel, dim3(1), dim3(kSmallThreads), 0, stream, pdl, ids, assignments, order, position,
                              lists, row_token, pp_of_flat, plan->status, range, shared_rows);
     }
     const int chunks = (assignments + kChunk - 1) / kChunk;
@@ -649,8 +704,8 @@ extern "C" int p92b_moe_permute_static(const int32_t* expert_ids, int assignment
     lists.tile_rows = 1;
     lists.tile_rows_wide = 1;
     lists.tile_prefix_wide = nullptr;
-    if (assignments <= kWarps * 1024) {
-        permute_small_kernel<<<1, 256, 0, stream>>>(expert_ids, assignments, order, position, lists, nullptr, nullptr,
+    if (assignments <= kSmallMax) {
+        permute_small_kernel<<<1, kSmallThreads, 0, stream>>>(expert_ids, assignments, order, position, lists, nullptr, nullptr,
                                                     status, IdRange(), -1);
         return cudaGetLastError();
     }
