@@ -754,8 +754,11 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_down_slab_kernel(const _
 // Quantises the token rows into the padded position space of the tensor-core
 // kernels: row pp gets the NVFP4 bytes of its token, and the scales go straight
 // into the 128x4-tiled layout (cuda/nvfp4_ops.cu:818-841 and :869-890 in one pass).
-// One warp per TOKEN: the row is read and quantised once (lane l owns 16-element blocks l, l+32, ...)
-// and written to the nine places it is needed, its eight routed slots and its shared-expert row.
+// The row is read and quantised once (lane l of a token's warps owns 16-element blocks l, l + 32 WARPS, ...) and
+// written to the nine places it is needed, its eight routed slots and its shared-expert row.  WARPS per token: 8 while
+// there are fewer tokens than would fill the chip with one each - a lane then has one block to read and nine pieces to
+// write instead of five of each one after the other (9.0 us at 64 and at 512 rows) - else 1.
+template <int WARPS>
 __global__ void __launch_bounds__(256) quantize_padded_kernel(const std::uint16_t* __restrict__ x,
                                                               const std::int32_t* __restrict__ pp_of_flat,
                                                               std::uint8_t* __restrict__ xq,
@@ -764,11 +767,12 @@ __global__ void __launch_bounds__(256) quantize_padded_kernel(const std::uint16_
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int token = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) / WARPS;
     if (token >= rows) return;
     const int blocks = hidden / 16;
     const int col_blocks = (blocks + 3) / 4;
-    constexpr int kMaxPerLane = 8;                   // hidden <= 4096
+    constexpr int kMaxPerLane = 8 / WARPS;           // hidden <= 4096
+    const int first = ((threadIdx.x >> 5) % WARPS) * 32 + lane;
     uint2 packed[kMaxPerLane];
     std::uint32_t scale_word[kMaxPerLane];           // lanes 0, 4, 8, ...: the scales of four neighbouring blocks
     // the nine destinations of the row, fetched before the row itself so that the stores wait for nothing
@@ -776,7 +780,7 @@ __global__ void __launch_bounds__(256) quantize_padded_kernel(const std::uint16_
     const int my_pp = lane <= kTop ? __ldg(pp_of_flat + place_index) : 0;
 #pragma unroll
     for (int j = 0; j < kMaxPerLane; ++j) {
-        const int b = lane + 32 * j;
+        const int b = first + 32 * WARPS * j;
         std::uint8_t scale_bits = 0;
         if (b < blocks) {                            // blocks is a multiple of 4: a quad of lanes is in or out together
             const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<std::size_t>(token) * hidden + b * 16);
@@ -803,7 +807,7 @@ __global__ void __launch_bounds__(256) quantize_padded_kernel(const std::uint16_
         std::uint8_t* row_s = xs + (pp >> 7) * col_blocks * 512 + (pp & 31) * 16 + ((pp >> 5) & 3) * 4;
 #pragma unroll
         for (int j = 0; j < kMaxPerLane; ++j) {
-            const int b = lane + 32 * j;
+            const int b = first + 32 * WARPS * j;
             if (b >= blocks) break;
             *reinterpret_cast<uint2*>(row_q + b * 8) = packed[j];
             if ((lane & 3) == 0) *reinterpret_cast<std::uint32_t*>(row_s + (b >> 2) * 512) = scale_word[j];
@@ -900,9 +904,9 @@ int tc_pad_align(int rows) { (void)rows; return 128; }
 cudaError_t launch_quantize_padded(const p92b_plan* plan, const std::uint16_t* x, int rows, cudaStream_t stream,
                                    bool pdl) {
     if (plan->hidden > 4096) return cudaErrorNotSupported;
-    const int warps = rows;                        // one per token
-    return launch_kernel(quantize_padded_kernel, dim3((warps + 7) / 8), dim3(256), 0, stream, pdl, x,
-                         static_cast<const std::int32_t*>(plan->pp_of_flat), plan->xq_pp, plan->xs_sw, rows,
+    const bool few = rows <= 1024;
+    return launch_kernel(few ? quantize_padded_kernel<8> : quantize_padded_kernel<1>, dim3(few ? rows : (rows + 7) / 8), dim3(256), 0,
+                         stream, pdl, x, static_cast<const std::int32_t*>(plan->pp_of_flat), plan->xq_pp, plan->xs_sw, rows,
                          plan->hidden, 1.0F);
 }
 
