@@ -187,10 +187,20 @@ def _ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
-def _stream() -> int:
-    import torch
+_raw_stream = None
 
-    return torch.cuda.current_stream().cuda_stream
+
+def _stream() -> int:
+    """Handle of the current stream of the current device."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+
+        torch.cuda.current_stream()          # initialises CUDA
+        # the handle without a Stream object around it, which costs as much as the rest of an operator call in Python
+        handle, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        _raw_stream = ((lambda: handle(device())) if handle and device else (lambda: torch.cuda.current_stream().cuda_stream))
+    return _raw_stream()
 
 
 def _require(t, dtype, name: str):
