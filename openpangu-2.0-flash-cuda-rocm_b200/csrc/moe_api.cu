@@ -193,6 +193,7 @@ int p92b_plan_create(p92b_plan** out, int max_rows, int hidden, int intermediate
         plan->mega_ret = c.take<unsigned long long>(static_cast<std::size_t>(16) * (kTop + 1) * 1280);
         plan->mega_trace = c.take<unsigned long long>(static_cast<std::size_t>(plan->sm_count) * 64);
         plan->w_norms = c.take<float>(kExperts);
+        plan->w_chains = c.take<std::uint16_t>(static_cast<std::size_t>(kExperts) * hidden);
         plan->router_stats = c.take<int>(2);
         plan->logit_partials = c.take<float>(std::min<std::size_t>(kRouterSplits * rows, kRouterPartialRows) * kExperts);
         plan->mega_hidden = c.take<unsigned long long>(static_cast<std::size_t>(16) * (hidden / 2));

@@ -326,6 +326,7 @@ struct p92b_plan {
     unsigned long long* mega_logits = nullptr;  // [8][16][256] router logits as {value, launch number} words, in eight copies
     unsigned long long* mega_ret = nullptr;     // [8][9][1280] down rows as {two BF16, launch number} words
     float* w_norms = nullptr;                   // [256] norms of the router rows (tensor-core router)
+    std::uint16_t* w_chains = nullptr;          // [256][H] the router rows in chain order (tensor-core router)
     float* logit_partials = nullptr;            // [min(kRouterSplits * max_rows, kRouterPartialRows)][256] partial logits of the K splits
     int* router_stats = nullptr;                // [2] large-batch router: logits recomputed exactly so far, tokens that took a whole row
     unsigned long long* mega_hidden = nullptr;  // [8][H/2] un-normalised output rows as tagged words (fused post-norm)

@@ -69,20 +69,38 @@ __host__ __device__ constexpr std::uint32_t idesc_bf16(int m, int n) {
            (static_cast<std::uint32_t>(m >> 4) << 24);
 }
 
-// ||w_e|| of one router row, by a warp.
-__device__ __forceinline__ void row_norm(const std::uint16_t* __restrict__ w, float* __restrict__ norms, int e, int hidden) {
+// ||w_e|| of one router row, by a warp; and, for hidden = 2,560, the row once more in the order in which the exact chains
+// take it: piece (c, lane) of 16 bytes holds columns lane + 32 (8 c + i), i = 0 .. 7, so that a lane of the repair kernel
+// reads eight steps of its chain with one load.
+constexpr int kChunksInRegisters = 80;                    // hidden / 32
+__device__ __forceinline__ void row_norm(const std::uint16_t* __restrict__ w, float* __restrict__ norms,
+                                         std::uint16_t* __restrict__ w_chains, int e, int hidden) {
     const int lane = threadIdx.x & 31;
     float s = 0.0F;
-    const uint4* row = reinterpret_cast<const uint4*>(w + static_cast<std::size_t>(e) * hidden);
-#pragma unroll 10
-    for (int v = lane; v < hidden / 8; v += 32) {
-        const uint4 q = __ldg(row + v);
-        const std::uint32_t words[4] = {q.x, q.y, q.z, q.w};
+    if (w_chains != nullptr) {
+        const std::uint16_t* row = w + static_cast<std::size_t>(e) * hidden + lane;
+        uint4* to = reinterpret_cast<uint4*>(w_chains + static_cast<std::size_t>(e) * hidden) + lane;
+#pragma unroll 5
+        for (int c = 0; c < kChunksInRegisters / 8; ++c) {
+            std::uint32_t v[8];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float lo = __uint_as_float(words[k] << 16), hi = __uint_as_float(words[k] & 0xffff0000U);
-            s = fmaf(lo, lo, s);
-            s = fmaf(hi, hi, s);
+            for (int i = 0; i < 8; ++i) v[i] = __ldg(row + 32 * (8 * c + i));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s = fmaf(__uint_as_float(v[i] << 16), __uint_as_float(v[i] << 16), s);
+            to[32 * c] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
+        }
+    } else {
+        const uint4* row = reinterpret_cast<const uint4*>(w + static_cast<std::size_t>(e) * hidden);
+#pragma unroll 10
+        for (int v = lane; v < hidden / 8; v += 32) {
+            const uint4 q = __ldg(row + v);
+            const std::uint32_t words[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float lo = __uint_as_float(words[k] << 16), hi = __uint_as_float(words[k] & 0xffff0000U);
+                s = fmaf(lo, lo, s);
+                s = fmaf(hi, hi, s);
+            }
         }
     }
 #pragma unroll
@@ -94,7 +112,8 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
                                                                      const __grid_constant__ CUtensorMap map_w,
                                                                      float* __restrict__ logits, int rows, int hidden,
                                                                      std::int32_t* status, const std::uint16_t* __restrict__ w,
-                                                                     float* __restrict__ norms) {
+                                                                     float* __restrict__ norms,
+                                                                     std::uint16_t* __restrict__ w_chains) {
     // gridDim.z > 1: block z takes a slice of the K blocks and writes its partial sums to slice z of `logits`
     // ([gridDim.z][rows][256]); the repair kernel adds the slices (small batches: 4 blocks would otherwise walk all of
     // K one after the other while 144 SMs idle)
@@ -180,7 +199,7 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
         // this expert tile (a kernel of its own in front of this one cost the chain 2 us)
         const int sharers = static_cast<int>(gridDim.x * gridDim.z) * 4;
         for (int i = static_cast<int>(blockIdx.x * gridDim.z + blockIdx.z) * 4 + (warp - 2); i < kExpTile; i += sharers) {
-            row_norm(w, norms, e0 + i, hidden);
+            row_norm(w, norms, w_chains, e0 + i, hidden);
         }
         const int quarter = warp & 3;                       // TMEM lanes 32 * quarter ..: the token rows of this warp
         if (k_blocks == 0) {
@@ -215,11 +234,6 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
     }
 }
 
-// 16-byte asynchronous copy global -> shared.
-__device__ __forceinline__ void copy16_async(void* dst_smem, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
-}
-
 // Exact logit of (token row in shared memory, router row in global memory) in the reference's T > 1 order.
 __device__ __forceinline__ float exact_logit(const std::uint16_t* __restrict__ x_row, const std::uint16_t* __restrict__ w_row,
                                              int hidden, int lane) {
@@ -234,13 +248,12 @@ __device__ __forceinline__ float exact_logit(const std::uint16_t* __restrict__ x
 }
 
 constexpr int kRepairWarps = 4;
-constexpr int kRepairDepth = 3;                // router rows in flight per warp (register variant)
 
-// CHUNKS = hidden / 32 > 0: the lane's columns of the token row (l, l+32, ...) stay in registers and every candidate's
-// router row is brought into shared memory by asynchronous 16-byte copies two candidates ahead (three buffers per warp:
-// the rows come from the L2 at about a microsecond each, and 171 MB of them at T=4096 make the L2-to-SM fabric the bound),
-// so a chain costs a shared-memory read, a shift and an fmaf per column instead of two 2-byte loads from the L2 that
-// the chain has to wait for.  CHUNKS = 0: any hidden size, token row in shared memory, router rows read in place.
+// CHUNKS = hidden / 32 > 0: the lane's columns of the token row (l, l+32, ...) stay in registers and the candidates' router
+// rows are read in chain order (row_norm) two at a time: ten 16-byte loads a row, two independent chains, three
+// instructions per column of a pair's row and no shared memory.  Rows brought into shared memory as they are cost a 2-byte
+// read, a shift and an fmaf per column of one dependent chain, and three blocks of four warps per SM (124 us at 16,384
+// tokens, 38 at 4,096).  CHUNKS = 0: any hidden size, token row in shared memory, router rows read in place.
 // WPT (warps per token) = 1: a warp does everything for its token, four tokens per block - the form for thousands of
 // tokens.  WPT = 8: one token per block; the eight warps each build the candidate list (the same list) and then share
 // the candidates' exact logits out among themselves, warp 0 finishes - a few hundred tokens would otherwise leave
@@ -251,7 +264,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     const std::uint16_t* __restrict__ x, const std::uint16_t* __restrict__ w, const float* __restrict__ bias,
     const float* __restrict__ w_norms, float* __restrict__ logits, std::int32_t* __restrict__ ids,
     float* __restrict__ weights, int rows, int hidden, float routed_scale, int* __restrict__ stats,
-    const float* __restrict__ partials, int splits) {
+    const float* __restrict__ partials, int splits, const std::uint16_t* __restrict__ w_chains) {
     extern __shared__ __align__(16) std::uint16_t repair_smem[];
     pdl_launch_dependents();
     pdl_wait();
@@ -260,8 +273,8 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     const int lane = threadIdx.x & 31;
     const int token = WPT > 1 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kRepairWarps + warp;
     if (token >= rows) return;                     // WPT > 1: the grid is exactly `rows` blocks
-    // per warp: [CHUNKS > 0: two router-row buffers | CHUNKS == 0: the token row], then 256 exact logits, then the candidate list
-    constexpr int kRowSlots = CHUNKS > 0 ? kRepairDepth : 1;
+    // per warp: [CHUNKS == 0: the token row], then 256 exact logits, then the candidate list
+    constexpr int kRowSlots = CHUNKS > 0 ? 0 : 1;
     std::uint16_t* x_row = repair_smem + static_cast<std::size_t>(warp) * kRowSlots * hidden;
     std::uint8_t* tail = reinterpret_cast<std::uint8_t*>(repair_smem + static_cast<std::size_t>(kWarps) * kRowSlots * hidden);
     float* exact_row = reinterpret_cast<float*>(tail) + (WPT > 1 ? 0 : warp) * kExperts;      // WPT > 1: one row per block
@@ -386,33 +399,46 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     constexpr int kStep = WPT > 1 ? WPT : 1;
     const int n_mine = n_cand > first ? (n_cand - first + kStep - 1) / kStep : 0;
     if constexpr (CHUNKS > 0) {
-        auto fetch = [&](int i) {
-            if (i < n_mine) {
-                const uint4* src = reinterpret_cast<const uint4*>(w + static_cast<std::size_t>(cand[first + i * kStep]) * hidden);
-                uint4* dst = reinterpret_cast<uint4*>(x_row + static_cast<std::size_t>(i % kRepairDepth) * hidden);
-                for (int v = lane; v < hidden / 8; v += 32) copy16_async(dst + v, src + v);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");       // an empty group keeps the count in step
-        };
-#pragma unroll
-        for (int i = 0; i < kRepairDepth - 1; ++i) fetch(i);
 #pragma unroll 1
-        for (int i = 0; i < n_mine; ++i) {
-            fetch(i + kRepairDepth - 1);                        // its buffer was last read by candidate i - 1
-            asm volatile("cp.async.wait_group %0;" ::"n"(kRepairDepth - 1) : "memory");
-            __syncwarp();
-            const std::uint16_t* w_row = x_row + static_cast<std::size_t>(i % kRepairDepth) * hidden + lane;
-            float value = 0.0F;
+        for (int i = 0; i < n_mine; i += 2) {
+            const int ea = cand[first + i * kStep];
+            const int eb = i + 1 < n_mine ? cand[first + (i + 1) * kStep] : ea;
+            const uint4* wa = reinterpret_cast<const uint4*>(w_chains + static_cast<std::size_t>(ea) * hidden) + lane;
+            const uint4* wb = reinterpret_cast<const uint4*>(w_chains + static_cast<std::size_t>(eb) * hidden) + lane;
+            float va = 0.0F, vb = 0.0F;
 #pragma unroll
-            for (int j = 0; j < CHUNKS; ++j) value = fmaf(xr[j], bf16_bits_to_float(w_row[32 * j]), value);
+            for (int h = 0; h < 2; ++h) {                         // half a row of both in flight
+                uint4 qa[CHUNKS / 16], qb[CHUNKS / 16];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) value += __shfl_down_sync(0xffffffffU, value, off);
-            if (lane == 0) {
-                const int e = cand[first + i * kStep];
-                exact_row[e] = value;
-                lg[e] = value;
+                for (int c = 0; c < CHUNKS / 16; ++c) {
+                    qa[c] = __ldg(wa + 32 * (h * (CHUNKS / 16) + c));
+                    qb[c] = __ldg(wb + 32 * (h * (CHUNKS / 16) + c));
+                }
+#pragma unroll
+                for (int c = 0; c < CHUNKS / 16; ++c) {
+                    const std::uint32_t ua[4] = {qa[c].x, qa[c].y, qa[c].z, qa[c].w};
+                    const std::uint32_t ub[4] = {qb[c].x, qb[c].y, qb[c].z, qb[c].w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int j = 8 * (h * (CHUNKS / 16) + c) + 2 * k;
+                        va = fmaf(xr[j], __uint_as_float(ua[k] << 16), va);
+                        vb = fmaf(xr[j], __uint_as_float(ub[k] << 16), vb);
+                        va = fmaf(xr[j + 1], __uint_as_float(ua[k] & 0xffff0000U), va);
+                        vb = fmaf(xr[j + 1], __uint_as_float(ub[k] & 0xffff0000U), vb);
+                    }
+                }
             }
-            __syncwarp();                                       // every lane is done with this buffer before it is refilled
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                va += __shfl_down_sync(0xffffffffU, va, off);
+                vb += __shfl_down_sync(0xffffffffU, vb, off);
+            }
+            if (lane == 0) {
+                exact_row[ea] = va;
+                lg[ea] = va;
+                exact_row[eb] = vb;
+                lg[eb] = vb;
+            }
         }
     } else {
 #pragma unroll 1
@@ -511,7 +537,7 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     if (st == cudaSuccess) st = make_operand_map(&map_w, router_w, kExperts, static_cast<std::size_t>(hidden) * 2, kExpTile);
     if (st != cudaSuccess) return cudaErrorNotSupported;
     if ((st = ensure_dynamic_smem<logits_tc_kernel>(kLogitSmem)) != cudaSuccess) return st;
-    const bool in_registers = hidden == 2560;
+    const bool in_registers = hidden == 32 * kChunksInRegisters;
     // small batches: K split over blocks of the logits kernel, and a block of eight warps per token in the repair
     const bool may_split = plan->logit_partials != nullptr && plan->max_rows >= rows && std::getenv("P92B_ROUTER_NO_SPLIT") == nullptr;
     const bool small = rows <= kRouterWideRows && may_split;
@@ -524,7 +550,7 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     const int splits = (k_blocks + per_split - 1) / per_split;                    // no empty slice
     constexpr int kWide = 8;
     const int repair_warps = small ? kWide : kRepairWarps;
-    const std::size_t repair_smem = static_cast<std::size_t>(repair_warps) * (in_registers ? kRepairDepth : 1) * hidden * 2 +
+    const std::size_t repair_smem = static_cast<std::size_t>(repair_warps) * (in_registers ? 0 : hidden) * 2 +
                                     static_cast<std::size_t>(repair_warps) * kExperts * (4 + 2);
     if (small) {
         st = in_registers ? ensure_dynamic_smem<route_repair_kernel<80, kWide>>(static_cast<int>(repair_smem))
@@ -537,19 +563,22 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     float* norms = plan->w_norms;
     float* approx_out = splits > 1 ? plan->logit_partials : plan->logits;
     st = launch_kernel(logits_tc_kernel, dim3((rows + kTokTile - 1) / kTokTile, kExperts / kExpTile, splits), dim3(kLogitThreads),
-                       kLogitSmem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status, router_w, norms);
+                       kLogitSmem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status, router_w, norms,
+                       in_registers ? plan->w_chains : nullptr);
     if (st != cudaSuccess) return st;
     const float* partials = splits > 1 ? plan->logit_partials : nullptr;
     if (small) {
         st = launch_kernel(in_registers ? route_repair_kernel<80, kWide> : route_repair_kernel<0, kWide>, dim3(rows),
                            dim3(kWide * 32), repair_smem, stream, pdl, x, router_w, bias,
                            static_cast<const float*>(norms), plan->logits, plan->ids, plan->route_weights, rows, hidden,
-                           routed_scale, plan->router_stats, partials, splits);
+                           routed_scale, plan->router_stats, partials, splits,
+                           static_cast<const std::uint16_t*>(plan->w_chains));
     } else {
         st = launch_kernel(in_registers ? route_repair_kernel<80, 1> : route_repair_kernel<0, 1>,
                            dim3((rows + kRepairWarps - 1) / kRepairWarps), dim3(kRepairWarps * 32), repair_smem, stream, pdl, x,
                            router_w, bias, static_cast<const float*>(norms), plan->logits, plan->ids,
-                           plan->route_weights, rows, hidden, routed_scale, plan->router_stats, partials, splits);
+                           plan->route_weights, rows, hidden, routed_scale, plan->router_stats, partials, splits,
+                           static_cast<const std::uint16_t*>(plan->w_chains));
     }
     plan->last_launches += 2;
     return st;
