@@ -503,7 +503,11 @@ struct DownSlab {
     static constexpr int kTmemCols = 512;                                           // 2 * 128 + 64 + 2 * 32 = 384
     static constexpr int kBarriers = 2 + 2 * kStages + 2 * kAccumBuffers;
     static constexpr int kSmemBytes = kBBytes + kStages * kStageBytes + kEpilogueWarps * kStoreBytes + kBarriers * 8 + 16 + 1024;
-    static constexpr int kGroups = 2;                                               // row-tile halves per slab
+    // An item is a slab and all of its row tiles, or half of them.  Between two items the tensor pipe waits for the next slab,
+    // so whole slabs are better (16,384 tokens: 289 us against 300) once there are enough of them to share out evenly; with
+    // three slabs per SM halves balance better (4,096 tokens: 118 us against 131; 64: 56 against 63).
+    static constexpr int kMaxGroups = 2;
+    static constexpr int kWholeSlabsPerSm = 6;
 };
 
 // Named barriers over the 128 threads of one epilogue group (barrier 0 is __syncthreads).
@@ -541,7 +545,6 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_down_slab_kernel(const _
     const int lane = threadIdx.x & 31;
     const int k_blocks = p.k_bytes / kBlockKBytes;              // <= 4, even
     const int chunks = k_blocks / 2;
-    const int tiles_per_group = p.m_tiles / C::kGroups;
 
     if (threadIdx.x == 0) {
         mbar_init(b_full, 1);
@@ -569,15 +572,18 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_down_slab_kernel(const _
     tc_fence_after();
     pdl_launch_dependents();
     const std::uint32_t tmem_base = *tmem_slot_ptr;
-    const int total_items = route_table.prefix[route_table.active_count] * C::kGroups;      // the prefix counts 128-row slabs here
+    const int slabs = route_table.prefix[route_table.active_count];                         // the prefix counts 128-row slabs here
+    const int groups = slabs >= C::kWholeSlabsPerSm * static_cast<int>(gridDim.x) ? 1 : C::kMaxGroups;
+    const int tiles_per_group = p.m_tiles / groups;
+    const int total_items = slabs * groups;
     auto give_up = [&]() {
         *abort_ptr = 1;
         atomicCAS(p.status, kStatusOk, kStatusWaitExpired);
     };
     // item -> (slab, first row tile); decode_item wants an index over (slab, row tile)
     auto decode = [&](int item, Item* it) {
-        const int slab = item / C::kGroups;
-        const int group = item - slab * C::kGroups;
+        const int slab = item / groups;
+        const int group = item - slab * groups;
         const bool ok = decode_item<C::kN>(p, route_table, slab * p.m_tiles + group * tiles_per_group, it);
         return ok;
     };
@@ -921,7 +927,7 @@ namespace {
 bool slab_shape(const p92b_plan* plan) {
     const int k_blocks = plan->intermediate / 2 / kBlockKBytes;
     return plan->wide_rows == 128 && k_blocks <= DownSlab::kKBlocksMax && k_blocks % 2 == 0 &&
-           (plan->hidden / kTileM) % DownSlab::kGroups == 0 && std::getenv("P92B_NO_DOWN_SLAB") == nullptr;
+           (plan->hidden / kTileM) % DownSlab::kMaxGroups == 0 && std::getenv("P92B_NO_DOWN_SLAB") == nullptr;
 }
 }  // namespace
 
