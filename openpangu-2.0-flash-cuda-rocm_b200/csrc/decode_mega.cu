@@ -200,6 +200,16 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
         tmem_alloc(smem_u32(&tmem_slot_word), kTmemCols);
         tmem_relinquish();
     }
+    // Every token uses the shared expert, so its weights need no routing: they go to the L2 now, while the memory is idle
+    // (4.4 MB; the routed experts' weights are not known yet), one chunk of the tile streams per block.
+    if (threadIdx.x == 64) {
+        const int g13_chunks = inter / kTile * (hidden / 256), g2_chunks = hidden / kTile * (inter / 512);
+        const std::size_t entry = static_cast<std::size_t>(p.bank.local_experts);
+        for (int c = block; c < g13_chunks + g2_chunks; c += grid) {
+            bulk_prefetch_l2(c < g13_chunks ? p.bank.g13 + (entry * g13_chunks + c) * kChunkBytes
+                                            : p.bank.g2 + (entry * g2_chunks + (c - g13_chunks)) * kChunkBytes, kChunkBytes);
+        }
+    }
     // the router rows and the bias do not depend on the kernel upstream: fetch them before waiting for it
     const int my_experts = block + grid < kExperts ? 2 : (block < kExperts ? 1 : 0);
     std::uint16_t* w_rows = reinterpret_cast<std::uint16_t*>(smem_raw + (base - smem_u32(smem_raw)));

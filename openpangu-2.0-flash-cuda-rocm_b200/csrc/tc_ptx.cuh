@@ -151,7 +151,12 @@ __device__ __forceinline__ void bulk_load(std::uint32_t dst, const void* src, st
                  : "memory");
 }
 
-// The same with an L2 policy: weights that are read once per launch are marked "evict first", so a
+// Asks for [src, src + bytes) to be brought into the L2; nothing waits for it.  Same alignment rules.
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src, std::uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
+// bulk_load with an L2 policy: weights that are read once per launch are marked "evict first", so a
 // 120 MB stream does not push everything else (code, routing tables, token rows) out of the L2.
 __device__ __forceinline__ std::uint64_t l2_policy_evict_first() {
     std::uint64_t policy;
