@@ -143,6 +143,44 @@ struct Stage {
     static constexpr int kSfBase = 256, kSfBufferCols = 64, kSfWeights = 16;
 };
 
+// Items that do not fill a last round of all blocks are cut into narrower ones, of 128 or 64 weight rows, where that ends
+// sooner.  What a K block costs is the bytes it brings in (60 bytes per cycle and SM), and the token rows come with
+// every width, so a narrow item is dearer per result but done in less time: the down product of a dense MLP of 3,807 rows
+// is 300 items on 148 SMs, two rounds and four items over; one of 64 rows is 10 items.
+struct Items {
+    int full;          // items of 256 weight rows, whole rounds of them
+    int parts;         // pieces per item after those: 1, 2 or 4
+    int total;         // full items and pieces
+};
+__device__ __forceinline__ Items share_out(int items, int blocks) {
+    Items s;
+    s.full = items / blocks * blocks;
+    const int over = items - s.full;
+    s.parts = 1;
+    int best = over > 0 ? Stage::kBytes : 0;
+#pragma unroll
+    for (int parts = 2; parts <= 4; parts *= 2) {
+        const int bytes = kWRows / parts * kBlockKBytes + kSfSlab + kTok * kBlockKBytes + kSfSlab;
+        const int cost = (over * parts + blocks - 1) / blocks * bytes;
+        if (cost < best) { best = cost; s.parts = parts; }
+    }
+    s.total = s.full + over * s.parts;
+    return s;
+}
+struct Piece {
+    Item it;
+    int width;         // weight rows: 256, 128 or 64
+    int first;         // the first of them within the item's 256
+};
+__device__ __forceinline__ bool decode_piece(const TcParams& p, const RouteTable& t, const Items& items, int index, Piece* piece) {
+    const int parts = index < items.full ? 1 : items.parts;
+    const int past = index - items.full;
+    const int item = parts == 1 ? index : items.full + past / parts;
+    piece->width = kWRows / parts;
+    piece->first = parts == 1 ? 0 : past % parts * piece->width;
+    return decode_item<kTok>(p, t, item, &piece->it);
+}
+
 // MODE 0: gate/up + SwiGLU + re-quantisation; p.m_tiles row tiles of 128 intermediate rows (gate and up rows of each).
 // MODE 1: one matrix, BF16 rows out; p.m_tiles pairs of the bank's 128-row tiles.
 // Roles as in expert_tc.cu: producer warp, MMA warp, sixteen epilogue warps; items (128-row token tile, weight tile).
@@ -198,7 +236,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
     tc_fence_after();
     pdl_launch_dependents();
     const std::uint32_t tmem_base = *tmem_slot_ptr;
-    const int total_items = route_table.prefix[route_table.active_count] * p.m_tiles;       // the prefix counts 128-row slabs here
+    const Items items = share_out(route_table.prefix[route_table.active_count] * p.m_tiles, gridDim.x);    // the prefix counts 128-row slabs here
+    const int total_items = items.total;
     auto give_up = [&]() {
         *abort_ptr = 1;
         atomicCAS(p.status, kStatusOk, kStatusWaitExpired);
@@ -209,8 +248,10 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
             int stage = 0;
             std::uint32_t phase = 0;
             for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
-                Item it;
-                if (!decode_item<kTok>(p, route_table, item, &it)) continue;
+                Piece piece;
+                if (!decode_piece(p, route_table, items, item, &piece)) continue;
+                const Item& it = piece.it;
+                const int half = piece.first / kTileM;          // narrow pieces: which of the two boxes
                 // token rows beyond the tile's last one are not loaded: their lanes compute on what the stage held
                 // before, and nothing reads them
                 const int boxes = (it.valid + 31) >> 5;
@@ -218,21 +259,32 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1U)) { give_up(); break; }
                     const std::uint32_t st = base + stage * Stage::kBytes;
-                    mbar_arrive_expect_tx(weight_bar(stage), kChunkBytes);
-                    if constexpr (MODE == 0) {
-                        bulk_load(st + Stage::kOffW,
-                                  p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes,
-                                  kChunkBytes, weight_bar(stage));
-                    } else {
-                        // K block kb of two neighbouring row tiles: a box and a scale slab from either tile's chunk
+                    if (piece.width == kWRows) {
+                        mbar_arrive_expect_tx(weight_bar(stage), kChunkBytes);
+                        if constexpr (MODE == 0) {
+                            bulk_load(st + Stage::kOffW,
+                                      p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes,
+                                      kChunkBytes, weight_bar(stage));
+                        } else {
+                            // K block kb of two neighbouring row tiles: a box and a scale slab from either tile's chunk
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const std::uint8_t* chunk = p.bank.g2 +
-                                ((static_cast<std::size_t>(it.entry) * p.m_tiles * 2 + it.m_tile * 2 + h) * (k_blocks / 2) + (kb >> 1)) * kChunkBytes;
-                            bulk_load(st + Stage::kOffW + h * kChunkBox, chunk + (kb & 1) * kChunkBox, kChunkBox, weight_bar(stage));
-                            bulk_load(st + Stage::kOffSfW + h * kSfSlab, chunk + kChunkScaleOffset + (kb & 1) * kChunkScaleBytes, kSfSlab,
-                                      weight_bar(stage));
+                            for (int h = 0; h < 2; ++h) {
+                                const std::uint8_t* chunk = p.bank.g2 +
+                                    ((static_cast<std::size_t>(it.entry) * p.m_tiles * 2 + it.m_tile * 2 + h) * (k_blocks / 2) + (kb >> 1)) * kChunkBytes;
+                                bulk_load(st + Stage::kOffW + h * kChunkBox, chunk + (kb & 1) * kChunkBox, kChunkBox, weight_bar(stage));
+                                bulk_load(st + Stage::kOffSfW + h * kSfSlab, chunk + kChunkScaleOffset + (kb & 1) * kChunkScaleBytes, kSfSlab,
+                                          weight_bar(stage));
+                            }
                         }
+                    } else {
+                        const int box = MODE == 0 ? half : kb & 1;
+                        const std::uint8_t* chunk = MODE == 0
+                            ? p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes
+                            : p.bank.g2 + ((static_cast<std::size_t>(it.entry) * p.m_tiles * 2 + it.m_tile * 2 + half) * (k_blocks / 2) + (kb >> 1)) * kChunkBytes;
+                        const std::uint32_t bytes = static_cast<std::uint32_t>(piece.width) * kBlockKBytes;
+                        mbar_arrive_expect_tx(weight_bar(stage), bytes + kSfSlab);
+                        bulk_load(st + Stage::kOffW, chunk + box * kChunkBox + piece.first % kTileM * kBlockKBytes, bytes, weight_bar(stage));
+                        bulk_load(st + Stage::kOffSfW, chunk + kChunkScaleOffset + box * kChunkScaleBytes, kSfSlab, weight_bar(stage));
                     }
                     mbar_arrive_expect_tx(token_bar(stage), boxes * (32 * kBlockKBytes) + kSfSlab);
                     if (boxes == 4) {
@@ -252,11 +304,13 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
             int stage = 0;
             std::uint32_t phase = 0;
             std::uint32_t accum_phase = 0;
-            constexpr std::uint32_t idesc = idesc_nvf4(kTok, kWRows);
             int sf_buffer = 0;
             for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
-                Item it;
-                if (!decode_item<kTok>(p, route_table, item, &it)) continue;
+                Piece piece;
+                if (!decode_piece(p, route_table, items, item, &piece)) continue;
+                const std::uint32_t idesc = idesc_nvf4(kTok, piece.width);
+                // 64 rows from the middle of a box: their scale factors sit two TMEM columns further
+                const std::uint32_t quarter = static_cast<std::uint32_t>(piece.first % kTileM) >> 5;
                 bool ok = true;
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!mbar_wait(weight_bar(stage), phase) || !mbar_wait(token_bar(stage), phase)) {
@@ -274,13 +328,13 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                         tc_copy_sf(sf_t + k * 4, desc_scale_atom(st + Stage::kOffSfT + k * 512));
                         // a 256-row operand takes eight columns per K step: its rows 0..127, then 128..255
                         tc_copy_sf(sf_w + k * 8, desc_scale_atom(st + Stage::kOffSfW + k * 512));
-                        tc_copy_sf(sf_w + k * 8 + 4, desc_scale_atom(st + Stage::kOffSfW + kSfSlab + k * 512));
+                        if (piece.width == kWRows) tc_copy_sf(sf_w + k * 8 + 4, desc_scale_atom(st + Stage::kOffSfW + kSfSlab + k * 512));
                     }
                     const std::uint64_t a_desc = desc_k_major_sw128(st + Stage::kOffT);
                     const std::uint64_t b_desc = desc_k_major_sw128(st + Stage::kOffW);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        mma_nvf4(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, sf_t + k * 4, sf_w + k * 8, kb > 0 || k > 0);
+                        mma_nvf4(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, sf_t + k * 4, sf_w + k * 8 + quarter, kb > 0 || k > 0);
                     }
                     tc_commit(empty_bar(stage));
                     sf_buffer ^= 1;
@@ -298,12 +352,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
         const int row = quarter * 32 + lane;                // token row of the tile
         std::uint32_t accum_phase = 0;
         for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
-            Item it;
-            if (!decode_item<kTok>(p, route_table, item, &it)) continue;
+            Piece piece;
+            if (!decode_piece(p, route_table, items, item, &piece)) continue;
+            const Item& it = piece.it;
             if (!mbar_wait(accum_full, accum_phase)) { give_up(); break; }
             accum_phase ^= 1U;
             tc_fence_after();
-            const bool mine = quarter * 32 < it.valid;      // warp uniform
+            const bool mine = quarter * 32 < it.valid && group * 64 < piece.width;      // warp uniform
+            const int column64 = piece.first + group * 64;  // of the item's 256 weight rows
             const int pp = it.pp0 + row;
             if constexpr (MODE == 0) {
                 std::uint32_t first[32], second[32];
@@ -315,14 +371,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(accum_empty);
-                if (row < it.valid) {
+                if (mine && row < it.valid) {
                     const float alpha_g = p.bank.alpha[it.entry * 3 + 0];
                     const float alpha_u = p.bank.alpha[it.entry * 3 + 1];
                     const int inter = p.m_total;
                     std::uint32_t scale0, scale1;
                     const uint2 q0 = swiglu_block16(first, first + 16, alpha_g, alpha_u, p.quant_scale, &scale0);
                     const uint2 q1 = swiglu_block16(second, second + 16, alpha_g, alpha_u, p.quant_scale, &scale1);
-                    const int column = it.m_tile * kTileM + group * 32;
+                    const int column = it.m_tile * kTileM + column64 / 2;
                     *reinterpret_cast<uint4*>(p.hq + static_cast<std::size_t>(pp) * (inter / 2) + (column >> 1)) = make_uint4(q0.x, q0.y, q1.x, q1.y);
                     const int sf_col = column >> 4;         // even: the two bytes are neighbours in the tiled layout
                     std::uint8_t* sf = p.hs + (static_cast<std::size_t>(pp >> 7) * (inter / 64) + (sf_col >> 2)) * 512 + (pp & 31) * 16 +
@@ -339,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                 if (lane == 0) mbar_arrive(accum_empty);
                 if (!mine) continue;
                 const long my_row = p.out_row != nullptr ? (row < it.valid ? p.out_row[it.dense0 + row] : 0) : pp;
-                store_rows64(p.out + static_cast<std::size_t>(it.m_tile) * kWRows + group * 64, p.m_total, my_row, it.valid - quarter * 32, w);
+                store_rows64(p.out + static_cast<std::size_t>(it.m_tile) * kWRows + column64, p.m_total, my_row, it.valid - quarter * 32, w);
             }
         }
     }

@@ -1,6 +1,6 @@
-"""The dense MLP of a few rows (its own pair of kernels up to 32 rows) against the CPU oracle.
+"""The dense MLP of a few rows (its own pair of kernels up to 20 rows) against the CPU oracle.
 
-Row counts sit on both sides of the column counts of the MMA (16, 32) and of the hand-over to the large-batch kernels;
+Row counts sit on both sides of the column count of the MMA (16) and of the hand-over to the large-batch kernels (20);
 shapes cover a K extent of the down product that its parts do not divide, fewer K blocks than parts, one part per tile
 (hidden 4096 has 32 tiles for 148 SMs: 4 parts) and the model's own MLP.  Both products accumulate in FP32 over FP4
 operands, so a result differs from the oracle's only where another order of the sums moves a SwiGLU value to the
@@ -43,7 +43,7 @@ def test_dense_few_rows_against_the_oracle(cuda, pkg, orc, hidden, inter):
     want = orc.bf16_to_f32(orc.dense_forward(_u16(x), np.stack(packed_np), np.stack(scales_np), np.array(alphas, np.float32),
                                              hidden, inter))
     plan = pkg.MoePlan(max_rows=most, hidden=hidden, intermediate=inter)
-    for rows in (1, 2, 15, 16, 17, 31, 32, 33):
+    for rows in (1, 2, 15, 16, 17, 20, 21, 31, 32, 33):
         if rows > most:
             continue
         out = torch.full((rows, hidden), float("nan"), dtype=torch.bfloat16, device="cuda")
@@ -55,5 +55,41 @@ def test_dense_few_rows_against_the_oracle(cuda, pkg, orc, hidden, inter):
         assert torch.equal(first.view(torch.int16), out.view(torch.int16))      # the parts are added in a fixed order
         got = orc.bf16_to_f32(_u16(out))
         assert np.linalg.norm(got - want[:rows]) <= 1e-2 * np.linalg.norm(want[:rows]), rows
+    plan.close()
+    bank.close()
+
+
+@pytest.mark.parametrize("hidden,inter", [(512, 1536), (768, 2048), (2560, 9216)])
+def test_dense_large_batch_equals_its_rows_sent_a_few_at_a_time(cuda, pkg, hidden, inter):
+    """The large-batch kernel cuts the items of its last round into pieces of 128 or 64 weight rows; 21 to 1,300 rows reach
+    every width at one shape or another.  Both sides accumulate the same FP4 products in FP32, in another order."""
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(inter)
+    entries = []
+    for rows, cols in ((inter, hidden), (inter, hidden), (hidden, inter)):
+        w = torch.empty((rows, cols), dtype=torch.float32, device="cuda").normal_(0, 0.02, generator=g).to(torch.bfloat16)
+        packed = torch.empty((rows, cols // 2), dtype=torch.uint8, device="cuda")
+        linear = torch.empty((rows, cols // 16), dtype=torch.uint8, device="cuda")
+        alpha = torch.empty(1, dtype=torch.float32, device="cuda")
+        pkg.nvfp4_pack_weight(w, packed, linear, alpha)
+        swizzled = torch.empty(pkg.nvfp4_swizzled_scale_bytes(rows, cols // 16), dtype=torch.uint8, device="cuda")
+        pkg.nvfp4_swizzle_scales(linear, swizzled, rows, cols // 16)
+        entries.append((packed, swizzled, alpha))
+    bank = pkg.ExpertBank(entries, first_expert=0, local_experts=0, hidden=hidden,
+                          intermediate=inter)
+    most = 1300
+    x = torch.empty((most, hidden), device="cuda").normal_(0, 1, generator=g).to(torch.bfloat16)
+    plan = pkg.MoePlan(max_rows=most, hidden=hidden, intermediate=inter)
+    want = torch.empty_like(x)
+    for r in range(0, most, 20):
+        n = min(20, most - r)
+        pkg.run_dense_rows(plan, bank, x[r:r + n], want[r:r + n], n)
+    for rows in (21, 33, 64, 128, 129, 400, 640, 1300):
+        out = torch.full((rows, hidden), float("nan"), dtype=torch.bfloat16, device="cuda")
+        pkg.run_dense_rows(plan, bank, x[:rows], out, rows)
+        torch.cuda.synchronize()
+        assert plan.status() == 0
+        got, ref = out.double(), want[:rows].double()
+        assert float((got - ref).norm()) <= 1e-2 * float(ref.norm()), rows
     plan.close()
     bank.close()
