@@ -495,16 +495,16 @@ int p92b_dense_forward(p92b_plan* plan, const p92b_bank* bank, const uint16_t* i
     if (dense_few_rows_applies(plan, rows)) return launch_dense_few_rows(plan, bank, input, output, rows, stream, pdl);
     // the MLP is the bank's last entry; every row is "routed" to it and to nothing else, so its rows sit at padded
     // positions 0 .. rows-1 in token order and the down product can write the caller's rows directly
-    cudaError_t st = launch_dense_lists(plan, rows, tc_tile_rows(rows), stream, pdl);
+    // 21 to 32 rows take the kernels of larger batches, with the tokens on the M side: 26 us a layer against 25 to 33
+    const int tile_class = rows > 20 ? std::max(rows, 33) : rows;
+    cudaError_t st = launch_dense_front(plan, input, rows, tc_tile_rows(tile_class), stream, pdl);
     if (st != cudaSuccess) return st;
-    st = launch_quantize_rows_to_pp(input, nullptr, plan->xq_pp, plan->xs_sw, rows, plan->hidden, stream, pdl);
-    if (st != cudaSuccess) return st;
-    st = launch_experts_tc(plan, bank, rows, false, stream, pdl);
+    st = launch_experts_tc(plan, bank, tile_class, false, stream, pdl);
     if (st != cudaSuccess) return st;
     TcIo io {};
     io.down_out = output;
-    st = launch_experts_tc(plan, bank, rows, true, stream, pdl, &io);
-    plan->last_launches += 3;
+    st = launch_experts_tc(plan, bank, tile_class, true, stream, pdl, &io);
+    plan->last_launches += 2;
     return st;
 }
 

@@ -499,12 +499,13 @@ cudaError_t launch_gather_quantized_rows(const std::uint8_t* packed, const std::
                                          bool pdl = false);
 cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int rows, bool down,
                               cudaStream_t stream, bool pdl = false, const TcIo* io = nullptr);
-// The dense MLP of up to 32 rows (dense_rows.cu).
+// The dense MLP of up to 20 rows (dense_rows.cu).
 bool dense_few_rows_applies(const p92b_plan* plan, int rows);
 cudaError_t launch_dense_few_rows(p92b_plan* plan, const p92b_bank* bank, const std::uint16_t* x, std::uint16_t* out, int rows,
                                   cudaStream_t stream, bool pdl);
-// Routing lists of a call in which every row goes to the bank's last entry only (the dense MLP).
-cudaError_t launch_dense_lists(p92b_plan* plan, int rows, int tile_rows, cudaStream_t stream, bool pdl = false);
+// Routing lists of a call in which every row goes to the bank's last entry only (the dense MLP), and its rows quantised.
+cudaError_t launch_dense_front(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream,
+                               bool pdl = false);
 // Pipelined host-buffer calls (moe_api.cu).  Three streams: the caller's (the block), one for rows coming in, one
 // for rows going out; two sets of staging rows used alternately.  begin: the copy-in of this call is enqueued on
 // the plan's in-stream (after the block of call n-2 has read the set) and `stream` is made to wait for it and for

@@ -493,29 +493,60 @@ __global__ void __launch_bounds__(256) route_fused_kernel(
     }
 }
 
-// Lists for a call without routing: all `rows` rows belong to entry 256 (the bank's last entry), which starts at
-// padded position 0; no routed expert has rows.
-__global__ void __launch_bounds__(256) dense_lists_kernel(RouteLists lists, int rows) {
+// Front of a call without routing (the dense MLP): all `rows` rows belong to entry 256 (the bank's last entry), which
+// starts at padded position 0, and no routed expert has rows; block 0 writes these lists, and every block quantises its
+// rows in place of the permutation and quantisation kernels.  WARPS per row: 8 while one per row would leave most of the
+// chip idle (33 to 64 rows: lists and a warp per row took 7 us in two kernels), else 1.
+template <int WARPS>
+__global__ void __launch_bounds__(256) dense_front_kernel(RouteLists lists, int rows, const std::uint16_t* __restrict__ x,
+                                                          std::uint8_t* __restrict__ xq, std::uint8_t* __restrict__ xs, int hidden,
+                                                          float quant_scale) {
     pdl_launch_dependents();
     pdl_wait();
-    const int e = threadIdx.x;
-    lists.counts[e] = 0;
-    lists.offsets[e] = 0;
-    lists.pp_off[e] = 0;
-    if (e == 0) {
-        lists.counts[kExperts] = rows;
-        lists.offsets[kExperts] = 0;
-        lists.offsets[kExperts + 1] = rows;
-        lists.active[0] = kExperts;
-        *lists.active_count = 1;
-        lists.pp_off[kExperts] = 0;
-        lists.pp_off[kExperts + 1] = (rows + lists.pad_align - 1) / lists.pad_align * lists.pad_align;
-        lists.tile_prefix[0] = 0;
-        lists.tile_prefix[1] = (rows + lists.tile_rows - 1) / lists.tile_rows;
-        if (lists.tile_prefix_wide != nullptr) {
-            lists.tile_prefix_wide[0] = 0;
-            lists.tile_prefix_wide[1] = (rows + lists.tile_rows_wide - 1) / lists.tile_rows_wide;
+    if (blockIdx.x == 0) {
+        const int e = threadIdx.x;
+        lists.counts[e] = 0;
+        lists.offsets[e] = 0;
+        lists.pp_off[e] = 0;
+        if (e == 0) {
+            lists.counts[kExperts] = rows;
+            lists.offsets[kExperts] = 0;
+            lists.offsets[kExperts + 1] = rows;
+            lists.active[0] = kExperts;
+            *lists.active_count = 1;
+            lists.pp_off[kExperts] = 0;
+            lists.pp_off[kExperts + 1] = (rows + lists.pad_align - 1) / lists.pad_align * lists.pad_align;
+            lists.tile_prefix[0] = 0;
+            lists.tile_prefix[1] = (rows + lists.tile_rows - 1) / lists.tile_rows;
+            if (lists.tile_prefix_wide != nullptr) {
+                lists.tile_prefix_wide[0] = 0;
+                lists.tile_prefix_wide[1] = (rows + lists.tile_rows_wide - 1) / lists.tile_rows_wide;
+            }
         }
+    }
+    const int warp = threadIdx.x >> 5;
+    const int row = (blockIdx.x * 8 + warp) / WARPS;
+    if (row >= rows) return;
+    const int blocks = hidden / 16;
+    const std::size_t col_blocks = static_cast<std::size_t>(blocks / 4);              // hidden is a multiple of 128
+    std::uint8_t* row_q = xq + static_cast<std::size_t>(row) * (hidden / 2);
+    std::uint8_t* row_s = xs + (row >> 7) * col_blocks * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+#pragma unroll 2
+    for (int b = warp % WARPS * 32 + (threadIdx.x & 31); b < blocks; b += 32 * WARPS) {
+        const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<std::size_t>(row) * hidden + b * 16);
+        const uint4 lo = __ldg(src);
+        const uint4 hi = __ldg(src + 1);
+        const std::uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            v[2 * i] = __uint_as_float(words[i] << 16);
+            v[2 * i + 1] = __uint_as_float(words[i] & 0xffff0000U);
+        }
+        std::uint8_t scale_bits;
+        const uint2 packed = quantize_block16(v, quant_scale, &scale_bits);
+        *reinterpret_cast<uint2*>(row_q + b * 8) = packed;
+        row_s[(b >> 2) * 512 + (b & 3)] = scale_bits;
     }
 }
 
@@ -523,7 +554,7 @@ __global__ void __launch_bounds__(256) dense_lists_kernel(RouteLists lists, int 
 
 int route_fused_max_rows() { return kFusedMaxRows; }
 
-cudaError_t launch_dense_lists(p92b_plan* plan, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
+cudaError_t launch_dense_front(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
     RouteLists lists {};
     lists.counts = plan->counts;
     lists.offsets = plan->offsets;
@@ -539,7 +570,9 @@ cudaError_t launch_dense_lists(p92b_plan* plan, int rows, int tile_rows, cudaStr
     lists.tile_prefix_wide = wide ? plan->tile_prefix_wide : nullptr;
     plan->wide_rows = wide ? 128 : 0;
     plan->last_launches += 1;
-    return launch_kernel(dense_lists_kernel, dim3(1), dim3(256), 0, stream, pdl, lists, rows);
+    const bool few = rows <= 1024;
+    return launch_kernel(few ? dense_front_kernel<8> : dense_front_kernel<1>, dim3(few ? rows : (rows + 7) / 8), dim3(256), 0, stream,
+                         pdl, lists, rows, x, plan->xq_pp, plan->xs_sw, plan->hidden, 1.0F);
 }
 
 cudaError_t launch_route_fused(p92b_plan* plan, const float* bias, float routed_scale, const std::uint16_t* x,
