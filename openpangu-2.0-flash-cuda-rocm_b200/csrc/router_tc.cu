@@ -6,8 +6,8 @@
 // those near the top-8 boundary matter.  Two kernels:
 //
 //   1. logits_tc_kernel      approximate logits of every (token, expert) as one BF16 x BF16 -> FP32 product on the
-//                            5th-generation tensor cores (tcgen05.mma kind::f16, M = 128 tokens, N = 64 experts per
-//                            block, operands by TMA, accumulator in TMEM), and beside it ||w_e||_2 of the 256 router
+//                            5th-generation tensor cores (tcgen05.mma kind::f16, M = 128 tokens, N = 64 to 256 experts
+//                            per block, operands by TMA, accumulator in TMEM), and beside it ||w_e||_2 of the 256 router
 //                            rows (the error bound below needs them);
 //   2. route_repair_kernel   one warp per token: corrected scores from the approximate logits, the approximate 8th
 //                            best, the candidate set = every expert whose approximate score is within 2 delta of it,
@@ -40,14 +40,17 @@ using namespace ptx;
 namespace {
 
 constexpr int kTokTile = 128;                 // M: tokens per block (TMEM lanes)
-constexpr int kExpTile = 64;                  // N: experts per block
 constexpr int kKBytes = 128;                  // one swizzle row: 64 BF16
 constexpr int kStageA = kTokTile * kKBytes;   // 16 KB
-constexpr int kStageB = kExpTile * kKBytes;   // 8 KB
-constexpr int kStageBytes = kStageA + kStageB;
-constexpr int kLogitStages = 8;
+// N: experts per block, 64, 128 or 256.  A block is bound by the bytes it brings in, and the token rows come once per expert
+// tile: with 64 experts a block 16,384 tokens took 50 us, four rounds of blocks that read every row four times.
+template <int N>
+struct Logits {
+    static constexpr int kStageBytes = kStageA + N * kKBytes;          // 24, 32 or 48 KB
+    static constexpr int kStages = 196 * 1024 / kStageBytes;          // 8, 6 or 4
+    static constexpr int kSmem = kStages * kStageBytes + 1024;
+};
 constexpr int kLogitThreads = 192;            // producer warp, MMA warp, four epilogue warps
-constexpr int kLogitSmem = kLogitStages * kStageBytes + 1024;
 constexpr float kLogitBound = 1.0F / 16384.0F;
 constexpr int kMaxCandidates = 24;
 
@@ -108,6 +111,7 @@ __device__ __forceinline__ void row_norm(const std::uint16_t* __restrict__ w, fl
     if (lane == 0) norms[e] = sqrtf(s) * 1.0001F;             // rounded up a little: it feeds a bound
 }
 
+template <int kExpTile>
 __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                      const __grid_constant__ CUtensorMap map_w,
                                                                      float* __restrict__ logits, int rows, int hidden,
@@ -117,6 +121,7 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
     // gridDim.z > 1: block z takes a slice of the K blocks and writes its partial sums to slice z of `logits`
     // ([gridDim.z][rows][256]); the repair kernel adds the slices (small batches: 4 blocks would otherwise walk all of
     // K one after the other while 144 SMs idle)
+    constexpr int kLogitStages = Logits<kExpTile>::kStages, kStageBytes = Logits<kExpTile>::kStageBytes;
     extern __shared__ std::uint8_t smem_raw[];
     __shared__ __align__(8) std::uint64_t barrier_words[2 * kLogitStages + 1];
     __shared__ std::uint32_t tmem_slot_word;
@@ -195,7 +200,7 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
             if (ok && k_blocks > 0) tc_commit(accum_bar);
         }
     } else {
-        // while the products run, the epilogue warps take the norms of the 64 router rows, shared out over the blocks of
+        // while the products run, the epilogue warps take the norms of the tile's router rows, shared out over the blocks of
         // this expert tile (a kernel of its own in front of this one cost the chain 2 us)
         const int sharers = static_cast<int>(gridDim.x * gridDim.z) * 4;
         for (int i = static_cast<int>(blockIdx.x * gridDim.z + blockIdx.z) * 4 + (warp - 2); i < kExpTile; i += sharers) {
@@ -534,16 +539,26 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     }
     CUtensorMap map_x, map_w;
     cudaError_t st = make_operand_map(&map_x, x, static_cast<std::size_t>(rows), static_cast<std::size_t>(hidden) * 2, kTokTile);
-    if (st == cudaSuccess) st = make_operand_map(&map_w, router_w, kExperts, static_cast<std::size_t>(hidden) * 2, kExpTile);
+    // the expert tile that brings the fewest bytes into the busiest SM
+    const int token_tiles = (rows + kTokTile - 1) / kTokTile;
+    int expert_tile = 64;
+    int least = 0;
+    for (int n = 64; n <= 256; n *= 2) {
+        const int cost = (token_tiles * (kExperts / n) + plan->sm_count - 1) / plan->sm_count * (kStageA + n * kKBytes);
+        if (least == 0 || cost < least) { least = cost; expert_tile = n; }
+    }
+    if (st == cudaSuccess) st = make_operand_map(&map_w, router_w, kExperts, static_cast<std::size_t>(hidden) * 2, expert_tile);
     if (st != cudaSuccess) return cudaErrorNotSupported;
-    if ((st = ensure_dynamic_smem<logits_tc_kernel>(kLogitSmem)) != cudaSuccess) return st;
+    if ((st = ensure_dynamic_smem<logits_tc_kernel<64>>(Logits<64>::kSmem)) != cudaSuccess) return st;
+    if ((st = ensure_dynamic_smem<logits_tc_kernel<128>>(Logits<128>::kSmem)) != cudaSuccess) return st;
+    if ((st = ensure_dynamic_smem<logits_tc_kernel<256>>(Logits<256>::kSmem)) != cudaSuccess) return st;
     const bool in_registers = hidden == 32 * kChunksInRegisters;
     // small batches: K split over blocks of the logits kernel, and a block of eight warps per token in the repair
     const bool may_split = plan->logit_partials != nullptr && plan->max_rows >= rows && std::getenv("P92B_ROUTER_NO_SPLIT") == nullptr;
     const bool small = rows <= kRouterWideRows && may_split;
     const int k_blocks = hidden * 2 / kKBytes;
     // as many slices as fill the chip: 8 up to 512 rows, 4 up to 1,024, 2 up to 2,304 (512 rows, 16 blocks: 12 us)
-    const int tiles = (rows + kTokTile - 1) / kTokTile * (kExperts / kExpTile);
+    const int tiles = token_tiles * (kExperts / expert_tile);
     const int wanted = may_split && rows <= kRouterSplitRows
                            ? std::max(1, std::min({kRouterSplits, plan->sm_count / tiles, kRouterPartialRows / rows})) : 1;
     const int per_split = (k_blocks + wanted - 1) / wanted;
@@ -562,8 +577,9 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     if (st != cudaSuccess) return st;
     float* norms = plan->w_norms;
     float* approx_out = splits > 1 ? plan->logit_partials : plan->logits;
-    st = launch_kernel(logits_tc_kernel, dim3((rows + kTokTile - 1) / kTokTile, kExperts / kExpTile, splits), dim3(kLogitThreads),
-                       kLogitSmem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status, router_w, norms,
+    const auto kernel = expert_tile == 64 ? logits_tc_kernel<64> : expert_tile == 128 ? logits_tc_kernel<128> : logits_tc_kernel<256>;
+    const int smem = expert_tile == 64 ? Logits<64>::kSmem : expert_tile == 128 ? Logits<128>::kSmem : Logits<256>::kSmem;
+    st = launch_kernel(kernel, dim3(token_tiles, kExperts / expert_tile, splits), dim3(kLogitThreads), smem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status, router_w, norms,
                        in_registers ? plan->w_chains : nullptr);
     if (st != cudaSuccess) return st;
     const float* partials = splits > 1 ? plan->logit_partials : nullptr;
