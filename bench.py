@@ -553,7 +553,7 @@ class SingleGpu:
         nvfp4_peak = yardstick if yardstick else 4 * pk["bf16_tflops"]
         t_flops = rows * FLOPS_PER_TOKEN / (nvfp4_peak * 1e12)
         ratios = ncu_ratios()
-        gu = ratios.get("expert_gu_pair_kernel")
+        gu = ratios.get("expert_rows_kernel<0>")
         gu_bytes = (distinct + 1) * 2 * (EXPERT_BYTES // 3) + rows * (HIDDEN // 2 + HIDDEN // 16) + real * (INTER // 2 + INTER // 16)
         gu_us = stage_us["gate_up_swiglu"]
         gu_gbs = gu_bytes / (gu_us * 1e-6) / 1e9
@@ -575,7 +575,7 @@ class SingleGpu:
                                                      "was refused by this torch build); vendor figure 9000"),
                                "flops_per_token": FLOPS_PER_TOKEN, "tensor_pipe_pct_ncu": gu["tensor_pipe_pct"] if gu else None,
                                "tensor_pipe_capture": gu["capture"] if gu else None},
-            "roofline": {"bound": "hbm", "kernel": "expert_gu_pair_kernel", "achieved": gu_gbs, "peak": pk["hbm_gbs"],
+            "roofline": {"bound": "hbm", "kernel": "expert_rows_kernel<0>", "achieved": gu_gbs, "peak": pk["hbm_gbs"],
                          "unit": "GB/s", "frac": gu_gbs / pk["hbm_gbs"], "peak_source": pk["source"], "bytes_per_launch": gu_bytes,
                          "us_per_launch": gu_us, "traffic": gu_bytes * gu["traffic_over_algorithmic"] if gu else None,
                          "traffic_source": (f"measured DRAM bytes / algorithmic bytes = {gu['traffic_over_algorithmic']} in the ncu "
