@@ -565,7 +565,7 @@ class SingleGpu:
             "padding_waste": {"padded_rows_over_real_rows": padded / real, "padded_rows": padded, "real_rows": real,
                               "mma_rows_over_real_rows_64_row_tiles": tiles64 / real,
                               "note": "every expert's rows start on a multiple of 128 padded positions (address space only); "
-                                      "the products run on 64-row token tiles, whose last tile per expert is partly empty"},
+                                      "both products run on 128-row token tiles, whose last tile per expert is partly empty"},
             "roofline_layer": {"t_bytes_us": t_bytes * 1e6, "t_flops_us": t_flops * 1e6,
                                "frac_of_max": max(t_bytes, t_flops) / (ms * 1e-3),
                                "nvfp4_dense_peak_tflops": nvfp4_peak,
