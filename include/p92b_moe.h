@@ -12,7 +12,9 @@
  *   - NVFP4 = two E2M1 values per byte, even element in the low nibble, one
  *     E4M3 scale per 16 elements along K, one FP32 per-tensor scale (alpha);
  *   - calls are asynchronous on `stream` (a cudaStream_t passed as void*; NULL
- *     is the default stream) and use the CURRENT device;
+ *     is the default stream) and use the CURRENT device; they are ordered like
+ *     any work of a stream: every array that a call reads, parameters included,
+ *     may be the output of the call queued just before it;
  *   - the return value is a cudaError_t: 0 success, cudaErrorInvalidValue for
  *     bad arguments, cudaErrorMemoryAllocation, cudaErrorNotSupported, or the
  *     launch error reported right after the launch

@@ -175,11 +175,20 @@ __global__ void __launch_bounds__(kEpThreads, 1) moe_decode_ep_kernel(const __gr
         tmem_alloc(smem_u32(&tmem_slot_word), kTmemCols);
         tmem_relinquish();
     }
-    // router rows and bias do not depend on the kernel upstream
     const int my_experts = block + grid < kExperts ? 2 : (block < kExperts ? 1 : 0);
     std::uint16_t* w_rows = reinterpret_cast<std::uint16_t*>(smem_raw + (base - smem_u32(smem_raw)));
     std::uint16_t* x_rows = w_rows + 2 * hidden;
     const int vec_per_row = hidden / 8;
+    // Router rows and bias may, like the token rows, be the output of the kernel just before this one: in front of the wait
+    // they only start on their way to the L2, which that kernel's stores still reach.
+    const int lines_per_row = hidden / 64;
+    for (int i = threadIdx.x; i < my_experts * lines_per_row; i += kEpThreads) {
+        const int r = i / lines_per_row;
+        prefetch_l2(p.router_w + static_cast<std::size_t>(block + r * grid) * hidden + (i - r * lines_per_row) * 64);
+    }
+    if (block == grid - 1 && threadIdx.x < kExperts / 32) prefetch_l2(p.bias + threadIdx.x * 32);
+    pdl_wait();
+    pdl_launch_dependents();
     for (int i = threadIdx.x; i < my_experts * vec_per_row; i += kEpThreads) {
         const int r = i / vec_per_row;
         const int c = i - r * vec_per_row;
@@ -187,8 +196,6 @@ __global__ void __launch_bounds__(kEpThreads, 1) moe_decode_ep_kernel(const __gr
                      reinterpret_cast<const uint4*>(p.router_w + static_cast<std::size_t>(block + r * grid) * hidden) + c);
     }
     for (int e = threadIdx.x; e < kExperts; e += kEpThreads) async_copy4(&rt.bias[e], p.bias + e);
-    pdl_wait();
-    pdl_launch_dependents();
     for (int i = threadIdx.x; i < rows * vec_per_row; i += kEpThreads) {
         const int r = i / vec_per_row;
         const int c = i - r * vec_per_row;

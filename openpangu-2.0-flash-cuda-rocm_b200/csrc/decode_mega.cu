@@ -120,13 +120,14 @@ struct Routing {                   // shared-memory copy, identical in every blo
     __align__(16) float bias[kExperts];
 };
 
-// Eight norm weights, one 16-byte load where the pointer allows it.
+// Eight norm weights, one 16-byte load where the pointer allows it.  Ordinary loads: the kernel upstream may have written
+// them, and a read-only load may be moved in front of the wait.
 __device__ __forceinline__ uint4 load_norm_weight(const std::uint16_t* w, bool aligned, int vec) {
-    if (aligned) return __ldg(reinterpret_cast<const uint4*>(w) + vec);
+    if (aligned) return __ldcg(reinterpret_cast<const uint4*>(w) + vec);
     std::uint32_t words[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        words[i] = static_cast<std::uint32_t>(__ldg(w + vec * 8 + 2 * i)) | (static_cast<std::uint32_t>(__ldg(w + vec * 8 + 2 * i + 1)) << 16);
+        words[i] = static_cast<std::uint32_t>(__ldcg(w + vec * 8 + 2 * i)) | (static_cast<std::uint32_t>(__ldcg(w + vec * 8 + 2 * i + 1)) << 16);
     }
     return make_uint4(words[0], words[1], words[2], words[3]);
 }
@@ -210,7 +211,6 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                                             : p.bank.g2 + (entry * g2_chunks + (c - g13_chunks)) * kChunkBytes, kChunkBytes);
         }
     }
-    // the router rows and the bias do not depend on the kernel upstream: fetch them before waiting for it
     const int my_experts = block + grid < kExperts ? 2 : (block < kExperts ? 1 : 0);
     std::uint16_t* w_rows = reinterpret_cast<std::uint16_t*>(smem_raw + (base - smem_u32(smem_raw)));
     // rows 64 bytes further apart than they are long: two neighbouring rows, read side by side by the halves of a warp,
@@ -218,8 +218,20 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     const int row_pitch = hidden + 32;
     std::uint16_t* x_rows = w_rows + 2 * row_pitch;
     const int vec_per_row = hidden / 8;
-    // (asynchronous 16-byte copies: the token rows below are requested behind them without waiting for these, so the
-    // block pays one round trip to the L2 for both, not two)
+    // Everything that the caller owns (token rows, router rows, bias, norm weights) may be the output of the kernel just before
+    // this one, so none of it is read before the wait.  The parameters only start on their way to the L2, which the
+    // stores of that kernel still reach: behind the wait the block then pays one round trip to the L2 for all of them.
+    const int lines_per_row = hidden / 64;
+    for (int i = threadIdx.x; i < my_experts * lines_per_row; i += kMegaThreads) {
+        const int r = i / lines_per_row;
+        prefetch_l2(p.router_w + static_cast<std::size_t>(block + r * grid) * hidden + (i - r * lines_per_row) * 64);
+    }
+    if (block == grid - 1) {
+        if (threadIdx.x < kExperts / 32) prefetch_l2(p.bias + threadIdx.x * 32);
+        if (p.pre_norm_w != nullptr && static_cast<int>(threadIdx.x) < lines_per_row) prefetch_l2(p.pre_norm_w + threadIdx.x * 64);
+    }
+    pdl_wait();
+    pdl_launch_dependents();
     for (int i = threadIdx.x; i < my_experts * vec_per_row; i += kMegaThreads) {
         const int r = i / vec_per_row;
         const int c = i - r * vec_per_row;
@@ -227,18 +239,16 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                      reinterpret_cast<const uint4*>(p.router_w + static_cast<std::size_t>(block + r * grid) * hidden) + c);
     }
     for (int e = threadIdx.x; e < kExperts; e += kMegaThreads) async_copy4(&rt.bias[e], p.bias + e);
-    // a thread below hidden / 8 owns eight columns of every row in the pre-norm: their weights, too, do not depend on upstream
-    const bool norm_thread = static_cast<int>(threadIdx.x) < vec_per_row;
-    uint4 pre_w = make_uint4(0U, 0U, 0U, 0U);
-    if (p.pre_norm_w != nullptr && norm_thread) pre_w = load_norm_weight(p.pre_norm_w, p.norm_w_aligned, threadIdx.x);
-    pdl_wait();                       // the token rows come from the kernel before this one
-    pdl_launch_dependents();
     for (int i = threadIdx.x; i < rows * vec_per_row; i += kMegaThreads) {
         const int r = i / vec_per_row;
         const int c = i - r * vec_per_row;
         async_copy16(reinterpret_cast<uint4*>(x_rows + r * row_pitch) + c,
                      reinterpret_cast<const uint4*>(p.x + static_cast<std::size_t>(r) * hidden) + c);
     }
+    // a thread below hidden / 8 owns eight columns of every row in the pre-norm and holds their weights
+    const bool norm_thread = static_cast<int>(threadIdx.x) < vec_per_row;
+    uint4 pre_w = make_uint4(0U, 0U, 0U, 0U);
+    if (p.pre_norm_w != nullptr && norm_thread) pre_w = load_norm_weight(p.pre_norm_w, p.norm_w_aligned, threadIdx.x);
     // the first tile number is asked for now and used after the routing, the atomic's latency in between; behind the
     // copies, because the store of its result makes the warp wait for the answer
     if (threadIdx.x == 0) first_tile_word = static_cast<int>(atomicAdd(tile_counter, 1U));

@@ -156,6 +156,9 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, std::uint32_t 
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
+// The same for one 128-byte line, from any address in it.
+__device__ __forceinline__ void prefetch_l2(const void* address) { asm volatile("prefetch.global.L2 [%0];" ::"l"(address)); }
+
 // bulk_load with an L2 policy: weights that are read once per launch are marked "evict first", so a
 // 120 MB stream does not push everything else (code, routing tables, token rows) out of the L2.
 __device__ __forceinline__ std::uint64_t l2_policy_evict_first() {
