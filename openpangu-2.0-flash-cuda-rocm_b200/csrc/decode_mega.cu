@@ -14,16 +14,18 @@
 //       every token (cuda/nvfp4_ops.cu:357-433), histogram, stable permutation
 //       (cuda/nvfp4_grouped.cu:117-132), active-expert list; block 0 also writes the
 //       routing products to global memory;
-//   P2  gate/up tiles (64 intermediate rows: one box of mixed gate and up rows) and P3 down tiles (128 output
-//       rows) through ONE TMA ring and one tcgen05 pipeline (same operand formats as expert_tc.cu).  The token side of gate/up is simply all
+//   P2  gate/up tiles (128 intermediate rows, gate and up, or half of them: one box of mixed gate and up rows) and P3
+//       down tiles (128 output rows) through ONE TMA ring and one tcgen05 pipeline (same operand formats as
+//       expert_tc.cu).  The token side of gate/up is simply all
 //       tokens in token order (N=16 columns cost nothing at M=128), so it does not depend
 //       on routing; the epilogue keeps the columns routed to the tile's expert.  A down
-//       tile needs the sixteen gate/up tiles of its expert: per-expert counters, no barrier,
+//       tile needs all gate/up tiles of its expert: per-expert counters, no barrier,
 //       and its weights are already in flight while the producer waits.  Tiles are handed
 //       out dynamically from one device-wide counter, gate/up tiles first, both in expert
-//       order: a block that falls behind simply takes fewer (a gate/up tile is 5 ring
-//       stages, a down tile 2, so the tail is fine-grained).  With one token the 144 gate/up tiles are
-//       one round of the 148 blocks (72 tiles of 128 rows left half the chip idle: 22.0 -> 18.8 us);
+//       order: a block that falls behind simply takes fewer (a gate/up tile is 10 or 5 ring
+//       stages, a down tile 2, so the tail is fine-grained).  With one token the 144 half tiles are
+//       one round of the 148 blocks (72 whole ones leave half the chip idle); with many tokens a tile's fixed
+//       costs count (kHalfTileRows);
 //   P4  weighted combine in slot order + shared expert (cuda/nvfp4_ops.cu:124-142,92-95):
 //       the down epilogue publishes its rows as {two BF16, launch number} words and the
 //       combining threads poll the words they need, so the combine of a token starts when
@@ -55,6 +57,9 @@ constexpr int kMegaWarps = kMegaThreads / 32;
 // with its own, now 1.0 us.
 constexpr int kReplicas = 8;
 constexpr int kEpilogueEnd = 6;                    // first warp behind the epilogue warps
+// Up to here gate/up tiles are halves, above whole ones; us per layer, halves against whole tiles: one token 18.9 / 20.6,
+// two 23.6 / 24.6, three 28.8 / 28.7, four 32.8 / 32.3, eight 52.4 / 51.1, sixteen 88.0 / 84.0.
+constexpr int kHalfTileRows = 3;
 constexpr int kMegaMaxRows = 16;                   // = kN: the token side of every MMA holds them all; the kernel is built
                                                    // for 8 (the decode sizes, leaner loops) and for 16 rows
 constexpr int kN = 16;                             // token columns of every MMA
@@ -145,7 +150,29 @@ __device__ __forceinline__ uint4 normalise8(uint4 x, float inverse, uint4 w) {
     return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-template <int R>
+// SwiGLU of one intermediate row and token, bf16(alpha * sum) for gate and up, and the activation quantiser over the
+// 16 neighbouring rows that the half warp holds: the even lanes get the byte of their row and the next, every lane the scale.
+struct RequantisedPair {
+    std::uint8_t packed, scale;
+};
+__device__ __forceinline__ RequantisedPair swiglu_requant(std::uint32_t gate_sum, std::uint32_t up_sum, float alpha_g, float alpha_u,
+                                                          float quant_scale) {
+    const float gv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(gate_sum) * alpha_g));
+    const float uv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(up_sum) * alpha_u));
+    const float h = bf16_bits_to_float(float_to_bf16_bits((gv / (1.0F + expf(-gv))) * uv));
+    float amax = fabsf(h);
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffU, amax, off));
+    const __nv_fp8_e4m3 scale(amax * (quant_scale / 6.0F));
+    const float decoded = static_cast<float>(scale);
+    const float multiplier = decoded == 0.0F ? 0.0F : quant_scale / decoded;
+    const float q = h * multiplier;
+    const float q_next = __shfl_xor_sync(0xffffffffU, q, 1);
+    return {static_cast<std::uint8_t>(__nv_fp4x2_e2m1(make_float2(q, q_next)).__x), scale.__x};
+}
+
+// R: rows that the kernel is built for; HALF: gate/up tiles are half tiles.
+template <int R, bool HALF>
 __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                       const __grid_constant__ CUtensorMap map_h,
                                                                       const MegaParams p) {
@@ -516,9 +543,11 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     }
     if (threadIdx.x == 0) stamp(3);
     // ------------------------------------------------------------ P2 + P3
-    const int gu_tiles = inter / (kTile / 2);    // 16: one box of a chunk, 64 intermediate rows
+    constexpr int kGuRows = HALF ? kTile / 2 : kTile;
+    constexpr int kGuKind = HALF ? 1 : 0;        // of a gate/up stage in issue_stage: two K blocks of one box, or one of both boxes
+    const int gu_tiles = inter / kGuRows;        // 16 or 8
     const int dn_tiles = hidden / kTile;         // 20
-    const int gu_stages = (hidden / 2) / kKB / 2; // 5 stages per gate/up tile, two K blocks each
+    const int gu_stages = (hidden / 2) / kKB / (HALF ? 2 : 1);
     const int dn_stages = (inter / 2) / kKB / 2; // 2 stages per down tile, two K blocks each
     const int gu_items = abort_word ? 0 : rt.n_active * gu_tiles;
     const int total_items = abort_word ? 0 : rt.n_active * (gu_tiles + dn_tiles);
@@ -560,26 +589,32 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                     if (sequence == 0 && s < 10) stamp(16 + s);
                     mbar_arrive_expect_tx(weight_bar(stage), kWeightTx);
                     if (kind == 0) {
-                        // K blocks 2s and 2s + 1 of one box: the same half of two neighbouring chunks
-                        const std::uint8_t* chunk = p.bank.g13 +
-                            ((static_cast<std::size_t>(entry) * (gu_tiles / 2) + (m_tile >> 1)) * (2 * gu_stages) + 2 * s) * kChunkBytes;
-                        const int half = m_tile & 1;
+                        const std::uint8_t* tile_chunks = p.bank.g13 +
+                            (static_cast<std::size_t>(entry) * (inter / kTile) + m_tile * kGuRows / kTile) * (hidden / 256) * kChunkBytes;
+                        if constexpr (HALF) {
+                            // K blocks 2s and 2s + 1 of one box: the same half of two neighbouring chunks
+                            const std::uint8_t* chunk = tile_chunks + static_cast<std::size_t>(2 * s) * kChunkBytes;
+                            const int half = m_tile & 1;
 #pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            bulk_load_hint(st + k * kChunkBox, chunk + k * kChunkBytes + half * kChunkBox, kChunkBox, weight_bar(stage), stream_policy);
-                            bulk_load_hint(st + kChunkScaleOffset + k * kChunkScaleBytes,
-                                           chunk + k * kChunkBytes + kChunkScaleOffset + half * kChunkScaleBytes, kChunkScaleBytes, weight_bar(stage),
-                                           stream_policy);
+                            for (int k = 0; k < 2; ++k) {
+                                bulk_load_hint(st + k * kChunkBox, chunk + k * kChunkBytes + half * kChunkBox, kChunkBox, weight_bar(stage), stream_policy);
+                                bulk_load_hint(st + kChunkScaleOffset + k * kChunkScaleBytes,
+                                               chunk + k * kChunkBytes + kChunkScaleOffset + half * kChunkScaleBytes, kChunkScaleBytes,
+                                               weight_bar(stage), stream_policy);
+                            }
+                        } else {
+                            bulk_load_hint(st, tile_chunks + static_cast<std::size_t>(s) * kChunkBytes, kChunkBytes, weight_bar(stage), stream_policy);
                         }
                         if (!rows_ready) {
                             if (!wait_counter(p.sync + 0, (p.epoch + 1U) * static_cast<unsigned>(grid))) { give_up(kStatusWaitExpired); ok = false; break; }
                             fence_proxy_async_all();      // ordinary stores of other blocks -> this block's TMA loads
                             rows_ready = true;
                         }
-                        mbar_arrive_expect_tx(token_bar(stage), 4 * kSlab);
-                        tma_load_2d(st + kOffB0, &map_x, token_bar(stage), (2 * s) * kKB, 0);
-                        tma_load_2d(st + kOffB1, &map_x, token_bar(stage), (2 * s + 1) * kKB, 0);
-                        bulk_load(st + kOffSfB0, p.xs_tok + static_cast<std::size_t>(s * 8) * 512, 2 * kSlab, token_bar(stage));
+                        constexpr int kBlocks = HALF ? 2 : 1;                    // K blocks of a stage
+                        mbar_arrive_expect_tx(token_bar(stage), kBlocks * 2 * kSlab);
+                        tma_load_2d(st + kOffB0, &map_x, token_bar(stage), kBlocks * s * kKB, 0);
+                        if constexpr (HALF) tma_load_2d(st + kOffB1, &map_x, token_bar(stage), (2 * s + 1) * kKB, 0);
+                        bulk_load(st + kOffSfB0, p.xs_tok + static_cast<std::size_t>(kBlocks * s * 4) * 512, kBlocks * kSlab, token_bar(stage));
                     } else {
                         bulk_load_hint(st, p.bank.g2 + ((static_cast<std::size_t>(entry) * dn_tiles + m_tile) * dn_stages + s) *
                                                            kChunkBytes,
@@ -646,7 +681,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                     }
                     tc_fence_after();
                     if (sequence == 0 && s < 10) stamp(26 + s);
-                    issue_stage(1, base + stage * kStage, kOffB1, kOffSfB0, sf_tmem + sf_buffer * kSfColsPerBuffer, accum,
+                    issue_stage(kind == 0 ? kGuKind : 1, base + stage * kStage, kOffB1, kOffSfB0, sf_tmem + sf_buffer * kSfColsPerBuffer, accum,
                                 idesc, s == 0);
                     tc_commit(empty_bar(stage));
                     if (sequence == 0 && s < 10) stamp(36 + s);
@@ -700,46 +735,48 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
             const int entry = expert == kExperts ? p.bank.local_experts : expert - p.bank.first_expert;
             const std::uint32_t lane_base = tmem_base + buffer * kAccumCols + (static_cast<std::uint32_t>(quarter * 32) << 16);
             if (kind == 0) {
-                // lanes 0..15 of the quarter hold the gate sums of 16 intermediate rows, lanes 16..31 their up sums.  Of a
-                // pair of token columns the lower half finishes the even one and the upper half the odd one: one exchange
-                // per pair and every lane has a gate and an up value.
                 const float alpha_g = p.bank.alpha[entry * 3 + 0];
                 const float alpha_u = p.bank.alpha[entry * 3 + 1];
-                const int row = m_tile * (kTile / 2) + quarter * 16 + (lane & 15);
-                const int sf_col = row >> 4;
-                const bool upper = (lane & 16) != 0;
-                std::uint32_t d[16];
-                tmem_load16(lane_base, d);
-                tmem_load_wait();
-#pragma unroll
-                for (int n = 0; n < R; n += 2) {
-                    const int pp_even = n < rows ? rt.pp_tok[slot][n] : -1;
-                    const int pp_odd = n + 1 < rows ? rt.pp_tok[slot][n + 1] : -1;
-                    if (pp_even < 0 && pp_odd < 0) continue;                         // warp uniform
-                    const std::uint32_t got = __shfl_xor_sync(0xffffffffU, upper ? d[n] : d[n + 1], 16);
-                    const std::uint32_t g = upper ? got : d[n];
-                    const std::uint32_t u = upper ? d[n + 1] : got;
-                    const float gv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(g) * alpha_g));
-                    const float uv = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(u) * alpha_u));
-                    const float h = bf16_bits_to_float(float_to_bf16_bits((gv / (1.0F + expf(-gv))) * uv));
-                    float amax = fabsf(h);
-#pragma unroll
-                    for (int off = 8; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffU, amax, off));
-                    const __nv_fp8_e4m3 scale(amax * (p.quant_scale / 6.0F));
-                    const float decoded = static_cast<float>(scale);
-                    const float multiplier = decoded == 0.0F ? 0.0F : p.quant_scale / decoded;
-                    const float q = h * multiplier;
-                    const float q_next = __shfl_xor_sync(0xffffffffU, q, 1);
-                    const int pp_signed = upper ? pp_odd : pp_even;
-                    if (pp_signed < 0) continue;                                     // no shuffle left in this round
-                    const std::size_t pp = static_cast<std::size_t>(pp_signed);
-                    if ((lane & 1) == 0) {
-                        p.hq[pp * (inter / 2) + (row >> 1)] =
-                            static_cast<std::uint8_t>(__nv_fp4x2_e2m1(make_float2(q, q_next)).__x);
-                    }
+                // stores byte and scale of intermediate row `row` for the token at padded position pp
+                auto store = [&](int row, int pp, RequantisedPair h) {
+                    const std::size_t at = static_cast<std::size_t>(pp);
+                    const int sf_col = row >> 4;
+                    if ((lane & 1) == 0) p.hq[at * (inter / 2) + (row >> 1)] = h.packed;
                     if ((lane & 15) == 0) {
-                        p.hs[((pp >> 7) * (inter / 64) + (sf_col >> 2)) * 512 + (pp & 31) * 16 + ((pp >> 5) & 3) * 4 +
-                             (sf_col & 3)] = scale.__x;
+                        p.hs[((at >> 7) * (inter / 64) + (sf_col >> 2)) * 512 + (at & 31) * 16 + ((at >> 5) & 3) * 4 + (sf_col & 3)] = h.scale;
+                    }
+                };
+                if constexpr (HALF) {
+                    // lanes 0..15 of the quarter hold the gate sums of 16 intermediate rows, lanes 16..31 their up sums.  Of
+                    // a pair of token columns the lower half finishes the even one and the upper half the odd one: one
+                    // exchange per pair and every lane has a gate and an up value.
+                    const int row = m_tile * kGuRows + quarter * 16 + (lane & 15);
+                    const bool upper = (lane & 16) != 0;
+                    std::uint32_t d[16];
+                    tmem_load16(lane_base, d);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int n = 0; n < R; n += 2) {
+                        const int pp_even = n < rows ? rt.pp_tok[slot][n] : -1;
+                        const int pp_odd = n + 1 < rows ? rt.pp_tok[slot][n + 1] : -1;
+                        if (pp_even < 0 && pp_odd < 0) continue;                     // warp uniform
+                        const std::uint32_t got = __shfl_xor_sync(0xffffffffU, upper ? d[n] : d[n + 1], 16);
+                        const RequantisedPair h = swiglu_requant(upper ? got : d[n], upper ? d[n + 1] : got, alpha_g, alpha_u, p.quant_scale);
+                        const int pp = upper ? pp_odd : pp_even;
+                        if (pp >= 0) store(row, pp, h);
+                    }
+                } else {
+                    const int row = m_tile * kGuRows + gu_tile_row(quarter, lane);
+                    std::uint32_t g[16], u[16];
+                    tmem_load16(lane_base, g);
+                    tmem_load16(lane_base + kAccumStride, u);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int n = 0; n < R; ++n) {
+                        const int pp = n < rows ? rt.pp_tok[slot][n] : -1;
+                        if (pp < 0) continue;                                        // warp uniform
+                        gu_exchange(g[n], u[n], lane, &g[n], &u[n]);
+                        store(row, pp, swiglu_requant(g[n], u[n], alpha_g, alpha_u, p.quant_scale));
                     }
                 }
                 __syncwarp();
@@ -900,11 +937,11 @@ cudaError_t launch_decode_mega(p92b_plan* plan, const p92b_bank* bank, const std
         plan->intermediate != 1024) {
         return cudaErrorNotSupported;
     }
-    const bool wide = rows > 8;
-    if (cudaError_t st = wide ? ensure_dynamic_smem<moe_decode_kernel<16>>(kMegaSmem) : ensure_dynamic_smem<moe_decode_kernel<8>>(kMegaSmem);
-        st != cudaSuccess) {
-        return st;
-    }
+    const auto kernel = rows <= kHalfTileRows ? moe_decode_kernel<8, true> : rows <= 8 ? moe_decode_kernel<8, false> : moe_decode_kernel<16, false>;
+    cudaError_t st = rows <= kHalfTileRows ? ensure_dynamic_smem<moe_decode_kernel<8, true>>(kMegaSmem)
+                     : rows <= 8           ? ensure_dynamic_smem<moe_decode_kernel<8, false>>(kMegaSmem)
+                                           : ensure_dynamic_smem<moe_decode_kernel<16, false>>(kMegaSmem);
+    if (st != cudaSuccess) return st;
     MegaParams p {};
     p.bank = bank->view;
     p.x = x;
@@ -942,10 +979,7 @@ cudaError_t launch_decode_mega(p92b_plan* plan, const p92b_bank* bank, const std
     p.hidden = plan->hidden;
     p.inter = plan->intermediate;
     plan->last_launches += 1;
-    return wide ? launch_kernel(moe_decode_kernel<16>, dim3(plan->sm_count), dim3(kMegaThreads), kMegaSmem, stream, pdl,
-                                plan->map_x_tok, plan->map_h[0], p)
-                : launch_kernel(moe_decode_kernel<8>, dim3(plan->sm_count), dim3(kMegaThreads), kMegaSmem, stream, pdl,
-                                plan->map_x_tok, plan->map_h[0], p);
+    return launch_kernel(kernel, dim3(plan->sm_count), dim3(kMegaThreads), kMegaSmem, stream, pdl, plan->map_x_tok, plan->map_h[0], p);
 }
 
 }  // namespace p92b

@@ -59,3 +59,24 @@ def test_top8_orders_scores_that_are_equal_or_nearly_equal(cuda, pkg, step):
         pkg.router_top8_rows(logits, torch.from_numpy(bias).cuda(), ids, weights, rows)
         assert np.array_equal(ids.cpu().numpy(), np.tile(want, (rows, 1)).astype(np.int32))
         assert np.array_equal(weights.cpu().numpy(), np.full((rows, 8), 0.3125, np.float32))    # 0.5 * 2.5 / 4, exact
+
+
+def test_decode_rows_equal_the_large_batch_at_both_gate_up_tiles(cuda, pkg, layer0):
+    """The fused decode kernel takes half gate/up tiles up to three rows and whole ones above, in a build for 8 and one for 16
+    rows: the first rows of a 64-row batch, sent alone, must come out with the batch's bits."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    x = synth.make_activations(78, 0, 64)
+    want = torch.empty_like(x)
+    plan = pkg.MoePlan(max_rows=64)
+    block = pkg.MoeBlock(layer0.bank, layer0.router_weight, layer0.bias, plan)
+    block.run_moe_rows(x, want, 64)
+    for rows in (2, 3, 4, 5, 8, 9, 15, 16):
+        for first in (0, 64 - rows):
+            out = torch.full((rows, x.shape[1]), float("nan"), dtype=torch.bfloat16, device="cuda")
+            block.run_moe_rows(x[first:first + rows], out, rows)
+            torch.cuda.synchronize()
+            assert plan.status() == 0 and plan.last_launches == 1
+            assert torch.equal(out.view(torch.int16), want[first:first + rows].view(torch.int16)), rows
+    plan.close()
