@@ -25,8 +25,11 @@ namespace {
 constexpr int kChunk = 256;          // flat indices per warp in the multi-block path
 constexpr int kWarps = 8;
 constexpr int kSmallWarps = 32;      // of the one-block path
-constexpr int kSmallChunk = 128;     // ids per warp there, at most
-constexpr int kSmallMax = kSmallWarps * kSmallChunk;      // 4,096: from there on the three-kernel form is quicker
+constexpr int kSmallChunk = 160;     // ids per warp there, at most
+// 5,120: the most that the block's 48 KB of shared memory hold.  At 4,104 it takes 12.3 us against 18.5 of the three-kernel
+// form (p92b_moe_permute_static; with a plan 10.3 against 16.4), at 5,120 12.4 against 18.5.
+constexpr int kSmallMax = kSmallWarps * kSmallChunk;
+static_assert(kSmallChunk % 32 == 0, "a warp's share is whole steps");
 
 // Which expert ids take part.  The whole range by default; an expert-parallel GPU that holds the ids of the whole
 // batch restricts the permutation to its own experts [first, first + count) - ids outside (other GPUs' experts, and
@@ -630,7 +633,6 @@ cudaError_t launch_permute(p92b_plan* plan, const std::int32_t* ids, int assignm
     plan->wide_rows = wide ? 128 : 0;
     std::int32_t* row_token = route_lists ? plan->row_token : nullptr;
     std::int32_t* pp_of_flat = padded ? plan->pp_of_flat : nullptr;
-    // one block up to 4,096 assignments; at 8,192 the three-kernel form was quicker (22 against 33 µs)
     if (assignments <= kSmallMax) {
         plan->last_launches += 1;
         return launch_kernel(permute_small_kernel, dim3(1), dim3(kSmallThreads), 0, stream, pdl, ids, assignments, order, position,

@@ -41,3 +41,20 @@ def test_router_logits_keep_their_order_of_sums(cuda, pkg, orc, batch, experts, 
     pkg.bf16_gemm_f32(x, w, out, batch)
     want = orc.router_logits(_u16(x), _u16(w), gemv_order=False)
     assert np.array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n", [1, 31, 4095, 4096, 4097, 4128, 5119, 5120, 5121, 8192])
+def test_permutation_either_side_of_the_one_block_form(cuda, pkg, n):
+    """A stable sort by expert id, whole numbers: sizes around whole steps of its warps and around its largest, 5,120."""
+    torch = cuda
+    ids = np.random.default_rng(n).integers(0, 256, size=n).astype(np.int32)
+    ids[: n // 3] = 77                                               # more of one expert than a warp's share holds
+    order, position = (torch.full((n,), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+    counts, offsets = (torch.full((k,), -1, dtype=torch.int32, device="cuda") for k in (256, 257))
+    pkg.moe_permute_static(torch.from_numpy(ids).cuda(), order, position, counts, offsets)
+    want = np.argsort(ids, kind="stable")
+    assert np.array_equal(order.cpu().numpy(), want)
+    assert np.array_equal(position.cpu().numpy()[want], np.arange(n))
+    assert np.array_equal(counts.cpu().numpy(), np.bincount(ids, minlength=256))
+    assert np.array_equal(offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(np.bincount(ids, minlength=256))]))
+    assert pkg.moe_permute_static_status() == 0
