@@ -1,6 +1,6 @@
 // The dense MLP for a few rows (decode, verify step): two kernels that stream the weights through every SM.
 //
-// With one matrix triple and up to 20 tokens the work is 3 x 9216 x 2560 FP4 weights, 40 MB or 6 us of HBM time, and the
+// With one matrix triple and a few tokens the work is 3 x 9216 x 2560 FP4 weights, 40 MB or 6 us of HBM time, and the
 // grouped kernels (expert_tc.cu) leave most of the chip idle on it: 72 gate/up tiles and 20 down tiles on 148 SMs, with a
 // list kernel and a one-block quantiser in front (28.3 us for four rows).  Here
 //   gate/up  a block owns half a tile, one box of 64 gate and 64 up rows (144 blocks), requests its weights before it
@@ -21,9 +21,7 @@ using namespace ptx;
 
 namespace {
 
-// Quantising in every block and adding up the parts cost 0.7 us per row and layer: 17 rows take 22.5 us a layer, 32 rows 33,
-// and the large-batch kernels 26 from 21 to 64 rows.
-constexpr int kRowsMax = 20;
+constexpr int kRowsMax = 32;                                 // that the kernels are built for
 constexpr int kPartsMax = 8;                                 // of K, down product
 constexpr int kTile = 128;
 constexpr int kKB = 128;                                     // bytes of a K block per row: 256 values
@@ -409,9 +407,18 @@ cudaError_t launch_both(const p92b_plan* plan, const DenseParams& p, cudaStream_
 
 }  // namespace
 
-// Up to kRowsMax rows; the token rows of a block have to fit its shared memory.
+// The token rows of a block have to fit its shared memory (hidden 4,096 at most), and the rows be few: quantising in every
+// block and adding up the parts cost 0.5 to 1 us per row, while the grouped kernels (expert_tc.cu) take nearly the same time
+// from 1 to 32 rows.  What those lose, idle SMs, grows with the intermediate size - until the blocks here need a second round.
+// Us a layer, few rows / grouped, at the last row count for the former and the first for the latter (hidden x intermediate):
+// 2560 x 9216: 18 rows 23.9 / 24.1, 19 rows 24.8 / 24.2; 2048 x 8192: 17 rows 21.6 / 21.6, 18 rows 22.1 / 21.7;
+// 1024 x 4096: 13 rows 15.5 / 16.4, 15 rows 16.9 / 16.5; 4096 x 4096: 13 rows 20.2 / 20.4, 14 rows 21.2 / 20.5;
+// 2560 x 1024: 10 rows 14.4 / 14.8, 11 rows 15.0 / 14.8; 512 x 1536: 10 rows 12.2 / 13.2, 11 rows 13.3 / 13.2;
+// 4096 x 14336, two rounds: 10 rows 35.1 / 35.3, 11 rows 36.1 / 35.4.
 bool dense_few_rows_applies(const p92b_plan* plan, int rows) {
-    return rows <= kRowsMax && plan->hidden <= 4096 && plan->hidden % 256 == 0 && plan->intermediate % 512 == 0;
+    const bool one_round = plan->intermediate / (kTile / 2) <= plan->sm_count;
+    const int most = one_round ? std::min(kRowsMax, 9 + plan->intermediate / 1024) : 10;
+    return rows <= most && plan->hidden <= 4096 && plan->hidden % 256 == 0 && plan->intermediate % 512 == 0;
 }
 
 cudaError_t launch_dense_few_rows(p92b_plan* plan, const p92b_bank* bank, const std::uint16_t* x, std::uint16_t* out, int rows,
@@ -431,7 +438,7 @@ cudaError_t launch_dense_few_rows(p92b_plan* plan, const p92b_bank* bank, const 
     p.inter = plan->intermediate;
     // parts of K: as many blocks as there are SMs (20 tiles: 7 parts), at least one K block each.  The sums lie in the
     // grouped kernels' output rows, which this call does not use: (257 * 127 or fewer, at least 1,152) rows x hidden
-    // BF16 values hold 8 parts x 20 rows x hidden FP32 values.
+    // BF16 values hold 8 parts x 32 rows x hidden FP32 values.
     p.parts = std::max(1, std::min({kPartsMax, plan->sm_count / (plan->hidden / kTile), plan->intermediate / 256}));
     p.partial = reinterpret_cast<float*>(plan->mixed_pp);
     if (static_cast<std::size_t>(p.parts) * rows * 4 > plan->pp_rows * 2) return cudaErrorInvalidValue;

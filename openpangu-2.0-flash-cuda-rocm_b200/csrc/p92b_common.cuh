@@ -499,7 +499,7 @@ cudaError_t launch_gather_quantized_rows(const std::uint8_t* packed, const std::
                                          bool pdl = false);
 cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int rows, bool down,
                               cudaStream_t stream, bool pdl = false, const TcIo* io = nullptr);
-// The dense MLP of up to 20 rows (dense_rows.cu).
+// The dense MLP of a few rows (dense_rows.cu, which says how few).
 bool dense_few_rows_applies(const p92b_plan* plan, int rows);
 cudaError_t launch_dense_few_rows(p92b_plan* plan, const p92b_bank* bank, const std::uint16_t* x, std::uint16_t* out, int rows,
                                   cudaStream_t stream, bool pdl);

@@ -1,6 +1,7 @@
-"""The dense MLP of a few rows (its own pair of kernels up to 20 rows) against the CPU oracle.
+"""The dense MLP of a few rows (its own pair of kernels) against the CPU oracle.
 
-Row counts sit on both sides of the column count of the MMA (16) and of the hand-over to the large-batch kernels (20);
+Row counts sit on both sides of the column count of the MMA (16), of the hand-over to the grouped kernels (after 9, 10 or 18
+rows at these shapes) and of the hand-over to the large-batch ones (32);
 shapes cover a K extent of the down product that its parts do not divide, fewer K blocks than parts, one part per tile
 (hidden 4096 has 32 tiles for 148 SMs: 4 parts) and the model's own MLP.  Both products accumulate in FP32 over FP4
 operands, so a result differs from the oracle's only where another order of the sums moves a SwiGLU value to the
@@ -38,12 +39,12 @@ def test_dense_few_rows_against_the_oracle(cuda, pkg, orc, hidden, inter):
         alphas.append(float(alpha))
     bank = pkg.ExpertBank(entries, first_expert=0, local_experts=0, hidden=hidden, intermediate=inter)
     # the oracle is row by row, so one call at the largest size has every row's result
-    most = 33 if inter < 9216 else 17
+    most = 33 if inter < 9216 else 19
     x = torch.empty((most, hidden), dtype=torch.float32, device="cuda").normal_(0, 1, generator=g).to(torch.bfloat16)
     want = orc.bf16_to_f32(orc.dense_forward(_u16(x), np.stack(packed_np), np.stack(scales_np), np.array(alphas, np.float32),
                                              hidden, inter))
     plan = pkg.MoePlan(max_rows=most, hidden=hidden, intermediate=inter)
-    for rows in (1, 2, 15, 16, 17, 20, 21, 31, 32, 33):
+    for rows in (1, 2, 9, 10, 11, 15, 16, 17, 18, 19, 20, 21, 31, 32, 33):
         if rows > most:
             continue
         out = torch.full((rows, hidden), float("nan"), dtype=torch.bfloat16, device="cuda")
