@@ -8,10 +8,12 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cfloat>
 #include <cstddef>
 #include <cstdint>
 #include <cstdlib>
+#include <mutex>
 
 #include "p92b_moe.h"
 
@@ -397,21 +399,24 @@ inline bool pdl_enabled() {
     return on;
 }
 
-// Opt-in to more than 48 KB of dynamic shared memory.  The attribute belongs to the (kernel, device)
-// pair, not to the process: a host that drives several GPUs from one process has to set it once on
-// each of them, so the "already done" flag is kept per device (one table per kernel through the
-// non-type template parameter).
+// Opt-in to dynamic shared memory.  The attribute belongs to the (kernel, device) pair, not to the process: a host that
+// drives several GPUs from one process has to set it once on each of them, so what has been set is kept per device (one
+// table per kernel through the non-type template parameter).  It is an upper limit for the launches to come, and some
+// kernels need more for one plan's sizes than for another's: a larger request raises it, a smaller one leaves it.
 constexpr int kMaxDevices = 64;
 template <auto Kernel>
 cudaError_t ensure_dynamic_smem(int bytes) {
-    static bool configured[kMaxDevices] = {};
+    static std::atomic<int> configured[kMaxDevices] = {};
+    static std::mutex raising;
     int device = 0;
     cudaError_t st = cudaGetDevice(&device);
     if (st != cudaSuccess) return st;
-    const bool tracked = device >= 0 && device < kMaxDevices;
-    if (tracked && configured[device]) return cudaSuccess;
+    if (device < 0 || device >= kMaxDevices) return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (configured[device].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+    const std::lock_guard<std::mutex> lock(raising);
+    if (configured[device].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
     st = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (st == cudaSuccess && tracked) configured[device] = true;
+    if (st == cudaSuccess) configured[device].store(bytes, std::memory_order_release);
     return st;
 }
 

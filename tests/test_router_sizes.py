@@ -1,0 +1,60 @@
+"""The tensor-core router with exact repair, at the sizes where its kernels change, against the operators that keep the
+reference's order of sums throughout (bf16_gemm_f32 and router_top8_rows, themselves held to the CPU oracle bit for bit)."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# K in eight slices and a block per token up to 256 rows, a warp per token above; eight slices up to 512, then fewer
+# (three from 1,153, two from 1,537) and none above 2,304 rows; tiles of 64 experts, of 128 from 4,737 and of 256 from 9,473
+# rows on (148 SMs).  Ends of these ranges, and odd sizes inside them.
+SIZES = [9, 17, 255, 256, 257, 300, 512, 513, 1025, 1152, 1153, 1200, 1536, 1537, 2304, 2305, 4736, 4737, 7001, 9000, 9472, 9473]
+
+
+def _check(torch, pkg, block, rows, x, bias):
+    plan, router = block.plan, block.router_weight
+    logits = torch.empty((rows, 256), dtype=torch.float32, device="cuda")
+    ids = torch.empty((rows, 8), dtype=torch.int32, device="cuda")
+    weights = torch.empty((rows, 8), dtype=torch.float32, device="cuda")
+    pkg.bf16_gemm_f32(x, router, logits, rows)
+    pkg.router_top8_rows(logits, bias, ids, weights, rows)
+    block.run_moe_rows(x, torch.empty_like(x), rows)
+    views = plan.views(rows)
+    assert plan.status() == 0
+    assert torch.equal(views["expert_ids"], ids)
+    assert torch.equal(views["expert_weights"], weights)
+    picked = ids.long()
+    assert torch.equal(torch.gather(views["logits"], 1, picked), torch.gather(logits, 1, picked))
+    # the others may deviate by 2^-14 |x| |w| without a wrong choice; they stay 8 times inside that
+    bound = 2.0 ** -14 * x.double().norm(dim=1, keepdim=True) * router.double().norm(dim=1)
+    assert bool(((views["logits"].double() - logits.double()).abs() <= 0.125 * bound).all())
+
+
+@pytest.mark.parametrize("rows", SIZES)
+def test_router_of_the_block_equals_the_exact_operators(cuda, pkg, layer0, rows):
+    torch = cuda
+    from p92moe_b200 import synth
+
+    plan = pkg.MoePlan(max_rows=rows)
+    plan.set_path(plan.PATH_TENSOR_CORE)
+    x = synth.make_activations(4500, rows, rows)
+    for bias in (layer0.bias, torch.zeros_like(layer0.bias)):             # without a bias the scores lie closer together
+        _check(torch, pkg, pkg.MoeBlock(layer0.bank, layer0.router_weight, bias, plan), rows, x, bias)
+    plan.close()
+
+
+def test_router_at_other_hidden_sizes(cuda, pkg):
+    """Hidden sizes other than 2,560 take the form that reads token row and router rows in place; its shared memory
+    grows with the size, so a larger plan behind a smaller one in the same process needs a higher limit."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    for hidden, inter in ((256, 512), (512, 512), (1024, 512), (4096, 512)):
+        bank = pkg.ExpertBank(synth.make_raw_layer_batched(11, 0, hidden=hidden, intermediate=inter).entries(), hidden=hidden,
+                              intermediate=inter)
+        router, bias = synth.make_router(11, 0, hidden=hidden)
+        for rows in (9, 100, 257, 1200, 2305):
+            plan = pkg.MoePlan(rows, hidden, inter)
+            x = synth.make_activations(11, rows, rows, hidden=hidden)
+            _check(torch, pkg, pkg.MoeBlock(bank, router, bias, plan), rows, x, bias)
+            plan.close()
+        bank.close()
