@@ -371,9 +371,10 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
             // Half a warp per chain set: lane l of a half runs columns 2l and 2l + 1 (mod 32) of one (token, router row)
             // pair with one 4-byte read per operand and step - 2-byte reads, a lane per column, keep the shared-memory
             // pipe busy for twice as long, which is what this phase is bound by.  The halves take the block's two router
-            // rows with the same token, or two tokens where the block has one router row.
+            // rows with the same token, or two tokens where the block has one router row; a block without any (more blocks
+            // than experts) has nothing to do.
             const int half = lane >> 4, l16 = lane & 15;
-            for (int q = warp; my_experts == 2 ? q < rows : 2 * q < rows; q += kMegaWarps) {
+            for (int q = warp; my_experts == 2 ? q < rows : 2 * q < rows * my_experts; q += kMegaWarps) {
                 const int t = my_experts == 2 ? q : min(2 * q + half, rows - 1);
                 const int r = my_experts == 2 ? half : 0;
                 const std::uint32_t* wr = reinterpret_cast<const std::uint32_t*>(w_rows + r * row_pitch) + l16;
