@@ -546,7 +546,6 @@ class SingleGpu:
         distinct = int((counts > 0).sum())
         real = rows * (TOP + 1)
         padded = int((np.ceil(counts / 128) * 128).sum() + math.ceil(rows / 128) * 128)
-        tiles64 = int((np.ceil(counts / 64) * 64).sum() + math.ceil(rows / 64) * 64)
         pk = peaks()
         t_bytes = layer_bytes(distinct, rows) / (pk["hbm_gbs"] * 1e9)
         yardstick = nvfp4_yardstick(torch)
@@ -563,8 +562,8 @@ class SingleGpu:
             "stage_us": stage_us, "distinct_routed_experts": distinct,
             "rows_per_expert": {"max": int(counts.max()), "mean": float(counts.mean()), "min": int(counts.min())},
             "padding_waste": {"padded_rows_over_real_rows": padded / real, "padded_rows": padded, "real_rows": real,
-                              "mma_rows_over_real_rows_64_row_tiles": tiles64 / real,
-                              "note": "every expert's rows start on a multiple of 128 padded positions (address space only); "
+                              "mma_rows_over_real_rows": padded / real,
+                              "note": "every expert's rows start on a multiple of 128 padded positions (address space only), and "
                                       "both products run on 128-row token tiles, whose last tile per expert is partly empty"},
             "roofline_layer": {"t_bytes_us": t_bytes * 1e6, "t_flops_us": t_flops * 1e6,
                                "frac_of_max": max(t_bytes, t_flops) / (ms * 1e-3),

@@ -15,12 +15,12 @@ using namespace ptx;
 constexpr int kTile = 128;                          // weight rows per tile (the MMA's M)
 constexpr int kKB = 128;                            // bytes per operand row per K block
 constexpr int kSlab = 2048;                         // one 128x4-tiled scale slab: 128 rows x 16 scales
-// Every stage starts with one 36,864-byte chunk of the bank's tile stream, copied as a whole: two 16 KB weight
-// boxes and their two scale slabs.  The token boxes and token scale slabs follow; their offsets depend on the
-// kernel's column count and are passed in.
+// Every stage starts with 36,864 bytes of weights in the layout of a chunk of the bank's tile stream, two 16 KB boxes and
+// their two scale slabs: one chunk as a whole or, for half a gate/up tile, the same box of two neighbouring chunks.  The
+// token boxes and token scale slabs follow; their offsets depend on the kernel's column count and are passed in.
 constexpr int kOffA0 = 0, kOffA1 = 16384, kOffSfA0 = 32768, kOffB0 = 36864;
 constexpr int kStages = 4;
-constexpr int kAccumStride = 32;                    // gate at +0, up at +32 inside an accumulator buffer
+constexpr int kAccumStride = 32;                    // box 0 at +0, box 1 at +32 inside an accumulator buffer
 constexpr int kAccumCols = 64;
 constexpr int kSfColsPerBuffer = 64;                // SFA0, SFA1, SFB0, SFB1 x 16 columns
 constexpr int kAccumBuffers = 4;                    // the issuer may run four tiles ahead of the epilogue
@@ -73,10 +73,11 @@ __device__ __forceinline__ void decode_tile(int code, int* kind, int* slot, int*
     *m_tile = code & 0xff;
 }
 
-// The products of one ring stage at shared-memory address `st`.  kind 0, a gate/up stage: one K block of the
-// tile's gate rows and of its up rows against the token box, into the two halves of the accumulator buffer.
-// kind 1, a down stage: two K blocks of the tile's rows against the two SwiGLU-row boxes, into one accumulator.
-// The stage's scale slabs are copied to the TMEM columns at `sfc` first (SFA0, SFA1, SFB0 and, for a down stage,
+// The products of one ring stage at shared-memory address `st`.  kind 0, a whole gate/up tile: one K block of its two
+// boxes (either holds gate rows and up rows, gu_box_row) against the token box, into the two halves of the accumulator
+// buffer.  kind 1, a down tile or half a gate/up tile: two K blocks of one box against their two token boxes, into one
+// accumulator.
+// The stage's scale slabs are copied to the TMEM columns at `sfc` first (SFA0, SFA1, SFB0 and, for kind 1,
 // SFB1, 16 columns each).  `first` is true for the first stage of a tile: its first product overwrites.
 __device__ __forceinline__ void issue_stage(int kind, std::uint32_t st, int off_b1, int off_sfb0, std::uint32_t sfc,
                                             std::uint32_t accum, std::uint32_t idesc, bool first) {

@@ -10,8 +10,6 @@
 // N = 64.
 #include "expert_common.cuh"
 
-#include <cstdlib>
-
 namespace p92b {
 
 using namespace ptx;
@@ -37,8 +35,9 @@ __device__ __forceinline__ uint4 scale_to_bf16x8(const std::uint32_t* v, float a
 // Stores 32 rows x 64 BF16 values; lane l holds row l's eight 16-byte pieces.  Stored as they are, one instruction
 // would touch 32 lines and write 16 bytes of each (a down product over 147,456 rows took 506 µs that way against 326).
 // An 8 x 8 transposition of the pieces inside every group of eight lanes - three exchange rounds - makes lane j of a
-// group hold piece j of the group's eight rows: one instruction then stores four whole 128-byte lines.  `row` = this lane's row number in the output, `valid` = rows that exist (warp uniform).
-__device__ __forceinline__ void store_rows64(std::uint16_t* out, int pitch, long row, int valid, uint4 (&w)[8]) {
+// group hold piece j of the group's eight rows: one instruction then stores four whole 128-byte lines.  `out` = the first of the
+// 32 rows in the output, `valid` = rows that exist (warp uniform).
+__device__ __forceinline__ void store_rows64(std::uint16_t* out, int pitch, int valid, uint4 (&w)[8]) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int d = 4; d >= 1; d >>= 1) {
@@ -60,8 +59,7 @@ __device__ __forceinline__ void store_rows64(std::uint16_t* out, int pitch, long
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int from = (lane & ~7) + r;
-        const long to = __shfl_sync(0xffffffffU, row, from);
-        if (from < valid) *reinterpret_cast<uint4*>(out + to * pitch + (lane & 7) * 8) = w[r];
+        if (from < valid) *reinterpret_cast<uint4*>(out + static_cast<std::size_t>(from) * pitch + (lane & 7) * 8) = w[r];
     }
 }
 
@@ -188,7 +186,7 @@ __device__ __forceinline__ bool decode_piece(const TcParams& p, const RouteTable
 // 64 columns into registers at once and the next item's products start after that read, not after the arithmetic.
 // What bounds it with full tiles: the shared-memory port.  A K block costs 48 KB of operand reads, 54 KB of arriving
 // copies and 6 KB of scale copies, 844 cycles at 128 bytes against 512 of tensor work; it runs at 907 (16,384 tokens:
-// 556 -> 393 us; 4,096 tokens: 202 -> 168 us, HBM floor 116).  A pair of blocks sharing the weight rows (cta_group::2,
+// 563 -> 394 us; 4,096 tokens: 201 -> 163 us, HBM floor 116).  A pair of blocks sharing the weight rows (cta_group::2,
 // 256-row token tiles) needs 594 cycles but pads every expert to 256 rows: 376 us and 200 us, not kept.  Token rows
 // gathered from token order (TMA tile::gather4, four rows per operation) take 46 ns per operation: 1,023 us.
 template <int MODE>
@@ -360,8 +358,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
             tc_fence_after();
             const bool mine = quarter * 32 < it.valid && group * 64 < piece.width;      // warp uniform
             const int column64 = piece.first + group * 64;  // of the item's 256 weight rows
-            const int pp = it.pp0 + row;
             if constexpr (MODE == 0) {
+                const int pp = it.pp0 + row;
                 std::uint32_t first[32], second[32];
                 if (mine) {
                     tmem_load32(lane_base + group * 64, first);            // gate and up sums of 16 intermediate rows
@@ -394,8 +392,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                 __syncwarp();
                 if (lane == 0) mbar_arrive(accum_empty);
                 if (!mine) continue;
-                const long my_row = p.out_row != nullptr ? (row < it.valid ? p.out_row[it.dense0 + row] : 0) : pp;
-                store_rows64(p.out + static_cast<std::size_t>(it.m_tile) * kWRows + column64, p.m_total, my_row, it.valid - quarter * 32, w);
+                std::uint16_t* first_row = p.out + static_cast<std::size_t>(it.pp0 + quarter * 32) * p.m_total;
+                store_rows64(first_row + static_cast<std::size_t>(it.m_tile) * kWRows + column64, p.m_total, it.valid - quarter * 32, w);
             }
         }
     }

@@ -996,9 +996,9 @@ cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int 
             case 1: return launch_tc<0, 32>(plan, plan->map_x[1], p, stream, pdl);
             default:
                 // Lists with 128-row tiles (every call of more than 32 rows except the expert-parallel ones that build
-                // their lists themselves): tokens on the M side.  It is the quicker form over the whole range: 107 against
-                // 109 us at 64 rows, 123 against 129 at 512 (both near the HBM time of the weights), 168 against 201 at
-                // 4,096, 389 against 563 at 16,384.
+                // their lists themselves): tokens on the M side.  It is the quicker form over the whole range: by 2 % at 64
+                // rows and 5 % at 512, where both run near the HBM time of the weights, 163 against 201 us at 4,096, 394
+                // against 563 at 16,384.
                 if (plan->wide_rows == 128) {
                     p.tile_prefix = plan->tile_prefix_wide;
                     return launch_expert_rows_gate_up(plan, p, stream, pdl);
@@ -1035,8 +1035,8 @@ cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int 
                 }
                 if (p.row_dest != nullptr) return cudaErrorNotSupported;
                 // any K: 128 x 256 tiles with the tokens on the M side (dense MLP, 3,807 rows: both products together 196 ->
-                // 141 us per layer); it stores 16 bytes at a time and computes whole token tiles of every entry
-                if (!(io != nullptr && io->skip_shared) && (reinterpret_cast<std::uintptr_t>(p.out) & 15U) == 0U) {
+                // 141 us per layer); it stores whole token tiles of every entry at their padded positions, 16 bytes at a time
+                if (p.out_row == nullptr && p.skip_shared == 0 && (reinterpret_cast<std::uintptr_t>(p.out) & 15U) == 0U) {
                     return launch_expert_rows_matrix(plan, p, stream, pdl);
                 }
                 return launch_tc<1, 128>(plan, plan->map_h[3], p, stream, pdl);

@@ -625,8 +625,8 @@ cudaError_t launch_permute(p92b_plan* plan, const std::int32_t* ids, int assignm
     const bool padded = route_lists && pad_align > 0;
     lists.pp_off = padded ? plan->pp_off : nullptr;
     lists.tile_prefix = padded ? plan->tile_prefix : nullptr;
-    // large batches: the down product takes token tiles twice as wide as the gate/up product (one
-    // accumulator per tile instead of two, so 128 columns still leave room for two buffers)
+    // more than 32 rows: a second prefix in 128-row tiles, which the kernels with the tokens on the M side and the slab kernel
+    // of the down product count in; the 64-row one stays for the operators on a caller's weights and the un-fused results
     const bool wide = padded && tile_rows == 64;
     lists.tile_rows_wide = wide ? 128 : lists.tile_rows;
     lists.tile_prefix_wide = wide ? plan->tile_prefix_wide : nullptr;
