@@ -14,6 +14,11 @@ using namespace ptx;
 constexpr int kTileM = 128;
 constexpr int kBlockKBytes = 128;                 // one swizzle row: 256 E2M1 values
 constexpr int kSfSlab = 2048;                     // 128 rows x 16 scales of one K block
+// Padded positions from one token tile of an expert to its next.  A tile's scale factors have to start at row 0 or 64 of a
+// 128-row scale tile (another row's are at an address that the MMA does not take), so tiles of 16 or 32 rows lie a
+// whole scale tile apart; an expert that no token picks twice has one such tile only.
+template <int N>
+constexpr int kTileStride = N < 64 ? 128 : N;
 
 struct TcParams {
     BankView bank;
@@ -93,7 +98,7 @@ __device__ __forceinline__ bool decode_item(const TcParams& p, const RouteTable&
     it->expert = t.expert[lo];
     it->entry = it->expert == kExperts ? p.bank.local_experts : it->expert - p.bank.first_expert;
     it->count = t.count[lo];
-    it->pp0 = t.pp_off[lo] + n_tile * N;
+    it->pp0 = t.pp_off[lo] + n_tile * kTileStride<N>;
     it->valid = min(N, it->count - n_tile * N);
     it->dense0 = t.offset[lo] + n_tile * N;
     if (p.skip_shared && it->expert == kExperts) return false;

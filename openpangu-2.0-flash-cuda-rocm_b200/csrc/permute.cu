@@ -92,7 +92,8 @@ __device__ __forceinline__ void load_chunk_ids(const std::int32_t* __restrict__ 
 }
 
 // Scatters one chunk.  running[e] (warp private) = first position of this chunk's rows of expert e, counted from
-// expert_base[e] (null: from 0); pp_delta[e] (shared memory, read only with pp_of_flat) = padded offset - offset of expert e.  The steps
+// expert_base[e] (null: from 0); pp_delta[e] (shared memory, read only with pp_of_flat) = padded offset - offset of expert e.
+// tile_shift > 0 (with expert_base): an expert's padded rows come in tiles of 1 << tile_shift, 128 positions apart.  The steps
 // of a chunk depend on one another through running[], so whatever a step reads has to be in shared memory or in
 // registers already: a global load per step is a round trip to the L2 per step.
 template <class T, class Order>
@@ -103,7 +104,8 @@ __device__ __forceinline__ void warp_scatter(const std::int32_t* __restrict__ id
                                              std::int32_t* __restrict__ row_token,
                                              const std::int32_t* pp_delta,
                                              std::int32_t* __restrict__ pp_of_flat,
-                                             const std::int16_t* cached = nullptr, IdRange range = IdRange()) {
+                                             const std::int16_t* cached = nullptr, IdRange range = IdRange(),
+                                             int tile_shift = 0) {
     const int lane = threadIdx.x & 31;
     __syncwarp();
     for (int step = begin; step < end; step += 32) {
@@ -123,11 +125,15 @@ __device__ __forceinline__ void warp_scatter(const std::int32_t* __restrict__ id
         const int rank = __popc(peers & ((1U << lane) - 1U));
         int pos = 0;
         if (valid) {
-            pos = running[e] + rank + (expert_base != nullptr ? expert_base[e] : 0);
+            const int of_expert = running[e] + rank;
+            pos = of_expert + (expert_base != nullptr ? expert_base[e] : 0);
             if (order != nullptr) order[pos] = static_cast<Order>(i);
             if (position != nullptr) position[i] = pos;
             if (row_token != nullptr) row_token[pos] = i / kTop;
-            if (pp_of_flat != nullptr) pp_of_flat[i] = pp_delta[e] + pos;
+            if (pp_of_flat != nullptr) {
+                const int gaps = tile_shift > 0 ? (of_expert >> tile_shift) * (128 - (1 << tile_shift)) : 0;
+                pp_of_flat[i] = pp_delta[e] + pos + gaps;
+            }
         }
         __syncwarp();
         if (valid && rank == 0) running[e] += static_cast<T>(__popc(peers));
@@ -164,7 +170,9 @@ __device__ __forceinline__ int block_exclusive_scan_256(int value, std::int32_t*
 // compact list of entries that have rows, shared expert first (it is the largest
 // group, so the persistent kernels start it first), and - for the tensor-core
 // kernels - a padded position space in which every entry's rows start on a
-// multiple of `pad_align`, plus the prefix of token-tile counts over the active list.
+// multiple of `pad_align`, plus the prefix of token-tile counts over the active list.  With tiles of 16 or 32 rows every
+// tile starts on such a multiple (expert_common.cuh, kTileStride): the positions that takes, 128 per assignment at most,
+// are what a plan reserves for as many experts with a row each.
 struct RouteLists {
     std::int32_t* counts;        // [257]
     std::int32_t* offsets;       // [258]
@@ -196,10 +204,10 @@ __device__ __forceinline__ void write_route_lists(int e, int count, int offset, 
     }
     if (lists.pp_off == nullptr) return;
     const int align = lists.pad_align;
-    const int padded = (count + align - 1) / align * align;
+    const int tiles = (count + lists.tile_rows - 1) / lists.tile_rows;
+    const int padded = lists.tile_rows < 64 ? tiles * align : (count + align - 1) / align * align;
     const int pp = block_exclusive_scan_256<PART>(padded, scan_scratch);
     lists.pp_off[e] = pp;
-    const int tiles = (count + lists.tile_rows - 1) / lists.tile_rows;
     const int shared_tiles = (rows + lists.tile_rows - 1) / lists.tile_rows;
     const int before = block_exclusive_scan_256<PART>(tiles, scan_scratch);
     if (count > 0) lists.tile_prefix[1 + slot] = shared_tiles + before;
@@ -283,8 +291,9 @@ __global__ void __launch_bounds__(kSmallThreads) permute_small_kernel(
         pp_delta[e] = (pp_of_flat != nullptr && lists.pp_off != nullptr) ? lists.pp_off[e] - offset : 0;       // write_route_lists stored both just above
     }
     __syncthreads();
+    const int tile_shift = pp_of_flat != nullptr && lists.tile_rows < 64 ? 31 - __clz(lists.tile_rows) : 0;
     warp_scatter(ids, begin, end, hist[warp], expert_base, order_image, position, static_cast<std::int32_t*>(nullptr), pp_delta,
-                 pp_of_flat, cached_ids[warp], range);
+                 pp_of_flat, cached_ids[warp], range, tile_shift);
     __syncthreads();
     for (int at = threadIdx.x; at < positions; at += kSmallThreads) {
         const int i = order_image[at];
