@@ -23,8 +23,8 @@
 // sigmoid's slope is at most 1/4; both the reference chain and the tensor-core sum differ from the true dot product by
 // at most (number of sequential roundings) * 2^-23 * sum|x_i w_i| <= that * ||x|| ||w||, with about 85 roundings in the
 // reference's order and fewer than 200 in the tensor core's; kLogitBound = 2^-14 is more than twice their sum; 4e-6
-// covers the fast-math sigmoid's own error on both sides.  A token whose candidate set would exceed 24 experts, or
-// that holds a non-finite logit, has its whole row recomputed exactly instead.
+// covers the fast-math sigmoid's own error on both sides.  A token whose candidate set would exceed 24 experts or
+// has fewer than eight, or that holds a non-finite logit, has its whole row recomputed exactly instead.
 //
 // The logits buffer keeps the approximate values except at the recomputed positions, which hold the exact ones.
 #include "p92b_common.cuh"
@@ -380,17 +380,19 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
         member[i] = __ballot_sync(0xffffffffU, score[i] >= eighth - 2.0F * delta);
         candidates += __popc(member[i]);
     }
-    const bool whole_row = !finite || candidates > kMaxCandidates;
+    // (fewer than eight: a NaN in the bias upset the 8th best, or fewer than eight experts are not masked by -infinity)
+    const bool whole_row = !finite || candidates > kMaxCandidates || candidates < kTop;
     if (whole_row) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) member[i] = 0xffffffffU;
     }
     // exact logits of the candidates (or of the whole row), into the logits buffer and into this warp's row
+    const float not_recomputed = __uint_as_float(0x7fc00000U);        // a NaN is picked behind every number
     if constexpr (WPT > 1) {
-        for (int e = threadIdx.x; e < kExperts; e += WPT * 32) exact_row[e] = -3.0e38F;
+        for (int e = threadIdx.x; e < kExperts; e += WPT * 32) exact_row[e] = not_recomputed;
         __syncthreads();                               // before any warp stores a result into the shared row
     } else {
-        for (int e = lane; e < kExperts; e += 32) exact_row[e] = -3.0e38F;   // non-candidates can never be selected
+        for (int e = lane; e < kExperts; e += 32) exact_row[e] = not_recomputed;
     }
     int n_cand = 0;
 #pragma unroll
@@ -465,62 +467,10 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
         atomicAdd(stats + 0, whole_row ? kExperts : candidates);
         if (whole_row) atomicAdd(stats + 1, 1);
     }
-    // The reference's top-8 over the exact values.  Every entry gets an order-preserving integer key of its corrected
-    // score; experts that were not recomputed (they cannot be in the top-8), NaN scores (a comparison never picks them)
-    // and entries already taken carry key 0, below every real score.
-    {
-        float raw[8];
-        std::uint32_t key[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = lane + 32 * i;
-            const float v = exact_row[e];
-            raw[i] = 1.0F / (1.0F + expf(-v));
-            const float corrected = raw[i] + bias[e];
-            const std::uint32_t bits = __float_as_uint(corrected);
-            const bool usable = v > -1.0e38F && corrected == corrected;
-            key[i] = usable ? (bits & 0x80000000U ? ~bits : bits | 0x80000000U) : 0U;
-        }
-        float chosen_weight = 0.0F;
-        int chosen_id = 0;
-#pragma unroll 1
-        for (int slot = 0; slot < 8; ++slot) {
-            // lane-local best: higher key, lower id on ties (ids ascend with i, the comparison is strict)
-            std::uint32_t best = key[0];
-            int at = 0;
-#pragma unroll
-            for (int i = 1; i < 8; ++i) {
-                if (key[i] > best) { best = key[i]; at = i; }
-            }
-            const std::uint32_t top = __reduce_max_sync(0xffffffffU, best);
-            float my_raw = 0.0F;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (i == at) my_raw = raw[i];
-            }
-            const int my_id = lane + 32 * at;
-            const int winner = static_cast<int>(__reduce_min_sync(0xffffffffU, best == top ? static_cast<std::uint32_t>(my_id) : 0xffffffffU));
-            const float winner_raw = __shfl_sync(0xffffffffU, my_raw, winner & 31);
-            if ((winner & 31) == lane) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if (i == at) key[i] = 0U;
-                }
-            }
-            if (lane == slot) {
-                chosen_weight = winner_raw;
-                chosen_id = winner;
-            }
-        }
-        float total = 0.0F;
-#pragma unroll
-        for (int slot = 0; slot < 8; ++slot) total += __shfl_sync(0xffffffffU, chosen_weight, slot);
-        const float multiplier = routed_scale / total;
-        if (lane < 8) {
-            ids[static_cast<std::size_t>(token) * kTop + lane] = chosen_id;
-            weights[static_cast<std::size_t>(token) * kTop + lane] = chosen_weight * multiplier;
-        }
-    }
+    // The reference's top-8 over the exact values.  (A selection of its own that gave taken, NaN and left-out experts one and
+    // the same key chose expert 0 again and again once fewer than eight scores were numbers.)
+    warp_top8(exact_row, bias, ids + static_cast<std::size_t>(token) * kTop, weights + static_cast<std::size_t>(token) * kTop,
+              routed_scale);
 }
 
 }  // namespace

@@ -58,3 +58,50 @@ def test_router_at_other_hidden_sizes(cuda, pkg):
             _check(torch, pkg, pkg.MoeBlock(bank, router, bias, plan), rows, x, bias)
             plan.close()
         bank.close()
+
+
+@pytest.mark.parametrize("rows", [9, 17, 64, 257, 300, 2305])
+@pytest.mark.parametrize("what", ["nan row", "infinite row", "six experts left", "nan bias", "infinite bias"])
+def test_router_of_the_block_with_scores_that_are_no_numbers(cuda, pkg, layer0, rows, what):
+    """Whatever a token holds, it names eight different experts, the ones that the exact operators name; and the other tokens
+    of the batch are not touched by it."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    x = synth.make_activations(4600, rows, rows)
+    bias = layer0.bias.clone()
+    odd = torch.zeros(rows, dtype=torch.bool, device="cuda")
+    if what == "nan row":
+        odd[::3] = True
+        x[odd, 11] = float("nan")
+    elif what == "infinite row":
+        odd[1::3] = True
+        x[odd, 11] = float("inf")
+    elif what == "six experts left":
+        bias[:250] = -float("inf")
+    elif what == "nan bias":
+        bias[[0, 5, 31, 40]] = float("nan")
+    else:
+        bias[77] = float("inf")
+    plan = pkg.MoePlan(max_rows=rows)
+    plan.set_path(plan.PATH_TENSOR_CORE)
+    logits = torch.empty((rows, 256), dtype=torch.float32, device="cuda")
+    ids = torch.empty((rows, 8), dtype=torch.int32, device="cuda")
+    weights = torch.empty((rows, 8), dtype=torch.float32, device="cuda")
+    pkg.bf16_gemm_f32(x, layer0.router_weight, logits, rows)
+    pkg.router_top8_rows(logits, bias, ids, weights, rows)
+    out = torch.zeros_like(x)
+    block = pkg.MoeBlock(layer0.bank, layer0.router_weight, bias, plan)
+    block.run_moe_rows(x, out, rows)
+    views = plan.views(rows)
+    assert plan.status() == 0
+    assert torch.equal(views["expert_ids"], ids)
+    ordered = ids.sort(dim=1).values
+    assert int(ordered.min()) >= 0 and int(ordered.max()) <= 255 and bool((ordered[:, 1:] > ordered[:, :-1]).all())
+    assert torch.equal(views["expert_weights"].nan_to_num(nan=-1.0), weights.nan_to_num(nan=-1.0))
+    if bool(odd.any()):
+        clean = torch.where(odd[:, None], torch.zeros_like(x), x)
+        want = torch.zeros_like(x)
+        block.run_moe_rows(clean, want, rows)
+        assert torch.equal(out[~odd].view(torch.int16), want[~odd].view(torch.int16))
+    plan.close()
