@@ -448,7 +448,7 @@ class SingleGpu:
         bytes_call = layer_bytes(d_mean, rows)
         pk = peaks()
         gbs = bytes_call / (us_per_call * 1e-6) / 1e9
-        kernel = "moe_decode_kernel" if rows <= 16 else "expert_tc_kernel (gate/up + down of a %d-launch chain)" % launches_per_call
+        kernel = "moe_decode_kernel" if rows <= 16 else "expert_rows_kernel<0> + expert_down_slab_kernel (gate/up + down of a %d-launch chain)" % launches_per_call
         ratio = ncu_ratios().get("moe_decode_kernel") if rows <= 16 else None
         rec = {
             "ms_per_step": ms, "value": rows / (ms * 1e-3), "unit": "tokens/s", "steps": steps * inner, "repeats": repeats,
@@ -663,7 +663,7 @@ def gpu_decode512_single(gpu: "SingleGpu", steps, warmup, min_seconds, sampler) 
     gbs = layer_bytes(d_mean, rows) * len(blocks) / (ms * 1e-3) / 1e9
     rec = {"ms_per_step": ms, "value": rows / (ms * 1e-3), "repeats": repeats, "status": plan.status(),
            "gpu_launches": plan.last_launches * len(blocks) * steps * repeats,
-           "roofline": {"bound": "hbm", "kernel": "expert_tc_kernel chain", "achieved": gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
+           "roofline": {"bound": "hbm", "kernel": "grouped gate/up and down products of the chain", "achieved": gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
                         "frac": gbs / pk["hbm_gbs"], "peak_source": pk["source"], "traffic": None,
                         "distinct_routed_experts_mean": d_mean}}
     plan.close()
@@ -792,7 +792,7 @@ class ExpertParallel:
             "gpu_launches": (launches * n_layers * steps * repeats) if launches else None,
             "us_per_layer_call": ms * 1e3 / n_layers,
             "roofline": {"bound": "hbm", "kernel": "moe_decode_ep_kernel (per-GPU shard)" if mode == "fused"
-                         else "expert_tc_kernel (per-GPU shard)", "achieved": gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
+                         else "grouped gate/up and down products (per-GPU shard)", "achieved": gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": gbs / pk["hbm_gbs"], "traffic": None, "peak_source": pk["source"],
                          "bytes_per_launch": bytes_call, "distinct_local_experts_last_layer": distinct,
                          "note": "per-GPU fraction of rank 0: its shard's bytes per layer over the step time"},
