@@ -15,6 +15,10 @@
  *     is the default stream) and use the CURRENT device; they are ordered like
  *     any work of a stream: every array that a call reads, parameters included,
  *     may be the output of the call queued just before it;
+ *   - rows of BF16 that a call reads, and the block's output rows, start on a
+ *     16-byte boundary; others are refused with cudaErrorInvalidValue unless
+ *     the call has a form for them (element-wise operators, RMSNorm, output of
+ *     the dense MLP);
  *   - the return value is a cudaError_t: 0 success, cudaErrorInvalidValue for
  *     bad arguments, cudaErrorMemoryAllocation, cudaErrorNotSupported, or the
  *     launch error reported right after the launch

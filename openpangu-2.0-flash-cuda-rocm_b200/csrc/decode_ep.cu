@@ -872,7 +872,8 @@ int p92b_ep_forward_fused(p92b_plan* plan, const p92b_bank* bank, p92b_ep_window
                           float routed_scale, void* stream_) {
     using namespace p92b;
     if (plan == nullptr || bank == nullptr || window == nullptr || input == nullptr || router_weight == nullptr ||
-        correction_bias == nullptr || output == nullptr || rows <= 0 || rows > window->rows_per_gpu) {
+        correction_bias == nullptr || output == nullptr || rows <= 0 || rows > window->rows_per_gpu ||
+        !aligned_to(16, input, router_weight) || !aligned_to(8, output)) {
         return cudaErrorInvalidValue;
     }
     if (window->bulk) return cudaErrorNotSupported;     // a large-batch window has another layout

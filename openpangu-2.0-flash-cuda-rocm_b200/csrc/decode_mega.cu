@@ -938,6 +938,7 @@ cudaError_t launch_decode_mega(p92b_plan* plan, const p92b_bank* bank, const std
         plan->intermediate != 1024) {
         return cudaErrorNotSupported;
     }
+    if (!aligned_to(16, x, router_w) || (post_norm_w == nullptr && !aligned_to(8, out))) return cudaErrorInvalidValue;
     const auto kernel = rows <= kHalfTileRows ? moe_decode_kernel<8, true> : rows <= 8 ? moe_decode_kernel<8, false> : moe_decode_kernel<16, false>;
     cudaError_t st = rows <= kHalfTileRows ? ensure_dynamic_smem<moe_decode_kernel<8, true>>(kMegaSmem)
                      : rows <= 8           ? ensure_dynamic_smem<moe_decode_kernel<8, false>>(kMegaSmem)

@@ -166,9 +166,6 @@ __device__ __forceinline__ uint4 pack_bf16x8(const float (&v)[8]) {
     }
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
-__host__ inline bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr) {
-    return ((reinterpret_cast<std::uintptr_t>(a) | reinterpret_cast<std::uintptr_t>(b) | reinterpret_cast<std::uintptr_t>(c)) & 15U) == 0U;
-}
 
 // SwiGLU, bf16( g / (1 + expf(-g)) * u ) with the fast-math expf and division of cuda/nvfp4_ops.cu:97-105.
 __device__ __forceinline__ float silu_times(float g, float u) { return (g / (1.0F + expf(-g))) * u; }
@@ -412,7 +409,9 @@ inline unsigned blocks_for(long n, int per_block) { return static_cast<unsigned>
 
 cudaError_t launch_quantize(const std::uint16_t* input, std::uint8_t* output, std::uint8_t* scales,
                             long groups, float global_scale, cudaStream_t stream, bool pdl) {
-    if (input == nullptr || output == nullptr || scales == nullptr || groups <= 0) return cudaErrorInvalidValue;
+    if (input == nullptr || output == nullptr || scales == nullptr || groups <= 0 || !aligned_to(16, input) || !aligned_to(8, output)) {
+        return cudaErrorInvalidValue;
+    }
     return launch_kernel(quantize_kernel, dim3(blocks_for(groups, 256)), dim3(256), 0, stream, pdl, input, output, scales, groups,
                          global_scale, static_cast<const float*>(nullptr));
 }
@@ -420,6 +419,7 @@ cudaError_t launch_quantize(const std::uint16_t* input, std::uint8_t* output, st
 cudaError_t launch_combine_shared(const std::uint16_t* mixed, const std::int32_t* mixed_index,
                                   const float* route_weights, std::uint16_t* output, int rows,
                                   int hidden, cudaStream_t stream, bool pdl) {
+    if (!aligned_to(16, output)) return cudaErrorInvalidValue;
     dim3 grid(blocks_for(hidden / 8, 256), rows);
     return launch_kernel(combine_shared_kernel, grid, dim3(256), 0, stream, pdl, mixed, mixed_index, route_weights,
                          output, rows, hidden);
@@ -476,7 +476,7 @@ int p92b_nvfp4_swizzle_scales(const uint8_t* linear, uint8_t* swizzled, int rows
 int p92b_nvfp4_pack_weight(const uint16_t* input, uint8_t* packed, uint8_t* scales, size_t elements,
                            float* weight_scale_2, void* stream) {
     if (input == nullptr || packed == nullptr || scales == nullptr || weight_scale_2 == nullptr ||
-        elements == 0 || elements % 16 != 0) {
+        elements == 0 || elements % 16 != 0 || !aligned_to(16, input) || !aligned_to(8, packed)) {
         return cudaErrorInvalidValue;
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -494,7 +494,8 @@ int p92b_nvfp4_pack_weight(const uint16_t* input, uint8_t* packed, uint8_t* scal
 int p92b_nvfp4_pack_weight_batch(const uint16_t* input, uint8_t* packed, uint8_t* scales, size_t elements_per_matrix,
                                  int matrices, float* weight_scale_2, void* stream) {
     if (input == nullptr || packed == nullptr || scales == nullptr || weight_scale_2 == nullptr || matrices <= 0 ||
-        matrices > 65535 || elements_per_matrix == 0 || elements_per_matrix % 16 != 0) {
+        matrices > 65535 || elements_per_matrix == 0 || elements_per_matrix % 16 != 0 || !aligned_to(16, input) ||
+        !aligned_to(8, packed)) {
         return cudaErrorInvalidValue;
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -513,7 +514,7 @@ int p92b_nvfp4_pack_weight_batch(const uint16_t* input, uint8_t* packed, uint8_t
 
 int p92b_swiglu(const uint16_t* gate, const uint16_t* up, uint16_t* output, int elements, void* stream) {
     if (gate == nullptr || up == nullptr || output == nullptr || elements <= 0) return cudaErrorInvalidValue;
-    const long vectors = aligned16(gate, up, output) ? elements / 8 : 0;
+    const long vectors = aligned_to(16, gate, up, output) ? elements / 8 : 0;
     return launch_kernel(swiglu_kernel, dim3(blocks_for(vectors + (elements - vectors * 8), 256)), dim3(256), 0,
                          static_cast<cudaStream_t>(stream), pdl_enabled(), gate, up, output, elements, vectors);
 }
@@ -524,7 +525,7 @@ int p92b_expert_combine_rows(const uint16_t* expert_rows, const float* route_wei
         experts <= 0 || elements <= 0) {
         return cudaErrorInvalidValue;
     }
-    const int vectors = aligned16(expert_rows, output) && elements % 8 == 0 ? elements / 8 : 0;
+    const int vectors = aligned_to(16, expert_rows, output) && elements % 8 == 0 ? elements / 8 : 0;
     dim3 grid(blocks_for(vectors + (elements - vectors * 8), 256), batch_rows);
     return launch_kernel(combine_rows_kernel, grid, dim3(256), 0, static_cast<cudaStream_t>(stream), pdl_enabled(), expert_rows,
                          route_weights, output, experts, elements, vectors);
@@ -549,7 +550,7 @@ int p92b_rmsnorm_strided(const uint16_t* input, int input_stride, const uint16_t
 
 int p92b_add_inplace(uint16_t* destination, const uint16_t* source, int elements, void* stream) {
     if (destination == nullptr || source == nullptr || elements <= 0) return cudaErrorInvalidValue;
-    const long vectors = aligned16(destination, source) ? elements / 8 : 0;
+    const long vectors = aligned_to(16, destination, source) ? elements / 8 : 0;
     return launch_kernel(add_kernel, dim3(blocks_for(vectors + (elements - vectors * 8), 256)), dim3(256), 0,
                          static_cast<cudaStream_t>(stream), pdl_enabled(), destination, source, elements, vectors);
 }

@@ -910,6 +910,7 @@ int tc_pad_align(int rows) { (void)rows; return 128; }
 cudaError_t launch_quantize_padded(const p92b_plan* plan, const std::uint16_t* x, int rows, cudaStream_t stream,
                                    bool pdl) {
     if (plan->hidden > 4096) return cudaErrorNotSupported;
+    if (!aligned_to(16, x)) return cudaErrorInvalidValue;
     const bool few = rows <= 1024;
     return launch_kernel(few ? quantize_padded_kernel<8> : quantize_padded_kernel<1>, dim3(few ? rows : (rows + 7) / 8), dim3(256), 0,
                          stream, pdl, x, static_cast<const std::int32_t*>(plan->pp_of_flat), plan->xq_pp, plan->xs_sw, rows,
@@ -918,7 +919,9 @@ cudaError_t launch_quantize_padded(const p92b_plan* plan, const std::uint16_t* x
 
 cudaError_t launch_quantize_rows_to_pp(const std::uint16_t* x, const std::int32_t* index, std::uint8_t* xq,
                                        std::uint8_t* xs, int n, int width, cudaStream_t stream, bool pdl) {
-    if (x == nullptr || xq == nullptr || xs == nullptr || n <= 0 || width <= 0 || width % 64 != 0) return cudaErrorInvalidValue;
+    if (x == nullptr || xq == nullptr || xs == nullptr || n <= 0 || width <= 0 || width % 64 != 0 || !aligned_to(16, x)) {
+        return cudaErrorInvalidValue;
+    }
     return launch_kernel(quantize_rows_to_pp_kernel, dim3((n + 7) / 8), dim3(256), 0, stream, pdl, x, index, xq, xs, n, width,
                          1.0F);
 }

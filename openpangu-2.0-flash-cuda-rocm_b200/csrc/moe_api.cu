@@ -65,7 +65,7 @@ int p92b_bank_create(p92b_bank** out, const p92b_expert_projection* host_entries
     const int entries = local_experts + 1;
     for (int i = 0; i < entries * 3; ++i) {
         if (host_entries[i].weight == nullptr || host_entries[i].scales_swizzled == nullptr ||
-            host_entries[i].alpha == nullptr) {
+            host_entries[i].alpha == nullptr || !aligned_to(16, host_entries[i].weight, host_entries[i].scales_swizzled)) {
             return cudaErrorInvalidValue;
         }
     }
@@ -488,6 +488,7 @@ int p92b_dense_forward(p92b_plan* plan, const p92b_bank* bank, const uint16_t* i
         return cudaErrorInvalidValue;
     }
     if (!plan->tc_ready || !bank->tc_ready) return cudaErrorNotSupported;
+    if (!aligned_to(16, input)) return cudaErrorInvalidValue;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     static const bool pdl = std::getenv("P92B_NO_PDL") == nullptr;
     plan->last_launches = 0;

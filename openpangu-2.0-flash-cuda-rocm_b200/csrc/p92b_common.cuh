@@ -393,6 +393,13 @@ cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, std::
     return cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
 }
 
+// Whether all pointers start on a multiple of `bytes` (a power of two).  Rows that a kernel reads or writes 8 or 16 bytes at
+// a time have to; calls with others are refused here, where the load would fault.
+template <class... P>
+inline bool aligned_to(std::size_t bytes, const P*... pointers) {
+    return ((reinterpret_cast<std::uintptr_t>(pointers) | ...) & (bytes - 1)) == 0U;
+}
+
 // Programmatic dependent launch is on unless P92B_NO_PDL is set (A/B timing).
 inline bool pdl_enabled() {
     static const bool on = std::getenv("P92B_NO_PDL") == nullptr;

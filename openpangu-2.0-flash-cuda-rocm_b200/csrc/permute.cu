@@ -589,7 +589,7 @@ cudaError_t launch_dense_front(p92b_plan* plan, const std::uint16_t* x, int rows
 
 cudaError_t launch_route_fused(p92b_plan* plan, const float* bias, float routed_scale, const std::uint16_t* x,
                                int rows, int pad_align, int tile_rows, cudaStream_t stream, bool pdl) {
-    if (rows <= 0 || rows > kFusedMaxRows) return cudaErrorInvalidValue;
+    if (rows <= 0 || rows > kFusedMaxRows || !aligned_to(16, x)) return cudaErrorInvalidValue;
     RouteLists lists {};
     lists.counts = plan->counts;
     lists.offsets = plan->offsets;

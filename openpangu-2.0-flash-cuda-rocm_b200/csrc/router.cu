@@ -360,7 +360,9 @@ cudaError_t launch_router_logits(const std::uint16_t* x, const std::uint16_t* w,
     if (gemv_order) {
         if (batch_rows != 1) return cudaErrorInvalidValue;
         return launch_kernel(logits_gemv_kernel, dim3(rows), dim3(256), 0, stream, pdl, x, w, out, rows, columns);
-    } else if (batch_rows <= 8) {
+    }
+    if (!aligned_to(16, x, w)) return cudaErrorInvalidValue;         // the forms below copy 16 bytes at a time
+    if (batch_rows <= 8) {
         // decode: the whole K extent of two expert rows and of every token in shared memory
         if (static_cast<std::size_t>(12) * columns * 2 > 200 * 1024) return cudaErrorInvalidValue;
         const dim3 grid((rows + 1) / 2);
