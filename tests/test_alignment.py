@@ -46,6 +46,7 @@ def test_block_refuses_rows_it_cannot_load(cuda, pkg, layer0, rows):
     torch = cuda
     bf16 = torch.bfloat16
     plan = pkg.MoePlan(max_rows=rows)
+    plan.set_path(plan.PATH_AUTO)
     block = pkg.MoeBlock(layer0.bank, layer0.router_weight, layer0.bias, plan)
     x, out = torch.zeros((rows, HIDDEN), dtype=bf16, device="cuda"), torch.zeros((rows, HIDDEN), dtype=bf16, device="cuda")
     _refused(pkg, block.run_moe_rows, _off(torch, (rows, HIDDEN), bf16), out, rows)

@@ -70,6 +70,7 @@ def test_decode_rows_equal_the_large_batch_at_both_gate_up_tiles(cuda, pkg, laye
     x = synth.make_activations(78, 0, 64)
     want = torch.empty_like(x)
     plan = pkg.MoePlan(max_rows=64)
+    plan.set_path(plan.PATH_AUTO)
     block = pkg.MoeBlock(layer0.bank, layer0.router_weight, layer0.bias, plan)
     block.run_moe_rows(x, want, 64)
     for rows in (2, 3, 4, 5, 8, 9, 15, 16):
