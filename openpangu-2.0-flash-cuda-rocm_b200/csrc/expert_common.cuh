@@ -120,5 +120,8 @@ __device__ __forceinline__ std::uint32_t bf16x2_bits(float low, float high) {
 // Large-batch products with the tokens on the M side (expert_rows.cu); p.tile_prefix counts 128-row tiles.
 cudaError_t launch_expert_rows_gate_up(const p92b_plan* plan, const expert::TcParams& p, cudaStream_t stream, bool pdl);
 cudaError_t launch_expert_rows_matrix(const p92b_plan* plan, expert::TcParams p, cudaStream_t stream, bool pdl);
+// Down product whose token rows stay in shared memory, where the K extent allows it; the one kernel that honours row_dest.
+bool down_slab_shape(int hidden, int intermediate);
+cudaError_t launch_expert_down_slab(const p92b_plan* plan, const expert::TcParams& p, cudaStream_t stream, bool pdl);
 
 }  // namespace p92b

@@ -405,7 +405,303 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
     }
 }
 
+// ---- down product whose token rows stay in shared memory ----------------------------------------------------
+// For a K extent of up to 1,024 a 128-token slab with all its K blocks (64 KB) and scale slabs (8 KB) is loaded ONCE per item and
+// only the weights stream past it, chunk by chunk of the bank; the slab's scale factors stay in TMEM.  An item is a slab and
+// all of the 128-row tiles of the weight, or half of them.
+// A tile is 1,024 cycles of products and 32 KB of results, so what happens between the accumulator and memory decides.  Two
+// teams of eight warps have an accumulator each and take the tiles in turn: a team has two tiles' time, and while one of them
+// stores the other reads; the weights of the first four chunks are requested before the wait for the gate/up kernel.  With the
+// weights on the M side and the results turned round through shared memory (the form before): 281 us at 16,384 tokens, even
+// routing, now 262 (1.2 GB, of which 755 MB are written); 4,096 skewed 119, now 110; 512 72, now 69.  One team of sixteen warps on one
+// accumulator of 256 columns took 283.
+struct Slab {
+    static constexpr int kKBlocksMax = 4;
+    static constexpr int kChunksMax = kKBlocksMax / 2;
+    static constexpr int kOffSf = kKBlocksMax * kTok * kBlockKBytes;                // scale slabs behind the boxes
+    static constexpr int kBytes = kOffSf + kKBlocksMax * kSfSlab;                   // 73,728
+    static constexpr int kStages = 4;                                               // of one chunk: 128 weight rows, two K blocks
+    static constexpr int kTeams = 2;
+    static constexpr int kTeamWarps = kEpiWarps / kTeams;
+    static constexpr int kBarriers = 2 * kStages + kChunksMax + 2 * kTeams;
+    static constexpr int kSmem = kBytes + kStages * kChunkBytes + kBarriers * 8 + 16 + 1024;
+    // TMEM: two accumulators, the slab's scale factors (16 columns per K block), two buffers of a chunk's (32)
+    static constexpr int kSfT = kTeams * kTileM, kSfW = kSfT + kKBlocksMax * 16;
+    // Whole slabs once there are enough of them to share out evenly; with three slabs per SM halves balance better.
+    static constexpr int kMaxGroups = 2;
+    static constexpr int kWholeSlabsPerSm = 6;
+};
+
+// 32 bytes of a row in two 16-byte halves.
+struct Piece32 {
+    uint4 lo, hi;
+};
+__device__ __forceinline__ void store_piece32(void* to, const Piece32& v) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(to), "r"(v.lo.x), "r"(v.lo.y), "r"(v.lo.z),
+                 "r"(v.lo.w), "r"(v.hi.x), "r"(v.hi.y), "r"(v.hi.z), "r"(v.hi.w) : "memory");
+}
+__device__ __forceinline__ uint4 shfl_xor4(uint4 v, int d) {
+    return make_uint4(__shfl_xor_sync(0xffffffffU, v.x, d), __shfl_xor_sync(0xffffffffU, v.y, d), __shfl_xor_sync(0xffffffffU, v.z, d),
+                      __shfl_xor_sync(0xffffffffU, v.w, d));
+}
+// Lane l holds row l's 64 values as four pieces of 32 bytes; afterwards piece (lane & 3) of rows (lane & ~3) + 0 .. 3: four lanes
+// then store a whole 128-byte line, eight lines per instruction.
+__device__ __forceinline__ void exchange_rows64(Piece32 (&w)[4]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 2; d >= 1; d >>= 1) {
+        const bool upper = (lane & d) != 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if ((q & d) != 0) continue;
+            const Piece32 give = upper ? w[q] : w[q + d];
+            const Piece32 got = {shfl_xor4(give.lo, d), shfl_xor4(give.hi, d)};
+            if (upper) w[q] = got; else w[q + d] = got;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, 1) expert_down_slab_kernel(const __grid_constant__ CUtensorMap map_t32,
+                                                                       const __grid_constant__ CUtensorMap map_t128, const TcParams p) {
+    extern __shared__ std::uint8_t smem_raw[];
+    __shared__ RouteTable route_table;
+    const std::uint32_t base = (smem_u32(smem_raw) + 1023U) & ~1023U;
+    const std::uint32_t ring = base + Slab::kBytes;
+    const std::uint32_t bars = ring + Slab::kStages * kChunkBytes;
+    auto full_bar = [&](int s) { return bars + 8U * s; };
+    auto empty_bar = [&](int s) { return bars + 8U * (Slab::kStages + s); };
+    auto slab_empty = [&](int c) { return bars + 8U * (2 * Slab::kStages + c); };
+    auto accum_full = [&](int t) { return bars + 8U * (2 * Slab::kStages + Slab::kChunksMax + t); };
+    auto accum_empty = [&](int t) { return bars + 8U * (2 * Slab::kStages + Slab::kChunksMax + Slab::kTeams + t); };
+    const std::uint32_t tmem_slot = bars + 8U * Slab::kBarriers;
+    volatile std::uint32_t* tmem_slot_ptr =
+        reinterpret_cast<volatile std::uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+    volatile std::uint32_t* abort_ptr = tmem_slot_ptr + 1;
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int chunks = p.k_bytes / kBlockKBytes / 2;            // <= 2
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < Slab::kStages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        for (int c = 0; c < Slab::kChunksMax; ++c) mbar_init(slab_empty(c), 1);
+        for (int t = 0; t < Slab::kTeams; ++t) {
+            mbar_init(accum_full(t), 1);
+            mbar_init(accum_empty(t), Slab::kTeamWarps);
+        }
+        *abort_ptr = 0;
+        fence_mbar_init();
+        prefetch_tensormap(&map_t32);
+        prefetch_tensormap(&map_t128);
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, kTmemAll);
+        tmem_relinquish();
+    }
+    // The SwiGLU rows come from the kernel just upstream, the routing lists from one further up.  Only the producer lane waits, and
+    // not before the ring is full of weights: as the blocks of the gate/up kernel leave, the memory already works for this one.
+    if (p.routing_is_upstream) pdl_wait();
+    load_route_table(p, &route_table);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_launch_dependents();
+    const std::uint32_t tmem_base = *tmem_slot_ptr;
+    const int slabs = route_table.prefix[route_table.active_count];                 // the prefix counts 128-row slabs here
+    const int groups = slabs >= Slab::kWholeSlabsPerSm * static_cast<int>(gridDim.x) ? 1 : Slab::kMaxGroups;
+    const int total_items = slabs * groups;
+    auto give_up = [&]() {
+        *abort_ptr = 1;
+        atomicCAS(p.status, kStatusOk, kStatusWaitExpired);
+    };
+    // item -> slab and the tiles [it->m_tile, *last) of the weight
+    auto decode = [&](int item, Item* it, int* last) {
+        const int slab = item / groups;
+        const int group = item - slab * groups;
+        const bool ok = decode_item<kTok>(p, route_table, slab * p.m_tiles, it);
+        it->m_tile = p.m_tiles * group / groups;
+        *last = p.m_tiles * (group + 1) / groups;
+        return ok;
+    };
+
+    if (warp == 0) {
+        if (elect_one()) {
+            int stage = 0;
+            std::uint32_t phase = 0, slab_phase = 0;
+            bool ok = true, upstream_done = p.routing_is_upstream != 0;
+            int requested = 0;                              // chunks of the first item whose weights were asked for before the wait
+            for (int item = blockIdx.x; item < total_items && !*abort_ptr && ok; item += gridDim.x) {
+                Item it;
+                int last;
+                if (!decode(item, &it, &last)) continue;
+                const int boxes = (it.valid + 31) >> 5;         // rows beyond the slab's last one are not loaded
+                const std::uint8_t* t_sf = p.b_sf + static_cast<std::size_t>(it.pp0 >> 7) * (p.k_bytes / 32) * 512;
+                const std::uint32_t slab_bytes = 2 * (boxes * (32 * kBlockKBytes) + kSfSlab);
+                const std::uint8_t* weights = p.bank.g2 + (static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * chunks * kChunkBytes;
+                auto request = [&](int s, int n) {          // chunk n of the item into stage s
+                    mbar_arrive_expect_tx(full_bar(s), kChunkBytes + (n < chunks ? slab_bytes : 0U));
+                    bulk_load(ring + s * kChunkBytes, weights + static_cast<std::size_t>(n) * kChunkBytes, kChunkBytes, full_bar(s));
+                };
+                if (!upstream_done) {
+                    requested = min(Slab::kStages, (last - it.m_tile) * chunks);
+                    for (int n = 0; n < requested; ++n) request(n, n);
+                    pdl_wait();
+                    upstream_done = true;
+                }
+                const int total = (last - it.m_tile) * chunks;
+                for (int n = 0; n < total; ++n) {
+                    if (n >= requested) {
+                        if (!mbar_wait(empty_bar(stage), phase ^ 1U)) { give_up(); ok = false; break; }
+                        request(stage, n);
+                    }
+                    if (n < chunks) {
+                        // two K blocks of the slab follow as soon as the last products on the one before have read their place
+                        if (!mbar_wait(slab_empty(n), slab_phase ^ 1U)) { give_up(); ok = false; break; }
+#pragma unroll
+                        for (int o = 0; o < 2; ++o) {
+                            const int kb = 2 * n + o;
+                            const std::uint32_t to = base + kb * kTok * kBlockKBytes;
+                            if (boxes == 4) {
+                                tma_load_2d(to, &map_t128, full_bar(stage), kb * kBlockKBytes, it.pp0);
+                            } else {
+                                for (int b = 0; b < boxes; ++b) {
+                                    tma_load_2d(to + b * 32 * kBlockKBytes, &map_t32, full_bar(stage), kb * kBlockKBytes, it.pp0 + b * 32);
+                                }
+                            }
+                            bulk_load(base + Slab::kOffSf + kb * kSfSlab, t_sf + static_cast<std::size_t>(kb) * 4 * 512, kSfSlab, full_bar(stage));
+                        }
+                    }
+                    if (++stage == Slab::kStages) { stage = 0; phase ^= 1U; }
+                }
+                requested = 0;
+                slab_phase ^= 1U;
+            }
+            if (!upstream_done) pdl_wait();                 // no work at all: still order this grid after its predecessor
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
+            int stage = 0, turn = 0;                            // tiles so far
+            std::uint32_t phase = 0;
+            int sf_buffer = 0;
+            bool ok = true;
+            constexpr std::uint32_t idesc = idesc_nvf4(kTok, kTileM);
+            for (int item = blockIdx.x; item < total_items && !*abort_ptr && ok; item += gridDim.x) {
+                Item it;
+                int last;
+                if (!decode(item, &it, &last)) continue;
+                for (int tile = it.m_tile; tile < last && ok; ++tile, ++turn) {
+                    const int team = turn & 1;
+                    const std::uint32_t accum = tmem_base + team * kTileM;
+                    for (int c = 0; c < chunks; ++c) {
+                        if (!mbar_wait(full_bar(stage), phase)) { give_up(); ok = false; break; }
+                        if (c == 0 && !mbar_wait(accum_empty(team), ((turn >> 1) & 1U) ^ 1U)) { give_up(); ok = false; break; }
+                        tc_fence_after();
+                        const std::uint32_t st = ring + stage * kChunkBytes;
+                        const std::uint32_t sf_w = tmem_base + Slab::kSfW + sf_buffer * 32;
+#pragma unroll
+                        for (int o = 0; o < 2; ++o) {
+                            const int kb = 2 * c + o;
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                if (tile == it.m_tile) tc_copy_sf(tmem_base + Slab::kSfT + kb * 16 + k * 4, desc_scale_atom(base + Slab::kOffSf + kb * kSfSlab + k * 512));
+                                tc_copy_sf(sf_w + o * 16 + k * 4, desc_scale_atom(st + kChunkScaleOffset + o * kChunkScaleBytes + k * 512));
+                            }
+                        }
+#pragma unroll
+                        for (int o = 0; o < 2; ++o) {
+                            const int kb = 2 * c + o;
+                            const std::uint64_t a_desc = desc_k_major_sw128(base + kb * kTok * kBlockKBytes);
+                            const std::uint64_t b_desc = desc_k_major_sw128(st + o * kChunkBox);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                mma_nvf4(accum, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_base + Slab::kSfT + kb * 16 + k * 4, sf_w + o * 16 + k * 4,
+                                         kb > 0 || k > 0);
+                            }
+                        }
+                        tc_commit(empty_bar(stage));
+                        if (tile == last - 1) tc_commit(slab_empty(c));
+                        sf_buffer ^= 1;
+                        if (++stage == Slab::kStages) { stage = 0; phase ^= 1U; }
+                    }
+                    if (!ok) break;
+                    tc_commit(accum_full(team));
+                }
+            }
+        }
+    } else {
+        const int quarter = warp & 3;
+        const int team = (warp - 2) / Slab::kTeamWarps;
+        const int half = ((warp - 2) >> 2) & 1;             // which 64 of the tile's 128 output columns
+        const std::uint32_t accum = tmem_base + (static_cast<std::uint32_t>(quarter * 32) << 16) + team * kTileM + half * 64;
+        int turn = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < total_items && !*abort_ptr && ok; item += gridDim.x) {
+            Item it;
+            int last;
+            if (!decode(item, &it, &last)) continue;
+            const float alpha = p.bank.alpha[it.entry * 3 + 2];
+            const int valid = it.valid - quarter * 32;      // rows of this warp; warp uniform
+            // where the four rows that this lane stores parts of go: their places in the padded position space or, with a
+            // table, anywhere
+            std::uint16_t* rows4[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int from = (lane & ~3) + r;
+                const int pp = it.pp0 + quarter * 32 + from;
+                rows4[r] = p.row_dest == nullptr ? p.out + static_cast<std::size_t>(pp) * p.m_total : from < valid ? p.row_dest[pp] : p.out;
+                rows4[r] += half * 64 + (lane & 3) * 16;
+            }
+            for (int tile = it.m_tile; tile < last; ++tile, ++turn) {
+                if ((turn & 1) != team) continue;
+                if (!mbar_wait(accum_full(team), (turn >> 1) & 1U)) { give_up(); ok = false; break; }
+                tc_fence_after();
+                Piece32 w[4];
+                if (valid > 0) {
+                    std::uint32_t v[32];
+                    tmem_load32(accum, v);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) w[q] = {scale_to_bf16x8(v + q * 16, alpha), scale_to_bf16x8(v + q * 16 + 8, alpha)};
+                    tmem_load32(accum + 32, v);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) w[2 + q] = {scale_to_bf16x8(v + q * 16, alpha), scale_to_bf16x8(v + q * 16 + 8, alpha)};
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accum_empty(team));
+                if (valid <= 0) continue;
+                exchange_rows64(w);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    if ((lane & ~3) + r < valid) store_piece32(rows4[r] + tile * kTileM, w[r]);
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, kTmemAll);
+    }
+}
+
 }  // namespace
+
+bool down_slab_shape(int hidden, int intermediate) {
+    const int k_blocks = intermediate / 2 / kBlockKBytes;
+    return k_blocks <= Slab::kKBlocksMax && k_blocks % 2 == 0 && hidden % (Slab::kMaxGroups * kTileM) == 0;
+}
+
+cudaError_t launch_expert_down_slab(const p92b_plan* plan, const TcParams& p, cudaStream_t stream, bool pdl) {
+    if (cudaError_t st = ensure_dynamic_smem<expert_down_slab_kernel>(Slab::kSmem); st != cudaSuccess) return st;
+    return launch_kernel(expert_down_slab_kernel, dim3(plan->sm_count), dim3(kThreads), Slab::kSmem, stream, pdl, plan->map_h[1],
+                         plan->map_h[3], p);
+}
 
 cudaError_t launch_expert_rows_gate_up(const p92b_plan* plan, const TcParams& p, cudaStream_t stream, bool pdl) {
     if (cudaError_t st = ensure_dynamic_smem<expert_rows_kernel<0>>(Stage::kSmem); st != cudaSuccess) return st;

@@ -23,8 +23,7 @@
 //           up rows un-fused (MODE 2, the reference's project_expert_gate_up result).
 // Every role turns an item number into work from a copy of the routing lists in shared memory (RouteTable), and an
 // epilogue warp hands its accumulator buffer back as soon as it has read its columns into registers.
-// expert_down_slab_kernel serves the down product of large batches with the same three roles (a 128-token slab resident,
-// weights streaming past); their gate/up product, with the tokens on the M side, is in expert_rows.cu.
+// The products of more than 32 rows, with the tokens on the M side, are in expert_rows.cu.
 // Scale factors stay in the 128x4-tiled layout the reference keeps them in
 // (cuda/nvfp4_ops.cu:869-890): one 512-byte tile is exactly one tcgen05.cp atom.
 //
@@ -483,280 +482,6 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
     }
 }
 
-// ---- down product for large batches: the token slab stays in shared memory ---------------------------------
-// In the tile-by-tile down kernel half of what a block loads is the token slab, fetched again for each of the 20
-// row tiles of the weight, and a ring stage that waits for it is a stage less of weights in flight.  Here an item is (128-token slab of an expert, half of the row
-// tiles): the slab's four K blocks (64 KB) and their scale slabs (8 KB) are loaded ONCE and stay resident, their
-// scale factors stay in TMEM, and only weight chunks stream through the ring - half the bytes per result.
-// Needs the whole K extent of a slab in shared memory: intermediate sizes up to 1024.
-struct DownSlab {
-    static constexpr int kN = 128;
-    static constexpr int kKBlocksMax = 4;
-    static constexpr int kBBytes = kKBlocksMax * (kN * kBlockKBytes + kSfSlab);     // 73,728
-    static constexpr int kOffBSf = kKBlocksMax * kN * kBlockKBytes;                 // scale slabs behind the boxes
-    static constexpr int kStages = 3;                                               // one chunk (two K blocks of the weight) each
-    static constexpr int kStageBytes = kChunkBytes;
-    static constexpr int kStoreBytes = 16 * 32 * 2;                                 // per epilogue warp (a group of four shares 4 KB): 16 tokens x 32 rows of BF16
-    static constexpr int kAccumBuffers = 2;
-    static constexpr int kSfbCols = kKBlocksMax * 16;                               // resident for an item
-    static constexpr int kSfaCols = 2 * 16;                                         // per chunk, two buffers
-    static constexpr int kTmemCols = 512;                                           // 2 * 128 + 64 + 2 * 32 = 384
-    static constexpr int kBarriers = 2 + 2 * kStages + 2 * kAccumBuffers;
-    static constexpr int kSmemBytes = kBBytes + kStages * kStageBytes + kEpilogueWarps * kStoreBytes + kBarriers * 8 + 16 + 1024;
-    // An item is a slab and all of its row tiles, or half of them.  Between two items the tensor pipe waits for the next slab,
-    // so whole slabs are better (16,384 tokens: 289 us against 300) once there are enough of them to share out evenly; with
-    // three slabs per SM halves balance better (4,096 tokens: 118 us against 131; 64: 56 against 63).
-    static constexpr int kMaxGroups = 2;
-    static constexpr int kWholeSlabsPerSm = 6;
-};
-
-// Named barriers over the 128 threads of one epilogue group (barrier 0 is __syncthreads).
-__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
-__device__ __forceinline__ bool group_all(bool mine, int id) {
-    std::uint32_t all;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, %2, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(all)
-        : "r"(static_cast<std::uint32_t>(mine)), "r"(id)
-        : "memory");
-    return all != 0U;
-}
-
-__global__ void __launch_bounds__(kThreadsTc, 1) expert_down_slab_kernel(const __grid_constant__ CUtensorMap map_b,
-                                                                         const TcParams p) {
-    using C = DownSlab;
-    extern __shared__ std::uint8_t smem_raw[];
-    __shared__ RouteTable route_table;
-    const std::uint32_t base = (smem_u32(smem_raw) + 1023U) & ~1023U;
-    const std::uint32_t ring = base + C::kBBytes;
-    const std::uint32_t store_area = ring + C::kStages * C::kStageBytes;
-    const std::uint32_t bars = store_area + kEpilogueWarps * C::kStoreBytes;
-    const std::uint32_t b_full = bars, b_empty = bars + 8U;
-    auto weight_bar = [&](int s) { return bars + 8U * (2 + s); };
-    auto empty_bar = [&](int s) { return bars + 8U * (2 + C::kStages + s); };
-    auto accum_full = [&](int b) { return bars + 8U * (2 + 2 * C::kStages + b); };
-    auto accum_empty = [&](int b) { return bars + 8U * (2 + 2 * C::kStages + C::kAccumBuffers + b); };
-    const std::uint32_t tmem_slot = bars + 8U * C::kBarriers;
-    volatile std::uint32_t* tmem_slot_ptr =
-        reinterpret_cast<volatile std::uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
-    volatile std::uint32_t* abort_ptr = tmem_slot_ptr + 1;
-
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int k_blocks = p.k_bytes / kBlockKBytes;              // <= 4, even
-    const int chunks = k_blocks / 2;
-
-    if (threadIdx.x == 0) {
-        mbar_init(b_full, 1);
-        mbar_init(b_empty, 1);
-        for (int s = 0; s < C::kStages; ++s) {
-            mbar_init(weight_bar(s), 1);
-            mbar_init(empty_bar(s), 1);
-        }
-        for (int b = 0; b < C::kAccumBuffers; ++b) {
-            mbar_init(accum_full(b), 1);
-            mbar_init(accum_empty(b), kEpilogueWarps);
-        }
-        *abort_ptr = 0;
-        fence_mbar_init();
-        prefetch_tensormap(&map_b);
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, C::kTmemCols);
-        tmem_relinquish();
-    }
-    pdl_wait();                       // routing lists and the SwiGLU rows come from the kernels upstream
-    load_route_table(p, &route_table);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    pdl_launch_dependents();
-    const std::uint32_t tmem_base = *tmem_slot_ptr;
-    const int slabs = route_table.prefix[route_table.active_count];                         // the prefix counts 128-row slabs here
-    const int groups = slabs >= C::kWholeSlabsPerSm * static_cast<int>(gridDim.x) ? 1 : C::kMaxGroups;
-    const int tiles_per_group = p.m_tiles / groups;
-    const int total_items = slabs * groups;
-    auto give_up = [&]() {
-        *abort_ptr = 1;
-        atomicCAS(p.status, kStatusOk, kStatusWaitExpired);
-    };
-    // item -> (slab, first row tile); decode_item wants an index over (slab, row tile)
-    auto decode = [&](int item, Item* it) {
-        const int slab = item / groups;
-        const int group = item - slab * groups;
-        const bool ok = decode_item<C::kN>(p, route_table, slab * p.m_tiles + group * tiles_per_group, it);
-        return ok;
-    };
-
-    if (warp == 0) {
-        if (elect_one()) {
-            int stage = 0;
-            std::uint32_t phase = 0, b_phase = 0;
-            for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
-                Item it;
-                if (!decode(item, &it)) continue;
-                if (!mbar_wait(b_empty, b_phase ^ 1U)) { give_up(); break; }
-                b_phase ^= 1U;
-                mbar_arrive_expect_tx(b_full, k_blocks * (C::kN * kBlockKBytes + kSfSlab));
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    tma_load_2d(base + kb * C::kN * kBlockKBytes, &map_b, b_full, kb * kBlockKBytes, it.pp0);
-                    bulk_load(base + C::kOffBSf + kb * kSfSlab,
-                              p.b_sf + (static_cast<std::size_t>(it.pp0 >> 7) * (p.k_bytes / 32) + kb * 4) * 512, kSfSlab, b_full);
-                }
-                bool ok = true;
-                for (int t = 0; t < tiles_per_group && ok; ++t) {
-                    const int m_tile = it.m_tile + t;
-                    for (int c = 0; c < chunks; ++c) {
-                        if (!mbar_wait(empty_bar(stage), phase ^ 1U)) { give_up(); ok = false; break; }
-                        mbar_arrive_expect_tx(weight_bar(stage), kChunkBytes);
-                        bulk_load(ring + stage * C::kStageBytes,
-                                  p.bank.g2 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + m_tile) * chunks + c) * kChunkBytes,
-                                  kChunkBytes, weight_bar(stage));
-                        if (++stage == C::kStages) { stage = 0; phase ^= 1U; }
-                    }
-                }
-                if (!ok) break;
-            }
-        }
-    } else if (warp == 1) {
-        if (elect_one()) {
-            int stage = 0;
-            std::uint32_t phase = 0, b_phase = 0;
-            int buffer = 0;
-            std::uint32_t accum_phase[2] = {0U, 0U};
-            constexpr std::uint32_t idesc = idesc_nvf4(kTileM, C::kN);
-            const std::uint32_t sfb_tmem = tmem_base + C::kAccumBuffers * C::kN;
-            const std::uint32_t sfa_tmem = sfb_tmem + C::kSfbCols;
-            int sfa_buffer = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < total_items && !*abort_ptr && ok; item += gridDim.x) {
-                Item it;
-                if (!decode(item, &it)) continue;
-                if (!mbar_wait(b_full, b_phase)) { give_up(); break; }
-                b_phase ^= 1U;
-                tc_fence_after();
-                // the slab's scale factors: 16 TMEM columns per K block, kept for the whole item
-                for (int kb = 0; kb < k_blocks; ++kb) {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        tc_copy_sf(sfb_tmem + kb * 16 + k * 4, desc_scale_atom(base + C::kOffBSf + kb * kSfSlab + k * 512));
-                    }
-                }
-                for (int t = 0; t < tiles_per_group && ok; ++t) {
-                    if (!mbar_wait(accum_empty(buffer), accum_phase[buffer] ^ 1U)) { give_up(); ok = false; break; }
-                    tc_fence_after();
-                    const std::uint32_t accum = tmem_base + buffer * C::kN;
-                    for (int c = 0; c < chunks; ++c) {
-                        if (!mbar_wait(weight_bar(stage), phase)) { give_up(); ok = false; break; }
-                        tc_fence_after();
-                        const std::uint32_t st = ring + stage * C::kStageBytes;
-                        const std::uint32_t sfa = sfa_tmem + sfa_buffer * C::kSfaCols;
-#pragma unroll
-                        for (int o = 0; o < 2; ++o) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                tc_copy_sf(sfa + o * 16 + k * 4, desc_scale_atom(st + kChunkScaleOffset + o * kChunkScaleBytes + k * 512));
-                            }
-                        }
-#pragma unroll
-                        for (int o = 0; o < 2; ++o) {
-                            const int kb = 2 * c + o;
-                            const std::uint64_t a_desc = desc_k_major_sw128(st + o * kChunkBox);
-                            const std::uint64_t b_desc = desc_k_major_sw128(base + kb * C::kN * kBlockKBytes);
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                mma_nvf4(accum, a_desc + 2 * k, b_desc + 2 * k, idesc, sfa + o * 16 + k * 4,
-                                         sfb_tmem + kb * 16 + k * 4, kb > 0 || k > 0);
-                            }
-                        }
-                        tc_commit(empty_bar(stage));
-                        sfa_buffer ^= 1;
-                        if (++stage == C::kStages) { stage = 0; phase ^= 1U; }
-                    }
-                    if (!ok) break;
-                    tc_commit(accum_full(buffer));
-                    accum_phase[buffer] ^= 1U;
-                    buffer ^= 1;
-                }
-                if (!ok) break;
-                tc_commit(b_empty);           // every product that reads the slab has been issued and will have completed
-            }
-        }
-    } else {
-        const int quarter = warp & 3;
-        const int sub = (warp - 2) >> 2;
-        int buffer = 0;
-        std::uint32_t accum_phase[2] = {0U, 0U};
-        bool ok = true;
-        for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-            if (!group_all(*abort_ptr == 0U, 1 + sub)) break;       // the four warps of a group leave together
-            Item it;
-            if (!decode(item, &it)) continue;
-            const float alpha = p.bank.alpha[it.entry * 3 + 2];
-            const int hidden = p.m_total;
-            for (int t = 0; t < tiles_per_group; ++t) {
-                // the four warps of a group (one per 32-lane quarter of the accumulator) move in step: they share a
-                // staging area and its barriers, so a wait that ran out in one of them ends the tile for all four
-                if (!group_all(mbar_wait(accum_full(buffer), accum_phase[buffer]), 1 + sub)) { give_up(); ok = false; break; }
-                accum_phase[buffer] ^= 1U;
-                tc_fence_after();
-                const std::uint32_t lane_base = tmem_base + buffer * C::kN + (static_cast<std::uint32_t>(quarter * 32) << 16);
-                // A lane holds one weight row for 16 tokens; the output is token-major, so 2-byte stores would touch a
-                // 64-byte piece per instruction.  The group turns its 128 x 16 block round through 4 KB of shared
-                // memory and every lane stores 16 bytes: a token's 128 rows leave as one 256-byte run, which is what
-                // keeps a store that crosses NVLink (TcIo::row_dest) efficient.
-                std::uint16_t* stage_rows = reinterpret_cast<std::uint16_t*>(smem_raw + (store_area - smem_u32(smem_raw))) +
-                                            sub * (4 * C::kStoreBytes / 2);
-                const int first_row = (it.m_tile + t) * kTileM;
-                // a warp's two chunks of 16 columns (sub * 16 and 64 + sub * 16) go into registers first and the buffer
-                // back to the MMA lane at once; staging and stores follow
-                constexpr int kChunks = C::kN / (16 * (kEpilogueWarps / 4));
-                static_assert(kChunks == 2, "two chunks per warp and tile");
-                std::uint32_t d[kChunks][16];
-#pragma unroll
-                for (int q = 0; q < kChunks; ++q) {
-                    const int c0 = sub * 16 + q * 16 * (kEpilogueWarps / 4);
-                    if (c0 < it.valid) tmem_load16(lane_base + c0, d[q]);              // group uniform
-                }
-                tmem_load_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(accum_empty(buffer));
-                buffer ^= 1;
-#pragma unroll
-                for (int q = 0; q < kChunks; ++q) {
-                    const int c0 = sub * 16 + q * 16 * (kEpilogueWarps / 4);
-                    if (c0 >= it.valid) break;
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        stage_rows[j * kTileM + quarter * 32 + lane] = float_to_bf16_bits(__uint_as_float(d[q][j]) * alpha);
-                    }
-                    group_sync(1 + sub);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int v = lane + 32 * h;                 // this warp: 4 tokens x 16 pieces of 16 bytes
-                        const int j = quarter * 4 + (v >> 4);
-                        const int n = c0 + j;
-                        if (n < it.valid) {
-                            std::uint16_t* to = p.row_dest != nullptr ? p.row_dest[it.pp0 + n]
-                                                                      : p.out + static_cast<std::size_t>(it.pp0 + n) * hidden;
-                            *reinterpret_cast<uint4*>(to + first_row + (v & 15) * 8) =
-                                *reinterpret_cast<const uint4*>(stage_rows + j * kTileM + (v & 15) * 8);
-                        }
-                    }
-                    group_sync(1 + sub);
-                }
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc(tmem_base, C::kTmemCols);
-    }
-}
-
 // Quantises the token rows into the padded position space of the tensor-core
 // kernels: row pp gets the NVFP4 bytes of its token, and the scales go straight
 // into the 128x4-tiled layout (cuda/nvfp4_ops.cu:818-841 and :869-890 in one pass).
@@ -928,9 +653,7 @@ cudaError_t launch_quantize_rows_to_pp(const std::uint16_t* x, const std::int32_
 
 namespace {
 bool slab_shape(const p92b_plan* plan) {
-    const int k_blocks = plan->intermediate / 2 / kBlockKBytes;
-    return plan->wide_rows == 128 && k_blocks <= DownSlab::kKBlocksMax && k_blocks % 2 == 0 &&
-           (plan->hidden / kTileM) % DownSlab::kMaxGroups == 0 && std::getenv("P92B_NO_DOWN_SLAB") == nullptr;
+    return plan->wide_rows == 128 && down_slab_shape(plan->hidden, plan->intermediate) && std::getenv("P92B_NO_DOWN_SLAB") == nullptr;
 }
 }  // namespace
 
@@ -1032,9 +755,7 @@ cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int 
                 const bool plain = io == nullptr || (io->down_out == nullptr && io->out_row == nullptr && !io->skip_shared);
                 if (plain && slab_shape(plan)) {
                     // the token slab resident in shared memory, only weights streaming
-                    if (cudaError_t st = ensure_dynamic_smem<expert_down_slab_kernel>(DownSlab::kSmemBytes); st != cudaSuccess) return st;
-                    return launch_kernel(expert_down_slab_kernel, dim3(plan->sm_count), dim3(kThreadsTc), DownSlab::kSmemBytes,
-                                         stream, pdl, plan->map_h[3], p);
+                    return launch_expert_down_slab(plan, p, stream, pdl);
                 }
                 if (p.row_dest != nullptr) return cudaErrorNotSupported;
                 // any K: 128 x 256 tiles with the tokens on the M side (dense MLP, 3,807 rows: both products together 196 ->
