@@ -151,14 +151,41 @@ static __device__ __noinline__ void warp_top8_by_id(const float* __restrict__ lg
     }
 }
 
+// Words of the nine best, lane k's the k-th: an image of the corrected score whose low byte is 255 - id.  Whether any two
+// neighbours agree in the score's 24 bits.
+__device__ __forceinline__ bool top8_is_close(std::uint32_t word_of_slot) {
+    const int lane = threadIdx.x & 31;
+    const std::uint32_t above = __shfl_up_sync(0xffffffffU, word_of_slot, 1);
+    return __any_sync(0xffffffffU, lane >= 1 && lane <= kTop && (above >> 8) == (word_of_slot >> 8));
+}
+
+// Ids and weights from those words: the uncorrected sigmoid of the winners, summed in slot order and scaled by
+// routed_scale / total (:420,425-432).
+__device__ __forceinline__ int top8_id(std::uint32_t word_of_slot) { return kExperts - 1 - static_cast<int>(word_of_slot & 0xffU); }
+__device__ __forceinline__ void warp_top8_weights(std::uint32_t word_of_slot, const float* __restrict__ lg, float* __restrict__ weights,
+                                                  float routed_scale) {
+    const int lane = threadIdx.x & 31;
+    const int chosen_id = top8_id(word_of_slot);
+    const float chosen_weight = lane < 8 ? 1.0F / (1.0F + expf(-lg[chosen_id])) : 0.0F;
+    float total = 0.0F;
+#pragma unroll
+    for (int slot = 0; slot < 8; ++slot) total += __shfl_sync(0xffffffffU, chosen_weight, slot);
+    const float multiplier = routed_scale / total;
+    if (lane < 8) weights[lane] = chosen_weight * multiplier;
+}
+__device__ __forceinline__ void warp_top8_write(std::uint32_t word_of_slot, const float* __restrict__ lg, std::int32_t* __restrict__ ids,
+                                                float* __restrict__ weights, float routed_scale) {
+    const int lane = threadIdx.x & 31;
+    warp_top8_weights(word_of_slot, lg, weights, routed_scale);
+    if (lane < 8) ids[lane] = top8_id(word_of_slot);
+}
+
 // The same for scores whose nine highest differ in the upper 24 bits of their order-preserving image - all but about one
 // token in a thousand: the low byte of a 32-bit word then carries the expert id, so that one warp reduction per
 // round gives winner and id together, and a comparator of the lane-local ordering is one minimum and one maximum.  The
 // ninth round is there to see that the eighth and ninth differ; any two neighbours that agree in 24 bits send the whole
 // token through warp_top8_by_id, so ids, order and weights are the same bits in every case.
-__device__ __forceinline__ void warp_top8(const float* __restrict__ lg, const float* __restrict__ bias,
-                                          std::int32_t* __restrict__ ids, float* __restrict__ weights,
-                                          float routed_scale) {
+__device__ __forceinline__ std::uint32_t warp_top8_words(const float* __restrict__ lg, const float* __restrict__ bias) {
     const int lane = threadIdx.x & 31;
     std::uint32_t cand[8];
 #pragma unroll
@@ -194,22 +221,18 @@ __device__ __forceinline__ void warp_top8(const float* __restrict__ lg, const fl
         }
         if (lane == slot) mine = top;
     }
-    const std::uint32_t above = __shfl_up_sync(0xffffffffU, mine, 1);
-    if (__any_sync(0xffffffffU, lane >= 1 && lane <= kTop && (above >> 8) == (mine >> 8))) {
+    return mine;
+}
+
+__device__ __forceinline__ void warp_top8(const float* __restrict__ lg, const float* __restrict__ bias,
+                                          std::int32_t* __restrict__ ids, float* __restrict__ weights,
+                                          float routed_scale) {
+    const std::uint32_t words = warp_top8_words(lg, bias);
+    if (top8_is_close(words)) {
         warp_top8_by_id(lg, bias, ids, weights, routed_scale);
         return;
     }
-    const int chosen_id = kExperts - 1 - static_cast<int>(mine & 0xffU);
-    // weights: the uncorrected sigmoid of the winners, summed in slot order and scaled by routed_scale / total (:420,425-432)
-    const float chosen_weight = lane < 8 ? 1.0F / (1.0F + expf(-lg[chosen_id])) : 0.0F;
-    float total = 0.0F;
-#pragma unroll
-    for (int slot = 0; slot < 8; ++slot) total += __shfl_sync(0xffffffffU, chosen_weight, slot);
-    const float multiplier = routed_scale / total;
-    if (lane < 8) {
-        ids[lane] = chosen_id;
-        weights[lane] = chosen_weight * multiplier;
-    }
+    warp_top8_write(words, lg, ids, weights, routed_scale);
 }
 
 // Layout of one layer's expert weights inside the library (device memory).

@@ -75,7 +75,7 @@ __host__ __device__ constexpr std::uint32_t idesc_bf16(int m, int n) {
 // ||w_e|| of one router row, by a warp; and, for hidden = 2,560, the row once more in the order in which the exact chains
 // take it: piece (c, lane) of 16 bytes holds columns lane + 32 (8 c + i), i = 0 .. 7, so that a lane of the repair kernel
 // reads eight steps of its chain with one load.
-constexpr int kChunksInRegisters = 80;                    // hidden / 32
+constexpr int kChainSteps = 80;                           // hidden / 32
 __device__ __forceinline__ void row_norm(const std::uint16_t* __restrict__ w, float* __restrict__ norms,
                                          std::uint16_t* __restrict__ w_chains, int e, int hidden) {
     const int lane = threadIdx.x & 31;
@@ -84,7 +84,7 @@ __device__ __forceinline__ void row_norm(const std::uint16_t* __restrict__ w, fl
         const std::uint16_t* row = w + static_cast<std::size_t>(e) * hidden + lane;
         uint4* to = reinterpret_cast<uint4*>(w_chains + static_cast<std::size_t>(e) * hidden) + lane;
 #pragma unroll 5
-        for (int c = 0; c < kChunksInRegisters / 8; ++c) {
+        for (int c = 0; c < kChainSteps / 8; ++c) {
             std::uint32_t v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = __ldg(row + 32 * (8 * c + i));
@@ -254,67 +254,13 @@ __device__ __forceinline__ float exact_logit(const std::uint16_t* __restrict__ x
 
 constexpr int kRepairWarps = 4;
 
-// CHUNKS = hidden / 32 > 0: the lane's columns of the token row (l, l+32, ...) stay in registers and the candidates' router
-// rows are read in chain order (row_norm) two at a time: ten 16-byte loads a row, two independent chains, three
-// instructions per column of a pair's row and no shared memory.  Rows brought into shared memory as they are cost a 2-byte
-// read, a shift and an fmaf per column of one dependent chain, and three blocks of four warps per SM (124 us at 16,384
-// tokens, 38 at 4,096).  CHUNKS = 0: any hidden size, token row in shared memory, router rows read in place.
-// WPT (warps per token) = 1: a warp does everything for its token, four tokens per block - the form for thousands of
-// tokens.  WPT = 8: one token per block; the eight warps each build the candidate list (the same list) and then share
-// the candidates' exact logits out among themselves, warp 0 finishes - a few hundred tokens would otherwise leave
-// most SMs idle while every warp walks eight 2560-step chains one after the other.
-// `partials` (splits > 1): the approximate logits arrive as `splits` slices of partial sums ([splits][rows][256]).
-template <int CHUNKS, int WPT>
-__global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_repair_kernel(
-    const std::uint16_t* __restrict__ x, const std::uint16_t* __restrict__ w, const float* __restrict__ bias,
-    const float* __restrict__ w_norms, float* __restrict__ logits, std::int32_t* __restrict__ ids,
-    float* __restrict__ weights, int rows, int hidden, float routed_scale, int* __restrict__ stats,
-    const float* __restrict__ partials, int splits, const std::uint16_t* __restrict__ w_chains) {
-    extern __shared__ __align__(16) std::uint16_t repair_smem[];
-    pdl_launch_dependents();
-    pdl_wait();
-    constexpr int kWarps = WPT > 1 ? WPT : kRepairWarps;
-    const int warp = threadIdx.x >> 5;
+// Approximate logits of one token as a lane holds them: experts lane, lane + 32, ..., lane + 224.  `partials` (splits > 1): they
+// arrive as `splits` slices of partial sums ([splits][rows][256]); all loads of the slices are issued before the first sum,
+// one round trip and not one per slice, and the sums go to the logits buffer if `store`.
+__device__ __forceinline__ void load_approximate(float* __restrict__ lg, const float* __restrict__ partials, int splits, int rows,
+                                                 int token, bool store, float (&approx)[8]) {
     const int lane = threadIdx.x & 31;
-    const int token = WPT > 1 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kRepairWarps + warp;
-    if (token >= rows) return;                     // WPT > 1: the grid is exactly `rows` blocks
-    // per warp: [CHUNKS == 0: the token row], then 256 exact logits, then the candidate list
-    constexpr int kRowSlots = CHUNKS > 0 ? 0 : 1;
-    std::uint16_t* x_row = repair_smem + static_cast<std::size_t>(warp) * kRowSlots * hidden;
-    std::uint8_t* tail = reinterpret_cast<std::uint8_t*>(repair_smem + static_cast<std::size_t>(kWarps) * kRowSlots * hidden);
-    float* exact_row = reinterpret_cast<float*>(tail) + (WPT > 1 ? 0 : warp) * kExperts;      // WPT > 1: one row per block
-    std::uint16_t* cand = reinterpret_cast<std::uint16_t*>(tail + kWarps * kExperts * 4) + warp * kExperts;
-    float xr[CHUNKS > 0 ? CHUNKS : 1];
-    float square = 0.0F;
-    if constexpr (CHUNKS > 0) {
-        const std::uint16_t* xg = x + static_cast<std::size_t>(token) * hidden + lane;
-#pragma unroll
-        for (int j = 0; j < CHUNKS; ++j) xr[j] = bf16_bits_to_float(__ldg(xg + 32 * j));
-#pragma unroll
-        for (int j = 0; j < CHUNKS; ++j) square = fmaf(xr[j], xr[j], square);
-    } else {
-        for (int v = lane; v < hidden / 8; v += 32) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4*>(x + static_cast<std::size_t>(token) * hidden) + v);
-            reinterpret_cast<uint4*>(x_row)[v] = q;
-            const std::uint32_t words[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float lo = __uint_as_float(words[k] << 16), hi = __uint_as_float(words[k] & 0xffff0000U);
-                square = fmaf(lo, lo, square);
-                square = fmaf(hi, hi, square);
-            }
-        }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) square += __shfl_xor_sync(0xffffffffU, square, off);
-    const float x_norm = sqrtf(square) * 1.0001F;
-    __syncwarp();
-
-    float* lg = logits + static_cast<std::size_t>(token) * kExperts;
-    float approx[8], score[8];
-    bool finite = true;
     if (splits > 1) {
-        // all loads of the slices are issued before the first sum: one round trip, not one per slice
         float part[kRouterSplits][8];
 #pragma unroll
         for (int z = 0; z < kRouterSplits; ++z) {
@@ -329,133 +275,355 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
 #pragma unroll
             for (int z = 1; z < kRouterSplits; ++z) sum += part[z][i];
             approx[i] = sum;
-            if (WPT == 1 || warp == 0) lg[lane + 32 * i] = sum;           // the logits buffer holds the approximate values
+            if (store) lg[lane + 32 * i] = sum;
         }
     } else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) approx[i] = lg[lane + 32 * i];
     }
+}
+
+// The candidates of one token, member[i] a ballot over experts 32 i .. 32 i + 31: approximate corrected score within 2 delta of
+// the approximate 8th best.  All 256 if that cannot decide it (*whole_row): a logit that is no finite number, fewer than eight
+// candidates (a NaN in the bias, or fewer than eight experts that -infinity does not mask) or more than a warp takes.
+__device__ __forceinline__ int find_candidates(const float (&approx)[8], const float* __restrict__ bias, const float* __restrict__ w_norms,
+                                               float x_norm, unsigned (&member)[8], bool* whole_row) {
+    const int lane = threadIdx.x & 31;
+    bool finite = true;
+    float score[8], delta[8];
+    std::uint32_t key[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int e = lane + 32 * i;
         finite = finite && (fabsf(approx[i]) <= 3.0e38F);
         score[i] = 1.0F / (1.0F + expf(-approx[i])) + bias[e];
+        delta[i] = 0.25F * kLogitBound * x_norm * w_norms[e] + 4.0e-6F;
+        const std::uint32_t bits = __float_as_uint(score[i]);
+        key[i] = score[i] != score[i] ? 0U : (bits & 0x80000000U ? ~bits : bits | 0x80000000U);
     }
     finite = __all_sync(0xffffffffU, finite);
-    // approximate 8th best corrected score: eight rounds of (remove the current maximum), value only
-    float eighth = 0.0F;
-    {
-        float work[8];
+    // The eighth best: every lane orders its own eight, then eight rounds look at the heads.  Lanes that share a maximum give it
+    // up together: the eighth then comes out lower and the candidates are more, never fewer.
+#define P92B_ORDER(a, b)                                    \
+    {                                                       \
+        const std::uint32_t hi = max(key[a], key[b]);       \
+        key[b] = min(key[a], key[b]);                       \
+        key[a] = hi;                                        \
+    }
+    P92B_ORDER(0, 1) P92B_ORDER(2, 3) P92B_ORDER(4, 5) P92B_ORDER(6, 7)
+    P92B_ORDER(0, 2) P92B_ORDER(1, 3) P92B_ORDER(4, 6) P92B_ORDER(5, 7)
+    P92B_ORDER(1, 2) P92B_ORDER(5, 6)
+    P92B_ORDER(0, 4) P92B_ORDER(1, 5) P92B_ORDER(2, 6) P92B_ORDER(3, 7)
+    P92B_ORDER(2, 4) P92B_ORDER(3, 5)
+    P92B_ORDER(1, 2) P92B_ORDER(3, 4) P92B_ORDER(5, 6)
+#undef P92B_ORDER
+    std::uint32_t top = 0U;
+#pragma unroll 2
+    for (int round = 0; round < kTop; ++round) {
+        top = __reduce_max_sync(0xffffffffU, key[0]);
+        if (key[0] == top) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) work[i] = score[i];
-#pragma unroll 1
-        for (int round = 0; round < 8; ++round) {
-            float best = work[0];
-            int at = 0;
-#pragma unroll
-            for (int i = 1; i < 8; ++i) {
-                if (work[i] > best) { best = work[i]; at = i; }
-            }
-            const std::uint32_t bits = __float_as_uint(best);
-            const std::uint32_t key = bits & 0x80000000U ? ~bits : bits | 0x80000000U;
-            const std::uint32_t top = __reduce_max_sync(0xffffffffU, key);
-            const unsigned holders = __ballot_sync(0xffffffffU, key == top);
-            if (lane == __ffs(holders) - 1) {                 // one holder gives its maximum up
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if (i == at) work[i] = -3.0e38F;
-                }
-            }
-            const std::uint32_t top_bits = top & 0x80000000U ? top & 0x7fffffffU : ~top;
-            eighth = __uint_as_float(top_bits);
+            for (int i = 0; i < 7; ++i) key[i] = key[i + 1];
+            key[7] = 0U;
         }
     }
-    // candidates: approximate score within 2 delta of the approximate 8th
-    unsigned member[8];
+    const float eighth = __uint_as_float(top & 0x80000000U ? top & 0x7fffffffU : ~top);       // image 0: a NaN, nothing is within reach
     int candidates = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int e = lane + 32 * i;
-        const float delta = 0.25F * kLogitBound * x_norm * w_norms[e] + 4.0e-6F;
-        member[i] = __ballot_sync(0xffffffffU, score[i] >= eighth - 2.0F * delta);
+        member[i] = __ballot_sync(0xffffffffU, score[i] >= eighth - 2.0F * delta[i]);
         candidates += __popc(member[i]);
     }
-    // (fewer than eight: a NaN in the bias upset the 8th best, or fewer than eight experts are not masked by -infinity)
-    const bool whole_row = !finite || candidates > kMaxCandidates || candidates < kTop;
-    if (whole_row) {
+    *whole_row = !finite || candidates > kMaxCandidates || candidates < kTop;
+    if (*whole_row) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) member[i] = 0xffffffffU;
+        candidates = kExperts;
     }
-    // exact logits of the candidates (or of the whole row), into the logits buffer and into this warp's row
-    const float not_recomputed = __uint_as_float(0x7fc00000U);        // a NaN is picked behind every number
-    if constexpr (WPT > 1) {
-        for (int e = threadIdx.x; e < kExperts; e += WPT * 32) exact_row[e] = not_recomputed;
-        __syncthreads();                               // before any warp stores a result into the shared row
-    } else {
-        for (int e = lane; e < kExperts; e += 32) exact_row[e] = not_recomputed;
-    }
-    int n_cand = 0;
+    return candidates;
+}
+
+// The members in order of their ids, as a list in shared memory.
+__device__ __forceinline__ void list_candidates(const unsigned (&member)[8], std::uint16_t* cand) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        if ((member[i] >> lane) & 1U) cand[n_cand + __popc(member[i] & ((1U << lane) - 1U))] = static_cast<std::uint16_t>(lane + 32 * i);
-        n_cand += __popc(member[i]);
+        if ((member[i] >> lane) & 1U) cand[before + __popc(member[i] & ((1U << lane) - 1U))] = static_cast<std::uint16_t>(lane + 32 * i);
+        before += __popc(member[i]);
     }
     __syncwarp();
-    // this warp's share of the candidates: all of them (WPT = 1) or every WPT-th, starting with its own number
-    const int first = WPT > 1 ? warp : 0;
-    constexpr int kStep = WPT > 1 ? WPT : 1;
-    const int n_mine = n_cand > first ? (n_cand - first + kStep - 1) / kStep : 0;
-    if constexpr (CHUNKS > 0) {
-#pragma unroll 1
-        for (int i = 0; i < n_mine; i += 2) {
-            const int ea = cand[first + i * kStep];
-            const int eb = i + 1 < n_mine ? cand[first + (i + 1) * kStep] : ea;
-            const uint4* wa = reinterpret_cast<const uint4*>(w_chains + static_cast<std::size_t>(ea) * hidden) + lane;
-            const uint4* wb = reinterpret_cast<const uint4*>(w_chains + static_cast<std::size_t>(eb) * hidden) + lane;
-            float va = 0.0F, vb = 0.0F;
+}
+
+// Logits that were not recomputed: a NaN, picked behind every number.
+__device__ __forceinline__ void clear_exact_row(float* exact_row, int first, int threads) {
+    for (int e = first; e < kExperts; e += threads) exact_row[e] = __uint_as_float(0x7fc00000U);
+}
+
+// Two chains at once: a.x = fmaf(x.x, w.x, a.x) and the same for y, rounded (and denormals flushed) as fmaf in this file.
+__device__ __forceinline__ void fma_pair(float2& a, float2 x, float2 w) {
+    unsigned long long acc = *reinterpret_cast<unsigned long long*>(&a);
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %0;"
+        : "+l"(acc)
+        : "l"(*reinterpret_cast<const unsigned long long*>(&x)), "l"(*reinterpret_cast<const unsigned long long*>(&w)));
+    a = *reinterpret_cast<float2*>(&acc);
+}
+
+// The repair for hidden = 2,560.  The token row lies in shared memory in chain order (row_norm): piece (c, lane) of 16 bytes is
+// eight steps of a lane's chain, for the token as for a router row.
+// WPT (warps per token) = 1: a warp does everything for its token, four tokens per block - the form for more than a few hundred
+// tokens.  The exact logits go eight candidates at a time (there are 8.16 on average): eight independent chains as four pairs,
+// the router rows of the next step in flight, and a tree over the 32 lanes that halves the number of values with every step
+// instead of repeating itself per candidate.  (Two candidates at a time from a token row in registers, all 256 exact logits in
+// the selection: 96 us at 16,384 tokens, now 80; 31 at 4,096, now 28; 15 at 512, now 11; 12 at 64, now 9.6.)
+// WPT = 8 or 4: one token per block; its warps bring the row in together, each build the candidate list (the same list) and
+// then share the candidates out, one chain at a time; warp 0 finishes.
+template <int WPT>
+__global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 ? 2 : 4) route_repair_chains_kernel(
+    const std::uint16_t* __restrict__ x, const float* __restrict__ bias, const float* __restrict__ w_norms, float* __restrict__ logits,
+    std::int32_t* __restrict__ ids, float* __restrict__ weights, int rows, float routed_scale, int* __restrict__ stats,
+    const float* __restrict__ partials, int splits, const std::uint16_t* __restrict__ w_chains) {
+    constexpr int kHidden = 32 * kChainSteps;
+    constexpr int kPieces = kChainSteps / 8;                  // of 16 bytes, per lane
+    constexpr int kWarps = WPT > 1 ? WPT : kRepairWarps;
+    constexpr int kTokens = WPT > 1 ? 1 : kRepairWarps;             // per block
+    __shared__ uint4 x_chains[kTokens][kPieces * 32];
+    __shared__ float exact_rows[kTokens][kExperts];
+    __shared__ std::uint16_t cand_lists[kWarps][kExperts];
+    __shared__ float square_sums[kWarps];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int token = WPT > 1 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kRepairWarps + warp;
+    if (token >= rows) return;                     // WPT > 1: the grid is exactly `rows` blocks
+    uint4* const x_row = x_chains[WPT > 1 ? 0 : warp];
+    float* const exact_row = exact_rows[WPT > 1 ? 0 : warp];
+    std::uint16_t* const cand = cand_lists[warp];
+    float* const lg = logits + static_cast<std::size_t>(token) * kExperts;
+    std::int32_t* const my_ids = ids + static_cast<std::size_t>(token) * kTop;
+    float* const my_weights = weights + static_cast<std::size_t>(token) * kTop;
+    float approx[8];
+    float square = 0.0F;
+    {
+        const std::uint16_t* xg = x + static_cast<std::size_t>(token) * kHidden + lane;
+#pragma unroll 5
+        for (int c = WPT > 1 ? warp : 0; c < kPieces; c += WPT > 1 ? WPT : 1) {
+            std::uint32_t v[8];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {                         // half a row of both in flight
-                uint4 qa[CHUNKS / 16], qb[CHUNKS / 16];
+            for (int i = 0; i < 8; ++i) v[i] = __ldg(xg + 32 * (8 * c + i));
 #pragma unroll
-                for (int c = 0; c < CHUNKS / 16; ++c) {
-                    qa[c] = __ldg(wa + 32 * (h * (CHUNKS / 16) + c));
-                    qb[c] = __ldg(wb + 32 * (h * (CHUNKS / 16) + c));
-                }
-#pragma unroll
-                for (int c = 0; c < CHUNKS / 16; ++c) {
-                    const std::uint32_t ua[4] = {qa[c].x, qa[c].y, qa[c].z, qa[c].w};
-                    const std::uint32_t ub[4] = {qb[c].x, qb[c].y, qb[c].z, qb[c].w};
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int j = 8 * (h * (CHUNKS / 16) + c) + 2 * k;
-                        va = fmaf(xr[j], __uint_as_float(ua[k] << 16), va);
-                        vb = fmaf(xr[j], __uint_as_float(ub[k] << 16), vb);
-                        va = fmaf(xr[j + 1], __uint_as_float(ua[k] & 0xffff0000U), va);
-                        vb = fmaf(xr[j + 1], __uint_as_float(ub[k] & 0xffff0000U), vb);
-                    }
-                }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                va += __shfl_down_sync(0xffffffffU, va, off);
-                vb += __shfl_down_sync(0xffffffffU, vb, off);
-            }
-            if (lane == 0) {
-                exact_row[ea] = va;
-                lg[ea] = va;
-                exact_row[eb] = vb;
-                lg[eb] = vb;
-            }
+            for (int i = 0; i < 8; ++i) square = fmaf(__uint_as_float(v[i] << 16), __uint_as_float(v[i] << 16), square);
+            x_row[32 * c + lane] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
         }
-    } else {
+    }
+    load_approximate(lg, partials, splits, rows, token, WPT == 1 || warp == 0, approx);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) square += __shfl_xor_sync(0xffffffffU, square, off);
+    if constexpr (WPT > 1) {
+        if (lane == 0) square_sums[warp] = square;
+        __syncthreads();                            // the row and its parts of the norm
+        square = 0.0F;
+#pragma unroll
+        for (int v = 0; v < WPT; ++v) square += square_sums[v];
+    }
+    const float x_norm = sqrtf(square) * 1.0001F;
+    unsigned member[8];
+    bool whole_row;
+    const int n_cand = find_candidates(approx, bias, w_norms, x_norm, member, &whole_row);
+    list_candidates(member, cand);
+
+    const uint4* const w_lane = reinterpret_cast<const uint4*>(w_chains) + lane;
+    float mine = 0.0F;                              // lane i < n_cand <= 32: exact logit of candidate i
+    if constexpr (WPT > 1) {
 #pragma unroll 1
-        for (int i = 0; i < n_mine; ++i) {
-            const int e = cand[first + i * kStep];
-            const float value = exact_logit(x_row, w + static_cast<std::size_t>(e) * hidden, hidden, lane);
+        for (int i = warp; i < n_cand; i += WPT) {
+            const int e = cand[i];
+            const uint4* w = w_lane + e * (kPieces * 32);
+            uint4 q[kPieces];
+#pragma unroll
+            for (int c = 0; c < kPieces; ++c) q[c] = __ldg(w + 32 * c);
+            float value = 0.0F;
+#pragma unroll
+            for (int c = 0; c < kPieces; ++c) {
+                const uint4 xq = x_row[32 * c + lane];
+                const std::uint32_t xs[4] = {xq.x, xq.y, xq.z, xq.w}, ws[4] = {q[c].x, q[c].y, q[c].z, q[c].w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    value = fmaf(__uint_as_float(xs[k] << 16), __uint_as_float(ws[k] << 16), value);
+                    value = fmaf(__uint_as_float(xs[k] & 0xffff0000U), __uint_as_float(ws[k] & 0xffff0000U), value);
+                }
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) value += __shfl_down_sync(0xffffffffU, value, off);
             if (lane == 0) {
                 exact_row[e] = value;
                 lg[e] = value;
             }
+        }
+        __syncthreads();                                        // every warp's results are in the block's row
+        if (warp != 0) return;
+        if (lane < n_cand && !whole_row) mine = exact_row[cand[lane]];
+    } else {
+#pragma unroll 1
+        for (int first = 0; first < n_cand; first += 8) {
+            int at[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) at[k] = cand[min(first + k, n_cand - 1)] * (kPieces * 32);
+            float2 acc[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) acc[m] = make_float2(0.0F, 0.0F);
+            // a step of eight columns per lane; two sets of registers, the loads of one under way while the other is used
+            uint4 even[8], odd[8];
+            auto request = [&](uint4 (&q)[8], int c) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) q[k] = __ldg(w_lane + at[k] + 32 * c);
+            };
+            auto add = [&](const uint4 (&q)[8], int c) {
+                const uint4 xq = x_row[32 * c + lane];
+                const std::uint32_t xs[4] = {xq.x, xq.y, xq.z, xq.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float lo = __uint_as_float(xs[k] << 16), hi = __uint_as_float(xs[k] & 0xffff0000U);
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const std::uint32_t wa = k == 0 ? q[2 * m].x : k == 1 ? q[2 * m].y : k == 2 ? q[2 * m].z : q[2 * m].w;
+                        const std::uint32_t wb = k == 0 ? q[2 * m + 1].x : k == 1 ? q[2 * m + 1].y : k == 2 ? q[2 * m + 1].z : q[2 * m + 1].w;
+                        fma_pair(acc[m], make_float2(lo, lo), make_float2(__uint_as_float(wa << 16), __uint_as_float(wb << 16)));
+                        fma_pair(acc[m], make_float2(hi, hi), make_float2(__uint_as_float(wa & 0xffff0000U), __uint_as_float(wb & 0xffff0000U)));
+                    }
+                }
+            };
+            static_assert(kPieces % 2 == 0, "steps in pairs");
+            request(even, 0);
+#pragma unroll 1
+            for (int c = 0; c < kPieces; c += 2) {
+                request(odd, c + 1);
+                add(even, c);
+                if (c + 2 < kPieces) request(even, c + 2);
+                add(odd, c + 1);
+            }
+            // The reference's tree over the 32 chains (lane l takes lane l + 16's sum, then l + 8's, ...), for eight candidates at
+            // once: a lane hands half of its values to its partner and goes on with the other half, so that after the steps of
+            // 16, 8 and 4 lanes it is left with candidate lane / 4.  An addition's two operands are the tree's, in either order.
+            float v[8] = {acc[0].x, acc[0].y, acc[1].x, acc[1].y, acc[2].x, acc[2].y, acc[3].x, acc[3].y};
+#pragma unroll
+            for (int half = 4; half >= 1; half >>= 1) {
+                const int off = half * 4;
+                const bool upper = (lane & off) != 0;
+#pragma unroll
+                for (int m = 0; m < half; ++m) {
+                    const float got = __shfl_xor_sync(0xffffffffU, upper ? v[m] : v[m + half], off);
+                    v[m] = (upper ? v[m + half] : v[m]) + got;
+                }
+            }
+            float value = v[0];
+            value += __shfl_xor_sync(0xffffffffU, value, 2);
+            value += __shfl_xor_sync(0xffffffffU, value, 1);
+            const int k = first + (lane >> 2);
+            if ((lane & 3) == 0 && k < n_cand) {
+                exact_row[cand[k]] = value;
+                lg[cand[k]] = value;
+            }
+            const float of_mine = __shfl_sync(0xffffffffU, value, (lane & 7) * 4);
+            if (lane >= first && lane < first + 8) mine = of_mine;
+        }
+        __syncwarp();
+    }
+    if (lane == 0 && stats != nullptr) {
+        atomicAdd(stats + 0, n_cand);
+        if (whole_row) atomicAdd(stats + 1, 1);
+    }
+    // The reference's top-8 over the exact values.
+    if (whole_row) {
+        warp_top8(exact_row, bias, my_ids, my_weights, routed_scale);
+        return;
+    }
+    // One candidate per lane, words as in warp_top8: nine rounds, a lane gives its word up when it is the maximum.
+    const int my_e = lane < n_cand ? cand[lane] : 0;
+    std::uint32_t word = 0U;
+    if (lane < n_cand) {
+        const float corrected = 1.0F / (1.0F + expf(-mine)) + bias[my_e];
+        const std::uint32_t bits = __float_as_uint(corrected);
+        const std::uint32_t image = corrected != corrected ? 0U : (bits & 0x80000000U ? ~bits : bits | 0x80000000U);
+        word = (image & 0xffffff00U) | static_cast<std::uint32_t>(kExperts - 1 - my_e);
+    }
+    std::uint32_t of_slot = 0U;                    // lane k keeps the word of slot k, lane 8 the ninth
+#pragma unroll 3
+    for (int slot = 0; slot <= kTop; ++slot) {
+        const std::uint32_t top = __reduce_max_sync(0xffffffffU, word);
+        if (word == top) word = 0U;
+        if (lane == slot) of_slot = top;
+    }
+    if (top8_is_close(of_slot)) {
+        clear_exact_row(exact_row, lane, 32);
+        __syncwarp();
+        if (lane < n_cand) exact_row[my_e] = mine;
+        __syncwarp();
+        warp_top8_by_id(exact_row, bias, my_ids, my_weights, routed_scale);
+        return;
+    }
+    warp_top8_write(of_slot, exact_row, my_ids, my_weights, routed_scale);
+}
+
+// Any other hidden size: the token row in shared memory as it is, router rows read in place, one chain at a time.
+template <int WPT>
+__global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_repair_kernel(
+    const std::uint16_t* __restrict__ x, const std::uint16_t* __restrict__ w, const float* __restrict__ bias,
+    const float* __restrict__ w_norms, float* __restrict__ logits, std::int32_t* __restrict__ ids,
+    float* __restrict__ weights, int rows, int hidden, float routed_scale, int* __restrict__ stats,
+    const float* __restrict__ partials, int splits) {
+    extern __shared__ __align__(16) std::uint16_t repair_smem[];
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int kWarps = WPT > 1 ? WPT : kRepairWarps;
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int token = WPT > 1 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kRepairWarps + warp;
+    if (token >= rows) return;                     // WPT > 1: the grid is exactly `rows` blocks
+    // per warp: the token row, then 256 exact logits, then the candidate list
+    std::uint16_t* x_row = repair_smem + static_cast<std::size_t>(warp) * hidden;
+    std::uint8_t* tail = reinterpret_cast<std::uint8_t*>(repair_smem + static_cast<std::size_t>(kWarps) * hidden);
+    float* exact_row = reinterpret_cast<float*>(tail) + (WPT > 1 ? 0 : warp) * kExperts;      // WPT > 1: one row per block
+    std::uint16_t* cand = reinterpret_cast<std::uint16_t*>(tail + kWarps * kExperts * 4) + warp * kExperts;
+    float square = 0.0F;
+    for (int v = lane; v < hidden / 8; v += 32) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(x + static_cast<std::size_t>(token) * hidden) + v);
+        reinterpret_cast<uint4*>(x_row)[v] = q;
+        const std::uint32_t words[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float lo = __uint_as_float(words[k] << 16), hi = __uint_as_float(words[k] & 0xffff0000U);
+            square = fmaf(lo, lo, square);
+            square = fmaf(hi, hi, square);
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) square += __shfl_xor_sync(0xffffffffU, square, off);
+    const float x_norm = sqrtf(square) * 1.0001F;
+    __syncwarp();
+    float* lg = logits + static_cast<std::size_t>(token) * kExperts;
+    float approx[8];
+    load_approximate(lg, partials, splits, rows, token, WPT == 1 || warp == 0, approx);
+    unsigned member[8];
+    bool whole_row;
+    const int n_cand = find_candidates(approx, bias, w_norms, x_norm, member, &whole_row);
+    list_candidates(member, cand);
+    if constexpr (WPT > 1) {
+        clear_exact_row(exact_row, threadIdx.x, WPT * 32);
+        __syncthreads();                               // before any warp stores a result into the shared row
+    } else {
+        clear_exact_row(exact_row, lane, 32);
+        __syncwarp();
+    }
+    // this warp's share of the candidates: all of them (WPT = 1) or every WPT-th, starting with its own number
+#pragma unroll 1
+    for (int i = WPT > 1 ? warp : 0; i < n_cand; i += WPT) {
+        const int e = cand[i];
+        const float value = exact_logit(x_row, w + static_cast<std::size_t>(e) * hidden, hidden, lane);
+        if (lane == 0) {
+            exact_row[e] = value;
+            lg[e] = value;
         }
     }
     if constexpr (WPT > 1) {
@@ -464,7 +632,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     }
     __syncwarp();
     if (lane == 0 && stats != nullptr) {
-        atomicAdd(stats + 0, whole_row ? kExperts : candidates);
+        atomicAdd(stats + 0, n_cand);
         if (whole_row) atomicAdd(stats + 1, 1);
     }
     // The reference's top-8 over the exact values.  (A selection of its own that gave taken, NaN and left-out experts one and
@@ -502,7 +670,7 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     if ((st = ensure_dynamic_smem<logits_tc_kernel<64>>(Logits<64>::kSmem)) != cudaSuccess) return st;
     if ((st = ensure_dynamic_smem<logits_tc_kernel<128>>(Logits<128>::kSmem)) != cudaSuccess) return st;
     if ((st = ensure_dynamic_smem<logits_tc_kernel<256>>(Logits<256>::kSmem)) != cudaSuccess) return st;
-    const bool in_registers = hidden == 32 * kChunksInRegisters;
+    const bool chain_order = hidden == 32 * kChainSteps;
     // small batches: K split over blocks of the logits kernel, and a block of eight warps per token in the repair
     const bool may_split = plan->logit_partials != nullptr && plan->max_rows >= rows && std::getenv("P92B_ROUTER_NO_SPLIT") == nullptr;
     const bool small = rows <= kRouterWideRows && may_split;
@@ -515,36 +683,32 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     const int splits = (k_blocks + per_split - 1) / per_split;                    // no empty slice
     constexpr int kWide = 8;
     const int repair_warps = small ? kWide : kRepairWarps;
-    const std::size_t repair_smem = static_cast<std::size_t>(repair_warps) * (in_registers ? 0 : hidden) * 2 +
-                                    static_cast<std::size_t>(repair_warps) * kExperts * (4 + 2);
-    if (small) {
-        st = in_registers ? ensure_dynamic_smem<route_repair_kernel<80, kWide>>(static_cast<int>(repair_smem))
-                          : ensure_dynamic_smem<route_repair_kernel<0, kWide>>(static_cast<int>(repair_smem));
-    } else {
-        st = in_registers ? ensure_dynamic_smem<route_repair_kernel<80, 1>>(static_cast<int>(repair_smem))
-                          : ensure_dynamic_smem<route_repair_kernel<0, 1>>(static_cast<int>(repair_smem));
+    const std::size_t repair_smem = chain_order ? 0 : static_cast<std::size_t>(repair_warps) * (hidden * 2 + kExperts * (4 + 2));
+    if (!chain_order) {
+        st = small ? ensure_dynamic_smem<route_repair_kernel<kWide>>(static_cast<int>(repair_smem))
+                   : ensure_dynamic_smem<route_repair_kernel<1>>(static_cast<int>(repair_smem));
+        if (st != cudaSuccess) return st;
     }
-    if (st != cudaSuccess) return st;
     float* norms = plan->w_norms;
     float* approx_out = splits > 1 ? plan->logit_partials : plan->logits;
     const auto kernel = expert_tile == 64 ? logits_tc_kernel<64> : expert_tile == 128 ? logits_tc_kernel<128> : logits_tc_kernel<256>;
     const int smem = expert_tile == 64 ? Logits<64>::kSmem : expert_tile == 128 ? Logits<128>::kSmem : Logits<256>::kSmem;
     st = launch_kernel(kernel, dim3(token_tiles, kExperts / expert_tile, splits), dim3(kLogitThreads), smem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status, router_w, norms,
-                       in_registers ? plan->w_chains : nullptr);
+                       chain_order ? plan->w_chains : nullptr);
     if (st != cudaSuccess) return st;
     const float* partials = splits > 1 ? plan->logit_partials : nullptr;
-    if (small) {
-        st = launch_kernel(in_registers ? route_repair_kernel<80, kWide> : route_repair_kernel<0, kWide>, dim3(rows),
-                           dim3(kWide * 32), repair_smem, stream, pdl, x, router_w, bias,
-                           static_cast<const float*>(norms), plan->logits, plan->ids, plan->route_weights, rows, hidden,
-                           routed_scale, plan->router_stats, partials, splits,
+    // between the two, four warps per token up to what the chip holds at a time
+    const bool medium = chain_order && !small && rows <= 4 * plan->sm_count;
+    const dim3 repair_grid(small || medium ? rows : (rows + kRepairWarps - 1) / kRepairWarps), repair_block(repair_warps * 32);
+    if (chain_order) {
+        st = launch_kernel(small ? route_repair_chains_kernel<kWide> : medium ? route_repair_chains_kernel<4> : route_repair_chains_kernel<1>,
+                           repair_grid, repair_block, 0, stream, pdl, x, bias, static_cast<const float*>(norms), plan->logits, plan->ids,
+                           plan->route_weights, rows, routed_scale, plan->router_stats, partials, splits,
                            static_cast<const std::uint16_t*>(plan->w_chains));
     } else {
-        st = launch_kernel(in_registers ? route_repair_kernel<80, 1> : route_repair_kernel<0, 1>,
-                           dim3((rows + kRepairWarps - 1) / kRepairWarps), dim3(kRepairWarps * 32), repair_smem, stream, pdl, x,
-                           router_w, bias, static_cast<const float*>(norms), plan->logits, plan->ids,
-                           plan->route_weights, rows, hidden, routed_scale, plan->router_stats, partials, splits,
-                           static_cast<const std::uint16_t*>(plan->w_chains));
+        st = launch_kernel(small ? route_repair_kernel<kWide> : route_repair_kernel<1>, repair_grid, repair_block, repair_smem, stream,
+                           pdl, x, router_w, bias, static_cast<const float*>(norms), plan->logits, plan->ids, plan->route_weights, rows,
+                           hidden, routed_scale, plan->router_stats, partials, splits);
     }
     plan->last_launches += 2;
     return st;
