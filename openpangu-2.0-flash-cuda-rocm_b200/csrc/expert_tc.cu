@@ -482,10 +482,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
     }
 }
 
-// Quantises the token rows into the padded position space of the tensor-core
-// kernels: row pp gets the NVFP4 bytes of its token, and the scales go straight
-// into the 128x4-tiled layout (cuda/nvfp4_ops.cu:818-841 and :869-890 in one pass).
-// The row is read and quantised once (lane l of a token's warps owns 16-element blocks l, l + 32 WARPS, ...) and
+// Quantises the token rows into the padded position space of the tensor-core kernels: a row is read and quantised once and
 // written to the nine places it is needed, its eight routed slots and its shared-expert row.  WARPS per token: 8 while
 // there are fewer tokens than would fill the chip with one each - a lane then has one block to read and nine pieces to
 // write instead of five of each one after the other (9.0 us at 64 and at 512 rows) - else 1.
@@ -498,52 +495,17 @@ __global__ void __launch_bounds__(256) quantize_padded_kernel(const std::uint16_
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31;
-    const int token = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) / WARPS;
+    const int warp = threadIdx.x >> 5;
+    const int token = (blockIdx.x * (blockDim.x >> 5) + warp) / WARPS;
     if (token >= rows) return;
-    const int blocks = hidden / 16;
-    const int col_blocks = (blocks + 3) / 4;
-    constexpr int kMaxPerLane = 8 / WARPS;           // hidden <= 4096
-    const int first = ((threadIdx.x >> 5) % WARPS) * 32 + lane;
-    uint2 packed[kMaxPerLane];
-    std::uint32_t scale_word[kMaxPerLane];           // lanes 0, 4, 8, ...: the scales of four neighbouring blocks
     // the nine destinations of the row, fetched before the row itself so that the stores wait for nothing
     const int place_index = lane < kTop ? token * kTop + lane : rows * kTop + token;
     const int my_pp = lane <= kTop ? __ldg(pp_of_flat + place_index) : 0;
-#pragma unroll
-    for (int j = 0; j < kMaxPerLane; ++j) {
-        const int b = first + 32 * WARPS * j;
-        std::uint8_t scale_bits = 0;
-        if (b < blocks) {                            // blocks is a multiple of 4: a quad of lanes is in or out together
-            const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<std::size_t>(token) * hidden + b * 16);
-            const uint4 lo = __ldg(src);
-            const uint4 hi = __ldg(src + 1);
-            const std::uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-            float v[16];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                v[2 * i] = __uint_as_float(words[i] << 16);
-                v[2 * i + 1] = __uint_as_float(words[i] & 0xffff0000U);
-            }
-            packed[j] = quantize_block16(v, global_scale, &scale_bits);
-        }
-        std::uint32_t word = scale_bits;
-        word |= __shfl_down_sync(0xffffffffU, word, 1) << 8;
-        word |= __shfl_down_sync(0xffffffffU, word, 2) << 16;
-        scale_word[j] = word;
-    }
+    QuantisedRow<WARPS> row;
+    row.load(x + static_cast<std::size_t>(token) * hidden, hidden, warp % WARPS);
+    row.quantise(global_scale);
 #pragma unroll 1
-    for (int place = 0; place <= kTop; ++place) {
-        const std::size_t pp = static_cast<std::size_t>(__shfl_sync(0xffffffffU, my_pp, place));
-        std::uint8_t* row_q = xq + pp * (hidden / 2);
-        std::uint8_t* row_s = xs + (pp >> 7) * col_blocks * 512 + (pp & 31) * 16 + ((pp >> 5) & 3) * 4;
-#pragma unroll
-        for (int j = 0; j < kMaxPerLane; ++j) {
-            const int b = first + 32 * WARPS * j;
-            if (b >= blocks) break;
-            *reinterpret_cast<uint2*>(row_q + b * 8) = packed[j];
-            if ((lane & 3) == 0) *reinterpret_cast<std::uint32_t*>(row_s + (b >> 2) * 512) = scale_word[j];
-        }
-    }
+    for (int place = 0; place <= kTop; ++place) row.store(xq, xs, static_cast<std::size_t>(__shfl_sync(0xffffffffU, my_pp, place)));
 }
 
 // The same for rows that each have ONE destination (the dense MLP's token rows, the (row, slot) intermediate rows

@@ -418,7 +418,7 @@ int p92b_moe_forward_normed(p92b_plan* plan, const p92b_bank* bank, const uint16
     // for bit); in the stage table its two kernels are the "router logits" stage and the top-8 stage is empty
     bool routed = false;
     if (rows >= router_fast_min_rows()) {
-        st = launch_router_fast(plan, input, router_weight, correction_bias, rows, routed_scale, stream, pdl);
+        st = launch_router_fast(plan, input, router_weight, correction_bias, rows, routed_scale, stream, pdl, true);
         if (st == cudaSuccess) routed = true;
         else if (st != cudaErrorNotSupported) return st;
     }
@@ -435,13 +435,16 @@ int p92b_moe_forward_normed(p92b_plan* plan, const p92b_bank* bank, const uint16
         if ((st = mark()) != cudaSuccess) return st;
         if ((st = mark()) != cudaSuccess) return st;
         if ((st = mark()) != cudaSuccess) return st;
+    } else if (routed) {
+        if ((st = mark()) != cudaSuccess) return st;
+        if ((st = launch_scan_counts(plan, rows, tile_rows, stream, pdl)) != cudaSuccess) return st;
+        if ((st = mark()) != cudaSuccess) return st;
+        if ((st = launch_place_rows(plan, input, rows, tile_rows, stream, pdl)) != cudaSuccess) return st;
+        if ((st = mark()) != cudaSuccess) return st;
     } else {
-        if (!routed) {
-            st = launch_router_top8(plan->logits, correction_bias, plan->ids, plan->route_weights, rows, routed_scale, stream,
-                                    pdl);
-            if (st != cudaSuccess) return st;
-            plan->last_launches += 1;
-        }
+        st = launch_router_top8(plan->logits, correction_bias, plan->ids, plan->route_weights, rows, routed_scale, stream, pdl);
+        if (st != cudaSuccess) return st;
+        plan->last_launches += 1;
         if ((st = mark()) != cudaSuccess) return st;
         st = launch_permute(plan, plan->ids, rows * kTop, plan->order, plan->position, plan->counts, plan->offsets, true,
                             pad_align, tile_rows, stream, pdl);

@@ -78,6 +78,63 @@ __device__ __forceinline__ uint2 quantize_block16(const float (&v)[16], float gl
     return make_uint2(words[0], words[1]);
 }
 
+// A token row quantised by WARPS warps (this one is number `part` of them; a lane owns 16-element blocks first, first + 32 WARPS,
+// ..., PER_LANE at most) and its storing at padded positions: NVFP4 bytes row-major, scales in the 128x4-tiled layout
+// (cuda/nvfp4_ops.cu:818-841 and :869-890 in one pass).  hidden <= 512 WARPS PER_LANE, a multiple of 64.  In steps, so that
+// a kernel can have the row on its way while it finds out where the row goes.
+template <int WARPS, int PER_LANE = 8 / WARPS>
+struct QuantisedRow {
+    uint4 raw[PER_LANE][2];
+    uint2 packed[PER_LANE];
+    std::uint32_t scale_word[PER_LANE];              // lanes 0, 4, 8, ...: the scales of four neighbouring blocks
+    int first, blocks;
+
+    __device__ __forceinline__ void load(const std::uint16_t* __restrict__ row, int hidden, int part) {
+        blocks = hidden / 16;
+        first = part * 32 + static_cast<int>(threadIdx.x & 31);
+#pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) {
+            const int b = first + 32 * WARPS * j;
+            if (b < blocks) {                        // blocks is a multiple of 4: a quad of lanes is in or out together
+                const uint4* src = reinterpret_cast<const uint4*>(row + b * 16);
+                raw[j][0] = __ldg(src);
+                raw[j][1] = __ldg(src + 1);
+            }
+        }
+    }
+    __device__ __forceinline__ void quantise(float global_scale) {
+#pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) {
+            std::uint8_t scale_bits = 0;
+            if (first + 32 * WARPS * j < blocks) {
+                const std::uint32_t words[8] = {raw[j][0].x, raw[j][0].y, raw[j][0].z, raw[j][0].w, raw[j][1].x, raw[j][1].y, raw[j][1].z, raw[j][1].w};
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    v[2 * i] = __uint_as_float(words[i] << 16);
+                    v[2 * i + 1] = __uint_as_float(words[i] & 0xffff0000U);
+                }
+                packed[j] = quantize_block16(v, global_scale, &scale_bits);
+            }
+            std::uint32_t word = scale_bits;
+            word |= __shfl_down_sync(0xffffffffU, word, 1) << 8;
+            word |= __shfl_down_sync(0xffffffffU, word, 2) << 16;
+            scale_word[j] = word;
+        }
+    }
+    __device__ __forceinline__ void store(std::uint8_t* __restrict__ xq, std::uint8_t* __restrict__ xs, std::size_t pp) const {
+        std::uint8_t* row_q = xq + pp * (blocks * 8);
+        std::uint8_t* row_s = xs + (pp >> 7) * ((blocks + 3) / 4) * 512 + (pp & 31) * 16 + ((pp >> 5) & 3) * 4;
+#pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) {
+            const int b = first + 32 * WARPS * j;
+            if (b >= blocks) break;
+            *reinterpret_cast<uint2*>(row_q + b * 8) = packed[j];
+            if ((first & 3) == 0) *reinterpret_cast<std::uint32_t*>(row_s + (b >> 2) * 512) = scale_word[j];
+        }
+    }
+};
+
 // Top-8 of one token by one warp for any scores, equal ones included (warp_top8 below calls it when it meets scores too
 // close for its 24-bit keys): lane l holds experts l, l+32, ..., l+224 in registers.
 // Eight rounds of (local best, warp butterfly arg-max) with the reference's total order: higher
@@ -489,8 +546,13 @@ constexpr int kRouterSplits = 8;                // K splits of the tensor-core l
 constexpr int kRouterSplitRows = 2304;          // ... used up to this many rows: 18 token tiles x 4 expert tiles, twice, on 148 SMs
 constexpr int kRouterPartialRows = 4736;        // rows x slices of their scratch: 148 SMs / 4 expert tiles x 128 rows
 constexpr int kRouterWideRows = 256;            // a block per token in the repair up to here
+// `count_experts`: plan->chunk_hist gets the experts of every 32 tokens counted, for launch_place_rows.
 cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const std::uint16_t* router_w, const float* bias,
-                               int rows, float routed_scale, cudaStream_t stream, bool pdl);
+                               int rows, float routed_scale, cudaStream_t stream, bool pdl, bool count_experts = false);
+// Behind launch_router_fast with count_experts: routing lists, positions and the token rows quantised at their places
+// (permute.cu), what launch_permute and launch_quantize_padded do for ids that come from anywhere.
+cudaError_t launch_scan_counts(p92b_plan* plan, int rows, int tile_rows, cudaStream_t stream, bool pdl);
+cudaError_t launch_place_rows(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream, bool pdl);
 // tensor-core path (expert_tc.cu)
 cudaError_t make_operand_map(CUtensorMap* map, const void* base, std::size_t rows, std::size_t row_bytes,
                              int box_rows);

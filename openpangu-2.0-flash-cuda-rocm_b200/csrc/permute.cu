@@ -424,6 +424,114 @@ __global__ void __launch_bounds__(256) permute_scatter_kernel(
     }
 }
 
+// ---- places of the block's own routing -------------------------------------------------------
+// The tensor-core router has counted the experts of every chunk of 32 tokens while it chose them, a token's eight ids are
+// different, and so the rank of an assignment in its chunk is the number of earlier tokens of the chunk that have the expert
+// too: eight votes of a warp whose lane l holds token l's ids.  Positions, lists and the quantised row are then one pass
+// over the tokens instead of two kernels (up to 5,120 assignments; 512 rows: 13.7 + 6.4 us, now 9.4) or four (4,096 rows:
+// 6 + 12 + 12 + 22 us, now 12 + 24).
+// SCANNED: permute_scan_kernel has turned the counts into prefixes over the chunks and written the lists.  Otherwise, for few
+// chunks, every block adds the counts up for itself, one expert per thread, and block 0 writes the lists: a launch less.
+constexpr int kPlaceChunks = 16;                 // up to 512 tokens without a scan kernel
+constexpr int kPlacePad = 128;                   // an expert's rows start on a multiple of this
+template <int WARPS, bool SCANNED, int PER_LANE>
+__global__ void __launch_bounds__(256) place_rows_kernel(const std::uint16_t* __restrict__ x, const std::int32_t* __restrict__ ids,
+                                                         const std::int32_t* __restrict__ chunk_hist, RouteLists lists,
+                                                         std::int32_t* __restrict__ order, std::int32_t* __restrict__ position,
+                                                         std::int32_t* __restrict__ row_token, std::int32_t* __restrict__ pp_of_flat,
+                                                         std::uint8_t* __restrict__ xq, std::uint8_t* __restrict__ xs, int rows, int hidden,
+                                                         float global_scale) {
+    static_assert(SCANNED || WARPS == 8, "a block that adds the counts up serves one token");
+    __shared__ std::int32_t scan_scratch[kWarps];
+    __shared__ std::int32_t first_position[kExperts], first_place[kExperts];        // of this chunk's rows of an expert
+    __shared__ std::int32_t shared_place;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int token = (static_cast<int>(blockIdx.x) - (SCANNED ? 0 : 1)) * (kWarps / WARPS) + warp / WARPS;      // !SCANNED: block 0 has none
+    const int chunk = token >> 5;
+    const int in_chunk = token & 31;
+    QuantisedRow<WARPS, PER_LANE> row;             // the row is on its way while its places are found
+    if constexpr (SCANNED) {
+        if (token >= rows) return;
+        row.load(x + static_cast<std::size_t>(token) * hidden, hidden, warp % WARPS);
+    } else {
+        const int e = threadIdx.x;
+        const int chunks = (rows + 31) >> 5;
+        int count[kPlaceChunks];
+#pragma unroll
+        for (int c = 0; c < kPlaceChunks; ++c) count[c] = c < chunks ? __ldcg(chunk_hist + c * kExperts + e) : 0;
+        if (blockIdx.x > 0) row.load(x + static_cast<std::size_t>(token) * hidden, hidden, warp % WARPS);
+        int total = 0, before = 0;
+#pragma unroll
+        for (int c = 0; c < kPlaceChunks; ++c) {
+            if (c < chunk) before += count[c];
+            total += count[c];
+        }
+        // both prefixes in one scan: at most 4,096 assignments and 32 + 256 pads
+        const int pads = (total + kPlacePad - 1) / kPlacePad;
+        const int prefix = block_exclusive_scan_256(pads << 16 | total, scan_scratch);
+        if (blockIdx.x == 0) {
+            write_route_lists(e, total, prefix & 0xffff, rows * kTop, rows, lists, scan_scratch);
+            return;
+        }
+        first_position[e] = (prefix & 0xffff) + before;
+        first_place[e] = (prefix >> 16) * kPlacePad + before;
+        if (e == kExperts - 1) shared_place = ((prefix >> 16) + pads) * kPlacePad;
+        __syncthreads();
+    }
+    // lane l holds the ids of the chunk's token l
+    int id[kTop];
+    {
+        const int4* at = reinterpret_cast<const int4*>(ids + static_cast<std::size_t>(min(chunk * 32 + lane, token)) * kTop);
+        const int4 a = __ldcg(at), b = __ldcg(at + 1);
+        id[0] = a.x; id[1] = a.y; id[2] = a.z; id[3] = a.w;
+        id[4] = b.x; id[5] = b.y; id[6] = b.z; id[7] = b.w;
+    }
+    int my_id = 0, my_rank = 0;                      // lane k < 8: of the token's slot k
+#pragma unroll
+    for (int k = 0; k < kTop; ++k) {
+        const int e = __shfl_sync(0xffffffffU, id[k], in_chunk);
+        bool has = false;
+#pragma unroll
+        for (int i = 0; i < kTop; ++i) has = has || id[i] == e;
+        const int rank = __popc(__ballot_sync(0xffffffffU, has && lane < in_chunk));
+        if (lane == k) {
+            my_id = e & (kExperts - 1);
+            my_rank = rank;
+        }
+    }
+    int my_place = 0;
+    if (lane < kTop) {
+        int pos;
+        if constexpr (SCANNED) {
+            const int before = __ldcg(chunk_hist + static_cast<std::size_t>(chunk) * kExperts + my_id) + my_rank;
+            pos = __ldcg(lists.offsets + my_id) + before;
+            my_place = __ldcg(lists.pp_off + my_id) + before;
+        } else {
+            pos = first_position[my_id] + my_rank;
+            my_place = first_place[my_id] + my_rank;
+        }
+        if (WARPS == 1 || warp % WARPS == 0) {
+            const int i = token * kTop + lane;
+            order[pos] = i;
+            position[i] = pos;
+            row_token[pos] = token;
+            pp_of_flat[i] = my_place;
+        }
+    } else if (lane == kTop) {
+        if constexpr (SCANNED) my_place = __ldcg(lists.pp_off + kExperts) + token; else my_place = shared_place + token;
+        if (WARPS == 1 || warp % WARPS == 0) {
+            row_token[rows * kTop + token] = token;
+            pp_of_flat[rows * kTop + token] = my_place;
+        }
+    }
+    row.quantise(global_scale);
+#pragma unroll 1
+    for (int place = 0; place <= kTop; ++place) row.store(xq, xs, static_cast<std::size_t>(__shfl_sync(0xffffffffU, my_place, place)));
+}
+
 // ---- decode front end: top-8 + permutation + lists + NVFP4 token rows, one block ------------
 // For up to 8 tokens the three routing stages are a few microseconds of work each, so they run as
 // one 256-thread block instead of three launches: warp w ranks token w; thread e counts expert e
@@ -566,14 +674,16 @@ __global__ void __launch_bounds__(256) dense_front_kernel(RouteLists lists, int 
 
 int route_fused_max_rows() { return kFusedMaxRows; }
 
-cudaError_t launch_dense_front(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
+namespace {
+// The lists that the block's expert kernels read, at 128 padded positions per started 128 rows.
+RouteLists plan_lists(p92b_plan* plan, int tile_rows) {
     RouteLists lists {};
     lists.counts = plan->counts;
     lists.offsets = plan->offsets;
     lists.active = plan->active;
     lists.active_count = plan->active_count;
     lists.enabled = true;
-    lists.pad_align = 128;
+    lists.pad_align = kPlacePad;
     lists.tile_rows = tile_rows;
     lists.pp_off = plan->pp_off;
     lists.tile_prefix = plan->tile_prefix;
@@ -581,6 +691,12 @@ cudaError_t launch_dense_front(p92b_plan* plan, const std::uint16_t* x, int rows
     lists.tile_rows_wide = wide ? 128 : tile_rows;
     lists.tile_prefix_wide = wide ? plan->tile_prefix_wide : nullptr;
     plan->wide_rows = wide ? 128 : 0;
+    return lists;
+}
+}  // namespace
+
+cudaError_t launch_dense_front(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
+    const RouteLists lists = plan_lists(plan, tile_rows);
     plan->last_launches += 1;
     const bool few = rows <= 1024;
     return launch_kernel(few ? dense_front_kernel<8> : dense_front_kernel<1>, dim3(few ? rows : (rows + 7) / 8), dim3(256), 0, stream,
@@ -607,6 +723,28 @@ cudaError_t launch_route_fused(p92b_plan* plan, const float* bias, float routed_
     return launch_kernel(route_fused_kernel, dim3(1), dim3(256), 0, stream, pdl, plan->logits, bias, plan->ids,
                          plan->route_weights, routed_scale, rows, plan->order, plan->position, lists, plan->row_token,
                          plan->pp_of_flat, x, plan->xq_pp, plan->xs_sw, plan->hidden, 1.0F);
+}
+
+cudaError_t launch_scan_counts(p92b_plan* plan, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
+    const int chunks = (rows + 31) / 32;
+    if (chunks <= kPlaceChunks) return cudaSuccess;
+    plan->last_launches += 1;
+    return launch_kernel(permute_scan_kernel, dim3(chunks >= 64 ? kScanBlocksLarge : 1), dim3(kScanThreads), 0, stream, pdl,
+                         plan->chunk_hist, chunks, rows * kTop, plan_lists(plan, tile_rows), rows, plan->scan_blocks_done);
+}
+
+cudaError_t launch_place_rows(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
+    if (plan->hidden > 4096) return cudaErrorNotSupported;
+    if (!aligned_to(16, x)) return cudaErrorInvalidValue;
+    const bool scanned = (rows + 31) / 32 > kPlaceChunks;
+    const bool few = rows <= 1024;
+    plan->last_launches += 1;
+    return launch_kernel(!scanned ? place_rows_kernel<8, false, 1> : few ? place_rows_kernel<8, true, 1>
+                                  : plan->hidden <= 2560 ? place_rows_kernel<1, true, 5> : place_rows_kernel<1, true, 8>,
+                         dim3(!scanned ? rows + 1 : few ? rows : (rows + 7) / 8), dim3(256), 0, stream, pdl, x,
+                         static_cast<const std::int32_t*>(plan->ids), static_cast<const std::int32_t*>(plan->chunk_hist),
+                         plan_lists(plan, tile_rows), plan->order, plan->position, plan->row_token, plan->pp_of_flat, plan->xq_pp,
+                         plan->xs_sw, rows, plan->hidden, 1.0F);
 }
 
 cudaError_t launch_permute(p92b_plan* plan, const std::int32_t* ids, int assignments,

@@ -117,7 +117,8 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
                                                                      float* __restrict__ logits, int rows, int hidden,
                                                                      std::int32_t* status, const std::uint16_t* __restrict__ w,
                                                                      float* __restrict__ norms,
-                                                                     std::uint16_t* __restrict__ w_chains) {
+                                                                     std::uint16_t* __restrict__ w_chains,
+                                                                     uint4* __restrict__ counts_to_clear, int clear_vectors) {
     // gridDim.z > 1: block z takes a slice of the K blocks and writes its partial sums to slice z of `logits`
     // ([gridDim.z][rows][256]); the repair kernel adds the slices (small batches: 4 blocks would otherwise walk all of
     // K one after the other while 144 SMs idle)
@@ -200,6 +201,10 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
             if (ok && k_blocks > 0) tc_commit(accum_bar);
         }
     } else {
+        // the expert counts that the repair kernel adds to
+        const int block_index = static_cast<int>((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+        const int blocks = static_cast<int>(gridDim.x * gridDim.y * gridDim.z);
+        for (int i = block_index * 128 + static_cast<int>(threadIdx.x) - 64; i < clear_vectors; i += blocks * 128) counts_to_clear[i] = make_uint4(0U, 0U, 0U, 0U);
         // while the products run, the epilogue warps take the norms of the tile's router rows, shared out over the blocks of
         // this expert tile (a kernel of its own in front of this one cost the chain 2 us)
         const int sharers = static_cast<int>(gridDim.x * gridDim.z) * 4;
@@ -355,6 +360,15 @@ __device__ __forceinline__ void list_candidates(const unsigned (&member)[8], std
     __syncwarp();
 }
 
+// The token's experts, which lanes 0..7 have just written, into the counts of its chunk of 32 tokens (null: not wanted).
+__device__ __forceinline__ void count_experts(std::int32_t* chunk_hist, int token, const std::int32_t* ids) {
+    const int lane = threadIdx.x & 31;
+    if (chunk_hist != nullptr && lane < kTop) {
+        const int e = *reinterpret_cast<const volatile std::int32_t*>(ids + lane) & (kExperts - 1);
+        atomicAdd(chunk_hist + static_cast<std::size_t>(token >> 5) * kExperts + e, 1);
+    }
+}
+
 // Logits that were not recomputed: a NaN, picked behind every number.
 __device__ __forceinline__ void clear_exact_row(float* exact_row, int first, int threads) {
     for (int e = first; e < kExperts; e += threads) exact_row[e] = __uint_as_float(0x7fc00000U);
@@ -382,7 +396,7 @@ template <int WPT>
 __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 ? 2 : 4) route_repair_chains_kernel(
     const std::uint16_t* __restrict__ x, const float* __restrict__ bias, const float* __restrict__ w_norms, float* __restrict__ logits,
     std::int32_t* __restrict__ ids, float* __restrict__ weights, int rows, float routed_scale, int* __restrict__ stats,
-    const float* __restrict__ partials, int splits, const std::uint16_t* __restrict__ w_chains) {
+    const float* __restrict__ partials, int splits, const std::uint16_t* __restrict__ w_chains, std::int32_t* __restrict__ chunk_hist) {
     constexpr int kHidden = 32 * kChainSteps;
     constexpr int kPieces = kChainSteps / 8;                  // of 16 bytes, per lane
     constexpr int kWarps = WPT > 1 ? WPT : kRepairWarps;
@@ -537,6 +551,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 
     // The reference's top-8 over the exact values.
     if (whole_row) {
         warp_top8(exact_row, bias, my_ids, my_weights, routed_scale);
+        count_experts(chunk_hist, token, my_ids);
         return;
     }
     // One candidate per lane, words as in warp_top8: nine rounds, a lane gives its word up when it is the maximum.
@@ -561,9 +576,10 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 
         if (lane < n_cand) exact_row[my_e] = mine;
         __syncwarp();
         warp_top8_by_id(exact_row, bias, my_ids, my_weights, routed_scale);
-        return;
+    } else {
+        warp_top8_write(of_slot, exact_row, my_ids, my_weights, routed_scale);
     }
-    warp_top8_write(of_slot, exact_row, my_ids, my_weights, routed_scale);
+    count_experts(chunk_hist, token, my_ids);
 }
 
 // Any other hidden size: the token row in shared memory as it is, router rows read in place, one chain at a time.
@@ -572,7 +588,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     const std::uint16_t* __restrict__ x, const std::uint16_t* __restrict__ w, const float* __restrict__ bias,
     const float* __restrict__ w_norms, float* __restrict__ logits, std::int32_t* __restrict__ ids,
     float* __restrict__ weights, int rows, int hidden, float routed_scale, int* __restrict__ stats,
-    const float* __restrict__ partials, int splits) {
+    const float* __restrict__ partials, int splits, std::int32_t* __restrict__ chunk_hist) {
     extern __shared__ __align__(16) std::uint16_t repair_smem[];
     pdl_launch_dependents();
     pdl_wait();
@@ -639,6 +655,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     // the same key chose expert 0 again and again once fewer than eight scores were numbers.)
     warp_top8(exact_row, bias, ids + static_cast<std::size_t>(token) * kTop, weights + static_cast<std::size_t>(token) * kTop,
               routed_scale);
+    count_experts(chunk_hist, token, ids + static_cast<std::size_t>(token) * kTop);
 }
 
 }  // namespace
@@ -648,7 +665,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
 int router_fast_min_rows() { return 9; }
 
 cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const std::uint16_t* router_w, const float* bias,
-                               int rows, float routed_scale, cudaStream_t stream, bool pdl) {
+                               int rows, float routed_scale, cudaStream_t stream, bool pdl, bool count_experts) {
     static const bool disabled = std::getenv("P92B_EXACT_LOGITS") != nullptr;
     const int hidden = plan->hidden;
     if (disabled || rows < router_fast_min_rows() || hidden % 64 != 0 || hidden > 8192 ||
@@ -694,9 +711,11 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     const auto kernel = expert_tile == 64 ? logits_tc_kernel<64> : expert_tile == 128 ? logits_tc_kernel<128> : logits_tc_kernel<256>;
     const int smem = expert_tile == 64 ? Logits<64>::kSmem : expert_tile == 128 ? Logits<128>::kSmem : Logits<256>::kSmem;
     st = launch_kernel(kernel, dim3(token_tiles, kExperts / expert_tile, splits), dim3(kLogitThreads), smem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status, router_w, norms,
-                       chain_order ? plan->w_chains : nullptr);
+                       chain_order ? plan->w_chains : nullptr, reinterpret_cast<uint4*>(plan->chunk_hist),
+                       count_experts ? (rows + 31) / 32 * kExperts / 4 : 0);
     if (st != cudaSuccess) return st;
     const float* partials = splits > 1 ? plan->logit_partials : nullptr;
+    std::int32_t* chunk_hist = count_experts ? plan->chunk_hist : nullptr;
     // between the two, four warps per token up to what the chip holds at a time
     const bool medium = chain_order && !small && rows <= 4 * plan->sm_count;
     const dim3 repair_grid(small || medium ? rows : (rows + kRepairWarps - 1) / kRepairWarps), repair_block(repair_warps * 32);
@@ -704,11 +723,11 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
         st = launch_kernel(small ? route_repair_chains_kernel<kWide> : medium ? route_repair_chains_kernel<4> : route_repair_chains_kernel<1>,
                            repair_grid, repair_block, 0, stream, pdl, x, bias, static_cast<const float*>(norms), plan->logits, plan->ids,
                            plan->route_weights, rows, routed_scale, plan->router_stats, partials, splits,
-                           static_cast<const std::uint16_t*>(plan->w_chains));
+                           static_cast<const std::uint16_t*>(plan->w_chains), chunk_hist);
     } else {
         st = launch_kernel(small ? route_repair_kernel<kWide> : route_repair_kernel<1>, repair_grid, repair_block, repair_smem, stream,
                            pdl, x, router_w, bias, static_cast<const float*>(norms), plan->logits, plan->ids, plan->route_weights, rows,
-                           hidden, routed_scale, plan->router_stats, partials, splits);
+                           hidden, routed_scale, plan->router_stats, partials, splits, chunk_hist);
     }
     plan->last_launches += 2;
     return st;

@@ -1,0 +1,37 @@
+"""Lists and places of the block's own routing, and batches in which a few experts have most of the tiles."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows", [9, 31, 32, 33, 255, 511, 512, 513, 1024, 1025, 1030, 2049])
+@pytest.mark.parametrize("popular", [0, 2])
+def test_places_of_the_routed_rows(cuda, pkg, layer0, rows, popular):
+    """The ranks come from chunks of 32 tokens, the sums over the chunks from every block up to 512 rows and from a kernel of
+    their own above; either side of these sizes the permutation is the stable sort of the ids, bit for bit, and an expert's
+    rows lie one behind the other from a multiple of 128 on, the shared expert's last."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    bias = layer0.bias.clone()
+    bias[[3, 255][:popular]] += 4.0
+    plan = pkg.MoePlan(max_rows=rows)
+    plan.set_path(plan.PATH_TENSOR_CORE)
+    x = synth.make_activations(91, rows, rows)
+    pkg.MoeBlock(layer0.bank, layer0.router_weight, bias, plan).run_moe_rows(x, torch.empty_like(x), rows)
+    views = {k: v.cpu().numpy() for k, v in plan.views(rows).items() if v is not None and v.dtype == torch.int32}
+    assert plan.status() == 0
+    plan.close()
+    ids = views["expert_ids"].reshape(-1)
+    want = np.argsort(ids, kind="stable")
+    counts = np.bincount(ids, minlength=256)
+    offsets = np.concatenate([[0], np.cumsum(counts)])
+    assert np.array_equal(views["order"], want)
+    assert np.array_equal(views["position"][want], np.arange(rows * 8))
+    assert np.array_equal(views["counts"], counts)
+    assert np.array_equal(views["offsets"], offsets)
+    base = np.concatenate([[0], np.cumsum((counts + 127) // 128 * 128)])
+    rank = views["position"] - offsets[ids]
+    assert np.array_equal(views["mixed_index"][: rows * 8], base[ids] + rank)
+    assert np.array_equal(views["mixed_index"][rows * 8:], base[256] + np.arange(rows))
