@@ -115,6 +115,36 @@ __device__ __forceinline__ std::uint32_t bf16x2_bits(float low, float high) {
     return *reinterpret_cast<const std::uint32_t*>(&pair);
 }
 
+// The tensor map of a matrix of the caller's table for the product kernel's loads: the host's map of a matrix of this shape
+// with the matrix's own address.  By a warp, through 128 bytes of shared memory; maps of matrices off a 16-byte boundary are
+// not built (the product kernel rejects them).
+__device__ __forceinline__ void build_table_map(const TableMaps& maps, int which, std::uint32_t* image) {
+    const int lane = threadIdx.x & 31;
+    const std::uint8_t* matrix = maps.table[which].weight;
+    if ((reinterpret_cast<std::uintptr_t>(matrix) & 15U) != 0U) return;
+    image[lane] = reinterpret_cast<const std::uint32_t*>(&maps.box)[lane];
+    __syncwarp();
+    if (lane == 0) tensormap_set_address(image, matrix);
+    __syncwarp();
+    tensormap_publish(maps.maps + which, image);
+}
+
+// A row that the caller has quantised in the reference's layout (packed [R][K/2], scales 128x4-tiled over the R rows), copied by
+// a warp to padded position pp.
+__device__ __forceinline__ void copy_quantised_row(const std::uint8_t* __restrict__ packed, const std::uint8_t* __restrict__ scales_swizzled,
+                                                   std::size_t src, std::uint8_t* __restrict__ xq, std::uint8_t* __restrict__ xs,
+                                                   std::size_t pp, int k_bytes) {
+    const int lane = threadIdx.x & 31;
+    const uint4* from = reinterpret_cast<const uint4*>(packed + src * k_bytes);
+    uint4* to = reinterpret_cast<uint4*>(xq + pp * k_bytes);
+    for (int v = lane; v < k_bytes / 16; v += 32) to[v] = __ldg(from + v);
+    const int scale_columns = k_bytes / 8;                       // K / 16
+    const int col_blocks = (scale_columns + 3) / 4;
+    const std::uint8_t* sf_from = scales_swizzled + (src >> 7) * col_blocks * 512 + (src & 31) * 16 + ((src >> 5) & 3) * 4;
+    std::uint8_t* sf_to = xs + (pp >> 7) * col_blocks * 512 + (pp & 31) * 16 + ((pp >> 5) & 3) * 4;
+    for (int c = lane; c < scale_columns; c += 32) sf_to[(c >> 2) * 512 + (c & 3)] = sf_from[(c >> 2) * 512 + (c & 3)];
+}
+
 }  // namespace expert
 
 // Large-batch products with the tokens on the M side (expert_rows.cu); p.tile_prefix counts 128-row tiles.

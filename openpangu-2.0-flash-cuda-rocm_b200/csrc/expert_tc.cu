@@ -745,37 +745,20 @@ __global__ void __launch_bounds__(256) gather_quantized_rows_kernel(const std::u
     __shared__ __align__(128) std::uint32_t map_image[8][32];
     pdl_launch_dependents();
     pdl_wait();
-    const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int gather_blocks = (assignments + 7) / 8;
     const int i = blockIdx.x * 8 + warp;
     if (static_cast<int>(blockIdx.x) >= gather_blocks) {
-        // a warp per matrix: the host's map of a matrix of this shape with the matrix's own address, so that the product
-        // kernel loads whole boxes by TMA; maps of matrices off a 16-byte boundary are not built (it rejects them)
+        // a warp per matrix of an active expert; slot 0 is the shared expert, which has no rows here
         const int m = i - gather_blocks * 8;
-        const int slot = 1 + m / maps.kinds;                          // slot 0 is the shared expert, which has no rows here
-        if (slot >= *maps.active_count) return;
-        const int which = maps.active[slot] * 3 + maps.first_kind + m % maps.kinds;
-        const std::uint8_t* matrix = maps.table[which].weight;
-        if ((reinterpret_cast<std::uintptr_t>(matrix) & 15U) != 0U) return;
-        map_image[warp][lane] = reinterpret_cast<const std::uint32_t*>(&maps.box)[lane];
-        __syncwarp();
-        if (lane == 0) tensormap_set_address(map_image[warp], matrix);
-        __syncwarp();
-        tensormap_publish(maps.maps + which, map_image[warp]);
+        const int slot = 1 + m / maps.kinds;
+        if (slot < *maps.active_count) build_table_map(maps, maps.active[slot] * 3 + maps.first_kind + m % maps.kinds, map_image[warp]);
         return;
     }
     if (i >= assignments) return;
     const std::size_t src = static_cast<std::size_t>(distinct_rows ? i : i / kTop);
     const std::size_t pp = static_cast<std::size_t>(pp_of_flat[i]);
-    const uint4* from = reinterpret_cast<const uint4*>(packed + src * k_bytes);
-    uint4* to = reinterpret_cast<uint4*>(xq + pp * k_bytes);
-    for (int v = lane; v < k_bytes / 16; v += 32) to[v] = __ldg(from + v);
-    const int scale_columns = k_bytes / 8;                       // K / 16
-    const int col_blocks = (scale_columns + 3) / 4;
-    const std::uint8_t* sf_from = scales_swizzled + (src >> 7) * col_blocks * 512 + (src & 31) * 16 + ((src >> 5) & 3) * 4;
-    std::uint8_t* sf_to = xs + (pp >> 7) * col_blocks * 512 + (pp & 31) * 16 + ((pp >> 5) & 3) * 4;
-    for (int c = lane; c < scale_columns; c += 32) sf_to[(c >> 2) * 512 + (c & 3)] = sf_from[(c >> 2) * 512 + (c & 3)];
+    copy_quantised_row(packed, scales_swizzled, src, xq, xs, pp, k_bytes);
 }
 }  // namespace
 

@@ -622,12 +622,9 @@ int p92b_project_expert_gate_up(p92b_plan* plan, const p92b_bank* bank, const in
     static const bool pdl = std::getenv("P92B_NO_PDL") == nullptr;
     plan->last_launches = 0;
     plan->last_path = 2;
-    // permutation of the caller's ids -> token rows quantised into the padded position space -> the grouped
+    // permutation of the caller's ids and token rows quantised into the padded position space -> the grouped
     // tcgen05 product with the epilogue that stores gate and up un-fused at their (row, slot) rows
-    cudaError_t st = launch_permute(plan, expert_ids, rows * kTop, plan->order, plan->position, plan->counts,
-                                    plan->offsets, true, tc_pad_align(rows), tc_tile_rows(rows), stream, pdl);
-    if (st != cudaSuccess) return st;
-    st = launch_quantize_padded(plan, input, rows, stream, pdl);
+    cudaError_t st = launch_token_assignments(plan, expert_ids, input, rows, tc_tile_rows(rows), false, stream, pdl);
     if (st != cudaSuccess) return st;
     TcIo io {};
     io.gate_out = gate_output;
@@ -635,7 +632,7 @@ int p92b_project_expert_gate_up(p92b_plan* plan, const p92b_bank* bank, const in
     io.out_row = plan->order;
     io.skip_shared = true;
     st = launch_experts_tc(plan, bank, rows, false, stream, pdl, &io);
-    plan->last_launches += 2;
+    plan->last_launches += 1;
     return st;
 }
 
@@ -650,12 +647,7 @@ int p92b_project_expert_down(p92b_plan* plan, const p92b_bank* bank, const int32
     static const bool pdl = std::getenv("P92B_NO_PDL") == nullptr;
     plan->last_launches = 0;
     plan->last_path = 2;
-    cudaError_t st = launch_permute(plan, expert_ids, rows * kTop, plan->order, plan->position, plan->counts,
-                                    plan->offsets, true, tc_pad_align(rows), tc_tile_rows(rows), stream, pdl);
-    if (st != cudaSuccess) return st;
-    // every (row, slot) intermediate row is quantised on its own (src/executor.cpp:85-91), to its padded position
-    st = launch_quantize_rows_to_pp(input_rows, plan->pp_of_flat, plan->hq_pp, plan->hs_sw, rows * kTop, plan->intermediate,
-                                    stream, pdl);
+    cudaError_t st = launch_token_assignments(plan, expert_ids, input_rows, rows, tc_tile_rows(rows), true, stream, pdl);
     if (st != cudaSuccess) return st;
     TcIo io {};
     io.down_out = output_rows;
@@ -663,7 +655,7 @@ int p92b_project_expert_down(p92b_plan* plan, const p92b_bank* bank, const int32
     io.skip_shared = true;
     io.wait_upstream = true;
     st = launch_experts_tc(plan, bank, rows, true, stream, pdl, &io);
-    plan->last_launches += 2;
+    plan->last_launches += 1;
     return st;
 }
 
@@ -730,12 +722,6 @@ int p92b_nvfp4_grouped_rows(p92b_grouped_plan* plan, const uint8_t* packed_input
     static const bool pdl = std::getenv("P92B_NO_PDL") == nullptr;
     p->last_launches = 0;
     p->last_path = 2;
-    const int assignments = batch_rows * kTop;
-    // the reference orders its problems by (kind, expert) with ties in the original order
-    // (cuda/nvfp4_grouped.cu:117-132); the same stable order groups the rows per expert here
-    cudaError_t st = launch_permute(p, expert_ids, assignments, p->order, p->position, p->counts, p->offsets, true,
-                                    tc_pad_align(batch_rows), tc_tile_rows(batch_rows), stream, pdl);
-    if (st != cudaSuccess) return st;
     TableMaps maps {};
     maps.table = expert_bank;
     maps.active = p->active;
@@ -744,9 +730,11 @@ int p92b_nvfp4_grouped_rows(p92b_grouped_plan* plan, const uint8_t* packed_input
     maps.box = p->map_table[down ? 1 : 0];
     maps.first_kind = projection_kind;
     maps.kinds = second_output != nullptr ? 2 : 1;
-    st = launch_gather_quantized_rows(packed_input, input_scales_swizzled, p->pp_of_flat, down ? p->hq_pp : p->xq_pp,
-                                      down ? p->hs_sw : p->xs_sw, assignments, plan->columns / 2,
-                                      expert_distinct_input_rows != 0, maps, stream, pdl);
+    // the reference orders its problems by (kind, expert) with ties in the original order
+    // (cuda/nvfp4_grouped.cu:117-132); the same stable order groups the rows per expert here
+    cudaError_t st = launch_quantised_assignments(p, expert_ids, batch_rows * kTop, tc_tile_rows(batch_rows), packed_input,
+                                                  input_scales_swizzled, down, plan->columns / 2, expert_distinct_input_rows != 0, maps,
+                                                  stream, pdl);
     if (st != cudaSuccess) return st;
     TcIo io {};
     io.table = expert_bank;
@@ -761,7 +749,7 @@ int p92b_nvfp4_grouped_rows(p92b_grouped_plan* plan, const uint8_t* packed_input
         io.single_matrix = !down;
     }
     st = launch_experts_tc(p, nullptr, batch_rows, down, stream, pdl, &io);
-    p->last_launches += 2;
+    p->last_launches += 1;
     return st;
 }
 

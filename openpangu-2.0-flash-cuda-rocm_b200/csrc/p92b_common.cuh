@@ -594,6 +594,13 @@ cudaError_t launch_gather_quantized_rows(const std::uint8_t* packed, const std::
                                          const std::int32_t* pp_of_flat, std::uint8_t* xq, std::uint8_t* xs, int assignments,
                                          int k_bytes, bool distinct_rows, const TableMaps& maps, cudaStream_t stream,
                                          bool pdl = false);
+// Fronts of the operators on the caller's expert ids: lists, permutation and the rows at their padded positions; quantised rows with
+// the maps of the matrices in place, or BF16 rows (down: one per assignment, else one per token).
+cudaError_t launch_quantised_assignments(p92b_plan* plan, const std::int32_t* ids, int assignments, int tile_rows,
+                                         const std::uint8_t* packed, const std::uint8_t* scales_swizzled, bool down, int k_bytes,
+                                         bool distinct_rows, const TableMaps& maps, cudaStream_t stream, bool pdl);
+cudaError_t launch_token_assignments(p92b_plan* plan, const std::int32_t* ids, const std::uint16_t* x, int rows, int tile_rows, bool down,
+                                     cudaStream_t stream, bool pdl);
 cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int rows, bool down,
                               cudaStream_t stream, bool pdl = false, const TcIo* io = nullptr);
 // The dense MLP of a few rows (dense_rows.cu, which says how few).

@@ -10,8 +10,7 @@
 // result is deterministic: each warp owns a contiguous chunk of flat indices,
 // ranks inside a 32-wide step come from a vote per id bit + popcount of the
 // lower lanes, and chunk bases come from an exclusive scan over (expert, chunk).
-#include "p92b_common.cuh"
-#include "tc_ptx.cuh"
+#include "expert_common.cuh"
 
 #include <cstdio>
 
@@ -532,6 +531,100 @@ __global__ void __launch_bounds__(256) place_rows_kernel(const std::uint16_t* __
     for (int place = 0; place <= kTop; ++place) row.store(xq, xs, static_cast<std::size_t>(__shfl_sync(0xffffffffU, my_place, place)));
 }
 
+// ---- lists, places and rows of a call on ids that come from the caller -------------------------------
+// Up to 512 assignments (64 tokens) the front of an operator call is one kernel: every block counts the experts for itself
+// (shared-memory atomics, a scan of the 256 counts), and a warp per assignment finds its rank from votes over the earlier ids,
+// its padded position, and brings its row there; block 0 writes the lists.  As permutation and row kernel the two took a
+// launch more: the operator sequence of four layers at four rows took 284 us, now 271.
+// SOURCE 0: rows of a caller that has quantised them, with the tensor maps of the matrices in place; 1: BF16 rows, quantised here.
+constexpr int kFrontMax = 512;
+struct FrontRows {
+    const std::uint8_t* packed;              // SOURCE 0
+    const std::uint8_t* scales_swizzled;
+    const std::uint16_t* rows;               // SOURCE 1
+    std::uint8_t* xq;
+    std::uint8_t* xs;
+    int width;                               // elements of a row
+    int distinct;                            // 1: a row per assignment, 0: the eight slots of a token share its row
+};
+template <int SOURCE>
+__global__ void __launch_bounds__(256) assignment_rows_kernel(const std::int32_t* __restrict__ ids, int assignments, RouteLists lists,
+                                                              std::int32_t* __restrict__ order, std::int32_t* __restrict__ position,
+                                                              std::int32_t* __restrict__ row_token, std::int32_t* __restrict__ pp_of_flat,
+                                                              std::int32_t* status, FrontRows from, const __grid_constant__ TableMaps maps) {
+    __shared__ __align__(128) std::uint32_t map_image[kWarps][32];
+    __shared__ std::int32_t cached_ids[kFrontMax];
+    __shared__ std::int32_t counts[kExperts], first_position[kExperts], first_place[kExperts];
+    __shared__ std::int32_t scan_scratch[kWarps];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int e = threadIdx.x;
+    counts[e] = 0;
+    __syncthreads();
+    for (int j = threadIdx.x; j < assignments; j += 256) {
+        const int id = ids[j];
+        if ((id < 0 || id >= kExperts) && blockIdx.x == 0) atomicCAS(status, kStatusOk, kStatusBadExpertId);
+        const int clamped = id < 0 ? 0 : (id >= kExperts ? kExperts - 1 : id);
+        cached_ids[j] = clamped;
+        atomicAdd(counts + clamped, 1);
+    }
+    __syncthreads();
+    // positions and padded positions in one scan: at most 512 assignments, each in a 128-row pad of its own
+    const int count = counts[e];
+    const bool spaced = lists.tile_rows < 64;                    // tiles of 16 or 32 rows lie a pad apart
+    const int pads = spaced ? (count + lists.tile_rows - 1) / lists.tile_rows : (count + kPlacePad - 1) / kPlacePad;
+    const int prefix = block_exclusive_scan_256(pads << 16 | count, scan_scratch);
+    first_position[e] = prefix & 0xffff;
+    first_place[e] = (prefix >> 16) * kPlacePad;
+    __syncthreads();
+    const int i = static_cast<int>(blockIdx.x) * kWarps + warp;
+    if (i < assignments) {
+        const int mine = cached_ids[i];
+        int rank = 0;
+        for (int step = 0; step < i; step += 32) {
+            const int j = step + lane;
+            rank += __popc(__ballot_sync(0xffffffffU, j < i && cached_ids[j] == mine));
+        }
+        const int gaps = spaced ? rank / lists.tile_rows * (kPlacePad - lists.tile_rows) : 0;
+        const int place = first_place[mine] + rank + gaps;
+        if (lane == 0) {
+            const int pos = first_position[mine] + rank;
+            order[pos] = i;
+            position[i] = pos;
+            row_token[pos] = i / kTop;
+            pp_of_flat[i] = place;
+        }
+        const std::size_t row = static_cast<std::size_t>(from.distinct ? i : i / kTop);
+        if constexpr (SOURCE == 0) {
+            if (rank == 0) {
+                for (int k = 0; k < maps.kinds; ++k) {
+                    expert::build_table_map(maps, mine * 3 + maps.first_kind + k, map_image[warp]);
+                    __syncwarp();
+                }
+            }
+            expert::copy_quantised_row(from.packed, from.scales_swizzled, row, from.xq, from.xs, place, from.width / 2);
+        } else {
+            QuantisedRow<1> quantised;
+            quantised.load(from.rows + row * from.width, from.width, 0);
+            quantised.quantise(1.0F);
+            quantised.store(from.xq, from.xs, place);
+        }
+    }
+    if (blockIdx.x == 0) {
+        const int rows = assignments / kTop;
+        write_route_lists(e, count, prefix & 0xffff, assignments, rows, lists, scan_scratch);
+        const int shared_place = __shfl_sync(0xffffffffU, ((prefix >> 16) + pads) * kPlacePad, 31);      // behind the last expert's: warp 7's lane 31
+        if (warp == kWarps - 1) {
+            for (int t = lane; t < rows; t += 32) {
+                row_token[assignments + t] = t;
+                pp_of_flat[assignments + t] = shared_place + t;
+            }
+        }
+    }
+}
+
 // ---- decode front end: top-8 + permutation + lists + NVFP4 token rows, one block ------------
 // For up to 8 tokens the three routing stages are a few microseconds of work each, so they run as
 // one 256-thread block instead of three launches: warp w ranks token w; thread e counts expert e
@@ -701,6 +794,56 @@ cudaError_t launch_dense_front(p92b_plan* plan, const std::uint16_t* x, int rows
     const bool few = rows <= 1024;
     return launch_kernel(few ? dense_front_kernel<8> : dense_front_kernel<1>, dim3(few ? rows : (rows + 7) / 8), dim3(256), 0, stream,
                          pdl, lists, rows, x, plan->xq_pp, plan->xs_sw, plan->hidden, 1.0F);
+}
+
+namespace {
+cudaError_t launch_assignment_rows(p92b_plan* plan, const std::int32_t* ids, int assignments, int tile_rows, const FrontRows& from,
+                                   const TableMaps* maps, cudaStream_t stream, bool pdl) {
+    plan->last_launches += 1;
+    const RouteLists lists = plan_lists(plan, tile_rows);
+    return launch_kernel(maps != nullptr ? assignment_rows_kernel<0> : assignment_rows_kernel<1>, dim3((assignments + kWarps - 1) / kWarps),
+                         dim3(256), 0, stream, pdl, ids, assignments, lists, plan->order, plan->position, plan->row_token,
+                         plan->pp_of_flat, plan->status, from, maps != nullptr ? *maps : TableMaps {});
+}
+}  // namespace
+
+cudaError_t launch_quantised_assignments(p92b_plan* plan, const std::int32_t* ids, int assignments, int tile_rows,
+                                         const std::uint8_t* packed, const std::uint8_t* scales_swizzled, bool down, int k_bytes,
+                                         bool distinct_rows, const TableMaps& maps, cudaStream_t stream, bool pdl) {
+    if (packed == nullptr || scales_swizzled == nullptr || assignments <= 0 || k_bytes % 16 != 0 || !aligned_to(16, packed)) {
+        return cudaErrorInvalidValue;
+    }
+    std::uint8_t* xq = down ? plan->hq_pp : plan->xq_pp;
+    std::uint8_t* xs = down ? plan->hs_sw : plan->xs_sw;
+    if (assignments <= kFrontMax) {
+        return launch_assignment_rows(plan, ids, assignments, tile_rows, FrontRows {packed, scales_swizzled, nullptr, xq, xs, 2 * k_bytes, distinct_rows},
+                                      &maps, stream, pdl);
+    }
+    cudaError_t st = launch_permute(plan, ids, assignments, plan->order, plan->position, plan->counts, plan->offsets, true, kPlacePad,
+                                    tile_rows, stream, pdl);
+    if (st != cudaSuccess) return st;
+    plan->last_launches += 1;
+    return launch_gather_quantized_rows(packed, scales_swizzled, plan->pp_of_flat, xq, xs, assignments, k_bytes, distinct_rows, maps,
+                                        stream, pdl);
+}
+
+cudaError_t launch_token_assignments(p92b_plan* plan, const std::int32_t* ids, const std::uint16_t* x, int rows, int tile_rows, bool down,
+                                     cudaStream_t stream, bool pdl) {
+    const int width = down ? plan->intermediate : plan->hidden;
+    if (!down && width > 4096) return cudaErrorNotSupported;
+    if (!aligned_to(16, x)) return cudaErrorInvalidValue;
+    if (rows * kTop <= kFrontMax && width <= 4096) {
+        return launch_assignment_rows(plan, ids, rows * kTop, tile_rows,
+                                      FrontRows {nullptr, nullptr, x, down ? plan->hq_pp : plan->xq_pp, down ? plan->hs_sw : plan->xs_sw, width, down},
+                                      nullptr, stream, pdl);
+    }
+    cudaError_t st = launch_permute(plan, ids, rows * kTop, plan->order, plan->position, plan->counts, plan->offsets, true, kPlacePad,
+                                    tile_rows, stream, pdl);
+    if (st != cudaSuccess) return st;
+    plan->last_launches += 1;
+    // the down operator's rows are the (row, slot) intermediate rows, each quantised on its own (src/executor.cpp:85-91)
+    return down ? launch_quantize_rows_to_pp(x, plan->pp_of_flat, plan->hq_pp, plan->hs_sw, rows * kTop, width, stream, pdl)
+                : launch_quantize_padded(plan, x, rows, stream, pdl);
 }
 
 cudaError_t launch_route_fused(p92b_plan* plan, const float* bias, float routed_scale, const std::uint16_t* x,

@@ -96,3 +96,37 @@ def test_rows_without_an_expert_are_counted_as_expert_0(cuda, pkg, layer0, rows)
     for got, want in zip(outs[1], outs[0]):
         assert torch.isfinite(want.float()).all() and _same_bits(torch, got, want)
     plan.close()
+
+
+@pytest.mark.parametrize("rows", [1, 2, 7, 16, 17, 33, 63, 64, 65])
+def test_fronts_of_the_operators_on_a_callers_ids(cuda, pkg, layer0, rows):
+    """Up to 64 rows one kernel counts, ranks and places, above two do; ids repeat within a token and leave the range.  Operators
+    on the bank and on weights in place go through different forms of it and give the same bits, and so do a batch's rows
+    and the same rows at the head of one of 72."""
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    ids = torch.randint(-2, 258, (72, 8), generator=g, device="cuda").to(torch.int32)
+    ids[::3, 4:] = 9                                              # an expert with more rows than the batch
+    x = torch.empty((72, HIDDEN), device="cuda").normal_(0, 1, generator=g).to(torch.bfloat16)
+    h = torch.empty((72 * 8, INTER), device="cuda").normal_(0, 1, generator=g).to(torch.bfloat16)
+    table = _table(torch, layer0.raw)
+    results = []
+    for n in (rows, 72):
+        plan = pkg.MoePlan(max_rows=n)
+        block = pkg.MoeBlock(layer0.bank, layer0.router_weight, layer0.bias, plan)
+        out = [torch.full((n * 8, width), float("nan"), dtype=torch.bfloat16, device="cuda") for width in (INTER, INTER, HIDDEN) * 2]
+        these = ids[:n].contiguous()
+        block.project_expert_gate_up(these, x[:n], out[0], out[1], n)
+        block.project_expert_down(these, h[:n * 8], out[2], n)
+        gate_up, down = pkg.GroupedPlan(n * 16, INTER, HIDDEN), pkg.GroupedPlan(n * 8, HIDDEN, INTER)
+        gate_up.grouped_rows(*_quantised(torch, pkg, x[:n]), table, these, out[3], out[4], 0, n, False)
+        down.grouped_rows(*_quantised(torch, pkg, h[:n * 8]), table, these, out[5], None, 2, n, True)
+        bad = int(((these < 0) | (these > 255)).any())
+        assert plan.status() == bad and gate_up.status() == bad and down.status() == bad
+        results.append(out)
+        for p in (plan, gate_up, down):
+            p.close()
+    for k in range(6):
+        assert torch.isfinite(results[0][k].float()).all()
+        assert _same_bits(torch, results[0][k], results[1][k][:rows * 8])
+        assert _same_bits(torch, results[0][k], results[0][k % 3])
