@@ -292,17 +292,9 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const std::uint16_t* 
 // Fused tail of the block: the weighted combine above (gathering each slot's
 // down row from position space), rounded to BF16 exactly where the reference
 // stores `hidden_`, then the shared expert's BF16 down row added and rounded
-// again (src/model.cpp:1505-1508 then :1571-1572).  Eight columns per thread.
-__global__ void __launch_bounds__(256) combine_shared_kernel(const std::uint16_t* __restrict__ mixed,
-                                                             const std::int32_t* __restrict__ mixed_index,
-                                                             const float* __restrict__ route_weights,
-                                                             std::uint16_t* __restrict__ output, int rows,
-                                                             int hidden) {
-    ptx::pdl_launch_dependents();
-    ptx::pdl_wait();
-    const int row = blockIdx.y;
-    const int c8 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c8 * 8 >= hidden) return;
+// again (src/model.cpp:1505-1508 then :1571-1572).  Eight columns of a row.
+__device__ __forceinline__ uint4 combine_shared8(const std::uint16_t* __restrict__ mixed, const std::int32_t* __restrict__ mixed_index,
+                                                 const float* __restrict__ route_weights, int rows, int hidden, int row, int c8) {
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.0F;
@@ -334,8 +326,77 @@ __global__ void __launch_bounds__(256) combine_shared_kernel(const std::uint16_t
         out_words[k] = static_cast<std::uint32_t>(float_to_bf16_bits(lo)) |
                        (static_cast<std::uint32_t>(float_to_bf16_bits(hi)) << 16);
     }
+    return make_uint4(out_words[0], out_words[1], out_words[2], out_words[3]);
+}
+
+__global__ void __launch_bounds__(256) combine_shared_kernel(const std::uint16_t* __restrict__ mixed,
+                                                             const std::int32_t* __restrict__ mixed_index,
+                                                             const float* __restrict__ route_weights,
+                                                             std::uint16_t* __restrict__ output, int rows,
+                                                             int hidden) {
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    const int row = blockIdx.y;
+    const int c8 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c8 * 8 >= hidden) return;
     *reinterpret_cast<uint4*>(output + static_cast<std::size_t>(row) * hidden + c8 * 8) =
-        make_uint4(out_words[0], out_words[1], out_words[2], out_words[3]);
+        combine_shared8(mixed, mixed_index, route_weights, rows, hidden, row, c8);
+}
+
+// The same with the RMSNorm behind the block (src/model.cpp:216-217,1215-1216) in the same pass: a block has its row together in
+// shared memory, where the norm's chains read it in the operator's order (rmsnorm_rows_kernel).  As a kernel of its own the norm
+// read and wrote every output row once more (3,807 rows with both norms: 416 us a call, now 411).
+constexpr int kCombineNormMaxHidden = 8192;
+__global__ void __launch_bounds__(1024) combine_shared_norm_kernel(const std::uint16_t* __restrict__ mixed,
+                                                                   const std::int32_t* __restrict__ mixed_index,
+                                                                   const float* __restrict__ route_weights,
+                                                                   const std::uint16_t* __restrict__ norm_weight,
+                                                                   std::uint16_t* __restrict__ output, int rows, int hidden, float epsilon) {
+    extern __shared__ __align__(16) std::uint16_t norm_row[];
+    __shared__ float warp_sums[8];
+    __shared__ float inverse_shared;
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    const int row = blockIdx.x;
+    const int c8 = threadIdx.x;
+    const bool mine = c8 * 8 < hidden;
+    uint4 value = make_uint4(0U, 0U, 0U, 0U);
+    if (mine) {
+        value = combine_shared8(mixed, mixed_index, route_weights, rows, hidden, row, c8);
+        reinterpret_cast<uint4*>(norm_row)[c8] = value;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    if (warp < 8) {
+        float square_sum = 0.0F;
+        for (int i = threadIdx.x; i < hidden; i += 256) {
+            const float v = bf16_bits_to_float(norm_row[i]);
+            square_sum = fmaf(v, v, square_sum);
+        }
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) square_sum += __shfl_down_sync(0xffffffffU, square_sum, offset);
+        if (lane == 0) warp_sums[warp] = square_sum;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        float total = lane < 8 ? warp_sums[lane] : 0.0F;
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_down_sync(0xffffffffU, total, offset);
+        if (lane == 0) inverse_shared = rsqrtf(total / static_cast<float>(hidden) + epsilon);
+    }
+    __syncthreads();
+    if (!mine) return;
+    const float inverse = inverse_shared;
+    std::uint32_t words[4] = {value.x, value.y, value.z, value.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const std::uint16_t* w = norm_weight + c8 * 8 + 2 * k;
+        const std::uint32_t lo = float_to_bf16_bits(__uint_as_float(words[k] << 16) * inverse * bf16_bits_to_float(__ldg(w)));
+        const std::uint32_t hi = float_to_bf16_bits(__uint_as_float(words[k] & 0xffff0000U) * inverse * bf16_bits_to_float(__ldg(w + 1)));
+        words[k] = lo | hi << 16;
+    }
+    *reinterpret_cast<uint4*>(output + static_cast<std::size_t>(row) * hidden + c8 * 8) = make_uint4(words[0], words[1], words[2], words[3]);
 }
 
 // Row-major packed weights + tiled scales of one matrix -> the chunk stream (see BankView).
@@ -423,6 +484,16 @@ cudaError_t launch_combine_shared(const std::uint16_t* mixed, const std::int32_t
     dim3 grid(blocks_for(hidden / 8, 256), rows);
     return launch_kernel(combine_shared_kernel, grid, dim3(256), 0, stream, pdl, mixed, mixed_index, route_weights,
                          output, rows, hidden);
+}
+
+cudaError_t launch_combine_shared_norm(const std::uint16_t* mixed, const std::int32_t* mixed_index, const float* route_weights,
+                                       const std::uint16_t* norm_weight, std::uint16_t* output, int rows, int hidden, float epsilon,
+                                       cudaStream_t stream, bool pdl) {
+    if (hidden > kCombineNormMaxHidden) return cudaErrorNotSupported;
+    if (!aligned_to(16, output)) return cudaErrorInvalidValue;
+    const unsigned threads = std::max(256U, blocks_for(hidden / 8, 32) * 32);          // the norm's 256 chains have a thread each
+    return launch_kernel(combine_shared_norm_kernel, dim3(rows), dim3(threads), static_cast<std::size_t>(hidden) * 2, stream, pdl, mixed,
+                         mixed_index, route_weights, norm_weight, output, rows, hidden, epsilon);
 }
 
 cudaError_t launch_rmsnorm(const std::uint16_t* input, const std::uint16_t* weight, std::uint16_t* output, int rows,

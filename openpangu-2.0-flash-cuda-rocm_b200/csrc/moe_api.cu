@@ -461,15 +461,19 @@ int p92b_moe_forward_normed(p92b_plan* plan, const p92b_bank* bank, const uint16
     st = launch_experts_tc(plan, bank, rows, true, stream, pdl);
     if (st != cudaSuccess) return st;
     if ((st = mark()) != cudaSuccess) return st;
-    st = launch_combine_shared(plan->mixed_pp, plan->pp_of_flat, plan->route_weights, output, rows, hidden, stream, pdl);
     plan->last_launches += 3;
-    if (st != cudaSuccess) return st;
-    if (post_norm_weight != nullptr) {
-        // in place: a block holds its whole row in shared memory before it writes
-        st = launch_rmsnorm(output, post_norm_weight, output, rows, hidden, hidden, hidden, norm_epsilon, stream, pdl);
-        if (st != cudaSuccess) return st;
-        plan->last_launches += 1;
+    st = post_norm_weight == nullptr ? cudaErrorNotSupported
+                                     : launch_combine_shared_norm(plan->mixed_pp, plan->pp_of_flat, plan->route_weights, post_norm_weight,
+                                                                  output, rows, hidden, norm_epsilon, stream, pdl);
+    if (st == cudaErrorNotSupported) {
+        st = launch_combine_shared(plan->mixed_pp, plan->pp_of_flat, plan->route_weights, output, rows, hidden, stream, pdl);
+        if (st == cudaSuccess && post_norm_weight != nullptr) {
+            // in place: a block holds its whole row in shared memory before it writes
+            st = launch_rmsnorm(output, post_norm_weight, output, rows, hidden, hidden, hidden, norm_epsilon, stream, pdl);
+            plan->last_launches += 1;
+        }
     }
+    if (st != cudaSuccess) return st;
     if (debug_sync && !plan->timing && (st = mark()) != cudaSuccess) return st;
     if (plan->timing) {
         if ((st = mark()) != cudaSuccess) return st;

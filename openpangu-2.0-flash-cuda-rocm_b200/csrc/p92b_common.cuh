@@ -536,6 +536,10 @@ cudaError_t launch_retile_table(const p92b_expert_projection* device_table, int 
 cudaError_t launch_combine_shared(const std::uint16_t* mixed, const std::int32_t* mixed_index,
                                   const float* route_weights, std::uint16_t* output, int rows,
                                   int hidden, cudaStream_t stream, bool pdl = false);
+// The same with the RMSNorm of the output rows; cudaErrorNotSupported above 8,192 columns: launch_rmsnorm behind it then.
+cudaError_t launch_combine_shared_norm(const std::uint16_t* mixed, const std::int32_t* mixed_index, const float* route_weights,
+                                       const std::uint16_t* norm_weight, std::uint16_t* output, int rows, int hidden, float epsilon,
+                                       cudaStream_t stream, bool pdl);
 cudaError_t launch_rmsnorm(const std::uint16_t* input, const std::uint16_t* weight, std::uint16_t* output, int rows,
                            int elements, int input_stride, int output_stride, float epsilon, cudaStream_t stream,
                            bool pdl = false);
