@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 const std::uint32_t* wr = reinterpret_cast<const std::uint32_t*>(w_rows + r * row_pitch) + l16;
                 const std::uint32_t* xr = reinterpret_cast<const std::uint32_t*>(x_rows + t * row_pitch) + l16;
                 float even = 0.0F, odd = 0.0F;
-#pragma unroll 8
+#pragma unroll 16
                 for (int j = 0; j < hidden / 32; ++j) {
                     const std::uint32_t wv = wr[16 * j], xv = xr[16 * j];
                     even = fmaf(__uint_as_float(xv << 16), __uint_as_float(wv << 16), even);
@@ -437,6 +437,9 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     }
 
     // ------------------------------------------------------------------ P1
+    // The lists need the ids only: a warp without a role in P2 computes its token's weights while the first tiles load.
+    int weights_of = -1;
+    std::uint32_t top_words = 0U;
     // (the last warp is left out: it is the one that waits for the fence above)
     constexpr int kPollers = kMegaThreads - 32;
     if (warp < kMegaWarps - 1) {
@@ -473,8 +476,18 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
         __syncwarp();
         asm volatile("bar.sync 3, %0;" ::"n"(kPollers) : "memory");
         if (threadIdx.x == 0) stamp(2);
-        for (int t = warp; t < rows && !abort_word; t += kMegaWarps - 1) {
-            warp_top8(rt.logits + t * kExperts, rt.bias, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
+        for (int t = kMegaWarps - 2 - warp; t < rows && !abort_word; t += kMegaWarps - 1) {
+            const float* lg = rt.logits + t * kExperts;
+            const std::uint32_t words = warp_top8_words(lg, rt.bias);
+            if (top8_is_close(words)) {
+                warp_top8_by_id(lg, rt.bias, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
+            } else if (warp >= kEpilogueEnd && t < kMegaWarps - 1) {
+                if (lane < kTop) rt.ids[t * kTop + lane] = top8_id(words);
+                weights_of = t;
+                top_words = words;
+            } else {
+                warp_top8_write(words, lg, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
+            }
         }
         if (threadIdx.x == 0) stamp(13);
     }
@@ -700,6 +713,10 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     } else if (warp >= kEpilogueEnd) {
         // the routing products go to global memory for the caller (ids, weights, permutation, histogram)
         constexpr int kHelpers = kMegaThreads - 32 * kEpilogueEnd;
+        if (weights_of >= 0) {
+            warp_top8_weights(top_words, rt.logits + weights_of * kExperts, rt.weights + weights_of * kTop, p.routed_scale);
+        }
+        asm volatile("bar.sync 2, %0;" ::"n"(kHelpers) : "memory");
         if (block == 0 && !abort_word) {
             for (int t = threadIdx.x - 32 * kEpilogueEnd; t < assignments; t += kHelpers) {
                 const int pos = rt.less[t] + rt.rank[t];
