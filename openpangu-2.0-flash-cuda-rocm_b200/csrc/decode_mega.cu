@@ -88,6 +88,7 @@ struct MegaParams {
     std::uint8_t* hs;              // tiled scales of hq
     std::uint16_t* mixed;          // [PP][H]
     unsigned long long* logits_tagged;   // [kReplicas][R][256] {value, launch number}
+    unsigned long long* choices;         // [kReplicas][R][8] {id, launch number, route weight, launch number}
     unsigned long long* ret;             // [8][9][1280] {two BF16, launch number}
     unsigned* sync;                // [0]: blocks that have finished P0 (monotonic across launches)
     std::int32_t* gu_done;         // [2][264] by launch parity: gate/up tiles finished per active slot, [257] tile counter
@@ -338,6 +339,12 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
         atomicCAS(p.status, kStatusOk, code);
     };
 
+    // From 9 rows on (the build for 16) the tokens are spread over as many blocks: a token's block polls its 256 words and ranks them,
+    // and every block polls the eight choices of every token.  With 148 blocks that each polled up to 4,096 words and ranked up
+    // to 16 tokens a layer of 13 rows took 71.9 us, now 70.4, and of 16 rows 83.8, now 81.1; at four rows the second poll costs more
+    // than it saves.
+    constexpr bool kSpreadRouting = R > 8;
+    constexpr int kCopies = kSpreadRouting ? 1 : kReplicas;
     // ------------------------------------------------------------------ P0
     {
         if (rows == 1) {
@@ -396,7 +403,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 if (my_experts == 2 || 2 * q + half < rows) {
                     const int e = block + r * grid;
                     if (l16 == 0) p.logits[static_cast<std::size_t>(t) * kExperts + e] = value;
-                    if (l16 < kReplicas) st_tagged(p.logits_tagged + (l16 * R + t) * kExperts + e, __float_as_uint(value), tag);
+                    if (l16 < kCopies) st_tagged(p.logits_tagged + (l16 * R + t) * kExperts + e, __float_as_uint(value), tag);
                 }
             }
         }
@@ -445,48 +452,83 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
     if (warp < kMegaWarps - 1) {
         for (int i = threadIdx.x; i < kMaxActive * R; i += kPollers) (&rt.pp_tok[0][0])[i] = -1;
         for (int i = threadIdx.x; i < kExperts; i += kPollers) rt.expert_mask[i] = 0U;
-        // logits come from all blocks of this launch: each word is polled until it carries this launch's number.  All of a
-        // thread's words are requested before the first is looked at, and only the missing ones again.
-        constexpr int kPerThread = (R * kExperts / 2 + kPollers - 1) / kPollers;        // pairs of words
-        const unsigned long long* const mine = p.logits_tagged + (block % kReplicas) * R * kExperts;
-        uint4 pair[kPerThread];
-        unsigned missing = 0U;
-#pragma unroll
-        for (int j = 0; j < kPerThread; ++j) {
-            if (2 * (static_cast<int>(threadIdx.x) + j * kPollers) < rows * kExperts) missing |= 1U << j;
-        }
-        const std::uint64_t poll_start = global_timer_ns();
-        while (missing != 0U) {
-#pragma unroll
-            for (int j = 0; j < kPerThread; ++j) {
-                if (missing >> j & 1U) pair[j] = ld_tagged_pair(mine + 2 * (threadIdx.x + j * kPollers));
+        if constexpr (kSpreadRouting) {
+            // token t's words are polled, and its experts chosen, by block t alone; every block then polls the choices
+            if (block < rows) {
+                if (threadIdx.x < kExperts / 2) {
+                    std::uint32_t first = 0U, second = 0U;
+                    if (!poll_tagged_pair(p.logits_tagged + block * kExperts + 2 * threadIdx.x, tag, &first, &second)) {
+                        give_up(kStatusWaitExpired);
+                    }
+                    reinterpret_cast<float2*>(rt.logits)[threadIdx.x] = make_float2(__uint_as_float(first), __uint_as_float(second));
+                }
+                __syncwarp();
+                asm volatile("bar.sync 3, %0;" ::"n"(kPollers) : "memory");
+                if (threadIdx.x == 0) stamp(2);
+                if (warp == 0 && !abort_word) {
+                    warp_top8(rt.logits, rt.bias, rt.ids, rt.weights, p.routed_scale);
+                    __syncwarp();
+                    for (int i = lane; i < kReplicas * kTop; i += 32) {
+                        unsigned long long* to = p.choices + 2 * ((i / kTop * R + block) * kTop + i % kTop);
+                        st_tagged(to, static_cast<std::uint32_t>(rt.ids[i % kTop]), tag);
+                        st_tagged(to + 1, __float_as_uint(rt.weights[i % kTop]), tag);
+                    }
+                    __syncwarp();
+                }
+                asm volatile("bar.sync 3, %0;" ::"n"(kPollers) : "memory");
             }
+            if (static_cast<int>(threadIdx.x) < assignments && !abort_word) {
+                std::uint32_t id = 0U, weight = 0U;
+                if (!poll_tagged_pair(p.choices + 2 * ((block % kReplicas) * R * kTop + static_cast<int>(threadIdx.x)), tag, &id, &weight)) {
+                    give_up(kStatusWaitExpired);
+                }
+                rt.ids[threadIdx.x] = static_cast<std::int32_t>(id);
+                rt.weights[threadIdx.x] = __uint_as_float(weight);
+            }
+        } else {
+            // logits come from all blocks of this launch: each word is polled until it carries this launch's number.  All of a
+            // thread's words are requested before the first is looked at, and only the missing ones again.
+            constexpr int kPerThread = (R * kExperts / 2 + kPollers - 1) / kPollers;        // pairs of words
+            const unsigned long long* const mine = p.logits_tagged + (block % kReplicas) * R * kExperts;
+            uint4 pair[kPerThread];
+            unsigned missing = 0U;
 #pragma unroll
             for (int j = 0; j < kPerThread; ++j) {
-                if ((missing >> j & 1U) && pair[j].y == tag && pair[j].w == tag) {
-                    reinterpret_cast<float2*>(rt.logits)[threadIdx.x + j * kPollers] = make_float2(__uint_as_float(pair[j].x), __uint_as_float(pair[j].z));
-                    missing &= ~(1U << j);
+                if (2 * (static_cast<int>(threadIdx.x) + j * kPollers) < rows * kExperts) missing |= 1U << j;
+            }
+            const std::uint64_t poll_start = global_timer_ns();
+            while (missing != 0U) {
+#pragma unroll
+                for (int j = 0; j < kPerThread; ++j) {
+                    if (missing >> j & 1U) pair[j] = ld_tagged_pair(mine + 2 * (threadIdx.x + j * kPollers));
+                }
+#pragma unroll
+                for (int j = 0; j < kPerThread; ++j) {
+                    if ((missing >> j & 1U) && pair[j].y == tag && pair[j].w == tag) {
+                        reinterpret_cast<float2*>(rt.logits)[threadIdx.x + j * kPollers] = make_float2(__uint_as_float(pair[j].x), __uint_as_float(pair[j].z));
+                        missing &= ~(1U << j);
+                    }
+                }
+                if (missing != 0U && global_timer_ns() - poll_start > 1000000000ULL) {
+                    give_up(kStatusWaitExpired);
+                    break;
                 }
             }
-            if (missing != 0U && global_timer_ns() - poll_start > 1000000000ULL) {
-                give_up(kStatusWaitExpired);
-                break;
-            }
-        }
-        __syncwarp();
-        asm volatile("bar.sync 3, %0;" ::"n"(kPollers) : "memory");
-        if (threadIdx.x == 0) stamp(2);
-        for (int t = kMegaWarps - 2 - warp; t < rows && !abort_word; t += kMegaWarps - 1) {
-            const float* lg = rt.logits + t * kExperts;
-            const std::uint32_t words = warp_top8_words(lg, rt.bias);
-            if (top8_is_close(words)) {
-                warp_top8_by_id(lg, rt.bias, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
-            } else if (warp >= kEpilogueEnd && t < kMegaWarps - 1) {
-                if (lane < kTop) rt.ids[t * kTop + lane] = top8_id(words);
-                weights_of = t;
-                top_words = words;
-            } else {
-                warp_top8_write(words, lg, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
+            __syncwarp();
+            asm volatile("bar.sync 3, %0;" ::"n"(kPollers) : "memory");
+            if (threadIdx.x == 0) stamp(2);
+            for (int t = kMegaWarps - 2 - warp; t < rows && !abort_word; t += kMegaWarps - 1) {
+                const float* lg = rt.logits + t * kExperts;
+                const std::uint32_t words = warp_top8_words(lg, rt.bias);
+                if (top8_is_close(words)) {
+                    warp_top8_by_id(lg, rt.bias, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
+                } else if (warp >= kEpilogueEnd && t < kMegaWarps - 1) {
+                    if (lane < kTop) rt.ids[t * kTop + lane] = top8_id(words);
+                    weights_of = t;
+                    top_words = words;
+                } else {
+                    warp_top8_write(words, lg, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
+                }
             }
         }
         if (threadIdx.x == 0) stamp(13);
@@ -981,6 +1023,7 @@ cudaError_t launch_decode_mega(p92b_plan* plan, const p92b_bank* bank, const std
     p.hs = plan->hs_sw;
     p.mixed = plan->mixed_pp;
     p.logits_tagged = plan->mega_logits;
+    p.choices = plan->mega_choices;
     p.ret = plan->mega_ret;
     p.sync = plan->mega_sync;
     p.gu_done = plan->gu_done;

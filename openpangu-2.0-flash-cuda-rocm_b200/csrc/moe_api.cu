@@ -190,6 +190,7 @@ int p92b_plan_create(p92b_plan** out, int max_rows, int hidden, int intermediate
         plan->ep_gu_done = c.take<std::int32_t>(2 * 264);
         plan->ep_logits = c.take<unsigned long long>(static_cast<std::size_t>(8) * kExperts);
         plan->mega_logits = c.take<unsigned long long>(static_cast<std::size_t>(kLogitReplicas) * 16 * kExperts);
+        plan->mega_choices = c.take<unsigned long long>(static_cast<std::size_t>(kLogitReplicas) * 16 * kTop * 2);
         plan->mega_ret = c.take<unsigned long long>(static_cast<std::size_t>(16) * (kTop + 1) * 1280);
         plan->mega_trace = c.take<unsigned long long>(static_cast<std::size_t>(plan->sm_count) * 64);
         plan->w_norms = c.take<float>(kExperts);

@@ -406,6 +406,7 @@ struct p92b_plan {
     std::int32_t* ep_gu_done = nullptr;   // [2][264] the same for the fused expert-parallel kernel
     unsigned long long* ep_logits = nullptr;    // [8][256] its router logits as tagged words
     unsigned long long* mega_logits = nullptr;  // [8][16][256] router logits as {value, launch number} words, in eight copies
+    unsigned long long* mega_choices = nullptr; // [8][16][8] experts and route weights of every token as tagged words, in eight copies
     unsigned long long* mega_ret = nullptr;     // [8][9][1280] down rows as {two BF16, launch number} words
     float* w_norms = nullptr;                   // [256] norms of the router rows (tensor-core router)
     std::uint16_t* w_chains = nullptr;          // [256][H] the router rows in chain order (tensor-core router)
