@@ -369,6 +369,7 @@ struct p92b_plan {
     int wide_rows = 0;                    // token tile tile_prefix_wide was last built for (0: not built)
     std::int32_t* pp_of_flat = nullptr;   // [9*max_rows] padded position of (row, slot), shared rows last
     std::int32_t* chunk_hist = nullptr;   // [chunks][256]
+    std::int32_t* span_hist = nullptr;    // [(chunks + 15) / 16][256] the same counts for 16 chunks at a time
     unsigned* scan_blocks_done = nullptr; // [1] blocks of the permutation's scan kernel that have finished (zero between calls)
     int chunks = 0;
     std::uint8_t* xq = nullptr;           // [max_rows][H/2]
@@ -551,7 +552,7 @@ constexpr int kRouterSplits = 8;                // K splits of the tensor-core l
 constexpr int kRouterSplitRows = 2304;          // ... used up to this many rows: 18 token tiles x 4 expert tiles, twice, on 148 SMs
 constexpr int kRouterPartialRows = 4736;        // rows x slices of their scratch: 148 SMs / 4 expert tiles x 128 rows
 constexpr int kRouterWideRows = 256;            // a block per token in the repair up to here
-// `count_experts`: plan->chunk_hist gets the experts of every 32 tokens counted, for launch_place_rows.
+// `count_experts`: plan->chunk_hist and span_hist get the experts of every 32 and every 512 tokens counted, for launch_place_rows.
 cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const std::uint16_t* router_w, const float* bias,
                                int rows, float routed_scale, cudaStream_t stream, bool pdl, bool count_experts = false);
 // Behind launch_router_fast with count_experts: routing lists, positions and the token rows quantised at their places

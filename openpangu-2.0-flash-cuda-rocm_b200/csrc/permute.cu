@@ -429,18 +429,22 @@ __global__ void __launch_bounds__(256) permute_scatter_kernel(
 // too: eight votes of a warp whose lane l holds token l's ids.  Positions, lists and the quantised row are then one pass
 // over the tokens instead of two kernels (up to 5,120 assignments; 512 rows: 13.7 + 6.4 us, now 9.4) or four (4,096 rows:
 // 6 + 12 + 12 + 22 us, now 12 + 24).
-// SCANNED: permute_scan_kernel has turned the counts into prefixes over the chunks and written the lists.  Otherwise, for few
-// chunks, every block adds the counts up for itself, one expert per thread, and block 0 writes the lists: a launch less.
-constexpr int kPlaceChunks = 16;                 // up to 512 tokens without a scan kernel
+// Every block adds the counts up for itself, one expert per thread: whole spans of 512 tokens, which the router counts too, and the
+// chunks of its own span; block 0 writes the lists.  At 8,192 tokens that is 31 words per thread from the L2.
+// SCANNED, above that: permute_scan_kernel has turned the counts into prefixes over the chunks and written the lists.  It takes 12 us;
+// at 16,384 tokens the words would cost the place kernel 9, at 4,096 they cost nothing that shows (whole calls 422.6 -> 416.9 us
+// without the scan kernel).
+constexpr int kPlaceRows = 8192;                 // up to here without a scan kernel
+constexpr int kSpanChunks = 16;                  // chunks of 32 tokens whose counts are also kept as one
 constexpr int kPlacePad = 128;                   // an expert's rows start on a multiple of this
 template <int WARPS, bool SCANNED, int PER_LANE>
 __global__ void __launch_bounds__(256) place_rows_kernel(const std::uint16_t* __restrict__ x, const std::int32_t* __restrict__ ids,
-                                                         const std::int32_t* __restrict__ chunk_hist, RouteLists lists,
+                                                         const std::int32_t* __restrict__ chunk_hist,
+                                                         const std::int32_t* __restrict__ span_hist, RouteLists lists,
                                                          std::int32_t* __restrict__ order, std::int32_t* __restrict__ position,
                                                          std::int32_t* __restrict__ row_token, std::int32_t* __restrict__ pp_of_flat,
                                                          std::uint8_t* __restrict__ xq, std::uint8_t* __restrict__ xs, int rows, int hidden,
                                                          float global_scale) {
-    static_assert(SCANNED || WARPS == 8, "a block that adds the counts up serves one token");
     __shared__ std::int32_t scan_scratch[kWarps];
     __shared__ std::int32_t first_position[kExperts], first_place[kExperts];        // of this chunk's rows of an expert
     __shared__ std::int32_t shared_place;
@@ -448,38 +452,47 @@ __global__ void __launch_bounds__(256) place_rows_kernel(const std::uint16_t* __
     pdl_wait();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int token = (static_cast<int>(blockIdx.x) - (SCANNED ? 0 : 1)) * (kWarps / WARPS) + warp / WARPS;      // !SCANNED: block 0 has none
+    // (the tokens of a block are of one chunk; !SCANNED: block 0 has none)
+    const int token = (static_cast<int>(blockIdx.x) - (SCANNED ? 0 : 1)) * (kWarps / WARPS) + warp / WARPS;
     const int chunk = token >> 5;
     const int in_chunk = token & 31;
     QuantisedRow<WARPS, PER_LANE> row;             // the row is on its way while its places are found
-    if constexpr (SCANNED) {
-        if (token >= rows) return;
-        row.load(x + static_cast<std::size_t>(token) * hidden, hidden, warp % WARPS);
-    } else {
+    if (token >= 0 && token < rows) row.load(x + static_cast<std::size_t>(token) * hidden, hidden, warp % WARPS);
+    if constexpr (!SCANNED) {
         const int e = threadIdx.x;
-        const int chunks = (rows + 31) >> 5;
-        int count[kPlaceChunks];
+        const int spans = (rows + 32 * kSpanChunks - 1) / (32 * kSpanChunks);
+        const int my_span = max(chunk, 0) / kSpanChunks;
+        // all of the span's chunks in one round trip
+        int of_chunk[kSpanChunks - 1];
 #pragma unroll
-        for (int c = 0; c < kPlaceChunks; ++c) count[c] = c < chunks ? __ldcg(chunk_hist + c * kExperts + e) : 0;
-        if (blockIdx.x > 0) row.load(x + static_cast<std::size_t>(token) * hidden, hidden, warp % WARPS);
-        int total = 0, before = 0;
-#pragma unroll
-        for (int c = 0; c < kPlaceChunks; ++c) {
-            if (c < chunk) before += count[c];
-            total += count[c];
+        for (int i = 0; i < kSpanChunks - 1; ++i) {
+            const int c = my_span * kSpanChunks + i;
+            of_chunk[i] = c < chunk ? __ldcg(chunk_hist + c * kExperts + e) : 0;
         }
-        // both prefixes in one scan: at most 4,096 assignments and 32 + 256 pads
+        int total = 0, before = 0;
+#pragma unroll 8
+        for (int s = 0; s < spans; ++s) {
+            const int n = __ldcg(span_hist + s * kExperts + e);
+            total += n;
+            if (s < my_span) before += n;
+        }
+#pragma unroll
+        for (int i = 0; i < kSpanChunks - 1; ++i) before += of_chunk[i];
+        // both prefixes in one scan: at most 65,536 assignments and 512 + 256 pads
+        static_assert(kPlaceRows * kTop < 1 << 18 && kPlaceRows * kTop / kPlacePad + kExperts < 1 << 13, "two fields of a word");
         const int pads = (total + kPlacePad - 1) / kPlacePad;
-        const int prefix = block_exclusive_scan_256(pads << 16 | total, scan_scratch);
+        const int prefix = block_exclusive_scan_256(pads << 18 | total, scan_scratch);
+        const int position0 = prefix & ((1 << 18) - 1), pad0 = prefix >> 18;
         if (blockIdx.x == 0) {
-            write_route_lists(e, total, prefix & 0xffff, rows * kTop, rows, lists, scan_scratch);
+            write_route_lists(e, total, position0, rows * kTop, rows, lists, scan_scratch);
             return;
         }
-        first_position[e] = (prefix & 0xffff) + before;
-        first_place[e] = (prefix >> 16) * kPlacePad + before;
-        if (e == kExperts - 1) shared_place = ((prefix >> 16) + pads) * kPlacePad;
+        first_position[e] = position0 + before;
+        first_place[e] = pad0 * kPlacePad + before;
+        if (e == kExperts - 1) shared_place = (pad0 + pads) * kPlacePad;
         __syncthreads();
     }
+    if (token >= rows) return;
     // lane l holds the ids of the chunk's token l
     int id[kTop];
     {
@@ -869,25 +882,27 @@ cudaError_t launch_route_fused(p92b_plan* plan, const float* bias, float routed_
 }
 
 cudaError_t launch_scan_counts(p92b_plan* plan, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
+    if (rows <= kPlaceRows) return cudaSuccess;
     const int chunks = (rows + 31) / 32;
-    if (chunks <= kPlaceChunks) return cudaSuccess;
     plan->last_launches += 1;
-    return launch_kernel(permute_scan_kernel, dim3(chunks >= 64 ? kScanBlocksLarge : 1), dim3(kScanThreads), 0, stream, pdl,
+    return launch_kernel(permute_scan_kernel, dim3(kScanBlocksLarge), dim3(kScanThreads), 0, stream, pdl,
                          plan->chunk_hist, chunks, rows * kTop, plan_lists(plan, tile_rows), rows, plan->scan_blocks_done);
 }
 
 cudaError_t launch_place_rows(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
     if (plan->hidden > 4096) return cudaErrorNotSupported;
     if (!aligned_to(16, x)) return cudaErrorInvalidValue;
-    const bool scanned = (rows + 31) / 32 > kPlaceChunks;
+    const bool scanned = rows > kPlaceRows;
     const bool few = rows <= 1024;
+    const bool narrow = plan->hidden <= 2560;
     plan->last_launches += 1;
-    return launch_kernel(!scanned ? place_rows_kernel<8, false, 1> : few ? place_rows_kernel<8, true, 1>
-                                  : plan->hidden <= 2560 ? place_rows_kernel<1, true, 5> : place_rows_kernel<1, true, 8>,
-                         dim3(!scanned ? rows + 1 : few ? rows : (rows + 7) / 8), dim3(256), 0, stream, pdl, x,
+    return launch_kernel(few       ? place_rows_kernel<8, false, 1>
+                         : scanned ? narrow ? place_rows_kernel<1, true, 5> : place_rows_kernel<1, true, 8>
+                                   : narrow ? place_rows_kernel<1, false, 5> : place_rows_kernel<1, false, 8>,
+                         dim3((few ? rows : (rows + 7) / 8) + (scanned ? 0 : 1)), dim3(256), 0, stream, pdl, x,
                          static_cast<const std::int32_t*>(plan->ids), static_cast<const std::int32_t*>(plan->chunk_hist),
-                         plan_lists(plan, tile_rows), plan->order, plan->position, plan->row_token, plan->pp_of_flat, plan->xq_pp,
-                         plan->xs_sw, rows, plan->hidden, 1.0F);
+                         static_cast<const std::int32_t*>(plan->span_hist), plan_lists(plan, tile_rows), plan->order, plan->position,
+                         plan->row_token, plan->pp_of_flat, plan->xq_pp, plan->xs_sw, rows, plan->hidden, 1.0F);
 }
 
 cudaError_t launch_permute(p92b_plan* plan, const std::int32_t* ids, int assignments,

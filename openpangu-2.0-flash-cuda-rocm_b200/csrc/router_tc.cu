@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
                                                                      std::int32_t* status, const std::uint16_t* __restrict__ w,
                                                                      float* __restrict__ norms,
                                                                      std::uint16_t* __restrict__ w_chains,
-                                                                     uint4* __restrict__ counts_to_clear, int clear_vectors) {
+                                                                     uint4* __restrict__ chunk_counts, int chunk_vectors,
+                                                                     uint4* __restrict__ span_counts, int span_vectors) {
     // gridDim.z > 1: block z takes a slice of the K blocks and writes its partial sums to slice z of `logits`
     // ([gridDim.z][rows][256]); the repair kernel adds the slices (small batches: 4 blocks would otherwise walk all of
     // K one after the other while 144 SMs idle)
@@ -204,7 +205,9 @@ __global__ void __launch_bounds__(kLogitThreads, 1) logits_tc_kernel(const __gri
         // the expert counts that the repair kernel adds to
         const int block_index = static_cast<int>((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
         const int blocks = static_cast<int>(gridDim.x * gridDim.y * gridDim.z);
-        for (int i = block_index * 128 + static_cast<int>(threadIdx.x) - 64; i < clear_vectors; i += blocks * 128) counts_to_clear[i] = make_uint4(0U, 0U, 0U, 0U);
+        for (int i = block_index * 128 + static_cast<int>(threadIdx.x) - 64; i < chunk_vectors + span_vectors; i += blocks * 128) {
+            (i < chunk_vectors ? chunk_counts[i] : span_counts[i - chunk_vectors]) = make_uint4(0U, 0U, 0U, 0U);
+        }
         // while the products run, the epilogue warps take the norms of the tile's router rows, shared out over the blocks of
         // this expert tile (a kernel of its own in front of this one cost the chain 2 us)
         const int sharers = static_cast<int>(gridDim.x * gridDim.z) * 4;
@@ -360,12 +363,14 @@ __device__ __forceinline__ void list_candidates(const unsigned (&member)[8], std
     __syncwarp();
 }
 
-// The token's experts, which lanes 0..7 have just written, into the counts of its chunk of 32 tokens (null: not wanted).
-__device__ __forceinline__ void count_experts(std::int32_t* chunk_hist, int token, const std::int32_t* ids) {
+// The token's experts, which lanes 0..7 have just written, into the counts of its chunk of 32 tokens and of its span of 512
+// (null: not wanted).
+__device__ __forceinline__ void count_experts(std::int32_t* chunk_hist, std::int32_t* span_hist, int token, const std::int32_t* ids) {
     const int lane = threadIdx.x & 31;
     if (chunk_hist != nullptr && lane < kTop) {
         const int e = *reinterpret_cast<const volatile std::int32_t*>(ids + lane) & (kExperts - 1);
         atomicAdd(chunk_hist + static_cast<std::size_t>(token >> 5) * kExperts + e, 1);
+        atomicAdd(span_hist + static_cast<std::size_t>(token >> 9) * kExperts + e, 1);
     }
 }
 
@@ -396,7 +401,8 @@ template <int WPT>
 __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 ? 2 : 4) route_repair_chains_kernel(
     const std::uint16_t* __restrict__ x, const float* __restrict__ bias, const float* __restrict__ w_norms, float* __restrict__ logits,
     std::int32_t* __restrict__ ids, float* __restrict__ weights, int rows, float routed_scale, int* __restrict__ stats,
-    const float* __restrict__ partials, int splits, const std::uint16_t* __restrict__ w_chains, std::int32_t* __restrict__ chunk_hist) {
+    const float* __restrict__ partials, int splits, const std::uint16_t* __restrict__ w_chains, std::int32_t* __restrict__ chunk_hist,
+    std::int32_t* __restrict__ span_hist) {
     constexpr int kHidden = 32 * kChainSteps;
     constexpr int kPieces = kChainSteps / 8;                  // of 16 bytes, per lane
     constexpr int kWarps = WPT > 1 ? WPT : kRepairWarps;
@@ -551,7 +557,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 
     // The reference's top-8 over the exact values.
     if (whole_row) {
         warp_top8(exact_row, bias, my_ids, my_weights, routed_scale);
-        count_experts(chunk_hist, token, my_ids);
+        count_experts(chunk_hist, span_hist, token, my_ids);
         return;
     }
     // One candidate per lane, words as in warp_top8: nine rounds, a lane gives its word up when it is the maximum.
@@ -579,7 +585,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 
     } else {
         warp_top8_write(of_slot, exact_row, my_ids, my_weights, routed_scale);
     }
-    count_experts(chunk_hist, token, my_ids);
+    count_experts(chunk_hist, span_hist, token, my_ids);
 }
 
 // Any other hidden size: the token row in shared memory as it is, router rows read in place, one chain at a time.
@@ -588,7 +594,8 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     const std::uint16_t* __restrict__ x, const std::uint16_t* __restrict__ w, const float* __restrict__ bias,
     const float* __restrict__ w_norms, float* __restrict__ logits, std::int32_t* __restrict__ ids,
     float* __restrict__ weights, int rows, int hidden, float routed_scale, int* __restrict__ stats,
-    const float* __restrict__ partials, int splits, std::int32_t* __restrict__ chunk_hist) {
+    const float* __restrict__ partials, int splits, std::int32_t* __restrict__ chunk_hist,
+    std::int32_t* __restrict__ span_hist) {
     extern __shared__ __align__(16) std::uint16_t repair_smem[];
     pdl_launch_dependents();
     pdl_wait();
@@ -655,7 +662,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     // the same key chose expert 0 again and again once fewer than eight scores were numbers.)
     warp_top8(exact_row, bias, ids + static_cast<std::size_t>(token) * kTop, weights + static_cast<std::size_t>(token) * kTop,
               routed_scale);
-    count_experts(chunk_hist, token, ids + static_cast<std::size_t>(token) * kTop);
+    count_experts(chunk_hist, span_hist, token, ids + static_cast<std::size_t>(token) * kTop);
 }
 
 }  // namespace
@@ -712,7 +719,8 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
     const int smem = expert_tile == 64 ? Logits<64>::kSmem : expert_tile == 128 ? Logits<128>::kSmem : Logits<256>::kSmem;
     st = launch_kernel(kernel, dim3(token_tiles, kExperts / expert_tile, splits), dim3(kLogitThreads), smem, stream, pdl, map_x, map_w, approx_out, rows, hidden, plan->status, router_w, norms,
                        chain_order ? plan->w_chains : nullptr, reinterpret_cast<uint4*>(plan->chunk_hist),
-                       count_experts ? (rows + 31) / 32 * kExperts / 4 : 0);
+                       count_experts ? (rows + 31) / 32 * kExperts / 4 : 0, reinterpret_cast<uint4*>(plan->span_hist),
+                       count_experts ? (rows + 511) / 512 * kExperts / 4 : 0);
     if (st != cudaSuccess) return st;
     const float* partials = splits > 1 ? plan->logit_partials : nullptr;
     std::int32_t* chunk_hist = count_experts ? plan->chunk_hist : nullptr;
@@ -723,11 +731,11 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
         st = launch_kernel(small ? route_repair_chains_kernel<kWide> : medium ? route_repair_chains_kernel<4> : route_repair_chains_kernel<1>,
                            repair_grid, repair_block, 0, stream, pdl, x, bias, static_cast<const float*>(norms), plan->logits, plan->ids,
                            plan->route_weights, rows, routed_scale, plan->router_stats, partials, splits,
-                           static_cast<const std::uint16_t*>(plan->w_chains), chunk_hist);
+                           static_cast<const std::uint16_t*>(plan->w_chains), chunk_hist, plan->span_hist);
     } else {
         st = launch_kernel(small ? route_repair_kernel<kWide> : route_repair_kernel<1>, repair_grid, repair_block, repair_smem, stream,
                            pdl, x, router_w, bias, static_cast<const float*>(norms), plan->logits, plan->ids, plan->route_weights, rows,
-                           hidden, routed_scale, plan->router_stats, partials, splits, chunk_hist);
+                           hidden, routed_scale, plan->router_stats, partials, splits, chunk_hist, plan->span_hist);
     }
     plan->last_launches += 2;
     return st;

@@ -5,12 +5,13 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [9, 31, 32, 33, 255, 511, 512, 513, 1024, 1025, 1030, 2049])
+@pytest.mark.parametrize("rows", [9, 31, 32, 33, 255, 511, 512, 513, 1024, 1025, 1030, 2049, 8192, 8193])
 @pytest.mark.parametrize("popular", [0, 2])
 def test_places_of_the_routed_rows(cuda, pkg, layer0, rows, popular):
-    """The ranks come from chunks of 32 tokens, the sums over the chunks from every block up to 512 rows and from a kernel of
-    their own above; either side of these sizes the permutation is the stable sort of the ids, bit for bit, and an expert's
-    rows lie one behind the other from a multiple of 128 on, the shared expert's last."""
+    """The ranks come from chunks of 32 tokens, the sums over the chunks from every block, through spans of 512 tokens, up to 8,192
+    rows and from a kernel of their own above; up to 1,024 rows a block has one token.  Either side of these sizes the
+    permutation is the stable sort of the ids, bit for bit, and an expert's rows lie one behind the other from a multiple of
+    128 on, the shared expert's last."""
     torch = cuda
     from p92moe_b200 import synth
 
