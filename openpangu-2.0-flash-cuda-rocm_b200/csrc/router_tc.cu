@@ -391,20 +391,23 @@ __device__ __forceinline__ void fma_pair(float2& a, float2 x, float2 w) {
 // The repair for hidden = 2,560.  The token row lies in shared memory in chain order (row_norm): piece (c, lane) of 16 bytes is
 // eight steps of a lane's chain, for the token as for a router row.
 // WPT (warps per token) = 1: a warp does everything for its token, four tokens per block - the form for more than a few hundred
-// tokens.  The exact logits go eight candidates at a time (there are 8.16 on average): eight independent chains as four pairs,
+// tokens.  The exact logits go four candidates at a time (there are 8.16 on average): four independent chains as two pairs,
 // the router rows of the next step in flight, and a tree over the 32 lanes that halves the number of values with every step
-// instead of repeating itself per candidate.  (Two candidates at a time from a token row in registers, all 256 exact logits in
-// the selection: 96 us at 16,384 tokens, now 80; 31 at 4,096, now 28; 15 at 512, now 11; 12 at 64, now 9.6.)
+// instead of repeating itself per candidate.  It waits for router rows more than it computes, so registers are worth warps:
+// with five blocks per SM whole calls of 3,807 and 16,384 rows take 385 and 1,116 us, with eight candidates and four blocks
+// 390 and 1,128, with six or seven blocks no less.  (Two candidates at a time from a token row in registers, all 256 exact
+// logits in the selection: 96 us at 16,384 tokens, 80 with eight at a time; 15 at 512, now 11; 12 at 64, now 9.6.)
 // WPT = 8 or 4: one token per block; its warps bring the row in together, each build the candidate list (the same list) and
 // then share the candidates out, one chain at a time; warp 0 finishes.
 template <int WPT>
-__global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 ? 2 : 4) route_repair_chains_kernel(
+__global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 ? 2 : WPT == 4 ? 4 : 5) route_repair_chains_kernel(
     const std::uint16_t* __restrict__ x, const float* __restrict__ bias, const float* __restrict__ w_norms, float* __restrict__ logits,
     std::int32_t* __restrict__ ids, float* __restrict__ weights, int rows, float routed_scale, int* __restrict__ stats,
     const float* __restrict__ partials, int splits, const std::uint16_t* __restrict__ w_chains, std::int32_t* __restrict__ chunk_hist,
     std::int32_t* __restrict__ span_hist) {
     constexpr int kHidden = 32 * kChainSteps;
     constexpr int kPieces = kChainSteps / 8;                  // of 16 bytes, per lane
+    constexpr int kBatch = 4;                                 // candidates at a time
     constexpr int kWarps = WPT > 1 ? WPT : kRepairWarps;
     constexpr int kTokens = WPT > 1 ? 1 : kRepairWarps;             // per block
     __shared__ uint4 x_chains[kTokens][kPieces * 32];
@@ -486,27 +489,27 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 
         if (lane < n_cand && !whole_row) mine = exact_row[cand[lane]];
     } else {
 #pragma unroll 1
-        for (int first = 0; first < n_cand; first += 8) {
-            int at[8];
+        for (int first = 0; first < n_cand; first += kBatch) {
+            int at[kBatch];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) at[k] = cand[min(first + k, n_cand - 1)] * (kPieces * 32);
-            float2 acc[4];
+            for (int k = 0; k < kBatch; ++k) at[k] = cand[min(first + k, n_cand - 1)] * (kPieces * 32);
+            float2 acc[kBatch / 2];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) acc[m] = make_float2(0.0F, 0.0F);
+            for (int m = 0; m < kBatch / 2; ++m) acc[m] = make_float2(0.0F, 0.0F);
             // a step of eight columns per lane; two sets of registers, the loads of one under way while the other is used
-            uint4 even[8], odd[8];
-            auto request = [&](uint4 (&q)[8], int c) {
+            uint4 even[kBatch], odd[kBatch];
+            auto request = [&](uint4 (&q)[kBatch], int c) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) q[k] = __ldg(w_lane + at[k] + 32 * c);
+                for (int k = 0; k < kBatch; ++k) q[k] = __ldg(w_lane + at[k] + 32 * c);
             };
-            auto add = [&](const uint4 (&q)[8], int c) {
+            auto add = [&](const uint4 (&q)[kBatch], int c) {
                 const uint4 xq = x_row[32 * c + lane];
                 const std::uint32_t xs[4] = {xq.x, xq.y, xq.z, xq.w};
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const float lo = __uint_as_float(xs[k] << 16), hi = __uint_as_float(xs[k] & 0xffff0000U);
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
+                    for (int m = 0; m < kBatch / 2; ++m) {
                         const std::uint32_t wa = k == 0 ? q[2 * m].x : k == 1 ? q[2 * m].y : k == 2 ? q[2 * m].z : q[2 * m].w;
                         const std::uint32_t wb = k == 0 ? q[2 * m + 1].x : k == 1 ? q[2 * m + 1].y : k == 2 ? q[2 * m + 1].z : q[2 * m + 1].w;
                         fma_pair(acc[m], make_float2(lo, lo), make_float2(__uint_as_float(wa << 16), __uint_as_float(wb << 16)));
@@ -523,13 +526,13 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 
                 if (c + 2 < kPieces) request(even, c + 2);
                 add(odd, c + 1);
             }
-            // The reference's tree over the 32 chains (lane l takes lane l + 16's sum, then l + 8's, ...), for eight candidates at
-            // once: a lane hands half of its values to its partner and goes on with the other half, so that after the steps of
-            // 16, 8 and 4 lanes it is left with candidate lane / 4.  An addition's two operands are the tree's, in either order.
-            float v[8] = {acc[0].x, acc[0].y, acc[1].x, acc[1].y, acc[2].x, acc[2].y, acc[3].x, acc[3].y};
+            // The reference's tree over the 32 chains (lane l takes lane l + 16's sum, then l + 8's, ...), for the batch at once: a
+            // lane hands half of its values to its partner and goes on with the other half, so that after the steps of 16 and 8
+            // lanes it is left with candidate lane / 8.  An addition's two operands are the tree's, in either order.
+            float v[kBatch] = {acc[0].x, acc[0].y, acc[1].x, acc[1].y};
 #pragma unroll
-            for (int half = 4; half >= 1; half >>= 1) {
-                const int off = half * 4;
+            for (int half = kBatch / 2; half >= 1; half >>= 1) {
+                const int off = half * (32 / kBatch);
                 const bool upper = (lane & off) != 0;
 #pragma unroll
                 for (int m = 0; m < half; ++m) {
@@ -538,15 +541,15 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32, WPT == 8 
                 }
             }
             float value = v[0];
-            value += __shfl_xor_sync(0xffffffffU, value, 2);
-            value += __shfl_xor_sync(0xffffffffU, value, 1);
-            const int k = first + (lane >> 2);
-            if ((lane & 3) == 0 && k < n_cand) {
+#pragma unroll
+            for (int off = 16 / kBatch; off > 0; off >>= 1) value += __shfl_xor_sync(0xffffffffU, value, off);
+            const int k = first + lane / (32 / kBatch);
+            if (lane % (32 / kBatch) == 0 && k < n_cand) {
                 exact_row[cand[k]] = value;
                 lg[cand[k]] = value;
             }
-            const float of_mine = __shfl_sync(0xffffffffU, value, (lane & 7) * 4);
-            if (lane >= first && lane < first + 8) mine = of_mine;
+            const float of_mine = __shfl_sync(0xffffffffU, value, lane % kBatch * (32 / kBatch));
+            if (lane >= first && lane < first + kBatch) mine = of_mine;
         }
         __syncwarp();
     }
