@@ -148,7 +148,7 @@ __device__ __forceinline__ void copy_quantised_row(const std::uint8_t* __restric
 }  // namespace expert
 
 // Large-batch products with the tokens on the M side (expert_rows.cu); p.tile_prefix counts 128-row tiles.
-cudaError_t launch_expert_rows_gate_up(const p92b_plan* plan, const expert::TcParams& p, cudaStream_t stream, bool pdl);
+cudaError_t launch_expert_rows_gate_up(const p92b_plan* plan, const expert::TcParams& p, bool scales_by_row, cudaStream_t stream, bool pdl);
 cudaError_t launch_expert_rows_matrix(const p92b_plan* plan, expert::TcParams p, cudaStream_t stream, bool pdl);
 // Down product whose token rows stay in shared memory, where the K extent allows it; the one kernel that honours row_dest.
 bool down_slab_shape(int hidden, int intermediate);

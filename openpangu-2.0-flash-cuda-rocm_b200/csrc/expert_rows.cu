@@ -21,6 +21,7 @@ constexpr int kTok = 128;                                   // token rows of a t
 constexpr int kWRows = 256;                                 // weight rows of a tile (N)
 constexpr int kEpiWarps = 16;                               // four per TMEM quarter
 constexpr int kThreads = 64 + 32 * kEpiWarps;
+constexpr int kThreadsByRow = kThreads + 32;                // and a warp that turns the token scales round
 
 constexpr int kTmemAll = 512;
 
@@ -184,21 +185,30 @@ __device__ __forceinline__ bool decode_piece(const TcParams& p, const RouteTable
 // Roles as in expert_tc.cu: producer warp, MMA warp, sixteen epilogue warps; items (128-row token tile, weight tile).
 // One accumulator only - two of 256 columns and the scale factors do not fit TMEM - so the epilogue warps take their
 // 64 columns into registers at once and the next item's products start after that read, not after the arithmetic.
-// What bounds it with full tiles: the shared-memory port.  A K block costs 48 KB of operand reads, 54 KB of arriving
-// copies and 6 KB of scale copies, 844 cycles at 128 bytes against 512 of tensor work; it runs at 907 (16,384 tokens:
-// 563 -> 394 us; 4,096 tokens: 201 -> 163 us, HBM floor 116).  A pair of blocks sharing the weight rows (cta_group::2,
-// 256-row token tiles) needs 594 cycles but pads every expert to 256 rows: 376 us and 200 us, not kept.  Token rows
-// gathered from token order (TMA tile::gather4, four rows per operation) take 46 ns per operation: 1,023 us.
-template <int MODE>
-__global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_constant__ CUtensorMap map_t32,
-                                                                  const __grid_constant__ CUtensorMap map_t128, const TcParams p) {
+// What bounds it with full tiles: a K block brings 54 KB into the SM, 864 cycles at 64 bytes, against 776 of the tensor pipe (512
+// of products, twelve scale copies of 22); it runs at about 910, and the four stages leave some 4 % more latency no room
+// (16,384 tokens: 563 -> 394 us; 4,096 tokens: 201 -> 163 us, HBM floor 116).  A pair of blocks sharing the weight rows
+// (cta_group::2, 256-row token tiles) pads every expert to 256 rows and took in 25 bytes per cycle and SM: dense MLP of 3,807
+// rows 230 us against 132, not kept.  Token rows gathered from token order (TMA tile::gather4, four rows per operation) take
+// 46 ns per operation: 1,023 us.
+// BY_ROW: the scales of a stage's 128 token rows come as 16 bytes per row, four K steps of four blocks, and the tensor core's copy
+// wants them as four slabs of [row % 32][row / 32][4 bytes].  One more warp turns them round where they lie: a lane has the 16 bytes
+// of rows l, l + 32, l + 64 and l + 96 and gives four words to each slab, four 16-byte loads and stores per K block of some 900
+// cycles, so that the kernels in front store a row's scales in 16-byte pieces.  The scales are requested ahead of the stage's other
+// bytes, on a barrier of their own, and are turned round before those have come: turned when all was there this kernel took 427 us
+// at 16,384 rows, with three barriers for the MMA lane to wait on 410, with one 400, as without the turning.
+// (One barrier per stage, not one for the weights and one for the tokens: dense MLP of 3,807 rows, two layers, 312.2 -> 309.5 us.)
+template <int MODE, bool BY_ROW>
+__global__ void __launch_bounds__(BY_ROW ? kThreadsByRow : kThreads, 1) expert_rows_kernel(const __grid_constant__ CUtensorMap map_t32,
+                                                                                            const __grid_constant__ CUtensorMap map_t128,
+                                                                                            const TcParams p) {
     extern __shared__ std::uint8_t smem_raw[];
     __shared__ RouteTable route_table;
     const std::uint32_t base = (smem_u32(smem_raw) + 1023U) & ~1023U;
     const std::uint32_t bars = base + Stage::kCount * Stage::kBytes;
-    auto weight_bar = [&](int s) { return bars + 8U * s; };
-    auto token_bar = [&](int s) { return bars + 8U * (Stage::kCount + s); };
-    auto empty_bar = [&](int s) { return bars + 8U * (2 * Stage::kCount + s); };
+    auto full_bar = [&](int s) { return bars + 8U * s; };                              // BY_ROW: and the token scales turned round
+    auto empty_bar = [&](int s) { return bars + 8U * (Stage::kCount + s); };
+    auto scale_bar = [&](int s) { return bars + 8U * (2 * Stage::kCount + s); };       // BY_ROW: token scales there, as they come
     const std::uint32_t accum_full = bars + 8U * (3 * Stage::kCount);
     const std::uint32_t accum_empty = accum_full + 8U;
     const std::uint32_t tmem_slot = bars + 8U * Stage::kBarriers;
@@ -212,9 +222,9 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < Stage::kCount; ++s) {
-            mbar_init(weight_bar(s), 1);
-            mbar_init(token_bar(s), 1);
+            mbar_init(full_bar(s), BY_ROW ? 2 : 1);
             mbar_init(empty_bar(s), 1);
+            mbar_init(scale_bar(s), 1);
         }
         mbar_init(accum_full, 1);
         mbar_init(accum_empty, kEpiWarps);
@@ -257,21 +267,26 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1U)) { give_up(); break; }
                     const std::uint32_t st = base + stage * Stage::kBytes;
+                    if constexpr (BY_ROW) {                 // ahead of the rest: turned round by the time that has come
+                        mbar_arrive_expect_tx(scale_bar(stage), kSfSlab);
+                        bulk_load(st + Stage::kOffSfT, t_sf + static_cast<std::size_t>(kb) * 4 * 512, kSfSlab, scale_bar(stage));
+                    }
+                    const std::uint32_t weight_bytes = piece.width == kWRows ? kChunkBytes : static_cast<std::uint32_t>(piece.width) * kBlockKBytes + kSfSlab;
+                    mbar_arrive_expect_tx(full_bar(stage), weight_bytes + boxes * (32 * kBlockKBytes) + (BY_ROW ? 0 : kSfSlab));
                     if (piece.width == kWRows) {
-                        mbar_arrive_expect_tx(weight_bar(stage), kChunkBytes);
                         if constexpr (MODE == 0) {
                             bulk_load(st + Stage::kOffW,
                                       p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes,
-                                      kChunkBytes, weight_bar(stage));
+                                      kChunkBytes, full_bar(stage));
                         } else {
                             // K block kb of two neighbouring row tiles: a box and a scale slab from either tile's chunk
 #pragma unroll
                             for (int h = 0; h < 2; ++h) {
                                 const std::uint8_t* chunk = p.bank.g2 +
                                     ((static_cast<std::size_t>(it.entry) * p.m_tiles * 2 + it.m_tile * 2 + h) * (k_blocks / 2) + (kb >> 1)) * kChunkBytes;
-                                bulk_load(st + Stage::kOffW + h * kChunkBox, chunk + (kb & 1) * kChunkBox, kChunkBox, weight_bar(stage));
+                                bulk_load(st + Stage::kOffW + h * kChunkBox, chunk + (kb & 1) * kChunkBox, kChunkBox, full_bar(stage));
                                 bulk_load(st + Stage::kOffSfW + h * kSfSlab, chunk + kChunkScaleOffset + (kb & 1) * kChunkScaleBytes, kSfSlab,
-                                          weight_bar(stage));
+                                          full_bar(stage));
                             }
                         }
                     } else {
@@ -279,20 +294,20 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                         const std::uint8_t* chunk = MODE == 0
                             ? p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes
                             : p.bank.g2 + ((static_cast<std::size_t>(it.entry) * p.m_tiles * 2 + it.m_tile * 2 + half) * (k_blocks / 2) + (kb >> 1)) * kChunkBytes;
-                        const std::uint32_t bytes = static_cast<std::uint32_t>(piece.width) * kBlockKBytes;
-                        mbar_arrive_expect_tx(weight_bar(stage), bytes + kSfSlab);
-                        bulk_load(st + Stage::kOffW, chunk + box * kChunkBox + piece.first % kTileM * kBlockKBytes, bytes, weight_bar(stage));
-                        bulk_load(st + Stage::kOffSfW, chunk + kChunkScaleOffset + box * kChunkScaleBytes, kSfSlab, weight_bar(stage));
+                        bulk_load(st + Stage::kOffW, chunk + box * kChunkBox + piece.first % kTileM * kBlockKBytes, weight_bytes - kSfSlab,
+                                  full_bar(stage));
+                        bulk_load(st + Stage::kOffSfW, chunk + kChunkScaleOffset + box * kChunkScaleBytes, kSfSlab, full_bar(stage));
                     }
-                    mbar_arrive_expect_tx(token_bar(stage), boxes * (32 * kBlockKBytes) + kSfSlab);
                     if (boxes == 4) {
-                        tma_load_2d(st + Stage::kOffT, &map_t128, token_bar(stage), kb * kBlockKBytes, it.pp0);
+                        tma_load_2d(st + Stage::kOffT, &map_t128, full_bar(stage), kb * kBlockKBytes, it.pp0);
                     } else {
                         for (int b = 0; b < boxes; ++b) {
-                            tma_load_2d(st + Stage::kOffT + b * 32 * kBlockKBytes, &map_t32, token_bar(stage), kb * kBlockKBytes, it.pp0 + b * 32);
+                            tma_load_2d(st + Stage::kOffT + b * 32 * kBlockKBytes, &map_t32, full_bar(stage), kb * kBlockKBytes, it.pp0 + b * 32);
                         }
                     }
-                    bulk_load(st + Stage::kOffSfT, t_sf + static_cast<std::size_t>(kb) * 4 * 512, kSfSlab, token_bar(stage));
+                    if constexpr (!BY_ROW) {
+                        bulk_load(st + Stage::kOffSfT, t_sf + static_cast<std::size_t>(kb) * 4 * 512, kSfSlab, full_bar(stage));
+                    }
                     if (++stage == Stage::kCount) { stage = 0; phase ^= 1U; }
                 }
             }
@@ -311,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                 const std::uint32_t quarter = static_cast<std::uint32_t>(piece.first % kTileM) >> 5;
                 bool ok = true;
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(weight_bar(stage), phase) || !mbar_wait(token_bar(stage), phase)) {
+                    if (!mbar_wait(full_bar(stage), phase)) {
                         give_up();
                         ok = false;
                         break;
@@ -341,6 +356,32 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const __grid_c
                 if (!ok) break;
                 tc_commit(accum_full);
                 accum_phase ^= 1U;
+            }
+        }
+    } else if (BY_ROW && warp == kThreads / 32) {
+        int stage = 0;
+        std::uint32_t phase = 0;
+        for (int item = blockIdx.x; item < total_items && !__any_sync(0xffffffffU, *abort_ptr != 0); item += gridDim.x) {
+            Piece piece;
+            if (!decode_piece(p, route_table, items, item, &piece)) continue;
+            bool ok = true;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                ok = __all_sync(0xffffffffU, mbar_wait(scale_bar(stage), phase));
+                if (!ok) break;
+                uint4* at = reinterpret_cast<uint4*>(smem_raw + (base - smem_u32(smem_raw)) + stage * Stage::kBytes + Stage::kOffSfT) + lane;
+                const uint4 a = at[0], b = at[32], c = at[64], d = at[96];
+                at[0] = make_uint4(a.x, b.x, c.x, d.x);
+                at[32] = make_uint4(a.y, b.y, c.y, d.y);
+                at[64] = make_uint4(a.z, b.z, c.z, d.z);
+                at[96] = make_uint4(a.w, b.w, c.w, d.w);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full_bar(stage));
+                if (++stage == Stage::kCount) { stage = 0; phase ^= 1U; }
+            }
+            if (!ok) {
+                give_up();
+                break;
             }
         }
     } else {
@@ -732,16 +773,21 @@ cudaError_t launch_expert_down_slab(const p92b_plan* plan, const TcParams& p, cu
                          plan->map_h[3], p);
 }
 
-cudaError_t launch_expert_rows_gate_up(const p92b_plan* plan, const TcParams& p, cudaStream_t stream, bool pdl) {
-    if (cudaError_t st = ensure_dynamic_smem<expert_rows_kernel<0>>(Stage::kSmem); st != cudaSuccess) return st;
-    return launch_kernel(expert_rows_kernel<0>, dim3(plan->sm_count), dim3(kThreads), Stage::kSmem, stream, pdl, plan->map_x[1],
+cudaError_t launch_expert_rows_gate_up(const p92b_plan* plan, const TcParams& p, bool scales_by_row, cudaStream_t stream, bool pdl) {
+    if (scales_by_row) {
+        if (cudaError_t st = ensure_dynamic_smem<expert_rows_kernel<0, true>>(Stage::kSmem); st != cudaSuccess) return st;
+        return launch_kernel(expert_rows_kernel<0, true>, dim3(plan->sm_count), dim3(kThreadsByRow), Stage::kSmem, stream, pdl,
+                             plan->map_x[1], plan->map_x[3], p);
+    }
+    if (cudaError_t st = ensure_dynamic_smem<expert_rows_kernel<0, false>>(Stage::kSmem); st != cudaSuccess) return st;
+    return launch_kernel(expert_rows_kernel<0, false>, dim3(plan->sm_count), dim3(kThreads), Stage::kSmem, stream, pdl, plan->map_x[1],
                          plan->map_x[3], p);
 }
 
 cudaError_t launch_expert_rows_matrix(const p92b_plan* plan, TcParams p, cudaStream_t stream, bool pdl) {
     p.m_tiles = p.m_total / kWRows;
-    if (cudaError_t st = ensure_dynamic_smem<expert_rows_kernel<1>>(Stage::kSmem); st != cudaSuccess) return st;
-    return launch_kernel(expert_rows_kernel<1>, dim3(plan->sm_count), dim3(kThreads), Stage::kSmem, stream, pdl, plan->map_h[1],
+    if (cudaError_t st = ensure_dynamic_smem<expert_rows_kernel<1, false>>(Stage::kSmem); st != cudaSuccess) return st;
+    return launch_kernel(expert_rows_kernel<1, false>, dim3(plan->sm_count), dim3(kThreads), Stage::kSmem, stream, pdl, plan->map_h[1],
                          plan->map_h[3], p);
 }
 

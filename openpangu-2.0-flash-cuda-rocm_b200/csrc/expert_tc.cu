@@ -678,6 +678,7 @@ cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int 
                                          : launch_tc<2, 64, 0>(plan, plan->map_x[2], p, stream, pdl);
             }
         }
+        if (io != nullptr && io->scales_by_row && (which != 2 || plan->wide_rows != 128)) return cudaErrorNotSupported;
         if (in_place) return cudaErrorNotSupported;              // the fused gate/up epilogue reads the bank's stream
         switch (which) {
             case 0: return launch_tc<0, 16>(plan, plan->map_x[0], p, stream, pdl);
@@ -689,7 +690,7 @@ cudaError_t launch_experts_tc(const p92b_plan* plan, const p92b_bank* bank, int 
                 // against 563 at 16,384.
                 if (plan->wide_rows == 128) {
                     p.tile_prefix = plan->tile_prefix_wide;
-                    return launch_expert_rows_gate_up(plan, p, stream, pdl);
+                    return launch_expert_rows_gate_up(plan, p, io != nullptr && io->scales_by_row, stream, pdl);
                 }
                 return launch_tc<0, 64>(plan, plan->map_x[2], p, stream, pdl);
         }

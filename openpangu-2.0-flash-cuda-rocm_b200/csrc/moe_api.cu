@@ -430,6 +430,7 @@ int p92b_moe_forward_normed(p92b_plan* plan, const p92b_bank* bank, const uint16
         plan->last_launches += 1;
     }
     if ((st = mark()) != cudaSuccess) return st;
+    TcIo front {};
     if (rows <= route_fused_max_rows()) {
         // top-8, permutation and token quantisation as one block (stages 1-3 of the timing table)
         st = launch_route_fused(plan, correction_bias, routed_scale, input, rows, pad_align, tile_rows, stream, pdl);
@@ -442,6 +443,7 @@ int p92b_moe_forward_normed(p92b_plan* plan, const p92b_bank* bank, const uint16
         if ((st = launch_scan_counts(plan, rows, tile_rows, stream, pdl)) != cudaSuccess) return st;
         if ((st = mark()) != cudaSuccess) return st;
         if ((st = launch_place_rows(plan, input, rows, tile_rows, stream, pdl)) != cudaSuccess) return st;
+        front.scales_by_row = place_scales_by_row(rows);
         if ((st = mark()) != cudaSuccess) return st;
     } else {
         st = launch_router_top8(plan->logits, correction_bias, plan->ids, plan->route_weights, rows, routed_scale, stream, pdl);
@@ -457,7 +459,7 @@ int p92b_moe_forward_normed(p92b_plan* plan, const p92b_bank* bank, const uint16
         if ((st = mark()) != cudaSuccess) return st;
         plan->last_launches += 1;
     }
-    st = launch_experts_tc(plan, bank, rows, false, stream, pdl);
+    st = launch_experts_tc(plan, bank, rows, false, stream, pdl, &front);
     if (st != cudaSuccess) return st;
     if ((st = mark()) != cudaSuccess) return st;
     st = launch_experts_tc(plan, bank, rows, true, stream, pdl);

@@ -82,6 +82,9 @@ __device__ __forceinline__ uint2 quantize_block16(const float (&v)[16], float gl
 // ..., PER_LANE at most) and its storing at padded positions: NVFP4 bytes row-major, scales in the 128x4-tiled layout
 // (cuda/nvfp4_ops.cu:818-841 and :869-890 in one pass).  hidden <= 512 WARPS PER_LANE, a multiple of 64.  In steps, so that
 // a kernel can have the row on its way while it finds out where the row goes.
+// BY_ROW (hidden a multiple of 256): the scales of 128 rows x one K block of 256 values - the same 2 KB - as 16 bytes per row instead
+// (TcIo::scales_by_row).  The tiled layout scatters a row's scales over 40 pieces of 4 bytes, which is what bounded the kernels that
+// place nine copies of every row: 80 -> 59 us at 16,384 rows, 27 -> 19 at 4,096 (without any scale stores 47 and 17).
 template <int WARPS, int PER_LANE = 8 / WARPS>
 struct QuantisedRow {
     uint4 raw[PER_LANE][2];
@@ -122,15 +125,18 @@ struct QuantisedRow {
             scale_word[j] = word;
         }
     }
+    template <bool BY_ROW = false>
     __device__ __forceinline__ void store(std::uint8_t* __restrict__ xq, std::uint8_t* __restrict__ xs, std::size_t pp) const {
         std::uint8_t* row_q = xq + pp * (blocks * 8);
-        std::uint8_t* row_s = xs + (pp >> 7) * ((blocks + 3) / 4) * 512 + (pp & 31) * 16 + ((pp >> 5) & 3) * 4;
+        std::uint8_t* row_s = xs + (pp >> 7) * ((blocks + 3) / 4) * 512 + (BY_ROW ? (pp & 127) * 16 : (pp & 31) * 16 + ((pp >> 5) & 3) * 4);
 #pragma unroll
         for (int j = 0; j < PER_LANE; ++j) {
             const int b = first + 32 * WARPS * j;
             if (b >= blocks) break;
             *reinterpret_cast<uint2*>(row_q + b * 8) = packed[j];
-            if ((first & 3) == 0) *reinterpret_cast<std::uint32_t*>(row_s + (b >> 2) * 512) = scale_word[j];
+            if ((first & 3) == 0) {
+                *reinterpret_cast<std::uint32_t*>(row_s + (BY_ROW ? (b >> 4) * 2048 + (b & 12) : (b >> 2) * 512)) = scale_word[j];
+            }
         }
     }
 };
@@ -558,6 +564,7 @@ cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const st
 // Behind launch_router_fast with count_experts: routing lists, positions and the token rows quantised at their places
 // (permute.cu), what launch_permute and launch_quantize_padded do for ids that come from anywhere.
 cudaError_t launch_scan_counts(p92b_plan* plan, int rows, int tile_rows, cudaStream_t stream, bool pdl);
+bool place_scales_by_row(int rows);             // the layout of the scales, TcIo::scales_by_row of the product behind it
 cudaError_t launch_place_rows(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream, bool pdl);
 // tensor-core path (expert_tc.cu)
 cudaError_t make_operand_map(CUtensorMap* map, const void* base, std::size_t rows, std::size_t row_bytes,
@@ -578,6 +585,8 @@ struct TcIo {
     int table_kind = 0;                     // with `table`, single-matrix products: which of the three matrices
     bool single_matrix = false;             // with `table`, token-row side: one matrix (gate or up alone), rows to down_out
     bool skip_shared = false;               // the call has no shared expert
+    bool scales_by_row = false;             // fused gate/up product with 128-row tiles: the token scales are laid out
+                                            // [128 rows][K block][row][16 bytes] instead of tiled (QuantisedRow)
     bool wait_upstream = false;             // down product: the kernel just upstream may still be waiting for ITS predecessor
                                             // when this one starts, so the routing lists may only be read after a wait
     std::uint16_t* const* row_dest = nullptr;   // down product of large batches only (down_slab_applies): [padded position] ->

@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(256) permute_scatter_kernel(
 // different, and so the rank of an assignment in its chunk is the number of earlier tokens of the chunk that have the expert
 // too: eight votes of a warp whose lane l holds token l's ids.  Positions, lists and the quantised row are then one pass
 // over the tokens instead of two kernels (up to 5,120 assignments; 512 rows: 13.7 + 6.4 us, now 9.4) or four (4,096 rows:
-// 6 + 12 + 12 + 22 us, now 12 + 24).
+// 6 + 12 + 12 + 22 us, now 12 + 24, with the scales by row 12 + 19).
 // Every block adds the counts up for itself, one expert per thread: whole spans of 512 tokens, which the router counts too, and the
 // chunks of its own span; block 0 writes the lists.  At 8,192 tokens that is 31 words per thread from the L2.
 // SCANNED, above that: permute_scan_kernel has turned the counts into prefixes over the chunks and written the lists.  It takes 12 us;
@@ -541,7 +541,9 @@ __global__ void __launch_bounds__(256) place_rows_kernel(const std::uint16_t* __
     }
     row.quantise(global_scale);
 #pragma unroll 1
-    for (int place = 0; place <= kTop; ++place) row.store(xq, xs, static_cast<std::size_t>(__shfl_sync(0xffffffffU, my_place, place)));
+    for (int place = 0; place <= kTop; ++place) {
+        row.template store<WARPS == 1>(xq, xs, static_cast<std::size_t>(__shfl_sync(0xffffffffU, my_place, place)));
+    }
 }
 
 // ---- lists, places and rows of a call on ids that come from the caller -------------------------------
@@ -889,11 +891,15 @@ cudaError_t launch_scan_counts(p92b_plan* plan, int rows, int tile_rows, cudaStr
                          plan->chunk_hist, chunks, rows * kTop, plan_lists(plan, tile_rows), rows, plan->scan_blocks_done);
 }
 
+// Up to 1,024 rows eight warps per row and tiled scales: the stores of the scales don't show there, and 64 rows, where the gate/up
+// product waits for memory throughout, took 747 us instead of 743 with scales by row.
+bool place_scales_by_row(int rows) { return rows > 1024; }
+
 cudaError_t launch_place_rows(p92b_plan* plan, const std::uint16_t* x, int rows, int tile_rows, cudaStream_t stream, bool pdl) {
     if (plan->hidden > 4096) return cudaErrorNotSupported;
     if (!aligned_to(16, x)) return cudaErrorInvalidValue;
     const bool scanned = rows > kPlaceRows;
-    const bool few = rows <= 1024;
+    const bool few = !place_scales_by_row(rows);
     const bool narrow = plan->hidden <= 2560;
     plan->last_launches += 1;
     return launch_kernel(few       ? place_rows_kernel<8, false, 1>

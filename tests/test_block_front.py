@@ -36,3 +36,28 @@ def test_places_of_the_routed_rows(cuda, pkg, layer0, rows, popular):
     rank = views["position"] - offsets[ids]
     assert np.array_equal(views["mixed_index"][: rows * 8], base[ids] + rank)
     assert np.array_equal(views["mixed_index"][rows * 8:], base[256] + np.arange(rows))
+
+
+@pytest.mark.parametrize("rows", [1024, 1025, 1153, 8193])
+@pytest.mark.parametrize("popular", [[], [3, 255]])
+def test_scales_stored_by_row(cuda, pkg, layer0, rows, popular):
+    """Above 1,024 rows the token scales reach the gate/up product as 16 bytes per row and K block and are turned round there.
+    The rows equal the same rows sent through the decode kernel, which has a layout of its own, bit for bit; the popular experts
+    have several tiles, the others one with a ragged end."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    bias = layer0.bias.clone()
+    bias[popular] += 4.0
+    x = synth.make_activations(92, rows, rows)
+    out = torch.full_like(x, float("nan"))
+    plan = pkg.MoePlan(max_rows=rows)
+    block = pkg.MoeBlock(layer0.bank, layer0.router_weight, bias, plan)
+    block.run_moe_rows(x, out, rows)
+    assert plan.status() == 0 and torch.isfinite(out.float()).all()
+    for first in (0, 120, rows - 16):
+        small = torch.empty_like(x[:16])
+        block.run_moe_rows(x[first:first + 16].contiguous(), small, 16)
+        assert plan.status() == 0
+        assert torch.equal(out[first:first + 16].view(torch.int16), small.view(torch.int16))
+    plan.close()
