@@ -253,12 +253,17 @@ __global__ void __launch_bounds__(BY_ROW ? kThreadsByRow : kThreads, 1) expert_r
 
     if (warp == 0) {
         if (elect_one()) {
+            const std::uint64_t stream_policy = l2_policy_evict_first();
             int stage = 0;
             std::uint32_t phase = 0;
             for (int item = blockIdx.x; item < total_items && !*abort_ptr; item += gridDim.x) {
                 Piece piece;
                 if (!decode_piece(p, route_table, items, item, &piece)) continue;
                 const Item& it = piece.it;
+                // The entry's only tile: nobody else reads these weights, and they are the first to leave the L2 again.  The rest
+                // stays there for the kernels behind (64 rows, four layers: 743 -> 730 us, 512 rows 462 -> 457.5, 2,048 rows 269 ->
+                // 262.5).  For every entry, the second tile's reads go to memory: 4,096 rows, down product 101 -> 121 us.
+                const bool once = it.count <= kTok;
                 const int half = piece.first / kTileM;          // narrow pieces: which of the two boxes
                 // token rows beyond the tile's last one are not loaded: their lanes compute on what the stage held
                 // before, and nothing reads them
@@ -275,9 +280,13 @@ __global__ void __launch_bounds__(BY_ROW ? kThreadsByRow : kThreads, 1) expert_r
                     mbar_arrive_expect_tx(full_bar(stage), weight_bytes + boxes * (32 * kBlockKBytes) + (BY_ROW ? 0 : kSfSlab));
                     if (piece.width == kWRows) {
                         if constexpr (MODE == 0) {
-                            bulk_load(st + Stage::kOffW,
-                                      p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes,
-                                      kChunkBytes, full_bar(stage));
+                            const std::uint8_t* from =
+                                p.bank.g13 + ((static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * k_blocks + kb) * kChunkBytes;
+                            if (once) {
+                                bulk_load_hint(st + Stage::kOffW, from, kChunkBytes, full_bar(stage), stream_policy);
+                            } else {
+                                bulk_load(st + Stage::kOffW, from, kChunkBytes, full_bar(stage));
+                            }
                         } else {
                             // K block kb of two neighbouring row tiles: a box and a scale slab from either tile's chunk
 #pragma unroll
@@ -602,6 +611,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_down_slab_kernel(const __g
             int stage = 0;
             std::uint32_t phase = 0, slab_phase = 0;
             bool ok = true, upstream_done = p.routing_is_upstream != 0;
+            const std::uint64_t stream_policy = l2_policy_evict_first();
             int requested = 0;                              // chunks of the first item whose weights were asked for before the wait
             for (int item = blockIdx.x; item < total_items && !*abort_ptr && ok; item += gridDim.x) {
                 Item it;
@@ -611,9 +621,15 @@ __global__ void __launch_bounds__(kThreads, 1) expert_down_slab_kernel(const __g
                 const std::uint8_t* t_sf = p.b_sf + static_cast<std::size_t>(it.pp0 >> 7) * (p.k_bytes / 32) * 512;
                 const std::uint32_t slab_bytes = 2 * (boxes * (32 * kBlockKBytes) + kSfSlab);
                 const std::uint8_t* weights = p.bank.g2 + (static_cast<std::size_t>(it.entry) * p.m_tiles + it.m_tile) * chunks * kChunkBytes;
+                const bool once = it.count <= kTok;             // its only slab: nobody else reads these weights (expert_rows_kernel)
                 auto request = [&](int s, int n) {          // chunk n of the item into stage s
                     mbar_arrive_expect_tx(full_bar(s), kChunkBytes + (n < chunks ? slab_bytes : 0U));
-                    bulk_load(ring + s * kChunkBytes, weights + static_cast<std::size_t>(n) * kChunkBytes, kChunkBytes, full_bar(s));
+                    const std::uint8_t* from = weights + static_cast<std::size_t>(n) * kChunkBytes;
+                    if (once) {
+                        bulk_load_hint(ring + s * kChunkBytes, from, kChunkBytes, full_bar(s), stream_policy);
+                    } else {
+                        bulk_load(ring + s * kChunkBytes, from, kChunkBytes, full_bar(s));
+                    }
                 };
                 if (!upstream_done) {
                     requested = min(Slab::kStages, (last - it.m_tile) * chunks);
