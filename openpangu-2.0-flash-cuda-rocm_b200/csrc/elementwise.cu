@@ -293,6 +293,13 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const std::uint16_t* 
 // down row from position space), rounded to BF16 exactly where the reference
 // stores `hidden_`, then the shared expert's BF16 down row added and rounded
 // again (src/model.cpp:1505-1508 then :1571-1572).  Eight columns of a row.
+// DONE_WITH: the rows read are marked to leave the L2 first.
+template <bool DONE_WITH>
+__device__ __forceinline__ uint4 mixed_piece(const std::uint16_t* at) {
+    const uint4* from = reinterpret_cast<const uint4*>(at);
+    if constexpr (DONE_WITH) return __ldcs(from); else return *from;
+}
+template <bool DONE_WITH>
 __device__ __forceinline__ uint4 combine_shared8(const std::uint16_t* __restrict__ mixed, const std::int32_t* __restrict__ mixed_index,
                                                  const float* __restrict__ route_weights, int rows, int hidden, int row, int c8) {
     float acc[8];
@@ -304,7 +311,7 @@ __device__ __forceinline__ uint4 combine_shared8(const std::uint16_t* __restrict
     for (int slot = 0; slot < kTop; ++slot) {
         const int pos = mixed_index[row * kTop + slot];
         w[slot] = route_weights[row * kTop + slot];
-        slot_rows[slot] = *reinterpret_cast<const uint4*>(mixed + static_cast<std::size_t>(pos) * hidden + c8 * 8);
+        slot_rows[slot] = mixed_piece<DONE_WITH>(mixed + static_cast<std::size_t>(pos) * hidden + c8 * 8);
     }
 #pragma unroll
     for (int slot = 0; slot < kTop; ++slot) {
@@ -315,8 +322,7 @@ __device__ __forceinline__ uint4 combine_shared8(const std::uint16_t* __restrict
             acc[2 * k + 1] = fmaf(__uint_as_float(words[k] & 0xffff0000U), w[slot], acc[2 * k + 1]);
         }
     }
-    const uint4 sh = *reinterpret_cast<const uint4*>(
-        mixed + static_cast<std::size_t>(mixed_index[rows * kTop + row]) * hidden + c8 * 8);
+    const uint4 sh = mixed_piece<DONE_WITH>(mixed + static_cast<std::size_t>(mixed_index[rows * kTop + row]) * hidden + c8 * 8);
     const std::uint32_t sw[4] = {sh.x, sh.y, sh.z, sh.w};
     std::uint32_t out_words[4];
 #pragma unroll
@@ -329,6 +335,7 @@ __device__ __forceinline__ uint4 combine_shared8(const std::uint16_t* __restrict
     return make_uint4(out_words[0], out_words[1], out_words[2], out_words[3]);
 }
 
+template <bool DONE_WITH>
 __global__ void __launch_bounds__(256) combine_shared_kernel(const std::uint16_t* __restrict__ mixed,
                                                              const std::int32_t* __restrict__ mixed_index,
                                                              const float* __restrict__ route_weights,
@@ -340,13 +347,14 @@ __global__ void __launch_bounds__(256) combine_shared_kernel(const std::uint16_t
     const int c8 = blockIdx.x * blockDim.x + threadIdx.x;
     if (c8 * 8 >= hidden) return;
     *reinterpret_cast<uint4*>(output + static_cast<std::size_t>(row) * hidden + c8 * 8) =
-        combine_shared8(mixed, mixed_index, route_weights, rows, hidden, row, c8);
+        combine_shared8<DONE_WITH>(mixed, mixed_index, route_weights, rows, hidden, row, c8);
 }
 
 // The same with the RMSNorm behind the block (src/model.cpp:216-217,1215-1216) in the same pass: a block has its row together in
 // shared memory, where the norm's chains read it in the operator's order (rmsnorm_rows_kernel).  As a kernel of its own the norm
 // read and wrote every output row once more (3,807 rows with both norms: 416 us a call, now 411).
 constexpr int kCombineNormMaxHidden = 8192;
+template <bool DONE_WITH>
 __global__ void __launch_bounds__(1024) combine_shared_norm_kernel(const std::uint16_t* __restrict__ mixed,
                                                                    const std::int32_t* __restrict__ mixed_index,
                                                                    const float* __restrict__ route_weights,
@@ -362,7 +370,7 @@ __global__ void __launch_bounds__(1024) combine_shared_norm_kernel(const std::ui
     const bool mine = c8 * 8 < hidden;
     uint4 value = make_uint4(0U, 0U, 0U, 0U);
     if (mine) {
-        value = combine_shared8(mixed, mixed_index, route_weights, rows, hidden, row, c8);
+        value = combine_shared8<DONE_WITH>(mixed, mixed_index, route_weights, rows, hidden, row, c8);
         reinterpret_cast<uint4*>(norm_row)[c8] = value;
     }
     __syncthreads();
@@ -477,12 +485,18 @@ cudaError_t launch_quantize(const std::uint16_t* input, std::uint8_t* output, st
                          global_scale, static_cast<const float*>(nullptr));
 }
 
+// The down rows are read here for the last time.  Marked to leave the L2 first, they make room for rows that are still there from
+// the down kernel instead of pushing them out: 2,048 rows 262.6 -> 257.8 us a call, 3,807 rows 392.7 -> 388.4.  Up to 1,024 rows all
+// of them fit (512 rows 452 without, 453.5 with the mark); of 16,384 rows' 755 MB next to nothing is still there, and the token rows
+// for the next call's router go instead (combine 157 -> 152 us, that router 5 later).
+static bool combine_done_with(int rows) { return rows > 1024 && rows <= 8192; }
+
 cudaError_t launch_combine_shared(const std::uint16_t* mixed, const std::int32_t* mixed_index,
                                   const float* route_weights, std::uint16_t* output, int rows,
                                   int hidden, cudaStream_t stream, bool pdl) {
     if (!aligned_to(16, output)) return cudaErrorInvalidValue;
     dim3 grid(blocks_for(hidden / 8, 256), rows);
-    return launch_kernel(combine_shared_kernel, grid, dim3(256), 0, stream, pdl, mixed, mixed_index, route_weights,
+    return launch_kernel(combine_done_with(rows) ? combine_shared_kernel<true> : combine_shared_kernel<false>, grid, dim3(256), 0, stream, pdl, mixed, mixed_index, route_weights,
                          output, rows, hidden);
 }
 
@@ -492,7 +506,7 @@ cudaError_t launch_combine_shared_norm(const std::uint16_t* mixed, const std::in
     if (hidden > kCombineNormMaxHidden) return cudaErrorNotSupported;
     if (!aligned_to(16, output)) return cudaErrorInvalidValue;
     const unsigned threads = std::max(256U, blocks_for(hidden / 8, 32) * 32);          // the norm's 256 chains have a thread each
-    return launch_kernel(combine_shared_norm_kernel, dim3(rows), dim3(threads), static_cast<std::size_t>(hidden) * 2, stream, pdl, mixed,
+    return launch_kernel(combine_done_with(rows) ? combine_shared_norm_kernel<true> : combine_shared_norm_kernel<false>, dim3(rows), dim3(threads), static_cast<std::size_t>(hidden) * 2, stream, pdl, mixed,
                          mixed_index, route_weights, norm_weight, output, rows, hidden, epsilon);
 }
 
