@@ -9,22 +9,26 @@
 //                            5th-generation tensor cores (tcgen05.mma kind::f16, M = 128 tokens, N = 64 to 256 experts
 //                            per block, operands by TMA, accumulator in TMEM), and beside it ||w_e||_2 of the 256 router
 //                            rows (the error bound below needs them);
-//   2. route_repair_kernel   one warp per token: corrected scores from the approximate logits, the approximate 8th
-//                            best, the candidate set = every expert whose approximate score is within 2 delta of it,
-//                            the candidates' logits recomputed in the reference's exact order, and the reference's
+//   2. route_repair_chains_kernel (route_repair_kernel for hidden sizes other than 2,560)   eight, four or one warp per token
+//                            by batch: corrected scores from the approximate logits, the approximate 8th best, the
+//                            candidate set = every expert whose exact score may be among the eight best, the
+//                            candidates' logits recomputed in the reference's exact order, and the reference's
 //                            top-8 (cuda/nvfp4_ops.cu:357-433: higher corrected score first, ties to the lower id,
 //                            weights from the uncorrected sigmoid, renormalised) taken over the exact values.
 //
-// Why that is exact.  Let delta bound |approximate - exact| of a corrected score.  An expert outside the candidate set
-// has approximate score < a8 - 2 delta (a8 = approximate 8th best), so its exact score is < a8 - delta, while each of
-// the eight approximately best experts has exact score >= a8 - delta: eight experts beat it, it is not in the exact
-// top-8.  Hence the exact top-8 is a subset of the candidates, and selecting among exactly recomputed candidates
-// gives the reference's ids and weights bit for bit.  delta = 0.25 * kLogitBound * ||x_t|| * ||w_e|| + 4e-6: the
-// sigmoid's slope is at most 1/4; both the reference chain and the tensor-core sum differ from the true dot product by
-// at most (number of sequential roundings) * 2^-23 * sum|x_i w_i| <= that * ||x|| ||w||, with about 85 roundings in the
-// reference's order and fewer than 200 in the tensor core's; kLogitBound = 2^-14 is more than twice their sum; 4e-6
-// covers the fast-math sigmoid's own error on both sides.  A token whose candidate set would exceed 24 experts or
-// has fewer than eight, or that holds a non-finite logit, has its whole row recomputed exactly instead.
+// Why that is exact.  Let delta_e bound |approximate - exact| of expert e's corrected score, a8 be the approximate 8th best
+// and reach the largest delta of the approximately best experts (score >= a8, eight at least).  An expert is left out if its
+// approximate score is < a8 - (reach + delta_e); its exact score is then < a8 - reach, while each of the approximately
+// best has exact score >= a8 - reach: eight experts beat it, it is not in the exact top-8.  (Its own bound twice is not
+// enough: an expert with a small router row was left out for experts with large ones whose exact scores were lower.)
+// Hence the exact top-8 is a subset of the candidates, and selecting among exactly recomputed candidates gives the
+// reference's ids and weights bit for bit.  delta_e = 0.25 * kLogitBound * ||x_t|| * ||w_e|| + 4e-6: the sigmoid's slope is
+// at most 1/4; both the reference chain and the tensor-core sum differ from the true dot product by at most (number of
+// sequential roundings) * (2^-24 rounded, 2^-23 cut off) * sum|x_i w_i| <= that * ||x|| ||w||, with hidden / 32 + 5 roundings in
+// the reference's order and hidden / 16 steps in the tensor core's; kLogitBound = 2^-14 is 2.5 times their sum at 2,560
+// columns and 1.6 times at 4,096 (twice as much is allowed above); 4e-6 covers the fast-math sigmoid's own error on both sides.  A token whose candidate set
+// would exceed 24 experts or has fewer than eight, that holds a non-finite logit, or for which a bound is no finite
+// number (squares that overflow), has its whole row recomputed exactly instead.
 //
 // The logits buffer keeps the approximate values except at the recomputed positions, which hold the exact ones.
 #include "p92b_common.cuh"
@@ -291,9 +295,10 @@ __device__ __forceinline__ void load_approximate(float* __restrict__ lg, const f
     }
 }
 
-// The candidates of one token, member[i] a ballot over experts 32 i .. 32 i + 31: approximate corrected score within 2 delta of
-// the approximate 8th best.  All 256 if that cannot decide it (*whole_row): a logit that is no finite number, fewer than eight
-// candidates (a NaN in the bias, or fewer than eight experts that -infinity does not mask) or more than a warp takes.
+// The candidates of one token, member[i] a ballot over experts 32 i .. 32 i + 31: approximate corrected score no further below
+// the approximate 8th best than the two bounds allow.  All 256 if that cannot decide it (*whole_row): a logit or a bound that is
+// no finite number, fewer than eight candidates (a NaN in the bias, or fewer than eight experts that -infinity does not
+// mask) or more than a warp takes.
 __device__ __forceinline__ int find_candidates(const float (&approx)[8], const float* __restrict__ bias, const float* __restrict__ w_norms,
                                                float x_norm, unsigned (&member)[8], bool* whole_row) {
     const int lane = threadIdx.x & 31;
@@ -303,9 +308,9 @@ __device__ __forceinline__ int find_candidates(const float (&approx)[8], const f
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int e = lane + 32 * i;
-        finite = finite && (fabsf(approx[i]) <= 3.0e38F);
         score[i] = 1.0F / (1.0F + expf(-approx[i])) + bias[e];
         delta[i] = 0.25F * kLogitBound * x_norm * w_norms[e] + 4.0e-6F;
+        finite = finite && fabsf(approx[i]) <= 3.0e38F && delta[i] <= 3.0e38F;
         const std::uint32_t bits = __float_as_uint(score[i]);
         key[i] = score[i] != score[i] ? 0U : (bits & 0x80000000U ? ~bits : bits | 0x80000000U);
     }
@@ -336,10 +341,14 @@ __device__ __forceinline__ int find_candidates(const float (&approx)[8], const f
         }
     }
     const float eighth = __uint_as_float(top & 0x80000000U ? top & 0x7fffffffU : ~top);       // image 0: a NaN, nothing is within reach
+    float reach = 0.0F;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) reach = score[i] >= eighth ? fmaxf(reach, delta[i]) : reach;
+    reach = __uint_as_float(__reduce_max_sync(0xffffffffU, __float_as_uint(reach)));         // (not negative: ordered as its bits)
     int candidates = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        member[i] = __ballot_sync(0xffffffffU, score[i] >= eighth - 2.0F * delta[i]);
+        member[i] = __ballot_sync(0xffffffffU, score[i] >= eighth - (reach + delta[i]));
         candidates += __popc(member[i]);
     }
     *whole_row = !finite || candidates > kMaxCandidates || candidates < kTop;
@@ -626,7 +635,7 @@ __global__ void __launch_bounds__((WPT > 1 ? WPT : kRepairWarps) * 32) route_rep
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) square += __shfl_xor_sync(0xffffffffU, square, off);
-    const float x_norm = sqrtf(square) * 1.0001F;
+    const float x_norm = sqrtf(square) * (hidden > 4096 ? 2.0002F : 1.0001F);          // (kLogitBound holds up to 4,096 columns)
     __syncwarp();
     float* lg = logits + static_cast<std::size_t>(token) * kExperts;
     float approx[8];

@@ -105,3 +105,58 @@ def test_router_of_the_block_with_scores_that_are_no_numbers(cuda, pkg, layer0, 
         block.run_moe_rows(clean, want, rows)
         assert torch.equal(out[~odd].view(torch.int16), want[~odd].view(torch.int16))
     plan.close()
+
+
+def _uneven_case(torch, hidden, rows, seed):
+    """Token rows whose columns are equal in pairs and router rows whose columns of a pair are opposite, the pairs anywhere: every
+    logit is zero but for the rounding of its sums, which grows with the norm of the router row.  Experts 0 - 3 are taken by their bias, eight experts of norms
+    far apart and eight of norm zero contend for the other four places, and each pair of sums in another order may rank
+    them differently."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    half = torch.empty((256, hidden // 2), device="cuda").normal_(generator=g)
+    scale = torch.zeros((256, 1), device="cuda")
+    scale[100:108, 0] = 2.0 ** torch.arange(5, 13, device="cuda")
+    router = (torch.cat([half, -half], 1) * scale).to(torch.bfloat16)
+    bias = torch.full((256,), -1.0, device="cuda")
+    bias[0:4] = 1.0
+    bias[50:58] = 0.0
+    bias[100:108] = 0.0
+    x = torch.empty((rows, hidden // 2), device="cuda").normal_(generator=g).to(torch.bfloat16)
+    columns = torch.randperm(hidden, generator=g, device="cuda")
+    return router[:, columns].contiguous(), bias, torch.cat([x, x], 1)[:, columns].contiguous()
+
+
+@pytest.mark.parametrize("hidden,rows", [(2560, 9), (2560, 100), (2560, 300), (2560, 4097), (1024, 100), (1024, 300)])
+def test_router_rows_of_very_different_norms(cuda, pkg, layer0, hidden, rows):
+    """How far an approximate logit may lie from the exact one depends on the norm of its own router row: an expert may only be
+    left out for being behind the eight best by its own bound and theirs together."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    router, bias, x = _uneven_case(torch, hidden, rows, 70 + rows)
+    inter = 1024 if hidden == 2560 else 512
+    bank = layer0.bank if hidden == 2560 else pkg.ExpertBank(
+        synth.make_raw_layer_batched(11, 0, hidden=hidden, intermediate=inter).entries(), hidden=hidden, intermediate=inter)
+    plan = pkg.MoePlan(rows, hidden, inter)
+    plan.set_path(plan.PATH_TENSOR_CORE)
+    _check(torch, pkg, pkg.MoeBlock(bank, router, bias, plan), rows, x, bias)
+    plan.close()
+
+
+@pytest.mark.parametrize("rows", [9, 300, 1000])
+@pytest.mark.parametrize("whose", ["token", "expert"])
+def test_router_with_a_norm_beyond_float(cuda, pkg, layer0, rows, whose):
+    """Squares that overflow leave a bound of infinity, or of no number where the other norm is zero, and then nothing is known of
+    that logit's deviation: the token is ranked by its exact scores all the same."""
+    torch = cuda
+    router, bias, x = _uneven_case(torch, 2560, rows, 90 + rows)
+    if whose == "token":
+        x[::2] *= 2.0 ** 66                        # most router rows are zero
+    else:
+        router[60] = torch.where(router[107] > 0, 1e30, -1e30)
+        bias[60] = 0.5
+        x[::2] = 0.0
+    plan = pkg.MoePlan(rows)
+    plan.set_path(plan.PATH_TENSOR_CORE)
+    _check(torch, pkg, pkg.MoeBlock(layer0.bank, router, bias, plan), rows, x, bias)
+    plan.close()
