@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const std::uint16_t* 
 // Fused tail of the block: the weighted combine above (gathering each slot's
 // down row from position space), rounded to BF16 exactly where the reference
 // stores `hidden_`, then the shared expert's BF16 down row added and rounded
-// again (src/model.cpp:1505-1508 then :1571-1572).  Eight columns of a row.
+// again (src/model.cpp:1505-1508 then :1571-1572).  Eight columns of a row.  shared_index: places of the shared expert's rows.
 // DONE_WITH: the rows read are marked to leave the L2 first.
 template <bool DONE_WITH>
 __device__ __forceinline__ uint4 mixed_piece(const std::uint16_t* at) {
@@ -301,7 +301,8 @@ __device__ __forceinline__ uint4 mixed_piece(const std::uint16_t* at) {
 }
 template <bool DONE_WITH>
 __device__ __forceinline__ uint4 combine_shared8(const std::uint16_t* __restrict__ mixed, const std::int32_t* __restrict__ mixed_index,
-                                                 const float* __restrict__ route_weights, int rows, int hidden, int row, int c8) {
+                                                 const std::int32_t* __restrict__ shared_index, const float* __restrict__ route_weights,
+                                                 int hidden, int row, int c8) {
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.0F;
@@ -322,7 +323,7 @@ __device__ __forceinline__ uint4 combine_shared8(const std::uint16_t* __restrict
             acc[2 * k + 1] = fmaf(__uint_as_float(words[k] & 0xffff0000U), w[slot], acc[2 * k + 1]);
         }
     }
-    const uint4 sh = mixed_piece<DONE_WITH>(mixed + static_cast<std::size_t>(mixed_index[rows * kTop + row]) * hidden + c8 * 8);
+    const uint4 sh = mixed_piece<DONE_WITH>(mixed + static_cast<std::size_t>(shared_index[row]) * hidden + c8 * 8);
     const std::uint32_t sw[4] = {sh.x, sh.y, sh.z, sh.w};
     std::uint32_t out_words[4];
 #pragma unroll
@@ -338,16 +339,16 @@ __device__ __forceinline__ uint4 combine_shared8(const std::uint16_t* __restrict
 template <bool DONE_WITH>
 __global__ void __launch_bounds__(256) combine_shared_kernel(const std::uint16_t* __restrict__ mixed,
                                                              const std::int32_t* __restrict__ mixed_index,
+                                                             const std::int32_t* __restrict__ shared_index,
                                                              const float* __restrict__ route_weights,
-                                                             std::uint16_t* __restrict__ output, int rows,
-                                                             int hidden) {
+                                                             std::uint16_t* __restrict__ output, int hidden) {
     ptx::pdl_launch_dependents();
     ptx::pdl_wait();
     const int row = blockIdx.y;
     const int c8 = blockIdx.x * blockDim.x + threadIdx.x;
     if (c8 * 8 >= hidden) return;
     *reinterpret_cast<uint4*>(output + static_cast<std::size_t>(row) * hidden + c8 * 8) =
-        combine_shared8<DONE_WITH>(mixed, mixed_index, route_weights, rows, hidden, row, c8);
+        combine_shared8<DONE_WITH>(mixed, mixed_index, shared_index, route_weights, hidden, row, c8);
 }
 
 // The same with the RMSNorm behind the block (src/model.cpp:216-217,1215-1216) in the same pass: a block has its row together in
@@ -357,9 +358,10 @@ constexpr int kCombineNormMaxHidden = 8192;
 template <bool DONE_WITH>
 __global__ void __launch_bounds__(1024) combine_shared_norm_kernel(const std::uint16_t* __restrict__ mixed,
                                                                    const std::int32_t* __restrict__ mixed_index,
+                                                                   const std::int32_t* __restrict__ shared_index,
                                                                    const float* __restrict__ route_weights,
                                                                    const std::uint16_t* __restrict__ norm_weight,
-                                                                   std::uint16_t* __restrict__ output, int rows, int hidden, float epsilon) {
+                                                                   std::uint16_t* __restrict__ output, int hidden, float epsilon) {
     extern __shared__ __align__(16) std::uint16_t norm_row[];
     __shared__ float warp_sums[8];
     __shared__ float inverse_shared;
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(1024) combine_shared_norm_kernel(const std::ui
     const bool mine = c8 * 8 < hidden;
     uint4 value = make_uint4(0U, 0U, 0U, 0U);
     if (mine) {
-        value = combine_shared8<DONE_WITH>(mixed, mixed_index, route_weights, rows, hidden, row, c8);
+        value = combine_shared8<DONE_WITH>(mixed, mixed_index, shared_index, route_weights, hidden, row, c8);
         reinterpret_cast<uint4*>(norm_row)[c8] = value;
     }
     __syncthreads();
@@ -495,9 +497,13 @@ cudaError_t launch_combine_shared(const std::uint16_t* mixed, const std::int32_t
                                   const float* route_weights, std::uint16_t* output, int rows,
                                   int hidden, cudaStream_t stream, bool pdl) {
     if (!aligned_to(16, output)) return cudaErrorInvalidValue;
-    dim3 grid(blocks_for(hidden / 8, 256), rows);
-    return launch_kernel(combine_done_with(rows) ? combine_shared_kernel<true> : combine_shared_kernel<false>, grid, dim3(256), 0, stream, pdl, mixed, mixed_index, route_weights,
-                         output, rows, hidden);
+    const auto kernel = combine_done_with(rows) ? combine_shared_kernel<true> : combine_shared_kernel<false>;
+    return launch_row_parts(rows, [&](int first, int part) {
+        const std::size_t at = static_cast<std::size_t>(first);
+        return launch_kernel(kernel, dim3(blocks_for(hidden / 8, 256), part), dim3(256), 0, stream, pdl, mixed, mixed_index + at * kTop,
+                             mixed_index + static_cast<std::size_t>(rows) * kTop + at, route_weights + at * kTop, output + at * hidden,
+                             hidden);
+    });
 }
 
 cudaError_t launch_combine_shared_norm(const std::uint16_t* mixed, const std::int32_t* mixed_index, const float* route_weights,
@@ -506,8 +512,9 @@ cudaError_t launch_combine_shared_norm(const std::uint16_t* mixed, const std::in
     if (hidden > kCombineNormMaxHidden) return cudaErrorNotSupported;
     if (!aligned_to(16, output)) return cudaErrorInvalidValue;
     const unsigned threads = std::max(256U, blocks_for(hidden / 8, 32) * 32);          // the norm's 256 chains have a thread each
-    return launch_kernel(combine_done_with(rows) ? combine_shared_norm_kernel<true> : combine_shared_norm_kernel<false>, dim3(rows), dim3(threads), static_cast<std::size_t>(hidden) * 2, stream, pdl, mixed,
-                         mixed_index, route_weights, norm_weight, output, rows, hidden, epsilon);
+    return launch_kernel(combine_done_with(rows) ? combine_shared_norm_kernel<true> : combine_shared_norm_kernel<false>, dim3(rows),
+                         dim3(threads), static_cast<std::size_t>(hidden) * 2, stream, pdl, mixed, mixed_index,
+                         mixed_index + static_cast<std::size_t>(rows) * kTop, route_weights, norm_weight, output, hidden, epsilon);
 }
 
 cudaError_t launch_rmsnorm(const std::uint16_t* input, const std::uint16_t* weight, std::uint16_t* output, int rows,
@@ -611,9 +618,13 @@ int p92b_expert_combine_rows(const uint16_t* expert_rows, const float* route_wei
         return cudaErrorInvalidValue;
     }
     const int vectors = aligned_to(16, expert_rows, output) && elements % 8 == 0 ? elements / 8 : 0;
-    dim3 grid(blocks_for(vectors + (elements - vectors * 8), 256), batch_rows);
-    return launch_kernel(combine_rows_kernel, grid, dim3(256), 0, static_cast<cudaStream_t>(stream), pdl_enabled(), expert_rows,
-                         route_weights, output, experts, elements, vectors);
+    return launch_row_parts(batch_rows, [&](int first, int part) {
+        const std::size_t at = static_cast<std::size_t>(first);
+        const dim3 grid(blocks_for(vectors + (elements - vectors * 8), 256), part);
+        return launch_kernel(combine_rows_kernel, grid, dim3(256), 0, static_cast<cudaStream_t>(stream), pdl_enabled(),
+                             expert_rows + at * experts * elements, route_weights + at * experts, output + at * elements, experts,
+                             elements, vectors);
+    });
 }
 
 int p92b_expert_combine(const uint16_t* expert_rows, const float* route_weights, uint16_t* output,

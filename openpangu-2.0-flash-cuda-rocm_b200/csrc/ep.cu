@@ -425,11 +425,15 @@ static int ep_combine_impl(p92b_plan* home_plan, p92b_plan* shared_plan, const p
     sp->wide_rows = 0;
     if ((st = launch_experts_tc(sp, bank, rows, false, stream)) != cudaSuccess) return st;
     if ((st = launch_experts_tc(sp, bank, rows, true, stream)) != cudaSuccess) return st;
-    dim3 grid((home_plan->hidden / 8 + 255) / 256, rows);
-    ep_combine_kernel<<<grid, 256, 0, stream>>>(returned_rows, fixed ? home_plan->pp_of_flat : home_plan->position,
-                                                home_plan->route_weights, sp->mixed_pp,
-                                                output, home_plan->hidden);
-    return cudaGetLastError();
+    const int hidden = home_plan->hidden;
+    const std::int32_t* position = fixed ? home_plan->pp_of_flat : home_plan->position;
+    return launch_row_parts(rows, [&](int first, int part) {
+        const std::size_t at = static_cast<std::size_t>(first);
+        ep_combine_kernel<<<dim3((hidden / 8 + 255) / 256, part), 256, 0, stream>>>(
+            returned_rows, position + at * kTop, home_plan->route_weights + at * kTop, sp->mixed_pp + at * hidden, output + at * hidden,
+            hidden);
+        return cudaGetLastError();
+    });
 }
 
 int p92b_ep_combine(p92b_plan* home_plan, p92b_plan* shared_plan, const p92b_bank* bank, const uint16_t* input,

@@ -416,11 +416,16 @@ int p92b_ep_forward_bulk(p92b_plan* plan, const p92b_bank* bank, p92b_ep_window*
                                                                       assignments, window->rank, world, rpg, hidden, epoch);
     }
     bulk_wait_kernel<<<1, 32, 0, stream>>>(flags + kMaxWorld, world, epoch, plan->status);
-    dim3 grid((hidden / 8 + 255) / 256, rows);
-    bulk_combine_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const std::uint16_t*>(mine + layout.results),
-                                                  plan->route_weights, plan->mixed_pp, plan->pp_off, output, rows, hidden);
+    const std::uint16_t* results = reinterpret_cast<const std::uint16_t*>(mine + layout.results);
+    st = launch_row_parts(rows, [&](int first, int part) {
+        const std::size_t at = static_cast<std::size_t>(first);
+        bulk_combine_kernel<<<dim3((hidden / 8 + 255) / 256, part), 256, 0, stream>>>(
+            results + at * kTop * hidden, plan->route_weights + at * kTop, plan->mixed_pp + at * hidden, plan->pp_off, output + at * hidden,
+            part, hidden);
+        return cudaGetLastError();
+    });
     plan->last_launches += 10;
-    if ((st = cudaGetLastError()) != cudaSuccess) return st;
+    if (st != cudaSuccess) return st;
     if (plan->timing) {
         if ((st = mark()) != cudaSuccess) return st;
         if ((st = cudaStreamSynchronize(stream)) != cudaSuccess) return st;

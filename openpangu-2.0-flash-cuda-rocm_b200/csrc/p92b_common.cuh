@@ -462,6 +462,18 @@ struct p92b_ep_window {
 
 namespace p92b {
 
+// A grid's y ends at 65,535, so a batch whose rows lie there is launched in parts: launch(first row, rows) for each.  (The
+// rows spread over y and z, or divided out of x, cost the operator sequence of 64 rows 0.7 and 0.3 % of a call.)
+constexpr int kGridRows = 65535;
+template <class Launch>
+cudaError_t launch_row_parts(int rows, Launch launch) {
+    for (int first = 0; first < rows; first += kGridRows) {
+        const cudaError_t st = launch(first, rows - first < kGridRows ? rows - first : kGridRows);
+        if (st != cudaSuccess) return st;
+    }
+    return cudaSuccess;
+}
+
 // Launch with or without programmatic dependent launch: with `pdl` the kernel may start while the
 // previous kernel in the stream is still draining, and must call ptx::pdl_wait() before it touches
 // anything that kernel writes.

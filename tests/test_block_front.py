@@ -61,3 +61,36 @@ def test_scales_stored_by_row(cuda, pkg, layer0, rows, popular):
         assert plan.status() == 0
         assert torch.equal(out[first:first + 16].view(torch.int16), small.view(torch.int16))
     plan.close()
+
+
+def test_batch_of_more_rows_than_a_grid_has_in_y(cuda, pkg):
+    """65,536 rows, with and without the norm behind the block: the bits of its two halves.  And the combine operator at as many."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    hidden, inter, rows = 256, 512, 65536
+    bank = pkg.ExpertBank(synth.make_raw_layer_batched(14, 0, hidden=hidden, intermediate=inter).entries(), hidden=hidden,
+                          intermediate=inter)
+    router, bias = synth.make_router(14, 0, hidden=hidden)
+    x = synth.make_activations(94, 0, rows, hidden=hidden)
+    weight = synth.make_activations(94, 1, 1, hidden=hidden).view(-1)
+    plan = pkg.MoePlan(rows, hidden, inter)
+    block = pkg.MoeBlock(bank, router, bias, plan)
+    half = rows // 2
+    for post in (None, weight):
+        out, want = torch.full_like(x, float("nan")), torch.empty_like(x)
+        block.run_moe_rows_normed(x, None, post, out, rows, 1e-5)
+        for first in (0, half):
+            block.run_moe_rows_normed(x[first:first + half], None, post, want[first:first + half], half, 1e-5)
+        assert plan.status() == 0
+        assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+    plan.close()
+    bank.close()
+    g = torch.Generator(device="cuda").manual_seed(15)
+    expert_rows = torch.empty((rows, 8, 24), device="cuda").normal_(generator=g).to(torch.bfloat16)
+    weights = torch.empty((rows, 8), device="cuda").uniform_(generator=g)
+    out, want = (torch.empty((rows, 24), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    pkg.expert_combine_rows(expert_rows, weights, out, rows, 8, 24)
+    for first in (0, half):
+        pkg.expert_combine_rows(expert_rows[first:], weights[first:], want[first:], half, 8, 24)
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
