@@ -63,6 +63,50 @@ def test_scales_stored_by_row(cuda, pkg, layer0, rows, popular):
     plan.close()
 
 
+@pytest.mark.parametrize("hidden,inter", [(256, 512), (512, 1024), (768, 512), (1024, 2048), (2816, 512), (4096, 1024)])
+@pytest.mark.parametrize("rows", [33, 1025, 2305, 8200])
+def test_block_at_other_shapes(cuda, pkg, orc, hidden, inter, rows):
+    """Places, token scales and products at hidden sizes with one K block to sixteen and K extents of the down product with one
+    chunk, two or four (the last beyond the form with the token rows in shared memory): the lists are the stable sort's,
+    and the rows equal the same rows in batches of eight, which take other kernels throughout, bit for bit.  The first rows
+    are held to the CPU oracle."""
+    torch = cuda
+    from p92moe_b200 import synth
+    from conftest import u16
+
+    raw = synth.make_raw_layer_batched(13, 0, hidden=hidden, intermediate=inter)
+    bank = pkg.ExpertBank(raw.entries(), hidden=hidden, intermediate=inter)
+    router, bias = synth.make_router(13, 0, hidden=hidden)
+    bias[[3, 255]] += 4.0
+    x = synth.make_activations(93, rows, rows, hidden=hidden)
+    out = torch.full_like(x, float("nan"))
+    plan = pkg.MoePlan(rows, hidden, inter)
+    block = pkg.MoeBlock(bank, router, bias, plan)
+    block.run_moe_rows(x, out, rows)
+    assert plan.status() == 0
+    views = {k: v.cpu().numpy() for k, v in plan.views(rows).items() if v is not None and v.dtype == torch.int32}
+    ids = views["expert_ids"].reshape(-1)
+    counts = np.bincount(ids, minlength=256)
+    base = np.concatenate([[0], np.cumsum((counts + 127) // 128 * 128)])
+    rank = np.empty(rows * 8, dtype=np.int64)
+    rank[np.argsort(ids, kind="stable")] = np.concatenate([np.arange(c) for c in counts])
+    assert np.array_equal(views["order"], np.argsort(ids, kind="stable"))
+    assert np.array_equal(views["mixed_index"][: rows * 8], base[ids] + rank)
+    assert np.array_equal(views["mixed_index"][rows * 8:], base[256] + np.arange(rows))
+    for first in (0, 16, rows // 2, rows - 8):
+        small = torch.empty_like(x[:8])
+        block.run_moe_rows(x[first:first + 8].contiguous(), small, 8)
+        assert plan.status() == 0
+        assert torch.equal(out[first:first + 8].view(torch.int16), small.view(torch.int16))
+    if rows == 33:
+        want = orc.moe_forward(u16(x[:4]), u16(router), bias.cpu().numpy(), raw.packed.cpu().numpy(), raw.scales_linear.cpu().numpy(),
+                               raw.alpha.cpu().numpy(), hidden, inter)
+        got, want = out[:4].float().cpu().numpy(), orc.bf16_to_f32(want)
+        assert np.linalg.norm(got - want) <= 1e-2 * np.linalg.norm(want)
+    plan.close()
+    bank.close()
+
+
 def test_batch_of_more_rows_than_a_grid_has_in_y(cuda, pkg):
     """65,536 rows, with and without the norm behind the block: the bits of its two halves.  And the combine operator at as many."""
     torch = cuda

@@ -206,3 +206,34 @@ def test_dense_entry_point_rejects_mismatched_shapes(cuda, pkg, layer0):
         pkg.run_dense_rows(plan, layer0.bank, x, x.clone(), 4)          # a 1024-wide expert bank with a 9216-wide plan
     assert err.value.code == 1
     plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,hidden,inter", [(64, 2560, 1024), (1024, 2560, 1024), (1025, 2560, 1024), (3807, 2560, 1024),
+                                               (8192, 2560, 1024), (8193, 2560, 1024), (33, 256, 512), (1100, 256, 512),
+                                               (20000, 256, 512), (300, 4096, 512), (1100, 4096, 512), (8, 8192, 512),
+                                               (8, 8448, 512)])
+def test_norm_behind_the_block_equals_the_operator(cuda, pkg, layer0, rows, hidden, inter):
+    """The norm folded into the combine, both forms of it and every width of its blocks, and the operator of its own that takes its
+    place above 8,192 columns: the bits of the block followed by the operator."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    if (hidden, inter) == (2560, 1024):
+        bank, router, bias = layer0.bank, layer0.router_weight, layer0.bias
+    else:
+        bank = pkg.ExpertBank(synth.make_raw_layer_batched(12, 0, hidden=hidden, intermediate=inter).entries(), hidden=hidden,
+                              intermediate=inter)
+        router, bias = synth.make_router(12, 0, hidden=hidden)
+    weight = _norm_weight(torch, 23, hidden)
+    x = synth.make_activations(79, rows, rows, hidden=hidden)
+    plan = pkg.MoePlan(rows, hidden, inter)
+    block = pkg.MoeBlock(bank, router, bias, plan)
+    plain, want, got = torch.empty_like(x), torch.empty_like(x), torch.full_like(x, float("nan"))
+    block.run_moe_rows(x, plain, rows)
+    pkg.rmsnorm(plain, weight, want, rows, hidden, EPS)
+    block.run_moe_rows_normed(x, None, weight, got, rows, EPS)
+    assert plan.status() == 0
+    assert float(want.float().abs().max()) > 0.0
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    plan.close()

@@ -160,3 +160,18 @@ def test_router_with_a_norm_beyond_float(cuda, pkg, layer0, rows, whose):
     plan.set_path(plan.PATH_TENSOR_CORE)
     _check(torch, pkg, pkg.MoeBlock(layer0.bank, router, bias, plan), rows, x, bias)
     plan.close()
+
+
+@pytest.mark.parametrize("above", [0, 1])
+def test_router_either_side_of_a_block_per_token(cuda, pkg, layer0, above):
+    """Up to four tokens per SM the repair has a block of four warps per token, above a warp."""
+    torch = cuda
+    from p92moe_b200 import synth
+
+    rows = 4 * torch.cuda.get_device_properties(0).multi_processor_count + above
+    plan = pkg.MoePlan(max_rows=rows)
+    plan.set_path(plan.PATH_TENSOR_CORE)
+    x = synth.make_activations(4700, rows, rows)
+    for bias in (layer0.bias, torch.zeros_like(layer0.bias)):
+        _check(torch, pkg, pkg.MoeBlock(layer0.bank, layer0.router_weight, bias, plan), rows, x, bias)
+    plan.close()
