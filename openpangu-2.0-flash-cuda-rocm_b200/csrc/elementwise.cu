@@ -488,16 +488,19 @@ cudaError_t launch_quantize(const std::uint16_t* input, std::uint8_t* output, st
 }
 
 // The down rows are read here for the last time.  Marked to leave the L2 first, they make room for rows that are still there from
-// the down kernel instead of pushing them out: 2,048 rows 262.6 -> 257.8 us a call, 3,807 rows 392.7 -> 388.4.  Up to 1,024 rows all
-// of them fit (512 rows 452 without, 453.5 with the mark); of 16,384 rows' 755 MB next to nothing is still there, and the token rows
-// for the next call's router go instead (combine 157 -> 152 us, that router 5 later).
-static bool combine_done_with(int rows) { return rows > 1024 && rows <= 8192; }
+// the down kernel instead of pushing them out: 2,048 rows 262.6 -> 257.8 us a call, 3,807 rows 392.7 -> 388.4; with 512 columns
+// 12,000 rows 223 -> 217 and 40,960 rows 638 -> 630.  Up to 1,024 rows it gains nothing at any width (512 rows 452 without, 453.5
+// with the mark; 900 rows of 4,096 columns 392 and 395).  What is still there is a matter of bytes: 11,000 rows (507 MB) 813 -> 802,
+// from 553 to 604 MB within 0.3 % either way at 2,560 and 4,096 columns; of 16,384 rows' 755 MB next to nothing is, and
+// the token rows for the next call's router go instead (combine 157 -> 152 us, that router 5 later).
+constexpr long kDoneWithBytes = 8192L * (kTop + 1) * 4096 * 2;
+static bool combine_done_with(int rows, int hidden) { return rows > 1024 && static_cast<long>(rows) * (kTop + 1) * hidden * 2 <= kDoneWithBytes; }
 
 cudaError_t launch_combine_shared(const std::uint16_t* mixed, const std::int32_t* mixed_index,
                                   const float* route_weights, std::uint16_t* output, int rows,
                                   int hidden, cudaStream_t stream, bool pdl) {
     if (!aligned_to(16, output)) return cudaErrorInvalidValue;
-    const auto kernel = combine_done_with(rows) ? combine_shared_kernel<true> : combine_shared_kernel<false>;
+    const auto kernel = combine_done_with(rows, hidden) ? combine_shared_kernel<true> : combine_shared_kernel<false>;
     return launch_row_parts(rows, [&](int first, int part) {
         const std::size_t at = static_cast<std::size_t>(first);
         return launch_kernel(kernel, dim3(blocks_for(hidden / 8, 256), part), dim3(256), 0, stream, pdl, mixed, mixed_index + at * kTop,
@@ -512,7 +515,7 @@ cudaError_t launch_combine_shared_norm(const std::uint16_t* mixed, const std::in
     if (hidden > kCombineNormMaxHidden) return cudaErrorNotSupported;
     if (!aligned_to(16, output)) return cudaErrorInvalidValue;
     const unsigned threads = std::max(256U, blocks_for(hidden / 8, 32) * 32);          // the norm's 256 chains have a thread each
-    return launch_kernel(combine_done_with(rows) ? combine_shared_norm_kernel<true> : combine_shared_norm_kernel<false>, dim3(rows),
+    return launch_kernel(combine_done_with(rows, hidden) ? combine_shared_norm_kernel<true> : combine_shared_norm_kernel<false>, dim3(rows),
                          dim3(threads), static_cast<std::size_t>(hidden) * 2, stream, pdl, mixed, mixed_index,
                          mixed_index + static_cast<std::size_t>(rows) * kTop, route_weights, norm_weight, output, hidden, epsilon);
 }
