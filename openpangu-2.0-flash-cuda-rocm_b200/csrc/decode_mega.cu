@@ -517,17 +517,17 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
             __syncwarp();
             asm volatile("bar.sync 3, %0;" ::"n"(kPollers) : "memory");
             if (threadIdx.x == 0) stamp(2);
-            for (int t = kMegaWarps - 2 - warp; t < rows && !abort_word; t += kMegaWarps - 1) {
+            static_assert(R <= kMegaWarps - 1 - kEpilogueEnd, "a warp without a role in P2 for every token");
+            const int t = kMegaWarps - 2 - warp;
+            if (t < rows && !abort_word) {
                 const float* lg = rt.logits + t * kExperts;
                 const std::uint32_t words = warp_top8_words(lg, rt.bias);
                 if (top8_is_close(words)) {
                     warp_top8_by_id(lg, rt.bias, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
-                } else if (warp >= kEpilogueEnd && t < kMegaWarps - 1) {
+                } else {
                     if (lane < kTop) rt.ids[t * kTop + lane] = top8_id(words);
                     weights_of = t;
                     top_words = words;
-                } else {
-                    warp_top8_write(words, lg, rt.ids + t * kTop, rt.weights + t * kTop, p.routed_scale);
                 }
             }
         }
