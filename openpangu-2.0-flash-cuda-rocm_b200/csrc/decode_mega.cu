@@ -531,11 +531,10 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
                 }
             }
         }
-        if (threadIdx.x == 0) stamp(13);
     }
     __syncthreads();
     if (!abort_word) {
-        if (threadIdx.x == 0) stamp(14);
+        if (threadIdx.x == 0) stamp(13);                     // every token ranked, or every choice seen
         // The ranking law of cuda/nvfp4_grouped.cu:117-132, position = #(smaller expert id) + #(same id,
         // smaller flat index), through one bit mask of tokens per expert (a token picks an expert at most
         // once): popcounts give the ranks, a scan over the 256 experts the offsets and the active slots.
