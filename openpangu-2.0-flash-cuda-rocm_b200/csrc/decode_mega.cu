@@ -10,10 +10,11 @@
 //       (cuda/nvfp4_ops.cu:818-841, scales written 128x4-tiled).  Each logit is published
 //       as an 8-byte word {value, launch number}; the quantised rows are covered by an
 //       arrive-only counter that only the TMA producer lanes wait on, later;
-//   P1  every block, redundantly and in shared memory: polls the logit words, top-8 of
-//       every token (cuda/nvfp4_ops.cu:357-433), histogram, stable permutation
-//       (cuda/nvfp4_grouped.cu:117-132), active-expert list; block 0 also writes the
-//       routing products to global memory;
+//   P1  every block, redundantly and in shared memory: up to eight rows it polls the logit words
+//       and ranks every token (top-8, cuda/nvfp4_ops.cu:357-433); from nine on token t's words are
+//       polled and ranked by block t alone, and every block polls the choices.  Then histogram, stable
+//       permutation (cuda/nvfp4_grouped.cu:117-132), active-expert list; block 0 also writes
+//       the routing products to global memory;
 //   P2  gate/up tiles (128 intermediate rows, gate and up, or half of them: one box of mixed gate and up rows) and P3
 //       down tiles (128 output rows) through ONE TMA ring and one tcgen05 pipeline (same operand formats as
 //       expert_tc.cu).  The token side of gate/up is simply all
@@ -50,15 +51,17 @@ namespace {
 // (T=13: 81 instead of 100 us per layer with both norms; T=1: 18.8 against 19.2 with eight warps, T=4: the same).
 constexpr int kMegaThreads = 512;
 constexpr int kMegaWarps = kMegaThreads / 32;
-// Every logit is published in eight places and a block polls one of them: all blocks need all words at the same moment,
-// and 148 readers of the same few lines queue up at the L2 slices that hold them.  For the same reason a block starts to
+// What all blocks poll - every logit up to eight rows, every choice from nine on - is published in eight places and a block
+// polls one of them: all blocks need all words at the same moment, and 148 readers of the same few lines queue up at the L2
+// slices that hold them.  For the same reason a block starts to
 // poll only when its own logits are out, asks again only for what is missing, and nobody polls the arrival counter
 // while it is being counted up: at four tokens the last reader had the logits 2.2 us after the average block was done
 // with its own, now 1.0 us.
 constexpr int kReplicas = 8;
 constexpr int kEpilogueEnd = 6;                    // first warp behind the epilogue warps
 // Up to here gate/up tiles are halves, above whole ones; us per layer, halves against whole tiles: one token 18.9 / 20.6,
-// two 23.6 / 24.6, three 28.8 / 28.7, four 32.8 / 32.3, eight 52.4 / 51.1, sixteen 88.0 / 84.0.
+// two 23.6 / 24.6, three 28.8 / 28.7, four 32.8 / 32.3, eight 52.4 / 51.1; sixteen 88.0 / 84.0, when every block ranked every
+// token (now 80.2 with whole tiles).
 constexpr int kHalfTileRows = 3;
 constexpr int kMegaMaxRows = 16;                   // = kN: the token side of every MMA holds them all; the kernel is built
                                                    // for 8 (the decode sizes, leaner loops) and for 16 rows
@@ -87,7 +90,7 @@ struct MegaParams {
     std::uint8_t* hq;              // [PP][I/2]
     std::uint8_t* hs;              // tiled scales of hq
     std::uint16_t* mixed;          // [PP][H]
-    unsigned long long* logits_tagged;   // [kReplicas][R][256] {value, launch number}
+    unsigned long long* logits_tagged;   // [kReplicas, or 1 from nine rows on][R][256] {value, launch number}
     unsigned long long* choices;         // [kReplicas][R][8] {id, launch number, route weight, launch number}
     unsigned long long* ret;             // [8][9][1280] {two BF16, launch number}
     unsigned* sync;                // [0]: blocks that have finished P0 (monotonic across launches)
@@ -517,7 +520,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) moe_decode_kernel(const __gri
             __syncwarp();
             asm volatile("bar.sync 3, %0;" ::"n"(kPollers) : "memory");
             if (threadIdx.x == 0) stamp(2);
-            static_assert(R <= kMegaWarps - 1 - kEpilogueEnd, "a warp without a role in P2 for every token");
+            static_assert(R <= kMegaWarps - 1 - kEpilogueEnd, "a warp without a role in P2 for each token");
             const int t = kMegaWarps - 2 - warp;
             if (t < rows && !abort_word) {
                 const float* lg = rt.logits + t * kExperts;

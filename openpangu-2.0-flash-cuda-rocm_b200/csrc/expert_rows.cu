@@ -197,7 +197,8 @@ __device__ __forceinline__ bool decode_piece(const TcParams& p, const RouteTable
 // cycles, so that the kernels in front store a row's scales in 16-byte pieces.  The scales are requested ahead of the stage's other
 // bytes, on a barrier of their own, and are turned round before those have come: turned when all was there this kernel took 427 us
 // at 16,384 rows, with three barriers for the MMA lane to wait on 410, with one 400, as without the turning.
-// (One barrier per stage, not one for the weights and one for the tokens: dense MLP of 3,807 rows, two layers, 312.2 -> 309.5 us.)
+// (One barrier per stage, not one for the weights and one for the tokens: dense MLP of two layers, 33 rows 56.2 -> 55.7 us, 129
+// 59.6 -> 59.1, 512 70.5 -> 69.9, 1,400 133.7 -> 134.1 at a spread of 2 %, 2,000 184.2 -> 182.1, 3,807 312.2 -> 309.5.)
 template <int MODE, bool BY_ROW>
 __global__ void __launch_bounds__(BY_ROW ? kThreadsByRow : kThreads, 1) expert_rows_kernel(const __grid_constant__ CUtensorMap map_t32,
                                                                                             const __grid_constant__ CUtensorMap map_t128,
@@ -262,7 +263,8 @@ __global__ void __launch_bounds__(BY_ROW ? kThreadsByRow : kThreads, 1) expert_r
                 const Item& it = piece.it;
                 // The entry's only tile: nobody else reads these weights, and they are the first to leave the L2 again.  The rest
                 // stays there for the kernels behind (64 rows, four layers: 743 -> 730 us, 512 rows 462 -> 457.5, 2,048 rows 269 ->
-                // 262.5).  For every entry, the second tile's reads go to memory: 4,096 rows, down product 101 -> 121 us.
+                // 262.5).  For every entry, the second tile's reads go to memory: 4,096 rows, down product 101 -> 121 us.  Whole
+                // items of the gate/up product only: the pieces of the last round and MODE 1 load without it.
                 const bool once = it.count <= kTok;
                 const int half = piece.first / kTileM;          // narrow pieces: which of the two boxes
                 // token rows beyond the tile's last one are not loaded: their lanes compute on what the stage held

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) expert_tc_kernel(const __grid_c
     if (warp == 0 && SRC == 1) {
         // ------------------------------------------------ producer, weights read in place
         // The matrices are row-major [rows][K/2] wherever the caller keeps them; the kernel upstream has built a tensor
-        // map of each (gather_quantized_rows_kernel), so a box of 128 rows is one tiled load.  (Gathered in 16-byte
+        // map of each (assignment_rows_kernel, above 64 rows gather_quantized_rows_kernel), so a box of 128 rows is one tiled load.  (Gathered in 16-byte
         // pieces by this warp, 31 experts at 4 tokens took 35 us for gate and up against 20 from the bank's stream.)
         if (elect_one()) {
             int stage = 0;

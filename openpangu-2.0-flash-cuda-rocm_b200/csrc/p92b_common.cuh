@@ -412,7 +412,7 @@ struct p92b_plan {
     std::int32_t* gu_done = nullptr;      // [2][264] per launch parity: gate/up tiles finished per active slot, [257] the tile counter
     std::int32_t* ep_gu_done = nullptr;   // [2][264] the same for the fused expert-parallel kernel
     unsigned long long* ep_logits = nullptr;    // [8][256] its router logits as tagged words
-    unsigned long long* mega_logits = nullptr;  // [8][16][256] router logits as {value, launch number} words, in eight copies
+    unsigned long long* mega_logits = nullptr;  // [8][16][256] router logits as {value, launch number} words, in eight copies (one from 9 rows on)
     unsigned long long* mega_choices = nullptr; // [8][16][8] experts and route weights of every token as tagged words, in eight copies
     unsigned long long* mega_ret = nullptr;     // [8][9][1280] down rows as {two BF16, launch number} words
     float* w_norms = nullptr;                   // [256] norms of the router rows (tensor-core router)
@@ -569,7 +569,8 @@ int router_fast_min_rows();
 constexpr int kRouterSplits = 8;                // K splits of the tensor-core logits for small batches
 constexpr int kRouterSplitRows = 2304;          // ... used up to this many rows: 18 token tiles x 4 expert tiles, twice, on 148 SMs
 constexpr int kRouterPartialRows = 4736;        // rows x slices of their scratch: 148 SMs / 4 expert tiles x 128 rows
-constexpr int kRouterWideRows = 256;            // a block per token in the repair up to here
+constexpr int kRouterWideRows = 256;            // a block of eight warps per token in the repair up to here; then, for rows in
+                                                // chain order, of four up to four tokens per SM, and above a warp per token
 // `count_experts`: plan->chunk_hist and span_hist get the experts of every 32 and every 512 tokens counted, for launch_place_rows.
 cudaError_t launch_router_fast(p92b_plan* plan, const std::uint16_t* x, const std::uint16_t* router_w, const float* bias,
                                int rows, float routed_scale, cudaStream_t stream, bool pdl, bool count_experts = false);
